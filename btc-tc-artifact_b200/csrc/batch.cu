@@ -208,7 +208,8 @@ struct btc_batch {
     std::vector<uint32_t> h_rowoff;
     std::vector<int32_t> h_nv;
     bool built = false;        // the geometry above belongs to a build that succeeded
-    bool row_index = false;    // the builds enqueue the row index (row-wise count)
+    bool row_store = false;    // the builds enqueue the row store (streaming count)
+    uint32_t max_col_blocks = 0;  // 64-column blocks the widest graph's columns span
     bool pending = false;      // an enqueued rebuild's status is not known yet
     uint32_t pending_cap = 0;  // the tile capacity that rebuild ran against
     cudaStream_t pending_stream = nullptr;
@@ -261,9 +262,8 @@ static uint32_t batch_capacity(const btc_batch* b)
 }
 
 // The build after the tile count: emit (indices, row_indices, indptr, the (cell word, tile
-// prefix) pairs, the tiles zeroed), fill, row masks and, when reserved, the row index of
-// the row-wise count (built on the device when the union averages 8 or more tiles per row
-// block) -- all against `cap` tiles, the device tile count deciding (more than cap:
+// prefix) pairs, the tiles zeroed), fill, row masks and, when reserved, the row store of
+// the streaming count -- all against `cap` tiles, the device tile count deciding (more than cap:
 // nothing is built and the overflow flag is set).
 static int batch_enqueue_tiles(btc_batch* b, const int32_t* d_src, const int32_t* d_dst, int64_t m,
                                uint32_t cap, cudaStream_t s)
@@ -297,15 +297,12 @@ static int batch_enqueue_tiles(btc_batch* b, const int32_t* d_src, const int32_t
     }
     BTC_TRY(launch_rowmask(g->tile_cols, g->blocks.as<uint32_t>(), cap, meta + kMetaTiles,
                            g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
-                           meta + kMetaRowMax, s));
-    if (b->row_index) {
-        unsigned long long* total = g->row_bsum.as<unsigned long long>();
-        BTC_TRY(launch_rowindex(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->n_row_blocks,
-                                g->rowmask.as<uint32_t>(), meta + kMetaTiles, cap,
-                                g->row_tot.as<uint32_t>(), reinterpret_cast<uint32_t*>(total + 1), total,
-                                g->row_off.as<uint32_t>(), g->row_ent.as<uint2>(),
-                                g->row_ent.bytes / sizeof(uint2), s));
-    }
+                           meta + kMetaRowMax, s, true, b->row_store));
+    g->row_index = false;
+    if (b->row_store)
+        BTC_TRY(launch_rowstore(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
+                                g->blocks.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
+                                meta + kMetaTiles, cap, meta, row_store_of(g), s));
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 
@@ -406,6 +403,7 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
     b->h_bmoff.resize((size_t)G + 1);
     b->h_rowoff.resize((size_t)G + 1);
     uint64_t rows = 0, words = 0;
+    b->max_col_blocks = 0;
     for (int32_t i = 0; i < G; ++i) {
         GraphSeg& sg = b->h_segs[(size_t)i];
         const uint64_t Ri = ((uint64_t)num_vertices[i] + 15) / 16;
@@ -418,6 +416,7 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
         sg.wpr = (uint32_t)((ncb + 31) / 32);
         sg.pad = 0;
         sg.bm_off = words;
+        b->max_col_blocks = std::max(b->max_col_blocks, ((uint32_t)num_vertices[i] + 63) / 64 + 1);
         b->h_rowoff[(size_t)i] = (uint32_t)rows;
         b->h_bmoff[(size_t)i] = words;
         rows += Ri;
@@ -494,16 +493,11 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
     BTC_TRY(g->row_indices.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
     BTC_TRY(g->blocks.reserve(sizeof(uint32_t) * TW * (tiles ? tiles : 1)));
     BTC_TRY(g->rowmask.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
-    // the row-wise count's row index, when the union averages 8 or more tiles per row
-    // block (then it has at least 8 edges per row block)
-    b->row_index = rows > 0 && (uint64_t)tiles >= 8ull * rows && m < (int64_t)0xffffffffll;
-    if (b->row_index) {
-        BTC_TRY(g->row_off.reserve(sizeof(uint32_t) * (16 * (size_t)rows + 1)));
-        BTC_TRY(g->row_ent.reserve(sizeof(uint2) * (size_t)m));
-        BTC_TRY(g->row_tot.reserve(sizeof(uint32_t) * (size_t)rows));
-        BTC_TRY(g->row_bsum.reserve(sizeof(unsigned long long) +
-                                    sizeof(uint32_t) * ((size_t)ri_scan_blocks((uint32_t)rows) + 1)));
-    }
+    // the streaming count's row store, when the union averages 8 or more tiles per row block
+    // (then it has at least 8 edges per row block) and there is the memory for it
+    b->row_store = rows > 0 && (uint64_t)tiles >= 8ull * rows && m < (int64_t)0xffffffffll &&
+                   // (an enqueued rebuild may fill the arrays to their capacity)
+                   reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * batch_capacity(b))) == BTC_OK;
     BTC_TRY(ensure_count_scratch(g));
     BTC_TRY(b->counts.reserve(sizeof(unsigned long long) * (size_t)G));
     BTC_TRY(batch_enqueue_tiles(b, d_src, d_dst, m, (uint32_t)tiles, s));
@@ -583,16 +577,25 @@ int btc_batch_count(btc_batch* b, int tau, btc_stream_t stream, unsigned long lo
     // after an enqueued rebuild the kernel reads the tile count (and the build's status)
     // from the device, within the capacity; the schedule follows the previous count
     const unsigned long long* build_meta = b->pending ? g->meta.as<unsigned long long>() : nullptr;
+    const uint32_t cap = b->pending ? b->pending_cap : g->num_tiles;
+    if (b->row_store && tau >= default_tau(g->tile_cols)) {
+        BTC_TRY(launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks, g->tile_cols, g->n_row_blocks, b->max_col_blocks, scr,
+                                    b->row_off.as<uint32_t>(), (uint32_t)b->num_graphs, counts,
+                                    g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), 0, cap, true,
+                                    build_meta, count_grid_size(g->tile_cols), stream));
+    } else {
+    if (b->row_store) ensure_row_index(g, build_meta ? build_meta + kMetaTiles : nullptr, cap, stream);
     BTC_TRY(launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                          g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(),
-                         b->pending ? b->pending_cap : g->num_tiles, g->n_row_blocks, tau, scr,
+                         cap, g->n_row_blocks, tau, scr,
                          stream, b->row_off.as<uint32_t>(), (uint32_t)b->num_graphs, counts,
                          g->rowmask.as<uint32_t>(), g->prefix.as<uint2>(), 0,
                          g->meta.as<unsigned long long>() + kMetaRowMax, 0, 0xffffffffu, build_meta,
                          g->num_tiles,
-                         b->row_index ? g->row_off.as<uint32_t>() : nullptr,
-                         b->row_index ? g->row_ent.as<uint2>() : nullptr, false,
+                         g->row_index ? g->row_off.as<uint32_t>() : nullptr,
+                         g->row_index ? g->row_ent.as<uint2>() : nullptr, false,
                          b->segs.as<GraphSeg>()));
+    }
     if (h_counts) {
         BTC_CUDA_TRY(cudaMemcpyAsync(h_counts, counts, bytes, cudaMemcpyDeviceToHost, stream));
         BTC_CUDA_TRY(cudaStreamSynchronize(stream));

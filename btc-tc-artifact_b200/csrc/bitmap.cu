@@ -370,13 +370,13 @@ k_fill_bm(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int6
           const int32_t* __restrict__ rank, uint64_t wpr, const uint32_t* __restrict__ bitmap,
           const uint2* __restrict__ cellpp, uint32_t* __restrict__ blocks,
           const unsigned long long* __restrict__ d_tiles, uint32_t cap, uint32_t* __restrict__ rowmask,
-          int32_t R)
+          bool always_masks, int32_t R)
 {
     const unsigned long long T = *d_tiles;
     if (T > cap) return;  // overflowed tile arrays: the builder redoes this step
-    // row-occupancy masks: wanted when row blocks average 8 or more tiles (the row-wise
-    // count's condition, on the device tile count)
-    if (T < 8ull * (unsigned long long)(R > 0 ? R : 0)) rowmask = nullptr;
+    // row-occupancy masks: wanted for the row store, and when row blocks average 8 or more
+    // tiles (the heavy counts' condition, on the device tile count)
+    if (!always_masks && T < 8ull * (unsigned long long)(R > 0 ? R : 0)) rowmask = nullptr;
     constexpr int C = 1 << LOG2C;
     constexpr int WPR = C / 32;
     constexpr int TW = 16 * WPR;
@@ -426,7 +426,8 @@ k_fill_bm(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int6
             }
 #pragma unroll
             for (int k = 0; k < U; ++k)
-                if (old[k] == 0u) atomicOr(&rowmask[tile[k]], 1u << (r[k] & 15u));
+                if (old[k] == 0u)
+                    atomicOr(&rowmask[tile[k]], 1u << ((r[k] & 15u) + (C == 128 ? (c[k] & 64u) / 4u : 0u)));
         } else {
 #pragma unroll
             for (int k = 0; k < U; ++k) {
@@ -541,7 +542,7 @@ int bitmap_emit_and_fill(const BuildGeom& g, const int32_t* src, const int32_t* 
                          uint2* cellpp, uint32_t* indices, uint32_t* row_indices,
                          uint32_t* indptr, uint32_t* blocks, unsigned long long* meta,
                          uint32_t cap, unsigned long long* host_meta, cudaStream_t s,
-                         uint32_t* rowmask)
+                         uint32_t* rowmask, bool always_masks)
 {
     const unsigned long long* meta_tiles = meta + kMetaTiles;
     const uint64_t wpr = bitmap_words_per_row(g);
@@ -570,11 +571,11 @@ int bitmap_emit_and_fill(const BuildGeom& g, const int32_t* src, const int32_t* 
         if (g.tile_cols == 128)
             bm::k_fill_bm<7><<<edge_grid(m), bm::kThreads, 0, s>>>(
                 src, dst, m, g.n, rank, wpr, bitmap, cellpp, blocks, meta_tiles, cap, rowmask,
-                g.n_row_blocks);
+                always_masks, g.n_row_blocks);
         else
             bm::k_fill_bm<5><<<edge_grid(m), bm::kThreads, 0, s>>>(
                 src, dst, m, g.n, rank, wpr, bitmap, cellpp, blocks, meta_tiles, cap, rowmask,
-                g.n_row_blocks);
+                always_masks, g.n_row_blocks);
     }
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
@@ -614,7 +615,7 @@ __global__ void k_rowmask(const uint32_t* __restrict__ blocks, uint32_t cap,
                           const unsigned long long* __restrict__ d_tiles,
                           const uint32_t* __restrict__ indptr, uint32_t R,
                           uint32_t* __restrict__ rowmask, unsigned long long* __restrict__ row_max,
-                          bool masks)
+                          bool masks, bool always)
 {
     const unsigned long long T = d_tiles ? *d_tiles : cap;
     if (T > cap) return;  // overflowed tile arrays: the builder redoes this step
@@ -626,9 +627,9 @@ __global__ void k_rowmask(const uint32_t* __restrict__ blocks, uint32_t cap,
         mx = max(mx, indptr[i + 1] - indptr[i]);
     mx = __reduce_max_sync(kFull, mx);
     if ((threadIdx.x & 31) == 0 && mx) atomicMax(row_max, (unsigned long long)mx);
-    // the masks serve only the heavy count variant, which reads them only when row
-    // blocks average 8 or more tiles (the same test on the same count)
-    if (!masks || (uint64_t)num_tiles < 8ull * (uint64_t)R) return;
+    // the masks serve the row store and the heavy count variants, which read them only when
+    // row blocks average 8 or more tiles (the same test on the same count)
+    if (!masks || (!always && (uint64_t)num_tiles < 8ull * (uint64_t)R)) return;
 
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < num_tiles;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -638,7 +639,7 @@ __global__ void k_rowmask(const uint32_t* __restrict__ blocks, uint32_t cap,
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
                 const uint4 v = reinterpret_cast<const uint4*>(b)[r];
-                m |= ((v.x | v.y | v.z | v.w) != 0u) ? (1u << r) : 0u;
+                m |= ((v.x | v.y) != 0u ? 1u << r : 0u) | ((v.z | v.w) != 0u ? 0x10000u << r : 0u);
             }
         } else {
 #pragma unroll
@@ -657,15 +658,16 @@ __global__ void k_rowmask(const uint32_t* __restrict__ blocks, uint32_t cap,
 
 int launch_rowmask(int tile_cols, const uint32_t* blocks, uint32_t cap,
                    const unsigned long long* d_tiles, const uint32_t* indptr, int32_t n_row_blocks,
-                   uint32_t* rowmask, unsigned long long* row_max, cudaStream_t s, bool masks)
+                   uint32_t* rowmask, unsigned long long* row_max, cudaStream_t s, bool masks,
+                   bool always)
 {
     const uint32_t R = n_row_blocks > 0 ? (uint32_t)n_row_blocks : 0u;
     if (cap || R) {
         const int grid = grid_for((int64_t)(masks ? max(cap, R) : R), 256);
         if (tile_cols == 128)
-            bm::k_rowmask<4><<<grid, 256, 0, s>>>(blocks, cap, d_tiles, indptr, R, rowmask, row_max, masks);
+            bm::k_rowmask<4><<<grid, 256, 0, s>>>(blocks, cap, d_tiles, indptr, R, rowmask, row_max, masks, always);
         else
-            bm::k_rowmask<1><<<grid, 256, 0, s>>>(blocks, cap, d_tiles, indptr, R, rowmask, row_max, masks);
+            bm::k_rowmask<1><<<grid, 256, 0, s>>>(blocks, cap, d_tiles, indptr, R, rowmask, row_max, masks, always);
     }
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }

@@ -30,7 +30,7 @@ int bitmap_mark_and_count(const BuildGeom&, const int32_t*, const int32_t*, int6
 int bitmap_emit_and_fill(const BuildGeom&, const int32_t*, const int32_t*, int64_t, const int32_t*,
                          const uint32_t*, const uint32_t*, uint2*, uint32_t*, uint32_t*, uint32_t*,
                          uint32_t*, unsigned long long*, uint32_t, unsigned long long*,
-                         cudaStream_t, uint32_t*);
+                         cudaStream_t, uint32_t*, bool);
 int launch_popcount_sum(int, const uint32_t*, uint64_t, unsigned long long*, cudaStream_t);
 int launch_indptr(const uint32_t*, uint32_t, int32_t, uint32_t*, cudaStream_t);
 int launch_density(int, const uint32_t*, uint32_t, unsigned long long*, cudaStream_t);
@@ -124,32 +124,58 @@ struct BuildPlan {
     bool degree;
     uint64_t bm_words;
     uint32_t cap;  // > 0: the post-count steps run against this tile capacity
-    bool row_index = false;  // build the row-wise count's row index (rowindex.cu)
+    bool row_store = false;  // build the streaming count's row store (rowstore.cu)
 };
 
-static bool row_index_possible(int64_t m, int32_t n_row_blocks)
+// Only a graph with at least 8 edges per row block can average 8 tiles per row block (every
+// tile holds an edge).
+static bool row_store_possible(int64_t m, int32_t n_row_blocks)
 {
     return n_row_blocks > 0 && m >= 8 * (int64_t)n_row_blocks && m < (int64_t)0xffffffffll;
 }
 
-static int reserve_row_index(btc_bitbsr* g, int64_t m, uint64_t R)
+RowStore row_store_of(const btc_bitbsr* g)
 {
-    BTC_TRY(g->row_off.reserve(sizeof(uint32_t) * (16 * R + 1)));
-    BTC_TRY(g->row_ent.reserve(sizeof(uint2) * (size_t)m));
-    BTC_TRY(g->row_tot.reserve(sizeof(uint32_t) * R));
-    return g->row_bsum.reserve(sizeof(unsigned long long) +
-                               sizeof(uint32_t) * ((size_t)ri_scan_blocks((uint32_t)R) + 1));
+    return RowStore{g->rs_off.as<uint32_t>(), g->rs_key.ptr, g->rs_bits.as<uint4>(),
+                    g->rs_first.as<uint32_t>()};
 }
 
-// The row index after the row masks (T = *d_tiles bounded by cap, or cap itself).
-static int enqueue_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap,
+int reserve_row_store(btc_bitbsr* g, uint64_t entries)
+{
+    const uint64_t R = (uint64_t)g->n_row_blocks;
+    BTC_TRY(g->rs_off.reserve(sizeof(uint32_t) * (17 * R + 1)));
+    const uint64_t chunks = row_store_chunks(entries, R);
+    if (chunks * kRowChunk > 0xffffffffull) return BTC_E_NOMEM;  // entries are numbered in 32 bits
+    BTC_TRY(g->rs_key.reserve((row_store_wide(g->n_row_blocks) ? sizeof(uint2) : sizeof(uint32_t)) * kRowLanes * chunks));
+    BTC_TRY(g->rs_bits.reserve(sizeof(uint4) * kRowLanes * chunks));
+    return g->rs_first.reserve(sizeof(uint32_t) * (chunks / kRowRun + 1));
+}
+
+// The row store after the tiles and row masks (T = *d_tiles bounded by cap, or cap itself).
+static int enqueue_row_store(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap,
                              cudaStream_t s)
 {
+    return launch_rowstore(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
+                           g->blocks.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(), d_tiles,
+                           cap, g->meta.as<unsigned long long>(), row_store_of(g), s);
+}
+
+void ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s)
+{
+    if (g->row_index) return;
+    const uint64_t R = (uint64_t)g->n_row_blocks;
+    const int64_t m = g->input_edges;
+    const uint64_t ent = std::min<uint64_t>((uint64_t)m, 16ull * cap);
+    if (!row_store_possible(m, g->n_row_blocks) || g->row_off.reserve(sizeof(uint32_t) * (16 * R + 1)) ||
+        g->row_ent.reserve(sizeof(uint2) * (size_t)ent) || g->row_tot.reserve(sizeof(uint32_t) * R) ||
+        g->row_bsum.reserve(sizeof(unsigned long long) +
+                            sizeof(uint32_t) * ((size_t)ri_scan_blocks((uint32_t)R) + 1)))
+        return;
     unsigned long long* total = g->row_bsum.as<unsigned long long>();
-    return launch_rowindex(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->n_row_blocks,
-                           g->rowmask.as<uint32_t>(), d_tiles, cap, g->row_tot.as<uint32_t>(),
-                           reinterpret_cast<uint32_t*>(total + 1), total, g->row_off.as<uint32_t>(),
-                           g->row_ent.as<uint2>(), g->row_ent.bytes / sizeof(uint2), s);
+    g->row_index = launch_rowindex(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->n_row_blocks,
+                                   g->rowmask.as<uint32_t>(), d_tiles, cap, g->row_tot.as<uint32_t>(),
+                                   reinterpret_cast<uint32_t*>(total + 1), total, g->row_off.as<uint32_t>(),
+                                   g->row_ent.as<uint2>(), g->row_ent.bytes / sizeof(uint2), s) == BTC_OK;
 }
 
 // Enqueues the build up to the tile count (bitmap path) or up to the tile segmentation
@@ -198,12 +224,15 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
                                          g->prefix.as<uint2>(), g->indices.as<uint32_t>(),
                                          g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(),
                                          g->blocks.as<uint32_t>(), meta, P.cap, g->d_hmeta, s,
-                                         g->rowmask.as<uint32_t>()));
-            // the fill pass set the row masks; this pass finds the longest row-block list
-            BTC_TRY(launch_rowmask(geom.tile_cols, g->blocks.as<uint32_t>(), P.cap,
-                                   meta + kMetaTiles, g->indptr.as<uint32_t>(), geom.n_row_blocks,
-                                   g->rowmask.as<uint32_t>(), meta + kMetaRowMax, s, false));
-            if (P.row_index) BTC_TRY(enqueue_row_index(g, meta + kMetaTiles, P.cap, s));
+                                         g->rowmask.as<uint32_t>(), P.row_store));
+            // the fill pass set the row masks; what is left is the row store, or only the
+            // longest row-block list
+            if (P.row_store)
+                BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, s));
+            else
+                BTC_TRY(launch_rowmask(geom.tile_cols, g->blocks.as<uint32_t>(), P.cap,
+                                       meta + kMetaTiles, g->indptr.as<uint32_t>(), geom.n_row_blocks,
+                                       g->rowmask.as<uint32_t>(), meta + kMetaRowMax, s, false));
         }
     } else {
         // ---- keys, sort, segmentation ---------------------------------------
@@ -227,14 +256,14 @@ static void build_key(const btc_bitbsr* g, const BuildPlan& P, BuildGraphKey* k)
     const void* w[] = {P.src, P.dst, g->meta.ptr, g->in_src.ptr, g->in_dst.ptr, g->keys0.ptr,
                        g->keys1.ptr, g->sort_scratch.ptr, g->deg.ptr, g->rank.ptr, g->bitmap.ptr,
                        g->prefix.ptr, g->tile_base.ptr, g->indices.ptr, g->row_indices.ptr,
-                       g->indptr.ptr, g->blocks.ptr, g->rowmask.ptr, g->d_hmeta, g->row_off.ptr,
-                       g->row_ent.ptr, g->row_tot.ptr, g->row_bsum.ptr};
+                       g->indptr.ptr, g->blocks.ptr, g->rowmask.ptr, g->d_hmeta, g->rs_off.ptr,
+                       g->rs_key.ptr, g->rs_bits.ptr, g->rs_first.ptr};
     static_assert(sizeof(w) / sizeof(w[0]) == kBuildKeyPtrs, "key layout");
     for (int i = 0; i < kBuildKeyPtrs; ++i) k->ptr[i] = w[i];
     k->m = P.m;
     k->n = P.n;
     k->tile_cols = P.geom.tile_cols;
-    k->flags = P.flags;
+    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u);
     k->cap = P.cap;
 }
 
@@ -304,7 +333,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     P.geom = make_geom(n, tile_cols);
     const BuildGeom& geom = P.geom;
     // the previous build of this handle, when it had the same geometry, predicts whether
-    // the graph averages 8 or more tiles per row block (the row index's condition)
+    // the graph averages 8 or more tiles per row block (the row store's condition)
     const bool prev_light = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks &&
                             g->num_tiles > 0 &&
                             (uint64_t)g->num_tiles < 8ull * (uint64_t)geom.n_row_blocks;
@@ -340,7 +369,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     P.use_bitmap = !(flags & BTC_BUILD_RADIX) && bm_bytes <= (4ull << 30) &&
                    bm_bytes <= 32ull * (uint64_t)m + (64ull << 20);
     g->used_bitmap = P.use_bitmap;
-    g->row_index = false;
+    g->row_store = g->row_index = false;
     P.degree = (flags & BTC_ORIENT_DEGREE) && n > 0;
     size_t key_cap = P.use_bitmap ? 0 : (size_t)m;
     if (P.degree && (size_t)n > key_cap) key_cap = (size_t)n;
@@ -358,14 +387,6 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     if (P.use_bitmap) {
         BTC_TRY(g->bitmap.reserve(sizeof(uint32_t) * (P.bm_words ? P.bm_words : 1)));
         BTC_TRY(g->prefix.reserve(sizeof(uint2) * (P.bm_words ? P.bm_words : 1)));
-        // the row-wise count's row index: only a graph with at least 8 edges per row block
-        // can average 8 tiles per row block (every tile holds an edge).  A rebuild whose
-        // previous graph of the same geometry averaged fewer skips it (a mesh would pay
-        // five launches that find nothing to do); should this graph average more after
-        // all, the count takes the tile-wise kernel, which needs no index.
-        P.row_index = row_index_possible(m, geom.n_row_blocks) && !prev_light;
-        if (P.row_index) BTC_TRY(reserve_row_index(g, m, (uint64_t)geom.n_row_blocks));
-        g->row_index = P.row_index;
     }
     BTC_TRY(g->indptr.reserve(sizeof(uint32_t) * ((size_t)geom.n_row_blocks + 1)));
     BTC_TRY(ensure_count_scratch(g));
@@ -382,6 +403,13 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         c = std::min<uint64_t>(c, g->blocks.bytes / (4 * TW));
         c = std::min<uint64_t>(c, g->rowmask.bytes / 4);
         P.cap = (uint32_t)std::min<uint64_t>(c, 0xffffffffull);
+        // The row store of the streaming count.  A rebuild whose previous graph of the same
+        // geometry averaged fewer than 8 tiles per row block skips it (a mesh counts faster
+        // tile-wise); should this graph average more after all, the count takes the
+        // tile-wise kernel, which needs no store.  So does a graph without the memory for it.
+        P.row_store = P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light &&
+                      reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * P.cap)) == BTC_OK;
+        g->row_store = P.row_store;
     }
 
     uint64_t* sorted = nullptr;
@@ -418,13 +446,18 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     BTC_TRY(g->row_indices.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
     BTC_TRY(g->blocks.reserve(sizeof(uint32_t) * TW * (tiles ? tiles : 1)));
     BTC_TRY(g->rowmask.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
+    // the tile count is known here: the row store exactly when the graph averages 8 or more
+    // tiles per row block
+    P.row_store = row_store_possible(m, geom.n_row_blocks) &&
+                  (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks &&
+                  reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * tiles)) == BTC_OK;
     if (P.use_bitmap) {
         BTC_TRY(bitmap_emit_and_fill(geom, P.d_src, P.d_dst, m, P.degree ? g->rank.as<int32_t>() : nullptr,
                                      g->bitmap.as<uint32_t>(), g->tile_base.as<uint32_t>(),
                                      g->prefix.as<uint2>(), g->indices.as<uint32_t>(),
                                      g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(),
                                      g->blocks.as<uint32_t>(), meta, (uint32_t)tiles, nullptr, s,
-                                     g->rowmask.as<uint32_t>()));
+                                     g->rowmask.as<uint32_t>(), P.row_store));
     } else {
         if (tiles)
             BTC_CUDA_TRY(cudaMemsetAsync(g->blocks.ptr, 0, sizeof(uint32_t) * TW * tiles, s));
@@ -435,18 +468,12 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
                               g->indptr.as<uint32_t>(), s));
     }
     // the bitmap path's fill pass set the row masks; the radix path's are computed here
-    BTC_TRY(launch_rowmask(tile_cols, g->blocks.as<uint32_t>(), g->num_tiles, nullptr,
-                           g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
-                           meta + kMetaRowMax, s, !P.use_bitmap));
-    // the tile count is known here: the index exactly when the graph averages 8 or more
-    // tiles per row block
-    P.row_index = P.use_bitmap && row_index_possible(m, geom.n_row_blocks) &&
-                  (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks;
-    if (P.row_index) {
-        BTC_TRY(reserve_row_index(g, m, (uint64_t)geom.n_row_blocks));
-        BTC_TRY(enqueue_row_index(g, nullptr, g->num_tiles, s));
-    }
-    g->row_index = P.row_index;
+    if (!P.use_bitmap || !P.row_store)
+        BTC_TRY(launch_rowmask(tile_cols, g->blocks.as<uint32_t>(), g->num_tiles, nullptr,
+                               g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
+                               meta + kMetaRowMax, s, !P.use_bitmap));
+    if (P.row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, s));
+    g->row_store = P.row_store;
     return BTC_OK;
 }
 
@@ -468,19 +495,28 @@ int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_o
     // after an enqueued build the kernel reads the tile count (and the build's status)
     // from the device; the capacity bounds it
     const unsigned long long* build_meta = g->pending ? g->meta.as<unsigned long long>() : nullptr;
+    const uint32_t cap = g->pending ? g->pending_cap : g->num_tiles;
+    // tiles averaging more than half of tau's bits: the tensor-core path's graphs
+    const bool dense = (uint64_t)g->input_edges * 2 > (uint64_t)tau * (uint64_t)g->num_tiles;
+    const bool whole = tile_begin == 0 && tile_end == 0xffffffffu;
+    // A caller's lower tau asks for the tensor cores, which only the tile kernels use.
+    if (g->row_store && tau >= default_tau(g->tile_cols) && !(dense && g->tile_cols == 128))
+        return launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks, g->tile_cols, g->n_row_blocks,
+                                   ((uint32_t)g->n + 63) / 64, scr, nullptr, 0, nullptr,
+                                   g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), tile_begin,
+                                   std::min(tile_end, cap), whole, build_meta, count_grid_size(g->tile_cols), s);
+    if (g->row_store && g->used_bitmap)
+        ensure_row_index(g, build_meta ? build_meta + kMetaTiles : nullptr, cap, s);
     return launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                         g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(),
-                        g->pending ? g->pending_cap : g->num_tiles, g->n_row_blocks, tau, scr, s,
+                        cap, g->n_row_blocks, tau, scr, s,
                         nullptr, 0, nullptr, g->rowmask.as<uint32_t>(),
                         g->used_bitmap ? g->prefix.as<uint2>() : nullptr,
                         bitmap_words_per_row(make_geom(g->n, g->tile_cols)),
                         g->meta.as<unsigned long long>() + kMetaRowMax, tile_begin, tile_end,
                         build_meta, g->num_tiles,
-                        g->used_bitmap && g->row_index ? g->row_off.as<uint32_t>() : nullptr,
-                        g->used_bitmap && g->row_index ? g->row_ent.as<uint2>() : nullptr,
-                        // tiles averaging more than half of tau's bits: the kernel variant
-                        // that keeps the tensor-core path's registers
-                        (uint64_t)g->input_edges * 2 > (uint64_t)tau * (uint64_t)g->num_tiles);
+                        g->row_index ? g->row_off.as<uint32_t>() : nullptr,
+                        g->row_index ? g->row_ent.as<uint2>() : nullptr, dense);
 }
 
 int resolve_build(btc_bitbsr* g)

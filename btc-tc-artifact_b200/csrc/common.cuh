@@ -111,6 +111,31 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(ptr); }
 };
 
+// Exclusive prefix of one value per thread over a CTA of kThreads (s_warp: a word per warp);
+// `total` is the sum.  Every thread of the CTA calls it.
+template <int kThreads>
+__device__ __forceinline__ uint32_t cta_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t& total)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, d);
+        if (lane >= d) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t wbase = 0;
+    total = 0;
+    for (int w = 0; w < kThreads / kWarp; ++w) {
+        const uint32_t x = s_warp[w];
+        if (w < warp) wbase += x;
+        total += x;
+    }
+    __syncthreads();
+    return wbase + incl - v;
+}
+
 // ---------------------------------------------------------------------------
 // Sort (radix.cu)
 // ---------------------------------------------------------------------------
@@ -191,15 +216,60 @@ int launch_count(int tile_cols, const uint32_t* indptr, const uint32_t* indices,
                  const uint32_t* row_off = nullptr, const uint2* row_ent = nullptr,
                  bool dense_tiles = false, const GraphSeg* segs = nullptr);
 
-// rowmask[t] bit r = tile t's row r has a bit, for t < T = *d_tiles (T = cap when d_tiles
+// rowmask[t] bit r = tile t's row r has a bit -- in 16x128 tiles in its first 64 columns,
+// and bit 16 + r in its last 64 (fold_rows joins them) -- for t < T = *d_tiles (T = cap when d_tiles
 // is null) when T >= 8 * n_row_blocks (the heavy count variant's condition), and
 // *row_max = max(*row_max, the most tiles in one row block), which picks the count
 // kernel's schedule (the caller zeroes it).  Runs after the tiles are filled.  Writes
 // nothing when T > cap (the tile arrays overflowed).
-// masks = false: only *row_max (the bitmap builder's fill pass sets the masks itself).
+// masks = false: only *row_max (the bitmap builder's fill pass sets the masks itself);
+// always = true: masks whatever T is (the row store reads them).
+__host__ __device__ __forceinline__ uint32_t fold_rows(uint32_t m) { return (m | (m >> 16)) & 0xFFFFu; }
 int launch_rowmask(int tile_cols, const uint32_t* blocks, uint32_t cap,
                    const unsigned long long* d_tiles, const uint32_t* indptr, int32_t n_row_blocks,
-                   uint32_t* rowmask, unsigned long long* row_max, cudaStream_t s, bool masks = true);
+                   uint32_t* rowmask, unsigned long long* row_max, cudaStream_t s, bool masks = true,
+                   bool always = false);
+
+// The rows of L in 64-column words (rowstore.cu), the streaming count kernel's operand.
+constexpr uint32_t kRowChunk = 16;  // entries per chunk: a row is whole chunks
+constexpr uint32_t kRowLanes = 8;   // words per chunk: entry i is in word i % 8, half i / 8
+constexpr uint32_t kRowRun = 4;     // chunks per first_row entry
+struct RowStore {
+    uint32_t* off;        // 17 R: row r of row block I has chunks [off[17 I + r], off[17 I + r + 1])
+    void* key;            // word: the two entries' column blocks (64 columns), 16 bits each,
+                          // or 32 when the graph has more of them (row_store_wide)
+    uint4* bits;          // word: the two entries' 64 bits each
+    uint32_t* first_row;  // the row that holds chunk kRowRun b; row blocks hold whole runs, from
+                          // chunk kRowRun on; chunk 0 is empty
+};
+// Whether column block ids need more than 16 bits: 16 n_row_blocks / 64 of them.
+inline bool row_store_wide(int64_t n_row_blocks) { return (n_row_blocks + 3) / 4 > 0x10000; }
+// Chunks that hold `entries` entries of a graph of R row blocks, at most.
+inline uint64_t row_store_chunks(uint64_t entries, uint64_t R)
+{
+    const uint64_t rows = 16 * R < entries ? 16 * R : entries;  // rows with an entry
+    const uint64_t blocks = R < entries ? R : entries;
+    return kRowRun + (entries + rows * (kRowChunk - 1)) / kRowChunk + blocks * (kRowRun - 1);
+}
+
+// Enqueues the row store of a Bit-BSR whose row masks exist (T = *d_tiles tiles, bounded by
+// cap, or cap when d_tiles is null; nothing when T > cap).  meta:
+// the build's metadata slots (kMetaRowChunks zero: it counts the chunks handed out); also
+// raises meta[kMetaRowMax] to the most tiles in one row block.
+int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indices, const uint32_t* blocks,
+                    int32_t n_row_blocks, const uint32_t* rowmask, const unsigned long long* d_tiles,
+                    uint32_t cap, unsigned long long* meta, const RowStore& out,
+                    cudaStream_t s);
+
+// The streaming count (count_stream.cu) of the sample tiles [tile_begin, tile_end), or of
+// all of them with `whole`.  rs_chunks: the store's meta[kMetaRowChunks].  max_col_blocks: the most 64-column blocks a row's columns can
+// span.  grid: the CTAs scr.partials has room for.
+int stream_blocks_per_sm_max();
+int launch_count_stream(const RowStore& rs, const unsigned long long* rs_chunks, int tile_cols,
+                        int32_t n_row_blocks, uint32_t max_col_blocks, CountScratch scr, const uint32_t* graph_rows, uint32_t num_graphs,
+                        unsigned long long* graph_counts, const uint32_t* row_indices,
+                        const uint32_t* indices, uint32_t tile_begin, uint32_t tile_end, bool whole,
+                        const unsigned long long* build_meta, int grid, cudaStream_t s);
 
 // Row index of the row-wise count kernel (rowindex.cu): for vertex u, ent[off[u],
 // off[u+1]) lists (column block, tile) of the tiles whose row u % 16 holds a bit, in tile
@@ -220,7 +290,8 @@ int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n
 
 // Device metadata slots of a build (uint64 each): valid keys, out-of-range flag, tile
 // count, unique edges, sort length, longest row-block list, tile-capacity overflow flag,
-// and the chunk-scan ticket (CTAs of the chunk popcount that have finished).
+// the chunk-scan ticket (CTAs of the chunk popcount that have finished), and the chunks of
+// the row store handed out.
 enum {
     kMetaValid = 0,
     kMetaBad = 1,
@@ -230,7 +301,8 @@ enum {
     kMetaRowMax = 5,
     kMetaOverflow = 6,
     kMetaTicket = 7,
-    kMetaSlots = 8
+    kMetaRowChunks = 8,
+    kMetaSlots = 9
 };
 
 // Queue/completion words of the count kernel: done (u32) at byte 0, work (u64) at 8.

@@ -648,8 +648,8 @@ k_count(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indice
                             if (found) pb = cp.y + __popc(cp.x & (bit - 1u));
                         }
                         if (found && rmask_g) {
-                            ra = rmask_g[pa];
-                            rb = rmask_g[pb];
+                            ra = fold_rows(rmask_g[pa]);
+                            rb = fold_rows(rmask_g[pb]);
                             found = (ra & s.rmask[jsel]) && (rb & s.cmask[jsel]);
                         }
                     }
@@ -817,7 +817,8 @@ int count_grid_size(int tile_cols)
 {
     const int rows = rows_blocks_per_sm(tile_cols);
     const int tile = tile_blocks_per_sm(tile_cols);
-    return (rows > tile ? rows : tile) * device_sm_count();
+    const int most = rows > tile ? rows : tile, stream = stream_blocks_per_sm_max();
+    return (most > stream ? most : stream) * device_sm_count();
 }
 
 int launch_count(int tile_cols, const uint32_t* indptr, const uint32_t* indices,

@@ -106,7 +106,7 @@ k_count_rows(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ i
     // row masks and the row index exist only when row blocks average 8 or more tiles
     const bool have_rm = rowmask != nullptr && (uint64_t)num_tiles >= 8ull * (uint64_t)(R > 0 ? R : 0);
     const bool have_ri = have_rm && row_off != nullptr && row_ent != nullptr;
-    auto rmask_of = [&](uint32_t t) -> uint32_t { return have_rm ? __ldg(rowmask + t) : 0xFFFFu; };
+    auto rmask_of = [&](uint32_t t) -> uint32_t { return have_rm ? fold_rows(__ldg(rowmask + t)) : 0xFFFFu; };
 
     // The (cell word, tile prefix) pair of row block J, column block K, and K's bit in it.
     // A batch union looks the cell up in the part of the bitmap of J's graph (sg, the

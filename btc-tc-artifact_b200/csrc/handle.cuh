@@ -24,13 +24,18 @@ struct btc_bitbsr {
     int64_t input_edges = 0;
     // Bit-BSR arrays (reference layout)
     btc200::DevBuf indptr, indices, row_indices, blocks, result, rowmask;
-    // row index of the row-wise count kernel (rowindex.cu): per-vertex list offsets and
-    // (column block, tile) entries, plus the scan's scratch
+    // row store of the streaming count (rowstore.cu): row starts, column blocks, bits and
+    // the row of every run of chunks
+    btc200::DevBuf rs_off, rs_key, rs_bits, rs_first;
+    // row index of the row-wise count kernel (rowindex.cu), made by the first count that
+    // takes it: per-vertex list offsets and (column block, tile) entries, plus the scan's
+    // scratch
     btc200::DevBuf row_off, row_ent, row_tot, row_bsum;
     // build workspace
     btc200::DevBuf in_src, in_dst, keys0, keys1, sort_scratch, tile_base, meta, deg, rank, bitmap, prefix;
     bool used_bitmap = false;
-    bool row_index = false;  // the last build made the row index (its graph can be heavy)
+    bool row_store = false;  // the last build made the row store (its graph can be heavy)
+    bool row_index = false;  // the row index of the last build's graph has been enqueued
     // count scratch
     btc200::DevBuf partials, done;
     unsigned long long* h_meta = nullptr;  // pinned and mapped, 8 slots
@@ -55,7 +60,7 @@ struct btc_bitbsr {
         btc200::DevBuf* all[] = {&indptr, &indices, &row_indices, &blocks, &result, &in_src, &in_dst,
                                  &keys0, &keys1, &sort_scratch, &tile_base, &meta, &deg, &rank,
                                  &bitmap, &prefix, &partials, &done, &rowmask, &row_off, &row_ent,
-                                 &row_tot, &row_bsum};
+                                 &row_tot, &row_bsum, &rs_off, &rs_key, &rs_bits, &rs_first};
         for (btc200::DevBuf* b : all) f(*b);
     }
     size_t device_bytes() const
@@ -95,6 +100,14 @@ struct btc_bitbsr {
 // num_tiles and returns the build's status (BTC_E_RANGE, BTC_E_CAPACITY or BTC_OK).
 int resolve_build(btc_bitbsr* g);
 
+
+btc200::RowStore row_store_of(const btc_bitbsr* g);
+// Reserves the row store of a graph with at most `entries` entries (BTC_E_NOMEM: the caller
+// goes on without one); no allocation when the buffers already hold it.
+int reserve_row_store(btc_bitbsr* g, uint64_t entries);
+// The row index of the row-wise count kernel, enqueued on s if this build's is not yet there.
+// Without the memory for it the kernel walks whole row blocks instead.
+void ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s);
 
 int default_tau(int tile_cols);
 int ensure_count_scratch(btc_bitbsr* g);

@@ -50,32 +50,10 @@ __global__ void k_ri_totals(const uint32_t* __restrict__ indptr, uint32_t R,
     for (uint64_t I = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) / kWarp; I < R; I += nw) {
         const uint32_t a = indptr[I], b = indptr[I + 1];
         uint32_t sum = 0;
-        for (uint32_t t = a + lane; t < b; t += kWarp) sum += __popc(rowmask[t]);
+        for (uint32_t t = a + lane; t < b; t += kWarp) sum += __popc(fold_rows(rowmask[t]));
         sum = __reduce_add_sync(kFull, sum);
         if (lane == 0) tot[I] = sum;
     }
-}
-
-__device__ __forceinline__ uint32_t cta_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t& total)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, incl, d);
-        if (lane >= d) incl += y;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    uint32_t wbase = 0;
-    total = 0;
-    for (int w = 0; w < kThreads / kWarp; ++w) {
-        const uint32_t x = s_warp[w];
-        if (w < warp) wbase += x;
-        total += x;
-    }
-    __syncthreads();
-    return wbase + incl - v;
 }
 
 // CTA c: sum of items [c*kScanTile, (c+1)*kScanTile) -> bsum[c]
@@ -90,7 +68,7 @@ __global__ void k_scan_reduce(const uint32_t* __restrict__ v, uint32_t n, uint32
         if (i < n) sum += v[i];
     }
     uint32_t total;
-    cta_exclusive_scan(sum, s_warp, total);
+    cta_exclusive_scan<kThreads>(sum, s_warp, total);
     if (threadIdx.x == 0) bsum[blockIdx.x] = total;
 }
 
@@ -107,7 +85,7 @@ __global__ void k_scan_apply(uint32_t* __restrict__ v, uint32_t n, const uint32_
         sum += x[k];
     }
     uint32_t total;
-    uint32_t run = bsum[blockIdx.x] + cta_exclusive_scan(sum, s_warp, total);
+    uint32_t run = bsum[blockIdx.x] + cta_exclusive_scan<kThreads>(sum, s_warp, total);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         const uint64_t i = base + k;
@@ -137,7 +115,7 @@ __global__ void k_ri_fill(const uint32_t* __restrict__ indptr, const uint32_t* _
         // ballot per row took 16.
         uint32_t cnt = 0;
         for (uint32_t t0 = a; t0 < b; t0 += kWarp) {
-            const uint32_t m = t0 + lane < b ? rowmask[t0 + lane] : 0u;
+            const uint32_t m = t0 + lane < b ? fold_rows(rowmask[t0 + lane]) : 0u;
             uint32_t q[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k)
@@ -157,7 +135,7 @@ __global__ void k_ri_fill(const uint32_t* __restrict__ indptr, const uint32_t* _
         if (I + 1 == R && lane == 16) off[16 * (uint64_t)R] = start;  // = the entry total
         for (uint32_t t0 = a; t0 < b; t0 += kWarp) {
             const uint32_t t = t0 + lane;
-            const uint32_t m = t < b ? rowmask[t] : 0u;
+            const uint32_t m = t < b ? fold_rows(rowmask[t]) : 0u;
             const uint32_t K = t < b ? indices[t] : 0u;
 #pragma unroll
             for (int r = 0; r < 16; ++r) {
