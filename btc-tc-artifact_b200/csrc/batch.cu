@@ -433,14 +433,7 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
     g->n_row_blocks = (int32_t)rows;
     g->input_edges = m;
     g->edges_known = false;
-    if (!g->h_meta) {
-        void* p = nullptr;
-        if (cudaMallocHost(&p, sizeof(unsigned long long) * kMetaSlots) != cudaSuccess) {
-            cudaGetLastError();
-            return BTC_E_NOMEM;
-        }
-        g->h_meta = static_cast<unsigned long long*>(p);
-    }
+    if (!g->h_meta && !(g->h_meta = host_slot_alloc())) return BTC_E_NOMEM;
     BTC_TRY(g->meta.reserve(sizeof(unsigned long long) * kMetaSlots));
     unsigned long long* meta = g->meta.as<unsigned long long>();
 

@@ -92,20 +92,15 @@ int ensure_count_scratch(btc_bitbsr* g)
 int ensure_host_meta(btc_bitbsr* g)
 {
     if (g->h_meta) return BTC_OK;
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(unsigned long long) * kMetaSlots,
-                      cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        return BTC_E_NOMEM;
-    }
+    unsigned long long* p = host_slot_alloc();
+    if (!p) return BTC_E_NOMEM;
     void* d = nullptr;
     if (cudaHostGetDevicePointer(&d, p, 0) != cudaSuccess) {
         cudaGetLastError();
-        cudaFreeHost(p);
+        host_slot_free(p);
         return BTC_E_CUDA;
     }
-    std::memset(p, 0, sizeof(unsigned long long) * kMetaSlots);
-    g->h_meta = static_cast<unsigned long long*>(p);
+    g->h_meta = p;
     g->d_hmeta = static_cast<unsigned long long*>(d);
     return BTC_OK;
 }
@@ -685,7 +680,8 @@ int btc_density_hist(btc_bitbsr* g, btc_stream_t stream, uint64_t* hist)
                                         cudaMemcpyDeviceToHost, stream) != cudaSuccess)
         st = BTC_E_CUDA;
     if (st == BTC_OK && cudaStreamSynchronize(stream) != cudaSuccess) st = BTC_E_CUDA;
-    d.release();
+    if (st == BTC_OK) d.release_idle();
+    else d.release();
     return st;
 }
 
@@ -737,11 +733,18 @@ int btc_convert_coo_to_bcsr_16x32_gpu(btc_bcsr_device* b, const int32_t* d_rows,
 void btc_bcsr_free(btc_bcsr_device* b)
 {
     if (!b) return;
-    if (b->indptr) cudaFree(b->indptr);
-    if (b->indices) cudaFree(b->indices);
-    if (b->blocks) cudaFree(b->blocks);
-    if (b->row_indices) cudaFree(b->row_indices);
-    if (b->result) cudaFree(b->result);
+    if (b->indptr || b->indices || b->blocks || b->row_indices || b->result) {
+        // (a failed wait gives the memory up: something may still use it)
+        if (cudaDeviceSynchronize() == cudaSuccess) {
+            dev_free(b->indptr);
+            dev_free(b->indices);
+            dev_free(b->blocks);
+            dev_free(b->row_indices);
+            dev_free(b->result);
+        } else {
+            cudaGetLastError();
+        }
+    }
     b->indptr = b->indices = b->blocks = b->row_indices = nullptr;
     b->result = nullptr;
 }

@@ -58,6 +58,20 @@ __host__ __device__ __forceinline__ int log2_exact(int x)
     return k;
 }
 
+// Device memory for handles and workspaces, from a pool the library keeps per device
+// (devmem.cu): a cudaMalloc and cudaFree pair of a fresh allocation cost 0.1 to 2 ms here, a
+// pair from the pool a few microseconds (a one-off build, count and free of an R-MAT scale
+// 16 graph, 17 buffers: 5.3-8.6 ms before).  The memory can be used on any stream once the
+// call returns.  dev_free does not wait: nothing may be using the memory any more.
+cudaError_t dev_alloc(void** p, size_t bytes);
+void dev_free(void* p);
+
+// A zeroed slot of kHostSlotWords uint64 in pinned, mapped, portable host memory (nullptr
+// without memory), and its return: nothing may be writing to it any more.
+constexpr size_t kHostSlotWords = 16;
+unsigned long long* host_slot_alloc();
+void host_slot_free(unsigned long long* s);
+
 // A grow-only device buffer.  reserve() keeps contents only when no reallocation
 // happens; callers treat it as scratch.
 struct DevBuf {
@@ -65,8 +79,7 @@ struct DevBuf {
     size_t bytes = 0;
     // Stream-ordered allocation, for an owner that uses the buffer on one stream only:
     // with `pool` and `stream` set, a growth frees and allocates in that stream's order
-    // (cudaFreeAsync / cudaMallocFromPoolAsync) instead of cudaFree's wait for the whole
-    // device.  `pooled` records how the current allocation was made.
+    // (cudaFreeAsync / cudaMallocFromPoolAsync) instead of waiting for the whole device.  `pooled` records how the current allocation was made.
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
     bool pooled = false;
@@ -91,13 +104,22 @@ struct DevBuf {
     cudaError_t allocate(size_t b)
     {
         pooled = pool != nullptr && stream != nullptr;
-        return pooled ? cudaMallocFromPoolAsync(&ptr, b, pool, stream) : cudaMalloc(&ptr, b);
+        return pooled ? cudaMallocFromPoolAsync(&ptr, b, pool, stream) : dev_alloc(&ptr, b);
     }
     void release()
     {
+        if (ptr && !pooled && cudaDeviceSynchronize() != cudaSuccess) {
+            cudaGetLastError();  // something may still use it: the memory is given up
+            ptr = nullptr;
+        }
+        release_idle();
+    }
+    // the same when nothing uses the buffer any more (the owner has waited)
+    void release_idle()
+    {
         if (ptr) {
             if (pooled) cudaFreeAsync(ptr, stream);
-            else cudaFree(ptr);
+            else dev_free(ptr);
         }
         ptr = nullptr;
         bytes = 0;
@@ -304,10 +326,14 @@ enum {
     kMetaRowChunks = 8,
     kMetaSlots = 9
 };
+static_assert(kMetaSlots <= kHostSlotWords, "a host slot holds the metadata");
 
 // Queue/completion words of the count kernel: done (u32) at byte 0, work (u64) at 8.
 constexpr size_t kCountCtlBytes = 16;
 
 int device_sm_count();
+// Id of the calling thread's current context (0 when it cannot be read): a device reset
+// gives the device a new one.
+unsigned long long current_context_id();
 
 }  // namespace btc200

@@ -1,0 +1,170 @@
+// devmem.cu -- the library's device memory: one stream-ordered pool per device (and context).
+//
+// Handles that live for one graph allocate some 20 buffers; with cudaMalloc and cudaFree
+// each of them maps and unmaps memory and waits for the device.  The pool keeps up to
+// kKeepBytes of freed memory for the next handle; what is above that goes back to the
+// device at the next wait.  Allocations are made on a stream of the pool's own and are
+// complete when dev_alloc returns, so a caller may use the memory on any stream; freed
+// memory is idle (dev_free's callers have waited), so it may be handed to any other.
+#include "common.cuh"
+
+#include <cuda.h>
+
+#include <cstring>
+#include <mutex>
+#include <vector>
+
+namespace btc200 {
+
+unsigned long long current_context_id()
+{
+    using GetCurrent = CUresult (*)(CUcontext*);
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    static GetCurrent get_current = nullptr;
+    static GetId get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<GetCurrent>(f);
+        f = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<GetId>(f);
+        cudaGetLastError();
+    });
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx) return 0;
+    if (get_id(ctx, &id) != CUDA_SUCCESS) return 0;
+    return id;
+}
+
+namespace {
+
+constexpr uint64_t kKeepBytes = 1ull << 30;
+
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
+    unsigned long long ctx_id = 0;  // the context it belongs to
+    bool tried = false;
+};
+
+// The current device's pool, made on first use in each context; false without pool support.
+bool pool_for_current_device(cudaMemPool_t* pool, cudaStream_t* stream)
+{
+    static std::mutex mu;
+    static DevicePool pools[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    const unsigned long long id = current_context_id();
+    std::lock_guard<std::mutex> lock(mu);
+    DevicePool& p = pools[dev];
+    if (!p.tried || (id != 0 && id != p.ctx_id)) {
+        p = DevicePool{};
+        p.tried = true;
+        int supported = 0;
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        uint64_t keep = kKeepBytes;
+        if (cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess ||
+            !supported || cudaMemPoolCreate(&p.pool, &props) != cudaSuccess) {
+            p.pool = nullptr;
+        } else if (cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+                   cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) != cudaSuccess) {
+            cudaMemPoolDestroy(p.pool);
+            p.pool = nullptr;
+        }
+        if (!p.pool) cudaGetLastError();
+        p.ctx_id = id ? id : current_context_id();
+    }
+    *pool = p.pool;
+    *stream = p.stream;
+    return p.pool != nullptr;
+}
+
+}  // namespace
+
+// Pinned, mapped host slots of kHostSlotWords uint64, carved from blocks that stay until the
+// process ends (64 KB holds 512 handles; cudaHostAlloc and cudaFreeHost cost 0.01 to 5 ms a
+// handle).
+namespace {
+
+constexpr size_t kSlotsPerBlock = 512;
+
+struct HostSlots {
+    std::mutex mu;
+    std::vector<unsigned long long*> free_slots;
+    unsigned long long ctx_id = 0;  // a device reset takes the blocks with it
+};
+HostSlots& host_slots()
+{
+    static HostSlots* h = new HostSlots;  // (outlives handles freed at exit)
+    return *h;
+}
+
+}  // namespace
+
+unsigned long long* host_slot_alloc()
+{
+    HostSlots& h = host_slots();
+    const unsigned long long id = current_context_id();
+    std::lock_guard<std::mutex> lock(h.mu);
+    int devices = 0;
+    // (contexts of several devices share portable memory; one device's reset is told apart)
+    if (cudaGetDeviceCount(&devices) == cudaSuccess && devices == 1 && id != h.ctx_id) {
+        h.free_slots.clear();
+        h.ctx_id = id;
+    }
+    if (h.free_slots.empty()) {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(unsigned long long) * kHostSlotWords * kSlotsPerBlock,
+                          cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (id == 0) h.ctx_id = current_context_id();  // (the allocation made the context)
+        for (size_t i = kSlotsPerBlock; i-- > 0;)
+            h.free_slots.push_back(static_cast<unsigned long long*>(p) + i * kHostSlotWords);
+    }
+    unsigned long long* s = h.free_slots.back();
+    h.free_slots.pop_back();
+    std::memset(s, 0, sizeof(unsigned long long) * kHostSlotWords);
+    return s;
+}
+
+void host_slot_free(unsigned long long* s)
+{
+    if (!s) return;
+    HostSlots& h = host_slots();
+    std::lock_guard<std::mutex> lock(h.mu);
+    h.free_slots.push_back(s);
+}
+
+cudaError_t dev_alloc(void** ptr, size_t bytes)
+{
+    cudaMemPool_t pool;
+    cudaStream_t stream;
+    if (!pool_for_current_device(&pool, &stream)) return cudaMalloc(ptr, bytes);
+    cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
+    if (e == cudaErrorMemoryAllocation) {
+        // give the kept memory back and try once more
+        cudaGetLastError();
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
+    }
+    return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+}
+
+void dev_free(void* p)
+{
+    // (cudaFree of pool memory returns it to its pool without a wait)
+    if (p) cudaFree(p);
+}
+
+}  // namespace btc200

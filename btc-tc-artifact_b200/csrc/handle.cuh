@@ -80,8 +80,16 @@ struct btc_bitbsr {
     }
     void release_all()
     {
-        for_each_buf([](btc200::DevBuf& b) { b.release(); });
-        if (h_meta) cudaFreeHost(h_meta);
+        // one wait for all the buffers that are not stream-ordered, and for the host slot
+        bool wait = h_meta != nullptr;
+        for_each_buf([&](btc200::DevBuf& b) { wait |= b.ptr && !b.pooled; });
+        if (wait && cudaDeviceSynchronize() != cudaSuccess) {
+            cudaGetLastError();
+            for_each_buf([](btc200::DevBuf& b) { b.release(); });
+            h_meta = nullptr;  // (given up: something may still write to it)
+        }
+        for_each_buf([](btc200::DevBuf& b) { b.release_idle(); });
+        btc200::host_slot_free(h_meta);
         h_meta = nullptr;
         d_hmeta = nullptr;
         if (meta_event) cudaEventDestroy(meta_event);

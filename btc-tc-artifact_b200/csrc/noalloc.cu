@@ -35,34 +35,6 @@ struct ScratchSetup {
 std::mutex g_setup_mu;
 ScratchSetup g_setup[kMaxDevices];
 
-// Unique id of the current context (driver API through the runtime's entry-point table,
-// so the library needs no link against libcuda); 0 when there is none yet.
-unsigned long long current_context_id()
-{
-    using GetCurrent = CUresult (*)(CUcontext*);
-    using GetId = CUresult (*)(CUcontext, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<GetCurrent>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<GetId>(f);
-        cudaGetLastError();
-    });
-    CUcontext ctx = nullptr;
-    unsigned long long id = 0;
-    if (!get_current || !get_id || get_current(&ctx) != CUDA_SUCCESS || !ctx) return 0;
-    if (get_id(ctx, &id) != CUDA_SUCCESS) return 0;
-    return id;
-}
-
 // Device address of g_noalloc_scratch on the current device.  In host code the array's
 // name is only a host-side handle, so the address comes from cudaGetSymbolAddress, with
 // the device current, once per device and context: a device reset (cudaDeviceReset)

@@ -118,6 +118,7 @@ int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n
     unsigned long long h[2] = {0, 0};
     BTC_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
     BTC_CUDA_TRY(cudaStreamSynchronize(s));
+    sc.b.release_idle();
     *L = h[1] ? (double)h[0] / (double)h[1] : 0.0;
     return BTC_OK;
 }

@@ -215,11 +215,8 @@ extern "C" int btc_preprocess_for_triangle_counting(int32_t* d_rows, int32_t* d_
     DevBuf k0, k1, scratch, tbase, meta;
     int st = BTC_OK;
     auto cleanup = [&]() {
-        k0.release();
-        k1.release();
-        scratch.release();
-        tbase.release();
-        meta.release();
+        cudaDeviceSynchronize();
+        for (DevBuf* b : {&k0, &k1, &scratch, &tbase, &meta}) b->release_idle();
     };
 #define PRE_TRY(x)                 \
     do {                           \
