@@ -574,7 +574,7 @@ int btc_batch_count(btc_batch* b, int tau, btc_stream_t stream, unsigned long lo
     if (b->row_store && tau >= default_tau(g->tile_cols)) {
         BTC_TRY(launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks, g->tile_cols, g->n_row_blocks, b->max_col_blocks, scr,
                                     b->row_off.as<uint32_t>(), (uint32_t)b->num_graphs, counts,
-                                    g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), 0, cap, true,
+                                    g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), 0, cap, true, true,
                                     build_meta, count_grid_size(g->tile_cols), stream));
     } else {
     if (b->row_store) ensure_row_index(g, build_meta ? build_meta + kMetaTiles : nullptr, cap, stream);

@@ -278,6 +278,8 @@ inline uint64_t row_store_chunks(uint64_t entries, uint64_t R)
 // cap, or cap when d_tiles is null; nothing when T > cap).  meta:
 // the build's metadata slots (kMetaRowChunks zero: it counts the chunks handed out); also
 // raises meta[kMetaRowMax] to the most tiles in one row block.
+// *out += the set bits of mask[0, n).
+int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* out, cudaStream_t s);
 int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indices, const uint32_t* blocks,
                     int32_t n_row_blocks, const uint32_t* rowmask, const unsigned long long* d_tiles,
                     uint32_t cap, unsigned long long* meta, const RowStore& out,
@@ -285,13 +287,14 @@ int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indic
 
 // The streaming count (count_stream.cu) of the sample tiles [tile_begin, tile_end), or of
 // all of them with `whole`.  rs_chunks: the store's meta[kMetaRowChunks].  max_col_blocks: the most 64-column blocks a row's columns can
-// span.  grid: the CTAs scr.partials has room for.
+// span.  lower: the matrix is a lower triangle (every handle's is; a caller's
+// Bit-BSR need not be).  grid: the CTAs scr.partials has room for.
 int stream_blocks_per_sm_max();
 int launch_count_stream(const RowStore& rs, const unsigned long long* rs_chunks, int tile_cols,
                         int32_t n_row_blocks, uint32_t max_col_blocks, CountScratch scr, const uint32_t* graph_rows, uint32_t num_graphs,
                         unsigned long long* graph_counts, const uint32_t* row_indices,
                         const uint32_t* indices, uint32_t tile_begin, uint32_t tile_end, bool whole,
-                        const unsigned long long* build_meta, int grid, cudaStream_t s);
+                        bool lower, const unsigned long long* build_meta, int grid, cudaStream_t s);
 
 // Row index of the row-wise count kernel (rowindex.cu): for vertex u, ent[off[u],
 // off[u+1]) lists (column block, tile) of the tiles whose row u % 16 holds a bit, in tile

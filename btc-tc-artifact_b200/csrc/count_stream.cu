@@ -89,7 +89,7 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
                CountScratch scr, const uint32_t* __restrict__ graph_rows, uint32_t num_graphs,
                unsigned long long* __restrict__ graph_counts, const uint32_t* __restrict__ row_indices,
                const uint32_t* __restrict__ indices, int log2c, uint32_t tile_begin, uint32_t tile_end,
-               bool whole, const unsigned long long* __restrict__ build_meta)
+               bool whole, bool lower, const unsigned long long* __restrict__ build_meta)
 {
     using Key = RowKey<kWide>;
     using KeyWord = typename Key::Word;
@@ -185,11 +185,12 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
         __syncwarp();
     };
 
-    // Samples: chunks [fa, fb) of the row whose chunks start at p0 (its chunks past fb hold
-    // only higher columns, which no sample's row can reach).
-    auto take_row = [&](uint32_t u, uint32_t p0, uint32_t fa, uint32_t fb) {
-        const bool small = fb - p0 <= (uint32_t)kGroups;
-        const uint32_t wb = fb * kRowLanes;  // words end
+    // Samples: chunks [fa, fb) of u's row, chunks [p0, p1).  In a lower triangle the chunks
+    // past fb hold only higher columns, which no sample's row can reach: they are left out.
+    auto take_row = [&](uint32_t u, uint32_t p0, uint32_t p1, uint32_t fa, uint32_t fb) {
+        if (lower) p1 = fb;
+        const bool small = p1 - p0 <= (uint32_t)kGroups;
+        const uint32_t wb = p1 * kRowLanes;  // words end
         const uint32_t w_first = p0 * kRowLanes + lane;
         KeyWord k0{};
         uint4 b0 = make_uint4(0u, 0u, 0u, 0u);
@@ -209,15 +210,15 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
             for (uint32_t w = w_first + kWarp; w < wb; w += kWarp) stage(key[w], bits[w]);
         const uint32_t span = Key::hi(key[wb - 1]) - K0;  // up to the row's last column block
         __syncwarp();
-        for (uint32_t c = small ? p0 * kRowLanes : fa * kRowLanes; c < wb; c += kWarp) {
+        for (uint32_t c = small ? p0 * kRowLanes : fa * kRowLanes; c < fb * kRowLanes; c += kWarp) {
             KeyWord K = k0;
             uint4 b = b0;
             if (!small && c + lane < wb) {
                 K = key[c + lane];
                 b = bits[c + lane];
             }
-            if (c + lane < fa * kRowLanes || c + lane >= wb) b = make_uint4(0u, 0u, 0u, 0u);
-            if (lane == 0 && c == p0 * kRowLanes && fa == p0) {
+            if (c + lane < fa * kRowLanes || c + lane >= fb * kRowLanes) b = make_uint4(0u, 0u, 0u, 0u);
+            if (lower && lane == 0 && c == p0 * kRowLanes && fa == p0) {
                 // the row's first neighbour has no lower one in the row
                 if (b.x) b.x &= b.x - 1;
                 else b.y &= b.y - 1;
@@ -272,8 +273,11 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
                 }
                 v += select_bit(w, r);
                 const uint32_t vo = v + (v >> 4);  // 17 offsets per row block
-                uint32_t r0 = off[vo], r1 = off[vo + 1];
-                if (i0 + lane >= total) r1 = r0;
+                uint32_t r0 = 0, r1 = 0;
+                if (i0 + lane < total && (lower || (v >> 4) < n_row_blocks)) {
+                    r0 = off[vo];
+                    r1 = off[vo + 1];
+                }
                 // list its row's chunks
                 for (;;) {
                     uint32_t at = r1 - r0;
@@ -289,12 +293,12 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
                     if (nid <= (uint32_t)kIdCap) break;
                     nid = kIdCap;
                     __syncwarp();
-                    walk(K0, span, p0, fb);
+                    walk(K0, span, p0, p1);
                 }
             }
         }
         __syncwarp();
-        if (nid) walk(K0, span, p0, fb);
+        if (nid) walk(K0, span, p0, p1);
         // empty the table again
         auto clear = [&](const KeyWord& k) {
             const uint32_t s0 = Key::lo(k) - K0, s1 = Key::hi(k) - K0;
@@ -346,8 +350,8 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
             while (todo) {
                 const int r = __ffs(todo) - 1;
                 todo &= todo - 1;
-                take_row(16u * I + r, __shfl_sync(kFull, o, r), __shfl_sync(kFull, fa, r),
-                         __shfl_sync(kFull, fb, r));
+                take_row(16u * I + r, __shfl_sync(kFull, o, r), __shfl_sync(kFull, o1, r),
+                         __shfl_sync(kFull, fa, r), __shfl_sync(kFull, fb, r));
             }
             // the next row block's first run
             const uint32_t end = __shfl_sync(kFull, o, 16);
@@ -423,7 +427,7 @@ int launch_count_stream(const RowStore& rs, const unsigned long long* rs_chunks,
                         int32_t n_row_blocks, uint32_t max_col_blocks, CountScratch scr, const uint32_t* graph_rows, uint32_t num_graphs,
                         unsigned long long* graph_counts, const uint32_t* row_indices,
                         const uint32_t* indices, uint32_t tile_begin, uint32_t tile_end, bool whole,
-                        const unsigned long long* build_meta, int grid, cudaStream_t s)
+                        bool lower, const unsigned long long* build_meta, int grid, cudaStream_t s)
 {
     const int size = row_store_wide(n_row_blocks) ? 3 : max_col_blocks <= 256 ? 0 : max_col_blocks <= 512 ? 1 : 2;
     const int v = 2 * size + (graph_counts ? 1 : 0);
@@ -432,7 +436,7 @@ int launch_count_stream(const RowStore& rs, const unsigned long long* rs_chunks,
     if (per_sm * device_sm_count() < grid) grid = per_sm * device_sm_count();
     stream_kernel(v)<<<grid, kSThreads, stream_smem(v), s>>>(
         rs.off, rs.key, rs.bits, rs.first_row, rs_chunks, (uint32_t)n_row_blocks, scr, graph_rows, num_graphs,
-        graph_counts, row_indices, indices, tile_cols == 128 ? 7 : 5, tile_begin, tile_end, whole,
+        graph_counts, row_indices, indices, tile_cols == 128 ? 7 : 5, tile_begin, tile_end, whole, lower,
         build_meta);
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }

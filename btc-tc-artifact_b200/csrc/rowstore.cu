@@ -278,7 +278,24 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
     if (w == 0 && lane == 0 && longest) atomicMax(&meta[kMetaRowMax], (unsigned long long)longest);
 }
 
+__global__ void k_mask_popcount(const uint32_t* __restrict__ mask, uint32_t n,
+                                unsigned long long* __restrict__ out)
+{
+    uint32_t sum = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x)
+        sum += __popc(mask[i]);
+    sum = __reduce_add_sync(kFull, sum);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(out, (unsigned long long)sum);
+}
+
 }  // namespace rs
+
+int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* out, cudaStream_t s)
+{
+    if (n) rs::k_mask_popcount<<<std::min<uint32_t>((n + 255) / 256, 4u * device_sm_count()), 256, 0, s>>>(mask, n, out);
+    return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+}
 
 int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indices, const uint32_t* blocks,
                     int32_t n_row_blocks, const uint32_t* rowmask, const unsigned long long* d_tiles,
