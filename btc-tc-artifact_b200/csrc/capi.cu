@@ -301,8 +301,9 @@ static bool launch_build_graph(btc_bitbsr* g, const BuildPlan& P, cudaStream_t s
     return cudaGraphLaunch(g->graph_exec, s) == cudaSuccess;
 }
 
+// tiles_only: the caller keeps the reference-shaped arrays alone, so no row store is made.
 static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
-                      int tile_cols, uint32_t flags, cudaStream_t s)
+                      int tile_cols, uint32_t flags, cudaStream_t s, bool tiles_only = false)
 {
     if (n < 0 || m < 0 || (uint64_t)m > kMaxEdges) return BTC_E_INVAL;
     if (m > 0 && (!src || !dst)) return BTC_E_INVAL;
@@ -443,7 +444,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     BTC_TRY(g->rowmask.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
     // the tile count is known here: the row store exactly when the graph averages 8 or more
     // tiles per row block
-    P.row_store = row_store_possible(m, geom.n_row_blocks) &&
+    P.row_store = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
                   (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks &&
                   reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * tiles)) == BTC_OK;
     if (P.use_bitmap) {
@@ -701,8 +702,13 @@ static int convert_struct(btc_bcsr_device* b, const int32_t* d_rows, const int32
     if (!b) return BTC_E_INVAL;
     std::memset(b, 0, sizeof(*b));
     btc_bitbsr* g = nullptr;
-    const int st = btc_build_bitbsr(d_rows, d_cols, nnz, num_rows, tile_cols, 0, nullptr, &g);
-    if (st != BTC_OK) return st;
+    g = new (std::nothrow) btc_bitbsr();
+    if (!g) return BTC_E_NOMEM;
+    const int st = build_into(g, d_rows, d_cols, nnz, num_rows, tile_cols, 0, nullptr, true);
+    if (st != BTC_OK) {
+        btc_free(g);
+        return st;
+    }
     // hand the arrays to the struct; it frees them one by one (btc_bcsr_free)
     b->indptr = g->indptr.as<uint32_t>();
     b->indices = g->indices.as<uint32_t>();

@@ -27,18 +27,27 @@ namespace {
 
 constexpr int kSThreads = 256;
 constexpr int kSWarps = kSThreads / kWarp;
-constexpr int kIdCap = 256;    // chunks listed per walk
+constexpr int kIdCap = 240;    // chunks listed per walk
 constexpr int kGroup = kRowLanes;  // lanes that read a chunk
 constexpr int kGroups = kWarp / kGroup;
 constexpr int kBatch = 4;      // chunks a group has in flight
+constexpr int kPastWords = 64;
+static_assert(kPastWords == 2 * kWarp, "a lane ranks two words");
 static_assert(kGroup == 8 && kIdCap % (kGroups * kBatch) == 0, "a walk's rounds are whole");
+
+// Tables of fewer than 1,024 slots are for graphs whose rows they always hold.
+template <int W>
+constexpr bool kPastTable = W >= 1024;
 
 template <int W>
 struct __align__(16) StreamSmem {
     uint2 tab[W + 2];          // u's row by K - K0; slot W stays zero
+    uint32_t past[kPastWords]; // column blocks of u's entries past the table, modulo 32 kPastWords
+    uint16_t rank[kPastWords]; // set bits of `past` before each word
     uint32_t ids[kIdCap];      // chunks of the neighbours' rows, read four at a time
 };
-static_assert(sizeof(uint2) * 2 % 16 == 0, "ids keep the 16-byte alignment");
+static_assert(sizeof(uint2) * 2 % 16 == 0 && kPastWords % 4 == 0, "ids keep the 16-byte alignment");
+static_assert(sizeof(StreamSmem<1024>) * kSWarps + 1184 <= 233472 / 3, "three CTAs per SM");
 
 template <int W>
 constexpr size_t stream_smem_bytes() { return sizeof(StreamSmem<W>) * kSWarps; }
@@ -101,6 +110,7 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
     const int grp = lane / kGroup, sub = lane % kGroup;
     StreamSmem<W>& s = reinterpret_cast<StreamSmem<W>*>(stream_smem_raw)[warp];
     for (int i = lane; i <= W; i += kWarp) s.tab[i] = make_uint2(0u, 0u);
+    for (int i = lane; i < kPastWords; i += kWarp) s.past[i] = 0u;
 
     // The chunks to take as samples, [kRowRun, e_hi), or with a tile range the row blocks
     // [I_lo, I_hi), the first and last of them cut by column.
@@ -129,30 +139,47 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
 
     uint32_t nid = 0;  // chunks listed
 
-    // |entry (k, x) AND u's row| for an entry past the table: bisects u's row, the chunks
-    // [p0, fb) of the store (entry i of a chunk sits in lane i % 8's word, half i / 8).
-    auto beyond = [&](uint32_t k, uint32_t x, uint32_t y, uint32_t p0, uint32_t fb) -> uint32_t {
+    // |entry AND u's row| for an entry past the table: slot >= W, bits (x, y); u's row is the
+    // chunks [p0, p1) of the store (entry i of a chunk sits in lane i % 8's word, half i / 8)
+    // and its entries from `after` on lie past the table.  Most look-ups match none of them,
+    // which their bit in `past` shows; a row that spans at most 32 kPastWords column blocks
+    // past the table has them one per bit, and the bits' ranks number its entries, else the
+    // row is bisected.  (Without `past` some lane of almost every round went on to the
+    // bisection where 1% of the look-ups pass the table: R-MAT scale 22 14.4 ms, 10.9 with
+    // it.  Ranks instead of bisection where 5% pass it, most of them matches: scale 18 in
+    // natural order 2.0 -> 1.1 ms.)
+    auto beyond = [&](uint32_t slot, uint32_t x, uint32_t y, uint32_t K0, uint32_t span, uint32_t after,
+                      uint32_t p0, uint32_t p1) -> uint32_t {
+        const uint32_t pb = (slot - (uint32_t)W) % (32u * kPastWords);
+        const uint32_t pw = s.past[pb / 32];
+        if (!((pw >> (pb & 31u)) & 1u)) return 0u;
         auto word = [&](uint32_t i) { return i / kRowChunk * kRowLanes + i % kRowLanes; };
         auto half = [&](uint32_t i) { return (i / kRowLanes) & 1u; };
-        auto key_at = [&](uint32_t i) {
-            const KeyWord w = key[word(i)];
-            return half(i) ? Key::hi(w) : Key::lo(w);
-        };
-        uint32_t lo = p0 * kRowChunk, hi = fb * kRowChunk;
-        const uint32_t end = hi;
-        while (lo < hi) {
-            const uint32_t mid = lo + ((hi - lo) >> 1);
-            if (key_at(mid) < k) lo = mid + 1;
-            else hi = mid;
+        uint32_t i;
+        if (span < (uint32_t)W + 32u * kPastWords) {
+            i = after + s.rank[pb / 32] + __popc(pw & ((1u << (pb & 31u)) - 1u));
+        } else {
+            auto key_at = [&](uint32_t j) {
+                const KeyWord w = key[word(j)];
+                return half(j) ? Key::hi(w) : Key::lo(w);
+            };
+            uint32_t hi = p1 * kRowChunk;
+            const uint32_t end = hi, k = slot + K0;
+            i = after;
+            while (i < hi) {
+                const uint32_t mid = i + ((hi - i) >> 1);
+                if (key_at(mid) < k) i = mid + 1;
+                else hi = mid;
+            }
+            if (i >= end || key_at(i) != k) return 0u;
         }
-        if (lo >= end || key_at(lo) != k) return 0u;
-        const uint4 v = bits[word(lo)];
-        return half(lo) ? __popc(v.z & x) + __popc(v.w & y) : __popc(v.x & x) + __popc(v.y & y);
+        const uint4 v = bits[word(i)];
+        return half(i) ? __popc(v.z & x) + __popc(v.w & y) : __popc(v.x & x) + __popc(v.y & y);
     };
 
-    // Counts u's row (its table, first column block K0, last one K0 + span; chunks [p0, fb))
+    // Counts u's row (its table, first column block K0, last one K0 + span; chunks [p0, p1))
     // against the listed chunks.
-    auto walk = [&](uint32_t K0, uint32_t span, uint32_t p0, uint32_t fb) {
+    auto walk = [&](uint32_t K0, uint32_t span, uint32_t after, uint32_t p0, uint32_t p1) {
         const uint32_t n = (nid + kGroups * kBatch - 1) / (kGroups * kBatch) * (kGroups * kBatch);
         if (nid + lane < n) s.ids[nid + lane] = 0u;  // chunk 0 is empty
         __syncwarp();
@@ -174,9 +201,11 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
                 const uint2 a0 = s.tab[min(s0, (uint32_t)W)], a1 = s.tab[min(s1, (uint32_t)W)];
                 part += __popc(a0.x & b[x].x) + __popc(a0.y & b[x].y) + __popc(a1.x & b[x].z) +
                         __popc(a1.y & b[x].w);
-                if (span >= (uint32_t)W) {
-                    if (s0 >= (uint32_t)W && s0 <= span) part += beyond(s0 + K0, b[x].x, b[x].y, p0, fb);
-                    if (s1 >= (uint32_t)W && s1 <= span) part += beyond(s1 + K0, b[x].z, b[x].w, p0, fb);
+                if (kPastTable<W> && span >= (uint32_t)W) {
+                    if (s0 >= (uint32_t)W && s0 <= span)
+                        part += beyond(s0, b[x].x, b[x].y, K0, span, after, p0, p1);
+                    if (s1 >= (uint32_t)W && s1 <= span)
+                        part += beyond(s1, b[x].z, b[x].w, K0, span, after, p0, p1);
                 }
             }
         }
@@ -199,17 +228,43 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
             b0 = bits[w_first];
         }
         const uint32_t K0 = __shfl_sync(kFull, Key::lo(k0), 0);
+        const uint32_t span = Key::hi(key[wb - 1]) - K0;  // up to the row's last column block
         // (padding entries have no bits and the row's last key)
+        uint32_t inside = 0;  // entries in the table
+        auto put = [&](uint32_t slot, uint32_t x, uint32_t y) {
+            if ((x | y) == 0u) return;
+            if (!kPastTable<W> || slot < (uint32_t)W) {
+                s.tab[slot] = make_uint2(x, y);
+                ++inside;
+            } else {
+                const uint32_t pb = (slot - (uint32_t)W) % (32u * kPastWords);
+                atomicOr(&s.past[pb / 32], 1u << (pb & 31u));
+            }
+        };
         auto stage = [&](const KeyWord& k, const uint4& b) {
-            const uint32_t s0 = Key::lo(k) - K0, s1 = Key::hi(k) - K0;
-            if ((b.x | b.y) != 0u && s0 < (uint32_t)W) s.tab[s0] = make_uint2(b.x, b.y);
-            if ((b.z | b.w) != 0u && s1 < (uint32_t)W) s.tab[s1] = make_uint2(b.z, b.w);
+            put(Key::lo(k) - K0, b.x, b.y);
+            put(Key::hi(k) - K0, b.z, b.w);
         };
         stage(k0, b0);
         if (!small)
             for (uint32_t w = w_first + kWarp; w < wb; w += kWarp) stage(key[w], bits[w]);
-        const uint32_t span = Key::hi(key[wb - 1]) - K0;  // up to the row's last column block
         __syncwarp();
+        uint32_t after = 0;  // the first entry past the table
+        if (kPastTable<W> && span >= (uint32_t)W) {
+            after = p0 * kRowChunk + __reduce_add_sync(kFull, inside);
+            if (span < (uint32_t)W + 32u * kPastWords) {
+                const uint32_t c0 = __popc(s.past[2 * lane]), c1 = __popc(s.past[2 * lane + 1]);
+                uint32_t incl = c0 + c1;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t y = __shfl_up_sync(kFull, incl, d);
+                    if (lane >= d) incl += y;
+                }
+                s.rank[2 * lane] = (uint16_t)(incl - c0 - c1);
+                s.rank[2 * lane + 1] = (uint16_t)(incl - c1);
+            }
+            __syncwarp();
+        }
         for (uint32_t c = small ? p0 * kRowLanes : fa * kRowLanes; c < fb * kRowLanes; c += kWarp) {
             KeyWord K = k0;
             uint4 b = b0;
@@ -293,30 +348,35 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
                     if (nid <= (uint32_t)kIdCap) break;
                     nid = kIdCap;
                     __syncwarp();
-                    walk(K0, span, p0, p1);
+                    walk(K0, span, after, p0, p1);
                 }
             }
         }
         __syncwarp();
-        if (nid) walk(K0, span, p0, p1);
+        if (nid) walk(K0, span, after, p0, p1);
         // empty the table again
         auto clear = [&](const KeyWord& k) {
             const uint32_t s0 = Key::lo(k) - K0, s1 = Key::hi(k) - K0;
             if (s0 < (uint32_t)W) s.tab[s0] = make_uint2(0u, 0u);
             if (s1 < (uint32_t)W) s.tab[s1] = make_uint2(0u, 0u);
         };
+        if (kPastTable<W> && span >= (uint32_t)W)
+            for (int i = lane; i < kPastWords; i += kWarp) s.past[i] = 0u;
         if (w_first < wb) clear(k0);
         if (!small)
             for (uint32_t w = w_first + kWarp; w < wb; w += kWarp) clear(key[w]);
         __syncwarp();
     };
 
-    // Work queue: `per` runs of kRowRun chunks each, or one row block each.  A warp's first
-    // grab is its own index, later ones are numbered by an atomic.
+    // Work queue: `per` chunks each, or one row block each.  A warp's first grab is its own
+    // index, later ones are numbered by an atomic.  A chunk of a hub row in natural order
+    // holds up to 1,024 neighbours with long rows, so grabs stay at one 32nd of an even
+    // share, one to eight chunks (R-MAT scale 18 in natural order: 2.83 ms with runs of
+    // four chunks and an eighth of a share, 2.05 with these).
     __syncwarp();
     const uint64_t nwarps = (uint64_t)gridDim.x * kSWarps;
-    const uint32_t work = whole ? (e_hi + kRowRun - 1) / kRowRun : I_hi - I_lo;
-    const uint64_t share = work / (nwarps * 8);
+    const uint32_t work = whole ? (e_hi > kRowRun ? e_hi - kRowRun : 0u) : I_hi - I_lo;
+    const uint64_t share = work / (nwarps * 32);
     const uint32_t per = whole ? (uint32_t)(share < 1 ? 1 : (share > 8 ? 8 : share)) : 1u;
     unsigned long long kq = (unsigned long long)blockIdx.x * kSWarps + warp;
     while (kq * per < work) {
@@ -325,9 +385,9 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
         // chunks [e0, e1), row block by row block
         uint32_t e0, e1, u;
         if (whole) {
-            e0 = max((uint32_t)(kq * per), 1u) * kRowRun;
-            e1 = (uint32_t)min((unsigned long long)e_hi, (kq * per + per) * kRowRun);
-            u = e0 < e1 ? first_row[e0 / kRowRun] : 0u;
+            e0 = kRowRun + (uint32_t)(kq * per);
+            e1 = min(e_hi, e0 + per);
+            u = first_row[e0 / kRowRun];
         } else {
             u = 16u * (I_lo + (uint32_t)kq);
             e0 = off[u + (u >> 4)];
@@ -374,10 +434,10 @@ constexpr int kVariants = 8;
 StreamKernel stream_kernel(int v)
 {
     switch (v) {
-    case 0: return k_count_stream<256, 3, false, false>;
-    case 1: return k_count_stream<256, 3, true, false>;
-    case 2: return k_count_stream<512, 3, false, false>;
-    case 3: return k_count_stream<512, 3, true, false>;
+    case 0: return k_count_stream<256, 4, false, false>;
+    case 1: return k_count_stream<256, 4, true, false>;
+    case 2: return k_count_stream<512, 4, false, false>;
+    case 3: return k_count_stream<512, 4, true, false>;
     case 4: return k_count_stream<1024, 3, false, false>;
     case 5: return k_count_stream<1024, 3, true, false>;
     case 6: return k_count_stream<1024, 3, false, true>;
