@@ -302,7 +302,7 @@ static int batch_enqueue_tiles(btc_batch* b, const int32_t* d_src, const int32_t
     if (b->row_store)
         BTC_TRY(launch_rowstore(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                                 g->blocks.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
-                                meta + kMetaTiles, cap, meta, row_store_of(g), s));
+                                meta + kMetaTiles, cap, false, meta, row_store_of(g), s));
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 

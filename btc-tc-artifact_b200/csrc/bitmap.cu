@@ -441,7 +441,7 @@ k_fill_bm(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int6
 
 // indptr[R] = tile count; the overflow flag; and, when host_meta (a device alias of
 // mapped pinned memory) is given, the build's status slots copied to the host.
-// The same for a graph without cells (n = 0), where no k_bm_emit runs.
+// The same where no k_bm_emit runs: a graph without cells (n = 0), the grouped builder.
 __global__ void k_set_last(uint32_t* __restrict__ indptr, int32_t R,
                            unsigned long long* __restrict__ meta, uint32_t cap,
                            unsigned long long* __restrict__ host_meta)
@@ -580,6 +580,13 @@ int bitmap_emit_and_fill(const BuildGeom& g, const int32_t* src, const int32_t* 
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 
+int launch_finish_tiles(uint32_t* indptr, int32_t R, unsigned long long* meta, uint32_t cap,
+                        unsigned long long* host_meta, cudaStream_t s)
+{
+    bm::k_set_last<<<1, 1, 0, s>>>(indptr, R, meta, cap, host_meta);
+    return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+}
+
 int launch_popcount_sum(int tile_cols, const uint32_t* blocks, uint64_t num_tiles,
                         unsigned long long* out, cudaStream_t s)
 {
@@ -610,6 +617,45 @@ int launch_bitmap_count(const uint32_t* bitmap, uint64_t W, uint32_t* chunk_coun
 
 namespace btc200 {
 namespace bm {
+// (cell word, tile prefix) pairs from the tiles: the first tile of each word collects the
+// word.  Words without a tile keep the zeros the caller wrote.
+__global__ void k_cells(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
+                        const uint32_t* __restrict__ row_indices, uint32_t cap,
+                        const unsigned long long* __restrict__ d_tiles, uint64_t wpr,
+                        const GraphSeg* __restrict__ segs, const uint32_t* __restrict__ graph_rows, uint32_t G,
+                        uint2* __restrict__ cellpp)
+{
+    const unsigned long long T = d_tiles ? *d_tiles : cap;
+    if (T > cap) return;
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < T;
+         t += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t I = row_indices[t];
+        uint64_t row = (uint64_t)I * wpr;
+        uint32_t cb0 = 0;
+        if (segs) {
+            uint32_t lo = 0, hi = G;
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (graph_rows[mid] <= I) lo = mid;
+                else hi = mid;
+            }
+            const GraphSeg sg = segs[lo];
+            row = sg.bm_off + (uint64_t)(I - sg.row_off) * sg.wpr;
+            cb0 = sg.cb_lo;
+        }
+        const uint32_t w = (indices[t] - cb0) >> 5;
+        if (t > indptr[I] && ((indices[t - 1] - cb0) >> 5) == w) continue;
+        const uint64_t end = indptr[I + 1];
+        uint32_t bits = 0;
+        for (uint64_t x = t; x < end; ++x) {
+            const uint32_t k = indices[x] - cb0;
+            if ((k >> 5) != w) break;
+            bits |= 1u << (k & 31u);
+        }
+        cellpp[row + w] = make_uint2(bits, (uint32_t)t);
+    }
+}
+
 template <int WPR>
 __global__ void k_rowmask(const uint32_t* __restrict__ blocks, uint32_t cap,
                           const unsigned long long* __restrict__ d_tiles,
@@ -655,6 +701,17 @@ __global__ void k_rowmask(const uint32_t* __restrict__ blocks, uint32_t cap,
     }
 }
 }  // namespace bm
+
+int launch_cells(const uint32_t* indptr, const uint32_t* indices, const uint32_t* row_indices, uint32_t cap,
+                 const unsigned long long* d_tiles, uint64_t words, uint64_t wpr, const GraphSeg* segs,
+                 const uint32_t* graph_rows, uint32_t G, uint2* cellpp, cudaStream_t s)
+{
+    if (cudaMemsetAsync(cellpp, 0, sizeof(uint2) * words, s) != cudaSuccess) return BTC_E_CUDA;
+    if (cap)
+        bm::k_cells<<<grid_for(cap, 256), 256, 0, s>>>(indptr, indices, row_indices, cap, d_tiles, wpr, segs,
+                                                       graph_rows, G, cellpp);
+    return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+}
 
 int launch_rowmask(int tile_cols, const uint32_t* blocks, uint32_t cap,
                    const unsigned long long* d_tiles, const uint32_t* indptr, int32_t n_row_blocks,

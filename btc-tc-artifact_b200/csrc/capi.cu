@@ -68,6 +68,17 @@ using namespace btc200;
 // tensor core above 1024 bits (half full), 16x32 tiles above 64 (the reference's value).
 int default_tau(int tile_cols) { return tile_cols == 128 ? 1024 : 64; }
 
+// Degree-ordered edge lists from this length on are grouped by row block (group.cu) instead
+// of marked and filled edge by edge: the tiles of a power-law graph this large do not stay
+// in L2 between zeroing and filling (R-MAT scale 18, 4.2M draws: 0.71 ms against 0.73 a
+// step; scale 19: 1.29 / 1.43; scale 22: build 9.3 -> 5.6 ms; scale 17: the same).  In
+// natural order the bitmap stays: meshes and communities have small tile arrays (27-point
+// mesh 100^3 0.61 ms against 0.69 grouped, 8 communities on 60,000 vertices 4.0 / 4.5) and a
+// power-law hub's row block is one CTA's work here (scale 18: 2.1 / 2.4); uniform graphs of
+// more than 3M edges would gain (800,000 vertices, 6.4M edges: 1.9 / 1.35 ms), but nothing
+// at hand tells them from a power-law graph.
+static constexpr int64_t kGroupEdges = 1 << 22;
+
 static constexpr uint64_t kMaxEdges = (1ull << 32) - (uint64_t)kSortTile;
 
 int ensure_count_scratch(btc_bitbsr* g)
@@ -116,6 +127,8 @@ struct BuildPlan {
     int32_t n;
     uint32_t flags;
     bool use_bitmap;
+    bool use_group;  // the grouped builder (group.cu)
+    uint64_t col_blocks;
     bool degree;
     uint64_t bm_words;
     uint32_t cap;  // > 0: the post-count steps run against this tile capacity
@@ -148,11 +161,20 @@ int reserve_row_store(btc_bitbsr* g, uint64_t entries)
 
 // The row store after the tiles and row masks (T = *d_tiles bounded by cap, or cap itself).
 static int enqueue_row_store(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap,
-                             cudaStream_t s)
+                             bool by_degree, cudaStream_t s)
 {
     return launch_rowstore(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                            g->blocks.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(), d_tiles,
-                           cap, g->meta.as<unsigned long long>(), row_store_of(g), s);
+                           cap, by_degree, g->meta.as<unsigned long long>(), row_store_of(g), s);
+}
+
+void ensure_cells(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, uint64_t words, uint64_t wpr,
+                  const GraphSeg* segs, const uint32_t* graph_rows, uint32_t G, cudaStream_t s)
+{
+    if (g->cells || 4 * words > 32ull * (uint64_t)g->input_edges + (64ull << 20) || g->prefix.reserve(sizeof(uint2) * (words ? words : 1)) != BTC_OK)
+        return;
+    g->cells = launch_cells(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->row_indices.as<uint32_t>(),
+                            cap, d_tiles, words, wpr, segs, graph_rows, G, g->prefix.as<uint2>(), s) == BTC_OK;
 }
 
 void ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s)
@@ -171,6 +193,15 @@ void ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t
                                    g->rowmask.as<uint32_t>(), d_tiles, cap, g->row_tot.as<uint32_t>(),
                                    reinterpret_cast<uint32_t*>(total + 1), total, g->row_off.as<uint32_t>(),
                                    g->row_ent.as<uint2>(), g->row_ent.bytes / sizeof(uint2), s) == BTC_OK;
+}
+
+static int enqueue_group_write(btc_bitbsr* g, const BuildPlan& P, uint32_t cap, cudaStream_t s)
+{
+    return group_write(P.geom.tile_cols, P.col_blocks, (uint32_t)P.geom.n_row_blocks, nullptr, 0,
+                       g->keys0.as<uint32_t>(), g->tile_base.as<uint32_t>(), g->indptr.as<uint32_t>(),
+                       g->meta.as<unsigned long long>(), cap, g->indices.as<uint32_t>(),
+                       g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(), g->rowmask.as<uint32_t>(),
+                       g->num_tiles, s);
 }
 
 // Enqueues the build up to the tile count (bitmap path) or up to the tile segmentation
@@ -223,7 +254,23 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
             // the fill pass set the row masks; what is left is the row store, or only the
             // longest row-block list
             if (P.row_store)
-                BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, s));
+                BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s));
+            else
+                BTC_TRY(launch_rowmask(geom.tile_cols, g->blocks.as<uint32_t>(), P.cap,
+                                       meta + kMetaTiles, g->indptr.as<uint32_t>(), geom.n_row_blocks,
+                                       g->rowmask.as<uint32_t>(), meta + kMetaRowMax, s, false));
+        }
+    } else if (P.use_group) {
+        const uint32_t R = (uint32_t)geom.n_row_blocks;
+        uint32_t* scratch = g->tile_base.as<uint32_t>();
+        BTC_TRY(group_edges(P.d_src, P.d_dst, P.m, P.n, P.n, rank, nullptr, nullptr, 0, nullptr, geom.tile_cols,
+                            P.col_blocks, k0, k1, g->keys0.as<uint32_t>(), scratch, g->indptr.as<uint32_t>(),
+                            scratch + group_scratch_words(R), meta, s));
+        if (P.cap) {
+            BTC_TRY(launch_finish_tiles(g->indptr.as<uint32_t>(), geom.n_row_blocks, meta, P.cap, g->d_hmeta, s));
+            BTC_TRY(enqueue_group_write(g, P, P.cap, s));
+            if (P.row_store)
+                BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s));
             else
                 BTC_TRY(launch_rowmask(geom.tile_cols, g->blocks.as<uint32_t>(), P.cap,
                                        meta + kMetaTiles, g->indptr.as<uint32_t>(), geom.n_row_blocks,
@@ -258,7 +305,7 @@ static void build_key(const btc_bitbsr* g, const BuildPlan& P, BuildGraphKey* k)
     k->m = P.m;
     k->n = P.n;
     k->tile_cols = P.geom.tile_cols;
-    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u);
+    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.use_group ? 0x40000000u : 0u);
     k->cap = P.cap;
 }
 
@@ -364,18 +411,35 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     const uint64_t bm_bytes = 4 * P.bm_words;
     P.use_bitmap = !(flags & BTC_BUILD_RADIX) && bm_bytes <= (4ull << 30) &&
                    bm_bytes <= 32ull * (uint64_t)m + (64ull << 20);
-    g->used_bitmap = P.use_bitmap;
-    g->row_store = g->row_index = false;
+    // Large edge lists are grouped by row block instead of marked and filled edge by edge
+    // (see kGroupEdges), and so is what the bitmap does not take.
+    P.col_blocks = (uint64_t)geom.n_col_blocks;
     P.degree = (flags & BTC_ORIENT_DEGREE) && n > 0;
-    size_t key_cap = P.use_bitmap ? 0 : (size_t)m;
+    P.use_group = !(flags & BTC_BUILD_RADIX) && group_possible(n, P.col_blocks) &&
+                  (!P.use_bitmap || (P.degree && m >= kGroupEdges));
+    if (P.use_group) {
+        const uint64_t R = (uint64_t)geom.n_row_blocks;
+        if (g->keys0.reserve(sizeof(uint64_t) * (size_t)(m ? m : 1)) != BTC_OK ||
+            g->keys1.reserve(sizeof(uint64_t) * (size_t)(m ? m : 1)) != BTC_OK ||
+            g->tile_base.reserve(sizeof(uint32_t) * (group_scratch_words((uint32_t)R) + ri_scan_blocks((uint32_t)R) + 1)) != BTC_OK) {
+            if (!P.use_bitmap) return BTC_E_NOMEM;
+            P.use_group = false;  // the bitmap may still fit
+        }
+        if (P.use_group) P.use_bitmap = false;
+    }
+    g->cells = P.use_bitmap;
+    g->row_store = g->row_index = false;
+    size_t key_cap = P.use_bitmap || P.use_group ? 0 : (size_t)m;
     if (P.degree && (size_t)n > key_cap) key_cap = (size_t)n;
     if (key_cap) {
         BTC_TRY(g->keys0.reserve(sizeof(uint64_t) * key_cap));
         BTC_TRY(g->keys1.reserve(sizeof(uint64_t) * key_cap));
         BTC_TRY(g->sort_scratch.reserve(sizeof(uint32_t) * radix_scratch_words(key_cap)));
     }
-    const size_t chunk_slots = P.use_bitmap ? bitmap_chunks(P.bm_words) : sort_tiles((size_t)m);
-    BTC_TRY(g->tile_base.reserve(sizeof(uint32_t) * (chunk_slots + 1)));
+    if (!P.use_group) {
+        const size_t chunk_slots = P.use_bitmap ? bitmap_chunks(P.bm_words) : sort_tiles((size_t)m);
+        BTC_TRY(g->tile_base.reserve(sizeof(uint32_t) * (chunk_slots + 1)));
+    }
     if (P.degree) {
         BTC_TRY(g->deg.reserve(sizeof(uint32_t) * (size_t)n));
         BTC_TRY(g->rank.reserve(sizeof(int32_t) * (size_t)n));
@@ -393,7 +457,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     // device tile count, and waits once at the end (or not at all with BTC_BUILD_ASYNC);
     // a count above the capacity is redone below at the right size.  A first build
     // waits for the count in between.
-    if (P.use_bitmap && g->indices.ptr && g->row_indices.ptr && g->blocks.ptr && g->rowmask.ptr) {
+    if ((P.use_bitmap || P.use_group) && g->indices.ptr && g->row_indices.ptr && g->blocks.ptr && g->rowmask.ptr) {
         uint64_t c = g->indices.bytes / 4;
         c = std::min<uint64_t>(c, g->row_indices.bytes / 4);
         c = std::min<uint64_t>(c, g->blocks.bytes / (4 * TW));
@@ -454,6 +518,9 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
                                      g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(),
                                      g->blocks.as<uint32_t>(), meta, (uint32_t)tiles, nullptr, s,
                                      g->rowmask.as<uint32_t>(), P.row_store));
+    } else if (P.use_group) {
+        BTC_TRY(launch_finish_tiles(g->indptr.as<uint32_t>(), geom.n_row_blocks, meta, (uint32_t)tiles, nullptr, s));
+        BTC_TRY(enqueue_group_write(g, P, (uint32_t)tiles, s));
     } else {
         if (tiles)
             BTC_CUDA_TRY(cudaMemsetAsync(g->blocks.ptr, 0, sizeof(uint32_t) * TW * tiles, s));
@@ -463,12 +530,13 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         BTC_TRY(launch_indptr(g->row_indices.as<uint32_t>(), g->num_tiles, geom.n_row_blocks,
                               g->indptr.as<uint32_t>(), s));
     }
-    // the bitmap path's fill pass set the row masks; the radix path's are computed here
-    if (!P.use_bitmap || !P.row_store)
+    // the bitmap and grouped builders set the row masks; the radix path's are computed here
+    const bool have_masks = P.use_bitmap || P.use_group;
+    if (!have_masks || !P.row_store)
         BTC_TRY(launch_rowmask(tile_cols, g->blocks.as<uint32_t>(), g->num_tiles, nullptr,
                                g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
-                               meta + kMetaRowMax, s, !P.use_bitmap));
-    if (P.row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, s));
+                               meta + kMetaRowMax, s, !have_masks));
+    if (P.row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, P.degree, s));
     g->row_store = P.row_store;
     return BTC_OK;
 }
@@ -501,14 +569,17 @@ int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_o
                                    ((uint32_t)g->n + 63) / 64, scr, nullptr, 0, nullptr,
                                    g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), tile_begin,
                                    std::min(tile_end, cap), whole, true, build_meta, count_grid_size(g->tile_cols), s);
-    if (g->row_store && g->used_bitmap)
-        ensure_row_index(g, build_meta ? build_meta + kMetaTiles : nullptr, cap, s);
+    const uint64_t wpr = bitmap_words_per_row(make_geom(g->n, g->tile_cols));
+    if (g->row_store) {
+        const unsigned long long* d_tiles = build_meta ? build_meta + kMetaTiles : nullptr;
+        ensure_cells(g, d_tiles, cap, wpr * (uint64_t)g->n_row_blocks, wpr, nullptr, nullptr, 0, s);
+        if (g->cells) ensure_row_index(g, d_tiles, cap, s);
+    }
     return launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                         g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(),
                         cap, g->n_row_blocks, tau, scr, s,
                         nullptr, 0, nullptr, g->rowmask.as<uint32_t>(),
-                        g->used_bitmap ? g->prefix.as<uint2>() : nullptr,
-                        bitmap_words_per_row(make_geom(g->n, g->tile_cols)),
+                        g->cells ? g->prefix.as<uint2>() : nullptr, wpr,
                         g->meta.as<unsigned long long>() + kMetaRowMax, tile_begin, tile_end,
                         build_meta, g->num_tiles,
                         g->row_index ? g->row_off.as<uint32_t>() : nullptr,
@@ -826,7 +897,7 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
     BTC_TRY(w.first.reserve(sizeof(uint32_t) * (chunks / kRowRun + 1)));
     const RowStore rs{w.off.as<uint32_t>(), w.key.ptr, w.bits.as<uint4>(), w.first.as<uint32_t>()};
     BTC_TRY(launch_rowstore(tile_cols, b->indptr, b->indices, b->blocks, b->n_row_blocks,
-                            w.rowmask.as<uint32_t>(), nullptr, T, meta, rs, nullptr));
+                            w.rowmask.as<uint32_t>(), nullptr, T, false, meta, rs, nullptr));
     BTC_TRY(launch_count_stream(rs, meta + kMetaRowChunks, tile_cols, b->n_row_blocks,
                                 ((uint32_t)b->n_row_blocks * 16u + 63) / 64, scr, nullptr, 0, nullptr,
                                 b->row_indices, b->indices, 0, T, true, false, nullptr,

@@ -33,7 +33,7 @@ struct btc_bitbsr {
     btc200::DevBuf row_off, row_ent, row_tot, row_bsum;
     // build workspace
     btc200::DevBuf in_src, in_dst, keys0, keys1, sort_scratch, tile_base, meta, deg, rank, bitmap, prefix;
-    bool used_bitmap = false;
+    bool cells = false;      // prefix holds the (cell word, tile prefix) pairs of the last build
     bool row_store = false;  // the last build made the row store (its graph can be heavy)
     bool row_index = false;  // the row index of the last build's graph has been enqueued
     // count scratch
@@ -115,6 +115,10 @@ btc200::RowStore row_store_of(const btc_bitbsr* g);
 int reserve_row_store(btc_bitbsr* g, uint64_t entries);
 // The row index of the row-wise count kernel, enqueued on s if this build's is not yet there.
 // Without the memory for it the kernel walks whole row blocks instead.
+// The cell pairs, enqueued on s if the last build made none (`words` of them; segs and
+// graph_rows for a batch).  Without the memory for them the count goes tile-wise.
+void ensure_cells(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, uint64_t words, uint64_t wpr,
+                  const btc200::GraphSeg* segs, const uint32_t* graph_rows, uint32_t G, cudaStream_t s);
 void ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s);
 
 int default_tau(int tile_cols);

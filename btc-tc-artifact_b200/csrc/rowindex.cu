@@ -156,6 +156,16 @@ __global__ void k_ri_fill(const uint32_t* __restrict__ indptr, const uint32_t* _
 // off: 16 R + 1 words; ent: ent_cap entries.  d_tiles / cap as for launch_rowmask.
 uint32_t ri_scan_blocks(uint32_t R) { return (R + ri::kScanTile - 1) / ri::kScanTile; }
 
+// v[0, n) to its exclusive prefix, *total to the sum; bsum: ri_scan_blocks(n) words.
+int launch_scan_u32(uint32_t* v, uint32_t n, uint32_t* bsum, unsigned long long* total, cudaStream_t s)
+{
+    const uint32_t nb = ri_scan_blocks(n);
+    if (nb) ri::k_scan_reduce<<<nb, ri::kThreads, 0, s>>>(v, n, bsum);
+    BTC_TRY(launch_tile_scan(bsum, nb, total, s));
+    if (nb) ri::k_scan_apply<<<nb, ri::kThreads, 0, s>>>(v, n, bsum);
+    return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+}
+
 int launch_rowindex(const uint32_t* indptr, const uint32_t* indices, int32_t n_row_blocks,
                     const uint32_t* rowmask, const unsigned long long* d_tiles, uint32_t cap,
                     uint32_t* tot, uint32_t* bsum, unsigned long long* total, uint32_t* off,

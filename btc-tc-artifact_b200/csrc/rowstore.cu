@@ -91,7 +91,7 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
           const uint32_t* __restrict__ blocks, uint32_t R, const uint32_t* __restrict__ rowmask,
           const unsigned long long* __restrict__ d_tiles, uint32_t cap,
           unsigned long long* __restrict__ meta, uint32_t* __restrict__ off, void* __restrict__ key_words,
-          uint4* __restrict__ bit_words, uint32_t* __restrict__ first_row)
+          uint4* __restrict__ bit_words, uint32_t* __restrict__ first_row, uint32_t len_lo, uint32_t len_hi)
 {
     constexpr int TW = 16 * (C / 32);
     constexpr int kPerTile = C == 128 ? 32 : 16;
@@ -127,9 +127,7 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
         bits[threadIdx.x] = make_uint2(0u, 0u);
     }
     uint32_t longest = 0;
-    for (uint64_t I = (uint64_t)blockIdx.x * kTeams + team; I < R; I += (uint64_t)gridDim.x * kTeams) {
-        const uint32_t a = indptr[I], b = indptr[I + 1];
-        longest = max(longest, b - a);
+    auto row_block = [&](uint64_t I, uint32_t a, uint32_t b) {
         // ---- the rows' entries (lane r < 16: row r's) -----------------------------------
         uint32_t K = 0, m0 = 0, m1 = 0;
         bool pair = false;
@@ -274,6 +272,12 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
             }
         }
         team_sync<kTeam>(team);
+    };
+    // Row blocks of more than len_lo tiles (0: all) and at most len_hi.
+    for (uint64_t I = (uint64_t)blockIdx.x * kTeams + team; I < R; I += (uint64_t)gridDim.x * kTeams) {
+        const uint32_t a = indptr[I], b = indptr[I + 1];
+        longest = max(longest, b - a);
+        if (b - a <= len_hi && (len_lo == 0 || b - a > len_lo)) row_block(I, a, b);
     }
     if (w == 0 && lane == 0 && longest) atomicMax(&meta[kMetaRowMax], (unsigned long long)longest);
 }
@@ -299,41 +303,43 @@ int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* o
 
 int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indices, const uint32_t* blocks,
                     int32_t n_row_blocks, const uint32_t* rowmask, const unsigned long long* d_tiles,
-                    uint32_t cap, unsigned long long* meta, const RowStore& out,
+                    uint32_t cap, bool by_degree, unsigned long long* meta, const RowStore& out,
                     cudaStream_t s)
 {
     const uint32_t R = n_row_blocks > 0 ? (uint32_t)n_row_blocks : 0u;
     if (R == 0) return BTC_OK;
-    const bool wide = row_store_wide(n_row_blocks);
     // Few row blocks leave the GPU idle, so eight warps share one (Erdos-Renyi 16384 / 16: 1,024
     // row blocks, 26 us with one warp, 19 with two, 13 with four, 9.7 with eight; R-MAT scale
     // 16: 107, 57, 40 us); from four row blocks per resident warp on, a team's barriers cost
     // more than they save (R-MAT scale 22: 0.98 ms with one warp, 1.10 with two, 1.40 with
     // eight; 256 mixed graphs: 0.31, 0.41 ms, 0.54 with four).
-    const int team = R <= 32u * (uint32_t)device_sm_count() ? 8 : 1;
-    const int grid = (int)std::min<uint64_t>(((uint64_t)R * team + rs::kWarps - 1) / rs::kWarps,
-                                             (uint64_t)device_sm_count() * 16);
-#define BTC_FILL(CC, WW, TT)                                                                                 \
-    rs::k_rs_fill<CC, WW, TT><<<grid, rs::kThreads, 0, s>>>(indptr, indices, blocks, R, rowmask, d_tiles, cap, \
-                                                            meta, out.off, out.key, out.bits, out.first_row)
-#define BTC_FILL_TEAM(CC, WW)           \
-    if (team == 8) BTC_FILL(CC, WW, 8); \
-    else BTC_FILL(CC, WW, 1)
-    if (tile_cols == 128) {
-        if (wide) {
-            BTC_FILL_TEAM(128, true);
-        } else {
-            BTC_FILL_TEAM(128, false);
-        }
+    // In natural order the long row blocks among many (a hub's: 8,192 tiles at R-MAT scale 18,
+    // 256 rounds of one warp) get a team in a second launch: 0.51 -> 0.22 ms there.  Degree
+    // order has none that long, and the second launch costs more than it gives (scale 22:
+    // 0.99 ms without it, 1.15 with).
+    constexpr uint32_t kLong = 512, kAny = 0xffffffffu;
+    const bool few = R <= 32u * (uint32_t)device_sm_count();
+    const uint32_t sms = (uint32_t)device_sm_count();
+    auto launch = [&](auto kernel, uint32_t per_cta, uint32_t len_lo, uint32_t len_hi) {
+        const uint32_t grid = std::min((R + per_cta - 1) / per_cta, sms * 16);
+        kernel<<<grid, rs::kThreads, 0, s>>>(indptr, indices, blocks, R, rowmask, d_tiles, cap, meta, out.off,
+                                             out.key, out.bits, out.first_row, len_lo, len_hi);
+    };
+    auto fill = [&](auto one, auto team) {
+        if (!few) launch(one, rs::kWarps, 0, by_degree ? kAny : kLong);
+        if (few || !by_degree) launch(team, 1, few ? 0 : kLong, kAny);
+    };
+    if (row_store_wide(n_row_blocks)) {
+        if (tile_cols == 128)
+            fill(rs::k_rs_fill<128, true, 1>, rs::k_rs_fill<128, true, 8>);
+        else
+            fill(rs::k_rs_fill<32, true, 1>, rs::k_rs_fill<32, true, 8>);
     } else {
-        if (wide) {
-            BTC_FILL_TEAM(32, true);
-        } else {
-            BTC_FILL_TEAM(32, false);
-        }
+        if (tile_cols == 128)
+            fill(rs::k_rs_fill<128, false, 1>, rs::k_rs_fill<128, false, 8>);
+        else
+            fill(rs::k_rs_fill<32, false, 1>, rs::k_rs_fill<32, false, 8>);
     }
-#undef BTC_FILL_TEAM
-#undef BTC_FILL
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 
