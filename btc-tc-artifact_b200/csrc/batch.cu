@@ -201,7 +201,7 @@ using namespace btc200;
 struct btc_batch {
     btc_bitbsr g;  // the union graph's Bit-BSR, workspace and count scratch
     int32_t num_graphs = 0;
-    DevBuf segs, e_off, bm_off, row_off, counts;
+    DevBuf segs, e_off, nv, bm_off, row_off, counts;
     std::vector<GraphSeg> h_segs;
     std::vector<int64_t> h_eoff;
     std::vector<uint64_t> h_bmoff;
@@ -218,6 +218,7 @@ struct btc_batch {
         g.release_all();
         segs.release();
         e_off.release();
+        nv.release();
         bm_off.release();
         row_off.release();
         counts.release();
@@ -375,19 +376,15 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
         // locality measured against its own graph's size
         double L = 0.0;
         if (flags & BTC_INPUT_ON_HOST) {
-            BTC_TRY(policy_locality(src, dst, m, 0, true, edge_offsets, num_vertices, (uint32_t)G, s, &L));
+            BTC_TRY(policy_locality(src, dst, m, 0, true, edge_offsets, num_vertices, (uint32_t)G, s, g->policy, &L));
         } else if (m > 0) {
-            DevBuf tmp;
             const size_t eb = sizeof(int64_t) * ((size_t)G + 1), nb = sizeof(int32_t) * (size_t)G;
-            int st = tmp.reserve(eb + nb);
-            if (st == BTC_OK && (cudaMemcpyAsync(tmp.ptr, edge_offsets, eb, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-                                 cudaMemcpyAsync(tmp.as<char>() + eb, num_vertices, nb, cudaMemcpyHostToDevice, s) != cudaSuccess))
-                st = BTC_E_CUDA;
-            if (st == BTC_OK)
-                st = policy_locality(src, dst, m, 0, false, tmp.as<int64_t>(),
-                                     reinterpret_cast<const int32_t*>(tmp.as<char>() + eb), (uint32_t)G, s, &L);
-            tmp.release();
-            BTC_TRY(st);
+            BTC_TRY(b->e_off.reserve(eb));
+            BTC_TRY(b->nv.reserve(nb));
+            BTC_CUDA_TRY(cudaMemcpyAsync(b->e_off.ptr, edge_offsets, eb, cudaMemcpyHostToDevice, s));
+            BTC_CUDA_TRY(cudaMemcpyAsync(b->nv.ptr, num_vertices, nb, cudaMemcpyHostToDevice, s));
+            BTC_TRY(policy_locality(src, dst, m, 0, false, b->e_off.as<int64_t>(), b->nv.as<int32_t>(), (uint32_t)G,
+                                    s, g->policy, &L));
         }
         BTC_TRY(btc_tile_policy_from_features(m, (int32_t)(n_sum > 0x7fffffff ? 0x7fffffff : n_sum), 0, L,
                                               &tile_cols, nullptr));
@@ -501,7 +498,7 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
 namespace btc200 {
 size_t batch_device_bytes(const btc_batch* b)
 {
-    return b->g.device_bytes() + b->segs.bytes + b->e_off.bytes + b->bm_off.bytes +
+    return b->g.device_bytes() + b->segs.bytes + b->e_off.bytes + b->nv.bytes + b->bm_off.bytes +
            b->row_off.bytes + b->counts.bytes;
 }
 }  // namespace btc200
@@ -514,7 +511,7 @@ btc_batch* batch_new_pooled(cudaMemPool_t pool, cudaStream_t s)
     btc_batch* b = new (std::nothrow) btc_batch();
     if (!b) return nullptr;
     b->g.set_pool(pool, s);
-    for (DevBuf* d : {&b->segs, &b->e_off, &b->bm_off, &b->row_off, &b->counts}) {
+    for (DevBuf* d : {&b->segs, &b->e_off, &b->nv, &b->bm_off, &b->row_off, &b->counts}) {
         d->pool = pool;
         d->stream = s;
     }

@@ -366,8 +366,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         else if ((flags & BTC_BUILD_ASYNC) && (g->tile_cols == 32 || g->tile_cols == 128))
             tile_cols = g->tile_cols;
         else
-            BTC_TRY(btc_select_tile_policy(src, dst, m, n, flags & BTC_INPUT_ON_HOST, s, &tile_cols,
-                                           nullptr));
+            BTC_TRY(policy_select(src, dst, m, n, flags & BTC_INPUT_ON_HOST, s, g->policy, &tile_cols, nullptr));
     }
     if (tile_cols != 32 && tile_cols != 128) return BTC_E_INVAL;
     BTC_CUDA_TRY(cudaGetDevice(&g->device));

@@ -332,8 +332,28 @@ int launch_cells(const uint32_t* indptr, const uint32_t* indices, const uint32_t
 // Id locality of an edge list for the tile policy (policy.cu): sampled share of edges
 // with |u - v| < 128 over the share uniform ids would give.  e_off / nv (nullable): the
 // batch layout, each edge measured against its own graph's vertex count.
+struct PolicyWords {
+    DevBuf dev;                          // two sums and a ticket
+    unsigned long long* host = nullptr;  // a host slot
+    bool dirty = false;                  // a call did not come to its end
+    void release()
+    {
+        if (host && cudaDeviceSynchronize() != cudaSuccess) {
+            cudaGetLastError();
+            host = nullptr;  // (something may still write to it)
+            dev.release();
+        }
+        dev.release_idle();
+        host_slot_free(host);
+        host = nullptr;
+    }
+};
 int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, bool on_host,
-                    const int64_t* e_off, const int32_t* nv, uint32_t G, cudaStream_t s, double* L);
+                    const int64_t* e_off, const int32_t* nv, uint32_t G, cudaStream_t s, PolicyWords& w,
+                    double* L);
+// btc_select_tile_policy with the caller's words.
+int policy_select(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, uint32_t flags, cudaStream_t s,
+                  PolicyWords& w, int* tile_cols, int* tau);
 
 // Device metadata slots of a build (uint64 each): valid keys, out-of-range flag, tile
 // count, unique edges, sort length, longest row-block list, tile-capacity overflow flag,

@@ -6,6 +6,9 @@
 // device at the next wait.  Allocations are made on a stream of the pool's own and are
 // complete when dev_alloc returns, so a caller may use the memory on any stream; freed
 // memory is idle (dev_free's callers have waited), so it may be handed to any other.
+// Allocations of kDirectBytes and more come from cudaMalloc: the pool would not keep them
+// and maps them more slowly (a new R-MAT scale 22 handle of 9 GB: 69 ms to build and count
+// with all of it pooled, 19.4 like this; scale 20, 1.9 GB: 9.6 / 3.7 ms).
 #include "common.cuh"
 
 #include <cuda.h>
@@ -45,6 +48,7 @@ unsigned long long current_context_id()
 namespace {
 
 constexpr uint64_t kKeepBytes = 1ull << 30;
+constexpr size_t kDirectBytes = 256ull << 20;
 
 struct DevicePool {
     cudaMemPool_t pool = nullptr;
@@ -150,7 +154,7 @@ cudaError_t dev_alloc(void** ptr, size_t bytes)
 {
     cudaMemPool_t pool;
     cudaStream_t stream;
-    if (!pool_for_current_device(&pool, &stream)) return cudaMalloc(ptr, bytes);
+    if (bytes >= kDirectBytes || !pool_for_current_device(&pool, &stream)) return cudaMalloc(ptr, bytes);
     cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
     if (e == cudaErrorMemoryAllocation) {
         // give the kept memory back and try once more

@@ -38,6 +38,7 @@ struct btc_bitbsr {
     bool row_index = false;  // the row index of the last build's graph has been enqueued
     // count scratch
     btc200::DevBuf partials, done;
+    btc200::PolicyWords policy;
     unsigned long long* h_meta = nullptr;  // pinned and mapped, 8 slots
     unsigned long long* d_hmeta = nullptr; // the device's address of h_meta
     bool edges_known = false;
@@ -77,6 +78,8 @@ struct btc_bitbsr {
             b.pool = pool;
             b.stream = s;
         });
+        policy.dev.pool = pool;
+        policy.dev.stream = s;
     }
     void release_all()
     {
@@ -88,6 +91,7 @@ struct btc_bitbsr {
             for_each_buf([](btc200::DevBuf& b) { b.release(); });
             h_meta = nullptr;  // (given up: something may still write to it)
         }
+        policy.release();
         for_each_buf([](btc200::DevBuf& b) { b.release_idle(); });
         btc200::host_slot_free(h_meta);
         h_meta = nullptr;

@@ -32,10 +32,12 @@ constexpr int32_t kNear = 128;  // |u - v| below this counts as local
 // Sample i reads edge i * step.  Adds the number of local edges and their expectation
 // under uniform ids (per sampled edge: the chance that two uniform ids in [0, n) lie
 // closer than kNear, about (2 kNear - 1) / n), scaled by 2^20 to stay integer.  With
-// e_off / nv (a batch), an edge's n is its own graph's.
+// e_off / nv (a batch), an edge's n is its own graph's.  out: two sums and a ticket, zero at
+// the start; the last CTA hands the sums to the host (mapped memory) and zeroes them.
 __global__ void k_locality(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m,
                            int32_t n, const int64_t* __restrict__ e_off, const int32_t* __restrict__ nv,
-                           uint32_t G, int64_t step, unsigned long long* __restrict__ out)
+                           uint32_t G, int64_t step, unsigned long long* __restrict__ out,
+                           volatile unsigned long long* host)
 {
     unsigned long long local = 0, expect = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < kSamples;
@@ -65,6 +67,14 @@ __global__ void k_locality(const int32_t* __restrict__ src, const int32_t* __res
     if ((threadIdx.x & 31) == 0) {
         atomicAdd(&out[0], local);
         atomicAdd(&out[1], expect);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&out[2], 1ull) == gridDim.x - 1) {
+        host[0] = atomicExch(&out[0], 0ull);
+        host[1] = atomicExch(&out[1], 0ull);
+        out[2] = 0ull;
+        __threadfence_system();
     }
 }
 
@@ -90,14 +100,18 @@ double locality_host(const int32_t* src, const int32_t* dst, int64_t m, int32_t 
     return expect > 0.0 ? local / expect : 0.0;
 }
 
+// Average degree 2m/n of at least 512.
+bool dense(int64_t m, int32_t n) { return n > 0 && 2.0 * (double)m / (double)n >= 512.0; }
+
 }  // namespace pol
 
 // Id locality of an edge list (see above): host arrays are sampled on the host, device
-// arrays by one small kernel and one wait on `s` (16 bytes of scratch, allocated here).
-// e_off / nv (optional, num_graphs + 1 and num_graphs entries, host or device like
-// src/dst): batch layout.
+// arrays by one small kernel and one wait on `s`.  e_off / nv (optional, num_graphs + 1 and
+// num_graphs entries, host or device like src/dst): batch layout.  w: the caller's words (a
+// handle keeps them: an allocation, a memset and a copy back cost a small graph's step 15 us).
 int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, bool on_host,
-                    const int64_t* e_off, const int32_t* nv, uint32_t G, cudaStream_t s, double* L)
+                    const int64_t* e_off, const int32_t* nv, uint32_t G, cudaStream_t s, PolicyWords& w,
+                    double* L)
 {
     *L = 0.0;
     if (m <= 0) return BTC_OK;
@@ -105,22 +119,37 @@ int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n
         *L = pol::locality_host(src, dst, m, n, e_off, nv, G);
         return BTC_OK;
     }
-    struct Scratch {
-        DevBuf b;
-        ~Scratch() { b.release(); }
-    } sc;
-    BTC_TRY(sc.b.reserve(2 * sizeof(unsigned long long)));
-    unsigned long long* d = sc.b.as<unsigned long long>();
-    BTC_CUDA_TRY(cudaMemsetAsync(d, 0, 2 * sizeof(unsigned long long), s));
+    if (!w.host && !(w.host = host_slot_alloc())) return BTC_E_NOMEM;
+    void* d_host = nullptr;
+    BTC_CUDA_TRY(cudaHostGetDevicePointer(&d_host, w.host, 0));
+    const bool fresh = w.dev.ptr == nullptr;
+    BTC_TRY(w.dev.reserve(3 * sizeof(unsigned long long)));
+    // (a call that failed on its way may have left something in them)
+    if (fresh || w.dirty) BTC_CUDA_TRY(cudaMemsetAsync(w.dev.ptr, 0, 3 * sizeof(unsigned long long), s));
+    w.dirty = true;
     const int64_t step = m > (int64_t)pol::kSamples ? m / (int64_t)pol::kSamples : 1;
-    pol::k_locality<<<pol::kGrid, pol::kThreads, 0, s>>>(src, dst, m, n, e_off, nv, G, step, d);
+    const int64_t samples = m < (int64_t)pol::kSamples ? m : (int64_t)pol::kSamples;
+    const int grid = (int)((samples + 4 * pol::kThreads - 1) / (4 * pol::kThreads));
+    pol::k_locality<<<grid, pol::kThreads, 0, s>>>(src, dst, m, n, e_off, nv, G, step,
+                                                   w.dev.as<unsigned long long>(),
+                                                   static_cast<unsigned long long*>(d_host));
     BTC_CUDA_TRY(cudaGetLastError());
-    unsigned long long h[2] = {0, 0};
-    BTC_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s));
     BTC_CUDA_TRY(cudaStreamSynchronize(s));
-    sc.b.release_idle();
+    w.dirty = false;
+    const volatile unsigned long long* h = w.host;
     *L = h[1] ? (double)h[0] / (double)h[1] : 0.0;
     return BTC_OK;
+}
+
+int policy_select(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, uint32_t flags, cudaStream_t s,
+                  PolicyWords& w, int* tile_cols, int* tau)
+{
+    if (n < 0 || m < 0 || !tile_cols || (m > 0 && (!src || !dst))) return BTC_E_INVAL;
+    double L = 0.0;
+    // (the locality decides only where neither the degree nor the ordering does)
+    if (!(flags & BTC_ORIENT_DEGREE) && !pol::dense(m, n))
+        BTC_TRY(policy_locality(src, dst, m, n, (flags & BTC_INPUT_ON_HOST) != 0, nullptr, nullptr, 0, s, w, &L));
+    return btc_tile_policy_from_features(m, n, flags, L, tile_cols, tau);
 }
 
 }  // namespace btc200
@@ -133,9 +162,8 @@ int btc_tile_policy_from_features(int64_t m, int32_t n, uint32_t flags, double l
                                   int* tile_cols, int* tau)
 {
     if (m < 0 || n < 0 || !tile_cols) return BTC_E_INVAL;
-    const double d = n > 0 ? 2.0 * (double)m / (double)n : 0.0;
     int C;
-    if (d >= 512.0) C = 32;
+    if (pol::dense(m, n)) C = 32;
     else if (flags & BTC_ORIENT_DEGREE) C = 128;
     else C = locality >= 16.0 ? 128 : 32;
     *tile_cols = C;
@@ -146,12 +174,10 @@ int btc_tile_policy_from_features(int64_t m, int32_t n, uint32_t flags, double l
 int btc_select_tile_policy(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
                            uint32_t flags, btc_stream_t stream, int* tile_cols, int* tau)
 {
-    if (n < 0 || m < 0 || !tile_cols || (m > 0 && (!src || !dst))) return BTC_E_INVAL;
-    double L = 0.0;
-    if (!(flags & BTC_ORIENT_DEGREE))
-        BTC_TRY(policy_locality(src, dst, m, n, (flags & BTC_INPUT_ON_HOST) != 0, nullptr, nullptr, 0,
-                                stream, &L));
-    return btc_tile_policy_from_features(m, n, flags, L, tile_cols, tau);
+    PolicyWords w;
+    const int st = policy_select(src, dst, m, n, flags, stream, w, tile_cols, tau);
+    w.release();
+    return st;
 }
 
 }  // extern "C"
