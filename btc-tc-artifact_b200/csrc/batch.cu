@@ -25,7 +25,9 @@ namespace btc200 {
 namespace bt {
 
 constexpr int kThreads = 256;
-constexpr int kWordsPerThread = 16;
+// Four words per thread: a chunk of a dense graph (communities: 32 tiles a word) is one CTA's
+// to name and to zero (256 mixed graphs: k_emit_b 245 us with sixteen, 200 with four).
+constexpr int kWordsPerThread = 4;
 constexpr int kChunk = kThreads * kWordsPerThread;
 
 // last g in [0, G) with off[g] <= x (off[0] == 0; equal offsets are empty graphs)
@@ -41,12 +43,31 @@ __device__ __forceinline__ uint32_t last_le(const T* __restrict__ off, uint32_t 
     return lo;
 }
 
-// Orients edge i of its graph to local (r, c), r > c.  false: self-loop or bad id.
-__device__ __forceinline__ bool local_edge(const int32_t* __restrict__ src,
-                                           const int32_t* __restrict__ dst, int64_t i,
-                                           const GraphSeg& s, uint32_t& r, uint32_t& c, bool& bad)
+// Edges in flight per thread of the edge passes.  A CTA takes runs of kEdges * kThreads
+// consecutive edges and a thread every kThreads-th of them, so that a thread's edges nearly
+// always share a graph, whose search and segment are then kept (a search per edge, eight
+// dependent loads, made the marking of 256 mixed graphs, 35M edges, take 423 us and the filling 453; 253 and
+// 406 like this, bound by the atomics: four edges in flight or more CTAs changed nothing).
+constexpr int kEdges = 8;
+
+struct EdgeGraph {
+    int64_t lo = 0, hi = 0;  // the edges of `s`
+    GraphSeg s{};
+    __device__ __forceinline__ void find(const GraphSeg* __restrict__ segs, const int64_t* __restrict__ e_off,
+                                         uint32_t G, int64_t i)
+    {
+        if (i >= lo && i < hi) return;
+        const uint32_t g = last_le<int64_t>(e_off, G, i);
+        lo = e_off[g];
+        hi = e_off[g + 1];
+        s = segs[g];
+    }
+};
+
+// Orients an edge of its graph to local (r, c), r > c.  false: self-loop or bad id.
+__device__ __forceinline__ bool local_edge(int32_t u, int32_t v, const GraphSeg& s, uint32_t& r, uint32_t& c,
+                                           bool& bad)
 {
-    const int32_t u = src[i], v = dst[i];
     bad = (u < 0) | (v < 0) | (u >= s.n) | (v >= s.n);
     if (bad || u == v) return false;
     r = (uint32_t)max(u, v);
@@ -70,16 +91,39 @@ k_mark_b(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64
          uint32_t* bitmap, unsigned long long* __restrict__ bad_count)
 {
     uint32_t nbad = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const GraphSeg s = segs[last_le<int64_t>(e_off, G, i)];
-        uint32_t r, c, bit;
-        bool bad;
-        if (local_edge(src, dst, i, s, r, c, bad)) {
-            const uint64_t w = cell_word<LOG2C>(s, r, c, bit);
-            if (!(bitmap[w] & bit)) atomicOr(&bitmap[w], bit);
+    EdgeGraph g;
+    for (int64_t i0 = (int64_t)blockIdx.x * (kEdges * kThreads) + threadIdx.x; i0 < m;
+         i0 += (int64_t)gridDim.x * (kEdges * kThreads)) {
+        int32_t u[kEdges], v[kEdges];
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k) {
+            const int64_t i = i0 + k * kThreads;
+            u[k] = i < m ? src[i] : 0;
+            v[k] = i < m ? dst[i] : 0;
         }
-        nbad += bad;
+        uint64_t w[kEdges];
+        uint32_t bit[kEdges];
+        bool ok[kEdges];
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k) {
+            const int64_t i = i0 + k * kThreads;
+            ok[k] = false;
+            w[k] = 0;
+            bit[k] = 0;
+            if (i >= m) continue;
+            g.find(segs, e_off, G, i);
+            uint32_t r, c;
+            bool bad;
+            ok[k] = local_edge(u[k], v[k], g.s, r, c, bad);
+            nbad += bad;
+            if (ok[k]) w[k] = cell_word<LOG2C>(g.s, r, c, bit[k]);
+        }
+        uint32_t cur[kEdges];
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k) cur[k] = ok[k] ? bitmap[w[k]] : 0xffffffffu;
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k)
+            if (!(cur[k] & bit[k]) && ok[k]) atomicOr(&bitmap[w[k]], bit[k]);
     }
     nbad = __reduce_add_sync(kFull, nbad);
     if ((threadIdx.x & 31) == 0 && nbad) atomicAdd(bad_count, (unsigned long long)nbad);
@@ -164,19 +208,44 @@ k_fill_b(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64
 {
     if (*tiles > cap) return;  // nothing was emitted
     constexpr int C = 1 << LOG2C;
-    constexpr int WPR = C / 32;
-    constexpr int TW = 16 * WPR;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const GraphSeg s = segs[last_le<int64_t>(e_off, G, i)];
-        uint32_t r, c, bit;
-        bool bad;
-        if (!local_edge(src, dst, i, s, r, c, bad)) continue;
-        const uint64_t w = cell_word<LOG2C>(s, r, c, bit);
-        const uint2 cp = cellpp[w];
-        const uint32_t t = cp.y + __popc(cp.x & (bit - 1u));
-        const uint32_t cl = (s.vbase + c) & (C - 1);
-        atomicOr(&blocks[(size_t)t * TW + (r & 15u) * WPR + (cl >> 5)], 1u << (cl & 31u));
+    constexpr int TW = 16 * (C / 32);
+    EdgeGraph g;
+    for (int64_t i0 = (int64_t)blockIdx.x * (kEdges * kThreads) + threadIdx.x; i0 < m;
+         i0 += (int64_t)gridDim.x * (kEdges * kThreads)) {
+        int32_t u[kEdges], v[kEdges];
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k) {
+            const int64_t i = i0 + k * kThreads;
+            u[k] = i < m ? src[i] : 0;
+            v[k] = i < m ? dst[i] : 0;
+        }
+        uint32_t place[kEdges], bit[kEdges];  // row and column in the tile, cell bit
+        uint2 cp[kEdges];
+        bool ok[kEdges];
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k) {
+            const int64_t i = i0 + k * kThreads;
+            ok[k] = false;
+            bit[k] = place[k] = 0;
+            uint64_t w = 0;
+            if (i < m) {
+                g.find(segs, e_off, G, i);
+                uint32_t r, c;
+                bool bad;
+                ok[k] = local_edge(u[k], v[k], g.s, r, c, bad);
+                if (ok[k]) {
+                    w = cell_word<LOG2C>(g.s, r, c, bit[k]);
+                    place[k] = ((r & 15u) << LOG2C) | ((g.s.vbase + c) & (C - 1));
+                }
+            }
+            cp[k] = ok[k] ? cellpp[w] : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (int k = 0; k < kEdges; ++k)
+            if (ok[k]) {
+                const uint32_t tile = cp[k].y + __popc(cp[k].x & (bit[k] - 1u));
+                atomicOr(&blocks[(size_t)tile * TW + (place[k] >> 5)], 1u << (place[k] & 31u));
+            }
     }
 }
 
@@ -286,15 +355,15 @@ static int batch_enqueue_tiles(btc_batch* b, const int32_t* d_src, const int32_t
             g->blocks.as<uint4>(), vec4);
     bt::k_set_last_b<<<1, 1, 0, s>>>(g->indptr.as<uint32_t>(), rows, meta, cap);
     if (m > 0 && words) {
-        const int egrid = grid_for((m + 3) / 4, bt::kThreads);
+        const int egrid = grid_for((m + bt::kEdges - 1) / bt::kEdges, bt::kThreads);
         if (g->tile_cols == 128)
-            bt::k_fill_b<7><<<egrid, bt::kThreads, 0, s>>>(d_src, d_dst, m, dsegs, deoff, G,
-                                                           g->prefix.as<uint2>(), g->blocks.as<uint32_t>(),
-                                                           meta + kMetaTiles, cap);
+            bt::k_fill_b<7><<<egrid, bt::kThreads, 0, s>>>(
+                d_src, d_dst, m, dsegs, deoff, G, g->prefix.as<uint2>(), g->blocks.as<uint32_t>(), meta + kMetaTiles,
+                cap);
         else
-            bt::k_fill_b<5><<<egrid, bt::kThreads, 0, s>>>(d_src, d_dst, m, dsegs, deoff, G,
-                                                           g->prefix.as<uint2>(), g->blocks.as<uint32_t>(),
-                                                           meta + kMetaTiles, cap);
+            bt::k_fill_b<5><<<egrid, bt::kThreads, 0, s>>>(
+                d_src, d_dst, m, dsegs, deoff, G, g->prefix.as<uint2>(), g->blocks.as<uint32_t>(), meta + kMetaTiles,
+                cap);
     }
     BTC_TRY(launch_rowmask(g->tile_cols, g->blocks.as<uint32_t>(), cap, meta + kMetaTiles,
                            g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
@@ -319,7 +388,7 @@ static int batch_enqueue_mark(btc_batch* b, const int32_t* d_src, const int32_t*
     if (!words) return BTC_OK;
     BTC_CUDA_TRY(cudaMemsetAsync(g->bitmap.ptr, 0, sizeof(uint32_t) * words, s));
     if (m > 0) {
-        const int egrid = grid_for((m + 3) / 4, bt::kThreads);
+        const int egrid = grid_for((m + bt::kEdges - 1) / bt::kEdges, bt::kThreads);
         if (g->tile_cols == 128)
             bt::k_mark_b<7><<<egrid, bt::kThreads, 0, s>>>(d_src, d_dst, m, b->segs.as<GraphSeg>(),
                                                            b->e_off.as<int64_t>(), (uint32_t)b->num_graphs,

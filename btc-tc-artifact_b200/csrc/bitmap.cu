@@ -27,8 +27,6 @@ namespace btc200 {
 namespace bm {
 
 constexpr int kThreads = 256;
-constexpr int kWordsPerThread = 16;
-constexpr int kChunk = kThreads * kWordsPerThread;  // 4096 words per CTA
 
 __device__ __forceinline__ bool orient(int32_t u, int32_t v, int32_t n, const int32_t* rank,
                                        uint32_t& r, uint32_t& c, bool& bad)
@@ -190,16 +188,17 @@ __device__ __forceinline__ uint32_t load_lower_words(const uint32_t* __restrict_
     return need;
 }
 
+template <int WPT>
 __global__ void __launch_bounds__(kThreads)
 k_bm_count(const uint32_t* __restrict__ bitmap, uint64_t W, uint32_t* __restrict__ chunk_count)
 {
     __shared__ uint32_t s_warp[kThreads / kWarp];
-    const uint64_t w0 = (uint64_t)blockIdx.x * kChunk + (uint64_t)threadIdx.x * kWordsPerThread;
-    uint32_t x[kWordsPerThread];
-    load_words<kWordsPerThread>(bitmap, w0, W, x);
+    const uint64_t w0 = (uint64_t)blockIdx.x * (kThreads * WPT) + (uint64_t)threadIdx.x * WPT;
+    uint32_t x[WPT];
+    load_words<WPT>(bitmap, w0, W, x);
     uint32_t s = 0;
 #pragma unroll
-    for (int k = 0; k < kWordsPerThread; ++k) s += __popc(x[k]);
+    for (int k = 0; k < WPT; ++k) s += __popc(x[k]);
     s = __reduce_add_sync(kFull, s);
     if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = s;
     __syncthreads();
@@ -605,12 +604,12 @@ int launch_popcount_sum(int tile_cols, const uint32_t* blocks, uint64_t num_tile
 }  // namespace btc200
 
 namespace btc200 {
-// Popcount per fixed 4096-word chunk (bm::kChunk; the batch builder's chunking, which
-// does not follow bitmap_chunks).
+// Popcount per 1024-word chunk (the batch builder's chunking, which does not follow
+// bitmap_chunks).
 int launch_bitmap_count(const uint32_t* bitmap, uint64_t W, uint32_t* chunk_count, cudaStream_t s)
 {
-    const uint64_t chunks = (W + bm::kChunk - 1) / bm::kChunk;
-    if (W) bm::k_bm_count<<<(unsigned)chunks, bm::kThreads, 0, s>>>(bitmap, W, chunk_count);
+    const uint64_t chunks = (W + bm::kThreads * 4 - 1) / (bm::kThreads * 4);
+    if (W) bm::k_bm_count<4><<<(unsigned)chunks, bm::kThreads, 0, s>>>(bitmap, W, chunk_count);
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 }  // namespace btc200
