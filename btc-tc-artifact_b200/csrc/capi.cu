@@ -128,6 +128,9 @@ struct BuildPlan {
     uint32_t flags;
     bool use_bitmap;
     bool use_group;  // the grouped builder (group.cu)
+    bool small;      // the one-launch builder (small.cu)
+    bool open_width; // ... which picks the tile width
+    uint32_t cap32, cap128;  // ... and the tiles the arrays hold at either
     uint64_t col_blocks;
     bool degree;
     uint64_t bm_words;
@@ -137,6 +140,16 @@ struct BuildPlan {
 
 // Only a graph with at least 8 edges per row block can average 8 tiles per row block (every
 // tile holds an edge).
+// Graphs the one-launch builder takes: SMALL_RULE.
+static constexpr int64_t kSmallEdges = 1 << 19;
+static constexpr size_t kSmallFirstBytes = 32ull << 20;
+static bool small_possible(int64_t m, int32_t n)
+{
+    if (m <= 0 || m > kSmallEdges || n <= 0) return false;
+    const BuildGeom g = make_geom(n, 32);
+    return bitmap_words_per_row(g) * (uint64_t)g.n_row_blocks <= (1ull << 20);
+}
+
 static bool row_store_possible(int64_t m, int32_t n_row_blocks)
 {
     return n_row_blocks > 0 && m >= 8 * (int64_t)n_row_blocks && m < (int64_t)0xffffffffll;
@@ -211,7 +224,7 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
 {
     const BuildGeom& geom = P.geom;
     unsigned long long* meta = g->meta.as<unsigned long long>();
-    BTC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(unsigned long long) * kMetaSlots, s));
+    if (!P.small) BTC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(unsigned long long) * kMetaSlots, s));
     if ((P.flags & BTC_INPUT_ON_HOST) && P.m > 0) {
         BTC_CUDA_TRY(cudaMemcpyAsync(g->in_src.ptr, P.src, sizeof(int32_t) * (size_t)P.m,
                                      cudaMemcpyHostToDevice, s));
@@ -240,7 +253,18 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
         rank = g->rank.as<int32_t>();
     }
 
-    if (P.use_bitmap) {
+    if (P.small) {
+        unsigned long long* w = g->small.as<unsigned long long>();
+        SmallBuild b{P.d_src, P.d_dst, P.m, P.n, P.open_width ? 0 : geom.tile_cols, g->bitmap.as<uint32_t>(),
+                     g->tile_base.as<uint32_t>(), g->prefix.as<uint2>(), g->indices.as<uint32_t>(),
+                     g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(), g->blocks.as<uint32_t>(),
+                     g->rowmask.as<uint32_t>(), P.cap128, P.cap32, meta, g->d_hmeta, w,
+                     reinterpret_cast<unsigned int*>(w + 2),
+                     std::max<int64_t>(P.m / (int64_t)kPolicySamples, 1),
+                     (uint32_t)std::min<int64_t>(P.m, (int64_t)kPolicySamples)};
+        BTC_TRY(launch_build_small(b, s));
+        if (P.row_store) BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, false, s));
+    } else if (P.use_bitmap) {
         BTC_TRY(bitmap_mark_and_count(geom, P.d_src, P.d_dst, P.m, rank, g->bitmap.as<uint32_t>(),
                                       g->tile_base.as<uint32_t>(), meta + kMetaBad,
                                       meta + kMetaTiles, s));
@@ -299,13 +323,14 @@ static void build_key(const btc_bitbsr* g, const BuildPlan& P, BuildGraphKey* k)
                        g->keys1.ptr, g->sort_scratch.ptr, g->deg.ptr, g->rank.ptr, g->bitmap.ptr,
                        g->prefix.ptr, g->tile_base.ptr, g->indices.ptr, g->row_indices.ptr,
                        g->indptr.ptr, g->blocks.ptr, g->rowmask.ptr, g->d_hmeta, g->rs_off.ptr,
-                       g->rs_key.ptr, g->rs_bits.ptr, g->rs_first.ptr};
+                       g->rs_key.ptr, g->rs_bits.ptr, g->rs_first.ptr, g->small.ptr};
     static_assert(sizeof(w) / sizeof(w[0]) == kBuildKeyPtrs, "key layout");
     for (int i = 0; i < kBuildKeyPtrs; ++i) k->ptr[i] = w[i];
     k->m = P.m;
     k->n = P.n;
     k->tile_cols = P.geom.tile_cols;
-    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.use_group ? 0x40000000u : 0u);
+    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.use_group ? 0x40000000u : 0u) |
+               (P.small ? 0x20000000u : 0u);
     k->cap = P.cap;
 }
 
@@ -350,14 +375,22 @@ static bool launch_build_graph(btc_bitbsr* g, const BuildPlan& P, cudaStream_t s
 
 // tiles_only: the caller keeps the reference-shaped arrays alone, so no row store is made.
 static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
-                      int tile_cols, uint32_t flags, cudaStream_t s, bool tiles_only = false)
+                      int tile_cols, uint32_t flags, cudaStream_t s, bool tiles_only = false,
+                      bool allow_small = true)
 {
     if (n < 0 || m < 0 || (uint64_t)m > kMaxEdges) return BTC_E_INVAL;
     if (m > 0 && (!src || !dst)) return BTC_E_INVAL;
     if (flags & ~(BTC_INPUT_ON_HOST | BTC_ORIENT_DEGREE | BTC_BUILD_RADIX | BTC_BUILD_ASYNC))
         return BTC_E_INVAL;
     if (g->pending) resolve_build(g);  // an enqueued build still owns the buffers
-    if (tile_cols == 0) {
+    // A small graph in natural order is built by one launch (small.cu), which also picks the
+    // tile width where it is open: device input, and not the degree's to decide.
+    bool small = allow_small && !(flags & (BTC_ORIENT_DEGREE | BTC_BUILD_RADIX)) && small_possible(m, n);
+    const bool open_width = small && tile_cols == 0 && !(flags & (BTC_INPUT_ON_HOST | BTC_BUILD_ASYNC)) &&
+                            !policy_dense(m, n);
+    if (open_width) {
+        tile_cols = 32;  // the larger cell grid, for the sizes below
+    } else if (tile_cols == 0) {
         // the engine's tile policy (policy.cu).  With degree ordering it needs only m and
         // n; otherwise it samples the edges (a wait), which an enqueued rebuild skips by
         // keeping the handle's width.
@@ -410,6 +443,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     const uint64_t bm_bytes = 4 * P.bm_words;
     P.use_bitmap = !(flags & BTC_BUILD_RADIX) && bm_bytes <= (4ull << 30) &&
                    bm_bytes <= 32ull * (uint64_t)m + (64ull << 20);
+    small = small && P.use_bitmap;
     // Large edge lists are grouped by row block instead of marked and filled edge by edge
     // (see kGroupEdges), and so is what the bitmap does not take.
     P.col_blocks = (uint64_t)geom.n_col_blocks;
@@ -451,6 +485,34 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     BTC_TRY(ensure_count_scratch(g));
 
     const size_t TW = (size_t)16 * (tile_cols / 32);
+    if (small) {
+        // a first build reserves a tile per edge (or per cell) instead of waiting for the count
+        if (!g->indices.ptr || !g->row_indices.ptr || !g->blocks.ptr || !g->rowmask.ptr) {
+            const uint64_t cells = (uint64_t)geom.n_row_blocks * (uint64_t)geom.n_col_blocks;
+            const uint64_t most = std::min<uint64_t>((uint64_t)m, cells);
+            const size_t bytes = (size_t)(open_width ? 256 : 4 * TW) * most;
+            if (bytes <= kSmallFirstBytes) {
+                BTC_TRY(g->indices.reserve(sizeof(uint32_t) * most));
+                BTC_TRY(g->row_indices.reserve(sizeof(uint32_t) * most));
+                BTC_TRY(g->rowmask.reserve(sizeof(uint32_t) * most));
+                BTC_TRY(g->blocks.reserve(bytes));
+            } else {
+                small = false;
+            }
+        }
+        if (small) {
+            const bool fresh = !g->small.ptr;
+            BTC_TRY(g->small.reserve(4 * sizeof(unsigned long long)));
+            BTC_TRY(g->tile_base.reserve(sizeof(uint32_t) * 2 * (size_t)device_sm_count()));
+            if (fresh || g->small_dirty)
+                BTC_CUDA_TRY(cudaMemsetAsync(g->small.ptr, 0, 4 * sizeof(unsigned long long), s));
+            g->small_dirty = true;  // until a wait has seen the build's end
+        } else if (open_width) {
+            return build_into(g, src, dst, m, n, 0, flags, s, tiles_only, false);
+        }
+    }
+    P.small = small;
+    P.open_width = open_width;
     // Tiles the arrays already hold room for (a rebuild): the bitmap path then enqueues
     // the whole build against that capacity, with every post-count kernel checking the
     // device tile count, and waits once at the end (or not at all with BTC_BUILD_ASYNC);
@@ -462,11 +524,17 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         c = std::min<uint64_t>(c, g->blocks.bytes / (4 * TW));
         c = std::min<uint64_t>(c, g->rowmask.bytes / 4);
         P.cap = (uint32_t)std::min<uint64_t>(c, 0xffffffffull);
+        const uint64_t rows = std::min<uint64_t>(g->indices.bytes / 4,
+                                                 std::min<uint64_t>(g->row_indices.bytes / 4, g->rowmask.bytes / 4));
+        P.cap32 = (uint32_t)std::min<uint64_t>(rows, g->blocks.bytes / 64);
+        P.cap128 = (uint32_t)std::min<uint64_t>(rows, g->blocks.bytes / 256);
         // The row store of the streaming count.  A rebuild whose previous graph of the same
         // geometry averaged fewer than 8 tiles per row block skips it (a mesh counts faster
         // tile-wise); should this graph average more after all, the count takes the
         // tile-wise kernel, which needs no store.  So does a graph without the memory for it.
-        P.row_store = P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light &&
+        // (A waiting build by one launch decides when it knows the tiles.)
+        P.row_store = !(small && !(flags & BTC_BUILD_ASYNC)) && !tiles_only &&
+                      P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light &&
                       reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * P.cap)) == BTC_OK;
         g->row_store = P.row_store;
     }
@@ -486,6 +554,22 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         g->pending_cap = P.cap;
         if (flags & BTC_BUILD_ASYNC) return BTC_OK;  // resolved by the next wait
         const int st2 = resolve_build(g);
+        if (small) {
+            if (st2 == BTC_E_CUDA) return st2;
+            if (open_width) {
+                tile_cols = (int)g->h_meta[kHostTileCols];
+                if (tile_cols != 32 && tile_cols != 128) return BTC_E_CUDA;
+                g->tile_cols = tile_cols;
+            }
+            if (st2 == BTC_E_CAPACITY)
+                return build_into(g, src, dst, m, n, tile_cols, flags, s, tiles_only, false);
+            if (st2 != BTC_OK) return st2;
+            g->row_store = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
+                           (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks &&
+                           reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * g->num_tiles)) == BTC_OK;
+            if (g->row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, false, s));
+            return BTC_OK;
+        }
         if (st2 != BTC_E_CAPACITY) return st2;
         // more tiles than the arrays hold: redo the post-count steps at the right size
         BTC_CUDA_TRY(cudaMemsetAsync(meta + kMetaOverflow, 0, sizeof(unsigned long long), s));
@@ -594,7 +678,10 @@ int resolve_build(btc_bitbsr* g)
         return g->failed = BTC_E_CUDA;
     }
     const unsigned long long* h = g->h_meta;
-    if (h[kMetaBad] != 0) {
+    g->small_dirty = g->small_dirty && h[kMetaOverflow] > 1;  // (2: a barrier of the small build gave up)
+    if (h[kMetaOverflow] > 1) {
+        g->failed = BTC_E_CUDA;
+    } else if (h[kMetaBad] != 0) {
         g->failed = BTC_E_RANGE;
     } else if (h[kMetaOverflow] != 0 || h[kMetaTiles] > g->pending_cap) {
         g->failed = BTC_E_CAPACITY;

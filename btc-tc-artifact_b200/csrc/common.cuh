@@ -332,6 +332,51 @@ int launch_cells(const uint32_t* indptr, const uint32_t* indices, const uint32_t
 // Id locality of an edge list for the tile policy (policy.cu): sampled share of edges
 // with |u - v| < 128 over the share uniform ids would give.  e_off / nv (nullable): the
 // batch layout, each edge measured against its own graph's vertex count.
+constexpr uint32_t kPolicySamples = 1u << 16;
+constexpr int32_t kPolicyNear = 128;  // |u - v| below this counts as local
+// One sampled edge: is it local, and the chance that two uniform ids are (2^20 = 1).
+__device__ __forceinline__ void policy_sample(int32_t u, int32_t v, int32_t n, unsigned long long& local,
+                                              unsigned long long& expect)
+{
+    if (u == v || u < 0 || v < 0 || u >= n || v >= n) return;
+    local += (u > v ? u - v : v - u) < kPolicyNear ? (1ull << 20) : 0ull;
+    expect += n > 2 * kPolicyNear ? ((2ull * kPolicyNear - 1ull) << 20) / (unsigned long long)n : (1ull << 20);
+}
+// A locality of at least 16, as btc_tile_policy_from_features decides it (the sums stay below
+// 2^37, so the quotient there rounds to 16 only where it is 16).
+__device__ __forceinline__ bool policy_is_local(unsigned long long local, unsigned long long expect)
+{
+    return expect != 0 && local >= 16 * expect;
+}
+// Whether the average degree alone decides for 16x32 tiles.
+bool policy_dense(int64_t m, int32_t n);
+
+// The one-launch builder of small graphs (small.cu).
+constexpr int kHostTileCols = 9;  // host slot: the width the policy picked
+struct SmallBuild {
+    const int32_t* src;
+    const int32_t* dst;
+    int64_t m;
+    int32_t n;
+    int tile_cols;       // 0: the policy's
+    uint32_t* words;     // cell words (of 16x32 tiles where the width is open)
+    uint32_t* counts;    // two per SM
+    uint2* cellpp;
+    uint32_t* indices;
+    uint32_t* row_indices;
+    uint32_t* indptr;
+    uint32_t* blocks;
+    uint32_t* rowmask;
+    uint32_t cap128, cap32;
+    unsigned long long* meta;
+    unsigned long long* host;  // the device's address of the status slots
+    unsigned long long* policy_sums;
+    unsigned int* bar;
+    int64_t step;
+    uint32_t samples;
+};
+int launch_build_small(const SmallBuild& b, cudaStream_t s);
+
 struct PolicyWords {
     DevBuf dev;                          // two sums and a ticket
     unsigned long long* host = nullptr;  // a host slot

@@ -5,7 +5,7 @@
 
 // Arguments and buffers of an enqueued build (a cached build graph replays only when
 // they are unchanged).
-constexpr int kBuildKeyPtrs = 23;
+constexpr int kBuildKeyPtrs = 24;
 struct BuildGraphKey {
     const void* ptr[kBuildKeyPtrs];
     int64_t m;
@@ -39,6 +39,8 @@ struct btc_bitbsr {
     // count scratch
     btc200::DevBuf partials, done;
     btc200::PolicyWords policy;
+    btc200::DevBuf small;     // the one-launch builder's sums and barrier (small.cu), zero between launches
+    bool small_dirty = false; // a launch may have left something in them
     unsigned long long* h_meta = nullptr;  // pinned and mapped, 8 slots
     unsigned long long* d_hmeta = nullptr; // the device's address of h_meta
     bool edges_known = false;
@@ -61,7 +63,7 @@ struct btc_bitbsr {
         btc200::DevBuf* all[] = {&indptr, &indices, &row_indices, &blocks, &result, &in_src, &in_dst,
                                  &keys0, &keys1, &sort_scratch, &tile_base, &meta, &deg, &rank,
                                  &bitmap, &prefix, &partials, &done, &rowmask, &row_off, &row_ent,
-                                 &row_tot, &row_bsum, &rs_off, &rs_key, &rs_bits, &rs_first};
+                                 &row_tot, &row_bsum, &rs_off, &rs_key, &rs_bits, &rs_first, &small};
         for (btc200::DevBuf* b : all) f(*b);
     }
     size_t device_bytes() const

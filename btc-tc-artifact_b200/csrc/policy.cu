@@ -26,8 +26,8 @@ namespace pol {
 
 constexpr int kThreads = 256;
 constexpr int kGrid = 64;
-constexpr uint32_t kSamples = 1u << 16;
-constexpr int32_t kNear = 128;  // |u - v| below this counts as local
+constexpr uint32_t kSamples = kPolicySamples;
+constexpr int32_t kNear = kPolicyNear;
 
 // Sample i reads edge i * step.  Adds the number of local edges and their expectation
 // under uniform ids (per sampled edge: the chance that two uniform ids in [0, n) lie
@@ -55,9 +55,7 @@ __global__ void k_locality(const int32_t* __restrict__ src, const int32_t* __res
             ng = nv[lo];
         }
         const int32_t u = src[e], v = dst[e];
-        if (u == v || u < 0 || v < 0 || u >= ng || v >= ng) continue;
-        local += (u > v ? u - v : v - u) < kNear ? (1ull << 20) : 0ull;
-        expect += ng > 2 * kNear ? ((2ull * kNear - 1ull) << 20) / (unsigned long long)ng : (1ull << 20);
+        policy_sample(u, v, ng, local, expect);
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -101,9 +99,14 @@ double locality_host(const int32_t* src, const int32_t* dst, int64_t m, int32_t 
 }
 
 // Average degree 2m/n of at least 512.
-bool dense(int64_t m, int32_t n) { return n > 0 && 2.0 * (double)m / (double)n >= 512.0; }
+bool dense(int64_t m, int32_t n)
+{
+    return n > 0 && 2.0 * (double)m / (double)n >= 512.0;
+}
 
 }  // namespace pol
+
+bool policy_dense(int64_t m, int32_t n) { return pol::dense(m, n); }
 
 // Id locality of an edge list (see above): host arrays are sampled on the host, device
 // arrays by one small kernel and one wait on `s`.  e_off / nv (optional, num_graphs + 1 and
