@@ -23,6 +23,8 @@
 // up), one write of the tiles: no sort.  Duplicate edges OR the same bit.
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace btc200 {
 namespace bm {
 
@@ -45,14 +47,19 @@ __device__ __forceinline__ bool orient(int32_t u, int32_t v, int32_t n, const in
 
 // Every cell bit is hit by all edges of its tile, so the word is read first and the
 // atomic is skipped when the bit is already set.  Bits only go from 0 to 1, so a
-// stale read can only cost a redundant atomic, never a missing one.
+// stale read can only cost a redundant atomic, never a missing one.  The L2 atomics are what
+// bounds it, so few edges are in flight: with eight per thread a mesh's edges had nearly all
+// read their word before the first of a tile set it (27-point mesh 64^3: 20.7 us, 16.1 with
+// two; 8 communities on 32,768 vertices 51.7 / 46.4; sparse graphs, whose tiles hold one
+// edge, the same).
+constexpr int kMarkEdges = 2;
 template <int LOG2C>
 __global__ void __launch_bounds__(kThreads)
 k_mark(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m, int32_t n,
        const int32_t* __restrict__ rank, uint64_t wpr, uint32_t* bitmap,
        unsigned long long* __restrict__ bad_count)
 {
-    constexpr int U = 8;  // edges in flight per thread
+    constexpr int U = kMarkEdges;
     uint32_t nbad = 0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < m; i0 += U * stride) {
@@ -369,10 +376,20 @@ k_fill_bm(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int6
           const int32_t* __restrict__ rank, uint64_t wpr, const uint32_t* __restrict__ bitmap,
           const uint2* __restrict__ cellpp, uint32_t* __restrict__ blocks,
           const unsigned long long* __restrict__ d_tiles, uint32_t cap, uint32_t* __restrict__ rowmask,
-          bool always_masks, int32_t R)
+          bool always_masks, int32_t R, const uint32_t* __restrict__ indptr,
+          unsigned long long* __restrict__ row_max)
 {
     const unsigned long long T = *d_tiles;
     if (T > cap) return;  // overflowed tile arrays: the builder redoes this step
+    if (row_max) {
+        // the longest row-block list, for the tile-wise count's schedule
+        uint32_t mx = 0;
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < R;
+             i += (int64_t)gridDim.x * blockDim.x)
+            mx = max(mx, indptr[i + 1] - indptr[i]);
+        mx = __reduce_max_sync(kFull, mx);
+        if ((threadIdx.x & 31) == 0 && mx) atomicMax(row_max, (unsigned long long)mx);
+    }
     // row-occupancy masks: wanted for the row store, and when row blocks average 8 or more
     // tiles (the heavy counts' condition, on the device tile count)
     if (!always_masks && T < 8ull * (unsigned long long)(R > 0 ? R : 0)) rowmask = nullptr;
@@ -468,6 +485,11 @@ __global__ void k_popcount_sum(const uint32_t* __restrict__ blocks, uint64_t wor
 int grid_for(int64_t work, int threads);
 int launch_tile_scan(uint32_t* per_tile, uint32_t ntiles, unsigned long long* total, cudaStream_t s);
 
+static int mark_grid(int64_t m)
+{
+    return std::min(grid_for((m + bm::kMarkEdges - 1) / bm::kMarkEdges, bm::kThreads), 8 * device_sm_count());
+}
+
 // one round of U = 8 edges per thread (the grid is capped at 16 CTAs per SM)
 static int edge_grid(int64_t m) { return grid_for((m + 7) / 8, bm::kThreads); }
 
@@ -508,10 +530,10 @@ int bitmap_mark_and_count(const BuildGeom& g, const int32_t* src, const int32_t*
     if (cudaMemsetAsync(bitmap, 0, sizeof(uint32_t) * W, s) != cudaSuccess) return BTC_E_CUDA;
     if (m > 0) {
         if (g.tile_cols == 128)
-            bm::k_mark<7><<<edge_grid(m), bm::kThreads, 0, s>>>(src, dst, m, g.n, rank, wpr, bitmap,
+            bm::k_mark<7><<<mark_grid(m), bm::kThreads, 0, s>>>(src, dst, m, g.n, rank, wpr, bitmap,
                                                                  meta_bad);
         else
-            bm::k_mark<5><<<edge_grid(m), bm::kThreads, 0, s>>>(src, dst, m, g.n, rank, wpr, bitmap,
+            bm::k_mark<5><<<mark_grid(m), bm::kThreads, 0, s>>>(src, dst, m, g.n, rank, wpr, bitmap,
                                                                  meta_bad);
     }
     const size_t chunks = bitmap_chunks(W);
@@ -541,9 +563,13 @@ int bitmap_emit_and_fill(const BuildGeom& g, const int32_t* src, const int32_t* 
                          uint2* cellpp, uint32_t* indices, uint32_t* row_indices,
                          uint32_t* indptr, uint32_t* blocks, unsigned long long* meta,
                          uint32_t cap, unsigned long long* host_meta, cudaStream_t s,
-                         uint32_t* rowmask, bool always_masks)
+                         uint32_t* rowmask, bool row_store)
 {
     const unsigned long long* meta_tiles = meta + kMetaTiles;
+    // with a row store to come: masks whatever the tile count, and the store's pass finds the
+    // longest list
+    const bool always_masks = row_store;
+    unsigned long long* row_max = row_store ? nullptr : meta + kMetaRowMax;
     const uint64_t wpr = bitmap_words_per_row(g);
     const uint64_t W = wpr * (uint64_t)g.n_row_blocks;
     const uint32_t vec4 = 4u * (uint32_t)(g.tile_cols / 32);  // 16-byte words per tile
@@ -570,11 +596,11 @@ int bitmap_emit_and_fill(const BuildGeom& g, const int32_t* src, const int32_t* 
         if (g.tile_cols == 128)
             bm::k_fill_bm<7><<<edge_grid(m), bm::kThreads, 0, s>>>(
                 src, dst, m, g.n, rank, wpr, bitmap, cellpp, blocks, meta_tiles, cap, rowmask,
-                always_masks, g.n_row_blocks);
+                always_masks, g.n_row_blocks, indptr, row_max);
         else
             bm::k_fill_bm<5><<<edge_grid(m), bm::kThreads, 0, s>>>(
                 src, dst, m, g.n, rank, wpr, bitmap, cellpp, blocks, meta_tiles, cap, rowmask,
-                always_masks, g.n_row_blocks);
+                always_masks, g.n_row_blocks, indptr, row_max);
     }
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }

@@ -140,7 +140,11 @@ struct BuildPlan {
 
 // Only a graph with at least 8 edges per row block can average 8 tiles per row block (every
 // tile holds an edge).
-// Graphs the one-launch builder takes: SMALL_RULE.
+// Graphs the one-launch builder takes, when the call waits: it saves about 17 us of launches
+// and waits whatever the size (Erdos-Renyi, a step: 1,000 vertices 83 -> 66 us, 16,384 / 16
+// 112 -> 91, 40,000 / 26, 520,000 draws 184 -> 168), which from 2^19 edges on is a few percent
+// and on a mesh of 1.5M edges nothing.  An enqueued rebuild replays a graph, whose launches
+// cost less than the barriers (16,384 / 16: 66 us, 71 by one launch).
 static constexpr int64_t kSmallEdges = 1 << 19;
 static constexpr size_t kSmallFirstBytes = 32ull << 20;
 static bool small_possible(int64_t m, int32_t n)
@@ -210,7 +214,7 @@ void ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t
 
 static int enqueue_group_write(btc_bitbsr* g, const BuildPlan& P, uint32_t cap, cudaStream_t s)
 {
-    return group_write(P.geom.tile_cols, P.col_blocks, (uint32_t)P.geom.n_row_blocks, nullptr, 0,
+    return group_write(P.geom.tile_cols, P.col_blocks, P.m, (uint32_t)P.geom.n_row_blocks, nullptr, 0,
                        g->keys0.as<uint32_t>(), g->tile_base.as<uint32_t>(), g->indptr.as<uint32_t>(),
                        g->meta.as<unsigned long long>(), cap, g->indices.as<uint32_t>(),
                        g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(), g->rowmask.as<uint32_t>(),
@@ -263,7 +267,6 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
                      std::max<int64_t>(P.m / (int64_t)kPolicySamples, 1),
                      (uint32_t)std::min<int64_t>(P.m, (int64_t)kPolicySamples)};
         BTC_TRY(launch_build_small(b, s));
-        if (P.row_store) BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, false, s));
     } else if (P.use_bitmap) {
         BTC_TRY(bitmap_mark_and_count(geom, P.d_src, P.d_dst, P.m, rank, g->bitmap.as<uint32_t>(),
                                       g->tile_base.as<uint32_t>(), meta + kMetaBad,
@@ -275,14 +278,8 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
                                          g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(),
                                          g->blocks.as<uint32_t>(), meta, P.cap, g->d_hmeta, s,
                                          g->rowmask.as<uint32_t>(), P.row_store));
-            // the fill pass set the row masks; what is left is the row store, or only the
-            // longest row-block list
-            if (P.row_store)
-                BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s));
-            else
-                BTC_TRY(launch_rowmask(geom.tile_cols, g->blocks.as<uint32_t>(), P.cap,
-                                       meta + kMetaTiles, g->indptr.as<uint32_t>(), geom.n_row_blocks,
-                                       g->rowmask.as<uint32_t>(), meta + kMetaRowMax, s, false));
+            // (the fill pass set the row masks, or found the longest row-block list)
+            if (P.row_store) BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s));
         }
     } else if (P.use_group) {
         const uint32_t R = (uint32_t)geom.n_row_blocks;
@@ -323,14 +320,13 @@ static void build_key(const btc_bitbsr* g, const BuildPlan& P, BuildGraphKey* k)
                        g->keys1.ptr, g->sort_scratch.ptr, g->deg.ptr, g->rank.ptr, g->bitmap.ptr,
                        g->prefix.ptr, g->tile_base.ptr, g->indices.ptr, g->row_indices.ptr,
                        g->indptr.ptr, g->blocks.ptr, g->rowmask.ptr, g->d_hmeta, g->rs_off.ptr,
-                       g->rs_key.ptr, g->rs_bits.ptr, g->rs_first.ptr, g->small.ptr};
+                       g->rs_key.ptr, g->rs_bits.ptr, g->rs_first.ptr};
     static_assert(sizeof(w) / sizeof(w[0]) == kBuildKeyPtrs, "key layout");
     for (int i = 0; i < kBuildKeyPtrs; ++i) k->ptr[i] = w[i];
     k->m = P.m;
     k->n = P.n;
     k->tile_cols = P.geom.tile_cols;
-    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.use_group ? 0x40000000u : 0u) |
-               (P.small ? 0x20000000u : 0u);
+    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.use_group ? 0x40000000u : 0u);
     k->cap = P.cap;
 }
 
@@ -385,9 +381,9 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     if (g->pending) resolve_build(g);  // an enqueued build still owns the buffers
     // A small graph in natural order is built by one launch (small.cu), which also picks the
     // tile width where it is open: device input, and not the degree's to decide.
-    bool small = allow_small && !(flags & (BTC_ORIENT_DEGREE | BTC_BUILD_RADIX)) && small_possible(m, n);
-    const bool open_width = small && tile_cols == 0 && !(flags & (BTC_INPUT_ON_HOST | BTC_BUILD_ASYNC)) &&
-                            !policy_dense(m, n);
+    bool small = allow_small && !(flags & (BTC_ORIENT_DEGREE | BTC_BUILD_RADIX | BTC_BUILD_ASYNC)) &&
+                 small_possible(m, n);
+    const bool open_width = small && tile_cols == 0 && !(flags & BTC_INPUT_ON_HOST) && !policy_dense(m, n);
     if (open_width) {
         tile_cols = 32;  // the larger cell grid, for the sizes below
     } else if (tile_cols == 0) {
@@ -532,9 +528,8 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         // geometry averaged fewer than 8 tiles per row block skips it (a mesh counts faster
         // tile-wise); should this graph average more after all, the count takes the
         // tile-wise kernel, which needs no store.  So does a graph without the memory for it.
-        // (A waiting build by one launch decides when it knows the tiles.)
-        P.row_store = !(small && !(flags & BTC_BUILD_ASYNC)) && !tiles_only &&
-                      P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light &&
+        // (A build by one launch decides when it knows the tiles.)
+        P.row_store = !small && !tiles_only && P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light &&
                       reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * P.cap)) == BTC_OK;
         g->row_store = P.row_store;
     }
@@ -615,7 +610,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     }
     // the bitmap and grouped builders set the row masks; the radix path's are computed here
     const bool have_masks = P.use_bitmap || P.use_group;
-    if (!have_masks || !P.row_store)
+    if (!have_masks || (P.use_group && !P.row_store))
         BTC_TRY(launch_rowmask(tile_cols, g->blocks.as<uint32_t>(), g->num_tiles, nullptr,
                                g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
                                meta + kMetaRowMax, s, !have_masks));

@@ -316,7 +316,7 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, in
                 const uint32_t* graph_rows, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
                 uint64_t* grouped, uint32_t* edges, uint32_t* scratch, uint32_t* indptr, uint32_t* bsum,
                 unsigned long long* meta, cudaStream_t s);
-int group_write(int tile_cols, uint64_t col_blocks, uint32_t R, const uint32_t* graph_rows, uint32_t G,
+int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R, const uint32_t* graph_rows, uint32_t G,
                 const uint32_t* edges, const uint32_t* scratch, const uint32_t* indptr,
                 const unsigned long long* meta, uint32_t cap, uint32_t* indices, uint32_t* row_indices,
                 uint32_t* blocks, uint32_t* rowmask, uint32_t tiles_hint, cudaStream_t s);

@@ -321,7 +321,6 @@ k_rb_scatter(const uint64_t* __restrict__ in, const uint32_t* __restrict__ d_m, 
 }
 
 // ---- tiles ---------------------------------------------------------------------------------
-constexpr int kTThreads = 128;
 constexpr uint32_t kTileBytes = 32768;  // tile buffer, at most
 constexpr uint32_t kDirect = 1u << 18;  // looks at an edge from which a row block is written directly
 
@@ -340,7 +339,7 @@ __device__ __forceinline__ uint32_t first_col_block(const uint32_t* __restrict__
     return (16u * graph_rows[lo]) >> LOG2C;
 }
 
-template <int LOG2C>
+template <int LOG2C, int kTThreads>
 __global__ void __launch_bounds__(kTThreads)
 k_count_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ rb_end, uint32_t R,
               uint32_t words, const uint32_t* __restrict__ graph_rows, uint32_t G,
@@ -374,7 +373,7 @@ k_count_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
     }
 }
 
-template <int LOG2C>
+template <int LOG2C, int kTThreads>
 __global__ void __launch_bounds__(kTThreads)
 k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ rb_end, uint32_t R,
               uint32_t words, const uint32_t* __restrict__ graph_rows, uint32_t G,
@@ -554,6 +553,11 @@ static int bucket_shift(int64_t rows)
     return s;
 }
 
+// Threads of a row block's CTA: one warp where the row blocks average at most 96 edges (a grid
+// of 7 points per vertex, 48 edges a row block: k_write_tiles 273 us with four warps, 190 with
+// one, k_count_tiles 93 / 65), four above (R-MAT scale 22 in degree order averages 256).
+static int row_block_threads(int64_t m, uint32_t R) { return m <= 96ll * R ? 32 : 128; }
+
 // Whether the grouped builder takes a matrix of n columns (a batch: the union) whose row
 // blocks span at most col_blocks column blocks each.
 bool group_possible(int64_t n, uint64_t col_blocks)
@@ -601,24 +605,27 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, in
     BTC_TRY(launch_scan_u32(rb_end, R, bsum, sum, s));
     if (m > 0) gp::k_rb_scatter<<<stiles, gp::kSThreads, 0, s>>>(grouped, d_m, rb_end, edges);
     const uint32_t words = (uint32_t)((col_blocks + 31) / 32);
-    const int tgrid = (int)std::min<uint32_t>(R, 32u * device_sm_count());
+    const int threads = row_block_threads(m, R);
+    const uint32_t grid = std::min<uint32_t>(R, 32u * device_sm_count() * (128 / threads));
+    auto count = [&](auto kernel) {
+        kernel<<<grid, threads, 4 * words, s>>>(edges, rb_end, R, words, graph_rows, G, indptr);
+    };
     if (tile_cols == 128)
-        gp::k_count_tiles<7><<<tgrid, gp::kTThreads, 4 * words, s>>>(edges, rb_end, R, words, graph_rows, G, indptr);
+        threads == 32 ? count(gp::k_count_tiles<7, 32>) : count(gp::k_count_tiles<7, 128>);
     else
-        gp::k_count_tiles<5><<<tgrid, gp::kTThreads, 4 * words, s>>>(edges, rb_end, R, words, graph_rows, G, indptr);
+        threads == 32 ? count(gp::k_count_tiles<5, 32>) : count(gp::k_count_tiles<5, 128>);
     return launch_scan_u32(indptr, R, bsum, meta + kMetaTiles, s);
 }
 
 // Tiles, indices, row_indices and row masks from the grouped edges (indptr[R] set), against
 // `cap` tiles: nothing when meta[kMetaTiles] is above it.
-int group_write(int tile_cols, uint64_t col_blocks, uint32_t R, const uint32_t* graph_rows, uint32_t G,
+int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R, const uint32_t* graph_rows, uint32_t G,
                 const uint32_t* edges, const uint32_t* scratch, const uint32_t* indptr,
                 const unsigned long long* meta, uint32_t cap, uint32_t* indices, uint32_t* row_indices,
                 uint32_t* blocks, uint32_t* rowmask, uint32_t tiles_hint, cudaStream_t s)
 {
     const uint32_t* rb_end = scratch + 3 * (size_t)gp::kBuckets + 1;
     const uint32_t words = (uint32_t)((col_blocks + 127) / 128 * 4);  // whole fours
-    const int grid = (int)std::min<uint32_t>(R, 32u * device_sm_count());
     // tiles built at once: one and a half times the average row block's, in 4 KB (a mesh's
     // row blocks: more CTAs) up to 16 KB (16x128) or 32 KB (16x32); 8 KB cost R-MAT scale 22
     // 15%, 32 KB 20%
@@ -628,19 +635,18 @@ int group_write(int tile_cols, uint64_t col_blocks, uint32_t R, const uint32_t* 
     const uint32_t NT = buf / tile_bytes;
     const size_t smem = buf + 4 * (size_t)NT + 8 * (size_t)words;
     const size_t most = gp::kTileBytes + 4 * (gp::kTileBytes / 64) + 8 * (size_t)gp::kMaxWords;
-    static std::atomic<bool> ok7[64], ok5[64];
-    if (tile_cols == 128) {
-        if (!gp::allow_smem(gp::k_write_tiles<7>, most, ok7)) return BTC_E_CUDA;
-        gp::k_write_tiles<7><<<grid, gp::kTThreads, smem, s>>>(edges, rb_end, R, words, graph_rows, G, indptr,
-                                                               meta + kMetaTiles, cap, indices, row_indices,
-                                                               reinterpret_cast<uint4*>(blocks), rowmask, NT);
-    } else {
-        if (!gp::allow_smem(gp::k_write_tiles<5>, most, ok5)) return BTC_E_CUDA;
-        gp::k_write_tiles<5><<<grid, gp::kTThreads, smem, s>>>(edges, rb_end, R, words, graph_rows, G, indptr,
-                                                               meta + kMetaTiles, cap, indices, row_indices,
-                                                               reinterpret_cast<uint4*>(blocks), rowmask, NT);
-    }
-    return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+    static std::atomic<bool> ok[4][64];
+    const int threads = row_block_threads(m, R);
+    const uint32_t grid = std::min<uint32_t>(R, 32u * device_sm_count() * (128 / threads));
+    auto write = [&](auto kernel, int which) {
+        if (!gp::allow_smem(kernel, most, ok[which])) return BTC_E_CUDA;
+        kernel<<<grid, threads, smem, s>>>(edges, rb_end, R, words, graph_rows, G, indptr, meta + kMetaTiles, cap,
+                                           indices, row_indices, reinterpret_cast<uint4*>(blocks), rowmask, NT);
+        return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+    };
+    if (tile_cols == 128)
+        return threads == 32 ? write(gp::k_write_tiles<7, 32>, 0) : write(gp::k_write_tiles<7, 128>, 1);
+    return threads == 32 ? write(gp::k_write_tiles<5, 32>, 2) : write(gp::k_write_tiles<5, 128>, 3);
 }
 
 }  // namespace btc200

@@ -5,7 +5,7 @@
 
 // Arguments and buffers of an enqueued build (a cached build graph replays only when
 // they are unchanged).
-constexpr int kBuildKeyPtrs = 24;
+constexpr int kBuildKeyPtrs = 23;
 struct BuildGraphKey {
     const void* ptr[kBuildKeyPtrs];
     int64_t m;
