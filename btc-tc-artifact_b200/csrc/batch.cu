@@ -25,10 +25,12 @@ namespace btc200 {
 namespace bt {
 
 constexpr int kThreads = 256;
-// Four words per thread: a chunk of a dense graph (communities: 32 tiles a word) is one CTA's
-// to name and to zero (256 mixed graphs: k_emit_b 245 us with sixteen, 200 with four).
-constexpr int kWordsPerThread = 4;
-constexpr int kChunk = kThreads * kWordsPerThread;
+// Words per thread of the chunk popcount and k_emit_b: one, so that a dense graph's chunk
+// (communities: 32 tiles a word) is not too much for its CTA to name and to zero (256 mixed
+// graphs: k_emit_b 245 us with sixteen, 204 with four, 144 with two, 104 with one); four where
+// the chunk counts, which one CTA scans, would be more than 32,768.
+constexpr uint64_t kFewWords = 32768ull * kThreads;
+inline uint64_t chunk_words(uint64_t words) { return words <= kFewWords ? kThreads : 4 * kThreads; }
 
 // last g in [0, G) with off[g] <= x (off[0] == 0; equal offsets are empty graphs)
 template <class T>
@@ -46,9 +48,10 @@ __device__ __forceinline__ uint32_t last_le(const T* __restrict__ off, uint32_t 
 // Edges in flight per thread of the edge passes.  A CTA takes runs of kEdges * kThreads
 // consecutive edges and a thread every kThreads-th of them, so that a thread's edges nearly
 // always share a graph, whose search and segment are then kept (a search per edge, eight
-// dependent loads, made the marking of 256 mixed graphs, 35M edges, take 423 us and the filling 453; 253 and
+// dependent loads, made the marking of 256 mixed graphs, 35M edges, take 423 us and the filling 453; 236 and
 // 406 like this, bound by the atomics: four edges in flight or more CTAs changed nothing).
 constexpr int kEdges = 8;
+constexpr int kMarkEdges = 4;  // (marking, 236 us: fewer atomics that another edge makes needless)
 
 struct EdgeGraph {
     int64_t lo = 0, hi = 0;  // the edges of `s`
@@ -92,20 +95,20 @@ k_mark_b(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64
 {
     uint32_t nbad = 0;
     EdgeGraph g;
-    for (int64_t i0 = (int64_t)blockIdx.x * (kEdges * kThreads) + threadIdx.x; i0 < m;
-         i0 += (int64_t)gridDim.x * (kEdges * kThreads)) {
-        int32_t u[kEdges], v[kEdges];
+    for (int64_t i0 = (int64_t)blockIdx.x * (kMarkEdges * kThreads) + threadIdx.x; i0 < m;
+         i0 += (int64_t)gridDim.x * (kMarkEdges * kThreads)) {
+        int32_t u[kMarkEdges], v[kMarkEdges];
 #pragma unroll
-        for (int k = 0; k < kEdges; ++k) {
+        for (int k = 0; k < kMarkEdges; ++k) {
             const int64_t i = i0 + k * kThreads;
             u[k] = i < m ? src[i] : 0;
             v[k] = i < m ? dst[i] : 0;
         }
-        uint64_t w[kEdges];
-        uint32_t bit[kEdges];
-        bool ok[kEdges];
+        uint64_t w[kMarkEdges];
+        uint32_t bit[kMarkEdges];
+        bool ok[kMarkEdges];
 #pragma unroll
-        for (int k = 0; k < kEdges; ++k) {
+        for (int k = 0; k < kMarkEdges; ++k) {
             const int64_t i = i0 + k * kThreads;
             ok[k] = false;
             w[k] = 0;
@@ -118,17 +121,18 @@ k_mark_b(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64
             nbad += bad;
             if (ok[k]) w[k] = cell_word<LOG2C>(g.s, r, c, bit[k]);
         }
-        uint32_t cur[kEdges];
+        uint32_t cur[kMarkEdges];
 #pragma unroll
-        for (int k = 0; k < kEdges; ++k) cur[k] = ok[k] ? bitmap[w[k]] : 0xffffffffu;
+        for (int k = 0; k < kMarkEdges; ++k) cur[k] = ok[k] ? bitmap[w[k]] : 0xffffffffu;
 #pragma unroll
-        for (int k = 0; k < kEdges; ++k)
+        for (int k = 0; k < kMarkEdges; ++k)
             if (!(cur[k] & bit[k]) && ok[k]) atomicOr(&bitmap[w[k]], bit[k]);
     }
     nbad = __reduce_add_sync(kFull, nbad);
     if ((threadIdx.x & 31) == 0 && nbad) atomicAdd(bad_count, (unsigned long long)nbad);
 }
 
+template <int WPT>
 __global__ void __launch_bounds__(kThreads)
 k_emit_b(const uint32_t* __restrict__ bitmap, uint64_t W, const GraphSeg* __restrict__ segs,
          const uint64_t* __restrict__ bm_off, uint32_t G, const uint32_t* __restrict__ chunk_base,
@@ -148,13 +152,13 @@ k_emit_b(const uint32_t* __restrict__ bitmap, uint64_t W, const GraphSeg* __rest
             blocks[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t w0 = (uint64_t)blockIdx.x * kChunk + (uint64_t)threadIdx.x * kWordsPerThread;
-    uint32_t x[kWordsPerThread];
+    const uint64_t w0 = (uint64_t)blockIdx.x * (kThreads * WPT) + (uint64_t)threadIdx.x * WPT;
+    uint32_t x[WPT];
 #pragma unroll
-    for (int k = 0; k < kWordsPerThread; ++k) x[k] = (w0 + k < W) ? bitmap[w0 + k] : 0u;
+    for (int k = 0; k < WPT; ++k) x[k] = (w0 + k < W) ? bitmap[w0 + k] : 0u;
     uint32_t mine = 0;
 #pragma unroll
-    for (int k = 0; k < kWordsPerThread; ++k) mine += __popc(x[k]);
+    for (int k = 0; k < WPT; ++k) mine += __popc(x[k]);
     uint32_t incl = mine;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -173,7 +177,7 @@ k_emit_b(const uint32_t* __restrict__ bitmap, uint64_t W, const GraphSeg* __rest
     uint64_t lw = w0 - s.bm_off;
     uint32_t rb = (uint32_t)(lw / s.wpr);
     uint32_t cw = (uint32_t)(lw - (uint64_t)rb * s.wpr);
-    for (int k = 0; k < kWordsPerThread; ++k) {
+    for (int k = 0; k < WPT; ++k) {
         const uint64_t w = w0 + k;
         if (w >= W) break;
         while (w >= bm_off[g + 1]) {  // next non-empty graph
@@ -261,7 +265,8 @@ __global__ void k_set_last_b(uint32_t* __restrict__ indptr, uint32_t R,
 
 int grid_for(int64_t work, int threads);
 int launch_tile_scan(uint32_t* per_tile, uint32_t ntiles, unsigned long long* total, cudaStream_t s);
-int launch_bitmap_count(const uint32_t* bitmap, uint64_t W, uint32_t* chunk_count, cudaStream_t s);
+int launch_bitmap_count(const uint32_t* bitmap, uint64_t W, uint64_t chunk_words, uint32_t* chunk_count,
+                        cudaStream_t s);
 
 }  // namespace btc200
 
@@ -341,18 +346,22 @@ static int batch_enqueue_tiles(btc_batch* b, const int32_t* d_src, const int32_t
     btc_bitbsr* g = &b->g;
     unsigned long long* meta = g->meta.as<unsigned long long>();
     const uint64_t words = b->h_bmoff[(size_t)b->num_graphs];
-    const size_t chunks = (size_t)((words + bt::kChunk - 1) / bt::kChunk);
+    const size_t chunks = (size_t)((words + bt::chunk_words(words) - 1) / bt::chunk_words(words));
     const GraphSeg* dsegs = b->segs.as<GraphSeg>();
     const int64_t* deoff = b->e_off.as<int64_t>();
     const uint32_t G = (uint32_t)b->num_graphs;
     const uint32_t rows = (uint32_t)g->n_row_blocks;
     const uint32_t vec4 = 4u * (uint32_t)(g->tile_cols / 32);
-    if (words)
-        bt::k_emit_b<<<(unsigned)chunks, bt::kThreads, 0, s>>>(
-            g->bitmap.as<uint32_t>(), words, dsegs, b->bm_off.as<uint64_t>(), G,
-            g->tile_base.as<uint32_t>(), g->prefix.as<uint2>(), g->indices.as<uint32_t>(),
-            g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(), meta + kMetaTiles, cap,
-            g->blocks.as<uint4>(), vec4);
+    if (words) {
+        auto emit = [&](auto kernel) {
+            kernel<<<(unsigned)chunks, bt::kThreads, 0, s>>>(
+                g->bitmap.as<uint32_t>(), words, dsegs, b->bm_off.as<uint64_t>(), G, g->tile_base.as<uint32_t>(),
+                g->prefix.as<uint2>(), g->indices.as<uint32_t>(), g->row_indices.as<uint32_t>(),
+                g->indptr.as<uint32_t>(), meta + kMetaTiles, cap, g->blocks.as<uint4>(), vec4);
+        };
+        if (bt::chunk_words(words) == bt::kThreads) emit(bt::k_emit_b<1>);
+        else emit(bt::k_emit_b<4>);
+    }
     bt::k_set_last_b<<<1, 1, 0, s>>>(g->indptr.as<uint32_t>(), rows, meta, cap);
     if (m > 0 && words) {
         const int egrid = grid_for((m + bt::kEdges - 1) / bt::kEdges, bt::kThreads);
@@ -383,7 +392,7 @@ static int batch_enqueue_mark(btc_batch* b, const int32_t* d_src, const int32_t*
     btc_bitbsr* g = &b->g;
     unsigned long long* meta = g->meta.as<unsigned long long>();
     const uint64_t words = b->h_bmoff[(size_t)b->num_graphs];
-    const size_t chunks = (size_t)((words + bt::kChunk - 1) / bt::kChunk);
+    const size_t chunks = (size_t)((words + bt::chunk_words(words) - 1) / bt::chunk_words(words));
     BTC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(unsigned long long) * kMetaSlots, s));
     if (!words) return BTC_OK;
     BTC_CUDA_TRY(cudaMemsetAsync(g->bitmap.ptr, 0, sizeof(uint32_t) * words, s));
@@ -398,7 +407,7 @@ static int batch_enqueue_mark(btc_batch* b, const int32_t* d_src, const int32_t*
                                                            b->e_off.as<int64_t>(), (uint32_t)b->num_graphs,
                                                            g->bitmap.as<uint32_t>(), meta + kMetaBad);
     }
-    BTC_TRY(launch_bitmap_count(g->bitmap.as<uint32_t>(), words, g->tile_base.as<uint32_t>(), s));
+    BTC_TRY(launch_bitmap_count(g->bitmap.as<uint32_t>(), words, bt::chunk_words(words), g->tile_base.as<uint32_t>(), s));
     BTC_TRY(launch_tile_scan(g->tile_base.as<uint32_t>(), (uint32_t)chunks, meta + kMetaTiles, s));
     return BTC_OK;
 }
@@ -531,7 +540,7 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
     }
 
     // ---- mark, count, scan; the tile count to size the arrays ----------------------
-    const size_t chunks = (size_t)((words + bt::kChunk - 1) / bt::kChunk);
+    const size_t chunks = (size_t)((words + bt::chunk_words(words) - 1) / bt::chunk_words(words));
     BTC_TRY(g->bitmap.reserve(sizeof(uint32_t) * (words ? words : 1)));
     BTC_TRY(g->prefix.reserve(sizeof(uint2) * (words ? words : 1)));
     BTC_TRY(g->tile_base.reserve(sizeof(uint32_t) * (chunks + 1)));

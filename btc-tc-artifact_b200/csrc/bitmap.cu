@@ -630,12 +630,14 @@ int launch_popcount_sum(int tile_cols, const uint32_t* blocks, uint64_t num_tile
 }  // namespace btc200
 
 namespace btc200 {
-// Popcount per 1024-word chunk (the batch builder's chunking, which does not follow
-// bitmap_chunks).
-int launch_bitmap_count(const uint32_t* bitmap, uint64_t W, uint32_t* chunk_count, cudaStream_t s)
+// Popcount per chunk of chunk_words words, 256 or 1,024 (the batch builder's chunking, which
+// does not follow bitmap_chunks).
+int launch_bitmap_count(const uint32_t* bitmap, uint64_t W, uint64_t chunk_words, uint32_t* chunk_count,
+                        cudaStream_t s)
 {
-    const uint64_t chunks = (W + bm::kThreads * 4 - 1) / (bm::kThreads * 4);
-    if (W) bm::k_bm_count<4><<<(unsigned)chunks, bm::kThreads, 0, s>>>(bitmap, W, chunk_count);
+    const unsigned chunks = (unsigned)((W + chunk_words - 1) / chunk_words);
+    if (W && chunk_words == bm::kThreads) bm::k_bm_count<1><<<chunks, bm::kThreads, 0, s>>>(bitmap, W, chunk_count);
+    else if (W) bm::k_bm_count<4><<<chunks, bm::kThreads, 0, s>>>(bitmap, W, chunk_count);
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 }  // namespace btc200
