@@ -282,7 +282,8 @@ struct btc_batch {
     std::vector<uint32_t> h_rowoff;
     std::vector<int32_t> h_nv;
     bool built = false;        // the geometry above belongs to a build that succeeded
-    bool row_store = false;    // the builds enqueue the row store (streaming count)
+    bool heavy = false;        // the builds make the row masks
+    bool row_store = false;    // ... and enqueue the row store (streaming count)
     uint32_t max_col_blocks = 0;  // 64-column blocks the widest graph's columns span
     bool pending = false;      // an enqueued rebuild's status is not known yet
     uint32_t pending_cap = 0;  // the tile capacity that rebuild ran against
@@ -376,7 +377,7 @@ static int batch_enqueue_tiles(btc_batch* b, const int32_t* d_src, const int32_t
     }
     BTC_TRY(launch_rowmask(g->tile_cols, g->blocks.as<uint32_t>(), cap, meta + kMetaTiles,
                            g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
-                           meta + kMetaRowMax, s, true, b->row_store));
+                           meta + kMetaRowMax, s, true, b->heavy));
     g->row_index = false;
     if (b->row_store)
         BTC_TRY(launch_rowstore(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
@@ -439,6 +440,7 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
         std::equal(num_vertices, num_vertices + G, b->h_nv.begin());
     if ((flags & BTC_BUILD_ASYNC) && !(flags & BTC_INPUT_ON_HOST) && same_geometry) {
         const uint32_t cap = batch_capacity(b);
+        if (stream_capturing(s)) g->captured = true;
         BTC_TRY(batch_enqueue_mark(b, src, dst, m, s));
         BTC_TRY(batch_enqueue_tiles(b, src, dst, m, cap, s));
         b->pending = true;
@@ -562,8 +564,9 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
     BTC_TRY(g->blocks.reserve(sizeof(uint32_t) * TW * (tiles ? tiles : 1)));
     BTC_TRY(g->rowmask.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
     // the streaming count's row store, when the union averages 8 or more tiles per row block
-    // (then it has at least 8 edges per row block) and there is the memory for it
-    b->row_store = rows > 0 && (uint64_t)tiles >= 8ull * rows && m < (int64_t)0xffffffffll &&
+    // (then it has at least 8 edges per row block), is not dense, and there is the memory for it
+    b->heavy = rows > 0 && (uint64_t)tiles >= 8ull * rows && m < (int64_t)0xffffffffll;
+    b->row_store = b->heavy && !dense_graph(tile_cols, m, (uint32_t)tiles, rows) &&
                    // (an enqueued rebuild may fill the arrays to their capacity)
                    reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * batch_capacity(b))) == BTC_OK;
     BTC_TRY(ensure_count_scratch(g));
@@ -652,7 +655,7 @@ int btc_batch_count(btc_batch* b, int tau, btc_stream_t stream, unsigned long lo
                                     g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), 0, cap, true, true,
                                     build_meta, count_grid_size(g->tile_cols), stream));
     } else {
-    if (b->row_store) ensure_row_index(g, build_meta ? build_meta + kMetaTiles : nullptr, cap, stream);
+    const bool index = b->heavy && ensure_row_index(g, build_meta ? build_meta + kMetaTiles : nullptr, cap, stream);
     BTC_TRY(launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                          g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(),
                          cap, g->n_row_blocks, tau, scr,
@@ -660,8 +663,8 @@ int btc_batch_count(btc_batch* b, int tau, btc_stream_t stream, unsigned long lo
                          g->rowmask.as<uint32_t>(), g->prefix.as<uint2>(), 0,
                          g->meta.as<unsigned long long>() + kMetaRowMax, 0, 0xffffffffu, build_meta,
                          g->num_tiles,
-                         g->row_index ? g->row_off.as<uint32_t>() : nullptr,
-                         g->row_index ? g->row_ent.as<uint2>() : nullptr, false,
+                         index ? g->row_off.as<uint32_t>() : nullptr,
+                         index ? g->row_ent.as<uint2>() : nullptr, false,
                          b->segs.as<GraphSeg>()));
     }
     if (h_counts) {

@@ -8,11 +8,12 @@
 //
 //   k_mark       one pass over the edges: orient (max,min), range-check, drop
 //                self-loops, set the cell bit (fire-and-forget atomicOr)
-//   k_bm_count_scan  popcount per 4096-word chunk; the last CTA to finish scans the
+//   k_bm_count_scan  popcount per chunk of words; the last CTA to finish scans the
 //                chunk counts into chunk bases and the tile total
 //   k_bm_emit    per word: exclusive tile prefix (kept for k_fill_bm), indices /
 //                row_indices of each set cell, indptr at row-block starts; each CTA
-//                zeroes its chunk's tiles, the last one writes indptr[R]
+//                zeroes its chunk's tiles
+//   k_set_last   indptr[R], the overflow flag and the host's status words
 //   k_fill_bm    second pass over the edges: tile = prefix[word] + popc(lower bits of
 //                the word); OR the edge's bit into the tile; where the count wants row
 //                masks (8 or more tiles per row block), the edge whose OR finds its tile
@@ -563,12 +564,11 @@ int bitmap_emit_and_fill(const BuildGeom& g, const int32_t* src, const int32_t* 
                          uint2* cellpp, uint32_t* indices, uint32_t* row_indices,
                          uint32_t* indptr, uint32_t* blocks, unsigned long long* meta,
                          uint32_t cap, unsigned long long* host_meta, cudaStream_t s,
-                         uint32_t* rowmask, bool row_store)
+                         uint32_t* rowmask, bool masks, bool row_store)
 {
     const unsigned long long* meta_tiles = meta + kMetaTiles;
-    // with a row store to come: masks whatever the tile count, and the store's pass finds the
-    // longest list
-    const bool always_masks = row_store;
+    // masks whatever the tile count; with a row store to come, its pass finds the longest list
+    const bool always_masks = masks;
     unsigned long long* row_max = row_store ? nullptr : meta + kMetaRowMax;
     const uint64_t wpr = bitmap_words_per_row(g);
     const uint64_t W = wpr * (uint64_t)g.n_row_blocks;
@@ -648,38 +648,23 @@ namespace bm {
 // word.  Words without a tile keep the zeros the caller wrote.
 __global__ void k_cells(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indices,
                         const uint32_t* __restrict__ row_indices, uint32_t cap,
-                        const unsigned long long* __restrict__ d_tiles, uint64_t wpr,
-                        const GraphSeg* __restrict__ segs, const uint32_t* __restrict__ graph_rows, uint32_t G,
-                        uint2* __restrict__ cellpp)
+                        const unsigned long long* __restrict__ d_tiles, uint64_t wpr, uint2* __restrict__ cellpp)
 {
     const unsigned long long T = d_tiles ? *d_tiles : cap;
     if (T > cap) return;
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < T;
          t += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t I = row_indices[t];
-        uint64_t row = (uint64_t)I * wpr;
-        uint32_t cb0 = 0;
-        if (segs) {
-            uint32_t lo = 0, hi = G;
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (graph_rows[mid] <= I) lo = mid;
-                else hi = mid;
-            }
-            const GraphSeg sg = segs[lo];
-            row = sg.bm_off + (uint64_t)(I - sg.row_off) * sg.wpr;
-            cb0 = sg.cb_lo;
-        }
-        const uint32_t w = (indices[t] - cb0) >> 5;
-        if (t > indptr[I] && ((indices[t - 1] - cb0) >> 5) == w) continue;
+        const uint32_t w = indices[t] >> 5;
+        if (t > indptr[I] && (indices[t - 1] >> 5) == w) continue;
         const uint64_t end = indptr[I + 1];
         uint32_t bits = 0;
         for (uint64_t x = t; x < end; ++x) {
-            const uint32_t k = indices[x] - cb0;
+            const uint32_t k = indices[x];
             if ((k >> 5) != w) break;
             bits |= 1u << (k & 31u);
         }
-        cellpp[row + w] = make_uint2(bits, (uint32_t)t);
+        cellpp[(uint64_t)I * wpr + w] = make_uint2(bits, (uint32_t)t);
     }
 }
 
@@ -727,16 +712,43 @@ __global__ void k_rowmask(const uint32_t* __restrict__ blocks, uint32_t cap,
         rowmask[t] = m;
     }
 }
+
+// Bits and number of up to 4,096 tiles, evenly spaced, to out[0] and out[1] (host memory).
+__global__ void __launch_bounds__(1024) k_sample_bits(const uint4* __restrict__ blocks, uint32_t T, uint32_t vec,
+                                                      volatile unsigned long long* __restrict__ out)
+{
+    __shared__ uint32_t s_bits;
+    if (threadIdx.x == 0) s_bits = 0;
+    __syncthreads();
+    const uint32_t step = (T + 4095u) / 4096u, N = (T + step - 1) / step;
+    uint32_t bits = 0;
+    for (uint32_t i = threadIdx.x; i < N * vec; i += 1024) {
+        const uint4 v = blocks[(uint64_t)(i / vec) * step * vec + i % vec];
+        bits += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+    }
+    bits = __reduce_add_sync(kFull, bits);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_bits, bits);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        out[0] = s_bits;
+        out[1] = N;
+    }
+}
 }  // namespace bm
 
+int launch_sample_bits(int tile_cols, const uint32_t* blocks, uint32_t T, unsigned long long* d_host, cudaStream_t s)
+{
+    bm::k_sample_bits<<<1, 1024, 0, s>>>(reinterpret_cast<const uint4*>(blocks), T, 4u * (uint32_t)(tile_cols / 32), d_host);
+    return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+}
+
 int launch_cells(const uint32_t* indptr, const uint32_t* indices, const uint32_t* row_indices, uint32_t cap,
-                 const unsigned long long* d_tiles, uint64_t words, uint64_t wpr, const GraphSeg* segs,
-                 const uint32_t* graph_rows, uint32_t G, uint2* cellpp, cudaStream_t s)
+                 const unsigned long long* d_tiles, uint64_t words, uint64_t wpr, uint2* cellpp,
+                 cudaStream_t s)
 {
     if (cudaMemsetAsync(cellpp, 0, sizeof(uint2) * words, s) != cudaSuccess) return BTC_E_CUDA;
     if (cap)
-        bm::k_cells<<<grid_for(cap, 256), 256, 0, s>>>(indptr, indices, row_indices, cap, d_tiles, wpr, segs,
-                                                       graph_rows, G, cellpp);
+        bm::k_cells<<<grid_for(cap, 256), 256, 0, s>>>(indptr, indices, row_indices, cap, d_tiles, wpr, cellpp);
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 

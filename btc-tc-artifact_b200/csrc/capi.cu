@@ -30,7 +30,7 @@ int bitmap_mark_and_count(const BuildGeom&, const int32_t*, const int32_t*, int6
 int bitmap_emit_and_fill(const BuildGeom&, const int32_t*, const int32_t*, int64_t, const int32_t*,
                          const uint32_t*, const uint32_t*, uint2*, uint32_t*, uint32_t*, uint32_t*,
                          uint32_t*, unsigned long long*, uint32_t, unsigned long long*,
-                         cudaStream_t, uint32_t*, bool);
+                         cudaStream_t, uint32_t*, bool, bool);
 int launch_popcount_sum(int, const uint32_t*, uint64_t, unsigned long long*, cudaStream_t);
 int launch_indptr(const uint32_t*, uint32_t, int32_t, uint32_t*, cudaStream_t);
 int launch_density(int, const uint32_t*, uint32_t, unsigned long long*, cudaStream_t);
@@ -67,6 +67,21 @@ using namespace btc200;
 // Measured on sm_100a (policy.cu, the tau sweep): 16x128 tiles switch to the binary
 // tensor core above 1024 bits (half full), 16x32 tiles above 64 (the reference's value).
 int default_tau(int tile_cols) { return tile_cols == 128 ? 1024 : 64; }
+
+// A row's walk costs the streaming count its neighbours' entries, however full they are; the
+// row-wise kernel's tensor cores take a dense tile's 16 rows at once.  Measured on communities
+// of 512 to 8,192 vertices, density 0.05 to 1, with and without edges between them (count
+// only, streaming / row-wise, by edges per tile and tiles per row block).  16x32: 149 and 16.5
+// 32 / 25 us, 99 and 16.5 44 / 46; 200 and 82 474 / 429, 160 and 82 376 / 429; 508 and 64 1.87 /
+// 1.16 ms, 305 and 65 1.10 / 1.18; 56 and 117 0.47 / 1.64 ms, 12 and 212 0.24 / 1.68: the line
+// is below every pair where the row-wise kernel wins.  16x128: 866 and 8.5 196 / 336 us, 1,156
+// and 8.5 256 / 219, 596 and 16.5 0.58 / 1.51 ms, 1,191 and 16.5 1.10 / 1.05.
+bool dense_graph(int tile_cols, int64_t m, uint32_t T, int64_t R)
+{
+    if (T == 0 || R <= 0) return false;
+    const double per_tile = (double)m / (double)T;
+    return tile_cols == 128 ? per_tile > 896.0 : per_tile > 64.0 + (double)T / (double)R;
+}
 
 // Degree-ordered edge lists from this length on are grouped by row block (group.cu) instead
 // of marked and filled edge by edge: the tiles of a power-law graph this large do not stay
@@ -135,7 +150,8 @@ struct BuildPlan {
     bool degree;
     uint64_t bm_words;
     uint32_t cap;  // > 0: the post-count steps run against this tile capacity
-    bool row_store = false;  // build the streaming count's row store (rowstore.cu)
+    bool heavy = false;      // the graph can average 8 tiles per row block: make its row masks
+    bool row_store = false;  // ... and the streaming count's row store (rowstore.cu)
 };
 
 // Only a graph with at least 8 edges per row block can average 8 tiles per row block (every
@@ -185,36 +201,62 @@ static int enqueue_row_store(btc_bitbsr* g, const unsigned long long* d_tiles, u
                            cap, by_degree, g->meta.as<unsigned long long>(), row_store_of(g), s);
 }
 
-void ensure_cells(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, uint64_t words, uint64_t wpr,
-                  const GraphSeg* segs, const uint32_t* graph_rows, uint32_t G, cudaStream_t s)
+bool stream_capturing(cudaStream_t s)
 {
-    if (g->cells || 4 * words > 32ull * (uint64_t)g->input_edges + (64ull << 20) || g->prefix.reserve(sizeof(uint2) * (words ? words : 1)) != BTC_OK)
-        return;
-    g->cells = launch_cells(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->row_indices.as<uint32_t>(),
-                            cap, d_tiles, words, wpr, segs, graph_rows, G, g->prefix.as<uint2>(), s) == BTC_OK;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;  // (the legacy stream beside a global capture: allocate nothing)
+    }
+    return st != cudaStreamCaptureStatusNone;
 }
 
-void ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s)
+// A buffer of at least `bytes`, without an allocation while a stream is capturing.
+static bool room(DevBuf& b, size_t bytes, bool capturing)
 {
-    if (g->row_index) return;
+    return capturing ? b.ptr && b.bytes >= bytes : b.reserve(bytes) == BTC_OK;
+}
+
+bool ensure_cells(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, uint64_t words, uint64_t wpr,
+                  cudaStream_t s)
+{
+    const bool capturing = stream_capturing(s), keep = !capturing && !d_tiles && !g->captured;
+    if (g->cells && (keep || !g->cells_lazy)) return true;
+    if (4 * words > 32ull * (uint64_t)g->input_edges + (64ull << 20) ||
+        !room(g->prefix, sizeof(uint2) * (words ? words : 1), capturing))
+        return false;
+    const bool made = launch_cells(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->row_indices.as<uint32_t>(),
+                                   cap, d_tiles, words, wpr, g->prefix.as<uint2>(), s) == BTC_OK;
+    if (keep) g->cells = g->cells_lazy = made;
+    return made;
+}
+
+bool ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s)
+{
+    const bool capturing = stream_capturing(s), keep = !capturing && !d_tiles && !g->captured;
+    if (g->row_index && keep) return true;
     const uint64_t R = (uint64_t)g->n_row_blocks;
     const int64_t m = g->input_edges;
     const uint64_t ent = std::min<uint64_t>((uint64_t)m, 16ull * cap);
-    if (!row_store_possible(m, g->n_row_blocks) || g->row_off.reserve(sizeof(uint32_t) * (16 * R + 1)) ||
-        g->row_ent.reserve(sizeof(uint2) * (size_t)ent) || g->row_tot.reserve(sizeof(uint32_t) * R) ||
-        g->row_bsum.reserve(sizeof(unsigned long long) +
-                            sizeof(uint32_t) * ((size_t)ri_scan_blocks((uint32_t)R) + 1)))
-        return;
+    if (!row_store_possible(m, g->n_row_blocks) ||
+        !room(g->row_off, sizeof(uint32_t) * (16 * R + 1), capturing) ||
+        !room(g->row_ent, sizeof(uint2) * (size_t)ent, capturing) ||
+        !room(g->row_tot, sizeof(uint32_t) * R, capturing) ||
+        !room(g->row_bsum, sizeof(unsigned long long) + sizeof(uint32_t) * ((size_t)ri_scan_blocks((uint32_t)R) + 1),
+              capturing))
+        return false;
     unsigned long long* total = g->row_bsum.as<unsigned long long>();
-    g->row_index = launch_rowindex(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->n_row_blocks,
-                                   g->rowmask.as<uint32_t>(), d_tiles, cap, g->row_tot.as<uint32_t>(),
-                                   reinterpret_cast<uint32_t*>(total + 1), total, g->row_off.as<uint32_t>(),
-                                   g->row_ent.as<uint2>(), g->row_ent.bytes / sizeof(uint2), s) == BTC_OK;
+    const bool made = launch_rowindex(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->n_row_blocks,
+                                      g->rowmask.as<uint32_t>(), d_tiles, cap, g->row_tot.as<uint32_t>(),
+                                      reinterpret_cast<uint32_t*>(total + 1), total, g->row_off.as<uint32_t>(),
+                                      g->row_ent.as<uint2>(), g->row_ent.bytes / sizeof(uint2), s) == BTC_OK;
+    if (keep) g->row_index = made;
+    return made;
 }
 
 static int enqueue_group_write(btc_bitbsr* g, const BuildPlan& P, uint32_t cap, cudaStream_t s)
 {
-    return group_write(P.geom.tile_cols, P.col_blocks, P.m, (uint32_t)P.geom.n_row_blocks, nullptr, 0,
+    return group_write(P.geom.tile_cols, P.col_blocks, P.m, (uint32_t)P.geom.n_row_blocks,
                        g->keys0.as<uint32_t>(), g->tile_base.as<uint32_t>(), g->indptr.as<uint32_t>(),
                        g->meta.as<unsigned long long>(), cap, g->indices.as<uint32_t>(),
                        g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(), g->rowmask.as<uint32_t>(),
@@ -277,15 +319,15 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
                                          g->prefix.as<uint2>(), g->indices.as<uint32_t>(),
                                          g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(),
                                          g->blocks.as<uint32_t>(), meta, P.cap, g->d_hmeta, s,
-                                         g->rowmask.as<uint32_t>(), P.row_store));
+                                         g->rowmask.as<uint32_t>(), P.heavy, P.row_store));
             // (the fill pass set the row masks, or found the longest row-block list)
             if (P.row_store) BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s));
         }
     } else if (P.use_group) {
         const uint32_t R = (uint32_t)geom.n_row_blocks;
         uint32_t* scratch = g->tile_base.as<uint32_t>();
-        BTC_TRY(group_edges(P.d_src, P.d_dst, P.m, P.n, P.n, rank, nullptr, nullptr, 0, nullptr, geom.tile_cols,
-                            P.col_blocks, k0, k1, g->keys0.as<uint32_t>(), scratch, g->indptr.as<uint32_t>(),
+        BTC_TRY(group_edges(P.d_src, P.d_dst, P.m, P.n, rank, geom.tile_cols, P.col_blocks,
+                            k0, k1, g->keys0.as<uint32_t>(), scratch, g->indptr.as<uint32_t>(),
                             scratch + group_scratch_words(R), meta, s));
         if (P.cap) {
             BTC_TRY(launch_finish_tiles(g->indptr.as<uint32_t>(), geom.n_row_blocks, meta, P.cap, g->d_hmeta, s));
@@ -326,7 +368,7 @@ static void build_key(const btc_bitbsr* g, const BuildPlan& P, BuildGraphKey* k)
     k->m = P.m;
     k->n = P.n;
     k->tile_cols = P.geom.tile_cols;
-    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.use_group ? 0x40000000u : 0u);
+    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.heavy ? 0x20000000u : 0u) | (P.use_group ? 0x40000000u : 0u);
     k->cap = P.cap;
 }
 
@@ -408,6 +450,9 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     const bool prev_light = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks &&
                             g->num_tiles > 0 &&
                             (uint64_t)g->num_tiles < 8ull * (uint64_t)geom.n_row_blocks;
+    // ... and whether it is dense, which the row store does not help
+    const bool prev_dense = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks &&
+                            dense_graph(tile_cols, m, g->num_tiles, geom.n_row_blocks);
     g->tile_cols = tile_cols;
     g->n = n;
     g->n_row_blocks = geom.n_row_blocks;
@@ -457,7 +502,8 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         if (P.use_group) P.use_bitmap = false;
     }
     g->cells = P.use_bitmap;
-    g->row_store = g->row_index = false;
+    g->heavy = g->row_store = g->row_index = g->cells_lazy = false;
+    if ((flags & BTC_BUILD_ASYNC) && stream_capturing(s)) g->captured = true;
     size_t key_cap = P.use_bitmap || P.use_group ? 0 : (size_t)m;
     if (P.degree && (size_t)n > key_cap) key_cap = (size_t)n;
     if (key_cap) {
@@ -529,8 +575,10 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         // tile-wise); should this graph average more after all, the count takes the
         // tile-wise kernel, which needs no store.  So does a graph without the memory for it.
         // (A build by one launch decides when it knows the tiles.)
-        P.row_store = !small && !tiles_only && P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light &&
+        P.heavy = !small && !tiles_only && P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light;
+        P.row_store = P.heavy && !prev_dense &&
                       reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * P.cap)) == BTC_OK;
+        g->heavy = P.heavy;
         g->row_store = P.row_store;
     }
 
@@ -559,8 +607,9 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
             if (st2 == BTC_E_CAPACITY)
                 return build_into(g, src, dst, m, n, tile_cols, flags, s, tiles_only, false);
             if (st2 != BTC_OK) return st2;
-            g->row_store = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
-                           (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks &&
+            g->heavy = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
+                       (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks;
+            g->row_store = g->heavy && !dense_graph(tile_cols, m, g->num_tiles, geom.n_row_blocks) &&
                            reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * g->num_tiles)) == BTC_OK;
             if (g->row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, false, s));
             return BTC_OK;
@@ -584,10 +633,11 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     BTC_TRY(g->row_indices.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
     BTC_TRY(g->blocks.reserve(sizeof(uint32_t) * TW * (tiles ? tiles : 1)));
     BTC_TRY(g->rowmask.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
-    // the tile count is known here: the row store exactly when the graph averages 8 or more
-    // tiles per row block
-    P.row_store = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
-                  (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks &&
+    // the tile count is known here: row masks exactly when the graph averages 8 or more tiles
+    // per row block, the row store when it is not dense besides
+    P.heavy = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
+              (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks;
+    P.row_store = P.heavy && !dense_graph(tile_cols, m, g->num_tiles, geom.n_row_blocks) &&
                   reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * tiles)) == BTC_OK;
     if (P.use_bitmap) {
         BTC_TRY(bitmap_emit_and_fill(geom, P.d_src, P.d_dst, m, P.degree ? g->rank.as<int32_t>() : nullptr,
@@ -595,7 +645,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
                                      g->prefix.as<uint2>(), g->indices.as<uint32_t>(),
                                      g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(),
                                      g->blocks.as<uint32_t>(), meta, (uint32_t)tiles, nullptr, s,
-                                     g->rowmask.as<uint32_t>(), P.row_store));
+                                     g->rowmask.as<uint32_t>(), P.heavy, P.row_store));
     } else if (P.use_group) {
         BTC_TRY(launch_finish_tiles(g->indptr.as<uint32_t>(), geom.n_row_blocks, meta, (uint32_t)tiles, nullptr, s));
         BTC_TRY(enqueue_group_write(g, P, (uint32_t)tiles, s));
@@ -615,6 +665,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
                                g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
                                meta + kMetaRowMax, s, !have_masks));
     if (P.row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, P.degree, s));
+    g->heavy = P.heavy;
     g->row_store = P.row_store;
     return BTC_OK;
 }
@@ -642,26 +693,28 @@ int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_o
     const bool dense = (uint64_t)g->input_edges * 2 > (uint64_t)tau * (uint64_t)g->num_tiles;
     const bool whole = tile_begin == 0 && tile_end == 0xffffffffu;
     // A caller's lower tau asks for the tensor cores, which only the tile kernels use.
-    if (g->row_store && tau >= default_tau(g->tile_cols) && !(dense && g->tile_cols == 128))
+    if (g->row_store && tau >= default_tau(g->tile_cols) &&
+        !dense_graph(g->tile_cols, g->input_edges, g->num_tiles, g->n_row_blocks))
         return launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks, g->tile_cols, g->n_row_blocks,
                                    ((uint32_t)g->n + 63) / 64, scr, nullptr, 0, nullptr,
                                    g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), tile_begin,
                                    std::min(tile_end, cap), whole, true, build_meta, count_grid_size(g->tile_cols), s);
     const uint64_t wpr = bitmap_words_per_row(make_geom(g->n, g->tile_cols));
-    if (g->row_store) {
+    bool cells = g->cells && !g->cells_lazy, index = false;
+    if (g->heavy) {
         const unsigned long long* d_tiles = build_meta ? build_meta + kMetaTiles : nullptr;
-        ensure_cells(g, d_tiles, cap, wpr * (uint64_t)g->n_row_blocks, wpr, nullptr, nullptr, 0, s);
-        if (g->cells) ensure_row_index(g, d_tiles, cap, s);
+        cells = ensure_cells(g, d_tiles, cap, wpr * (uint64_t)g->n_row_blocks, wpr, s);
+        index = cells && ensure_row_index(g, d_tiles, cap, s);
     }
     return launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                         g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(),
                         cap, g->n_row_blocks, tau, scr, s,
                         nullptr, 0, nullptr, g->rowmask.as<uint32_t>(),
-                        g->cells ? g->prefix.as<uint2>() : nullptr, wpr,
+                        cells ? g->prefix.as<uint2>() : nullptr, wpr,
                         g->meta.as<unsigned long long>() + kMetaRowMax, tile_begin, tile_end,
                         build_meta, g->num_tiles,
-                        g->row_index ? g->row_off.as<uint32_t>() : nullptr,
-                        g->row_index ? g->row_ent.as<uint2>() : nullptr, dense);
+                        index ? g->row_off.as<uint32_t>() : nullptr,
+                        index ? g->row_ent.as<uint2>() : nullptr, dense);
 }
 
 int resolve_build(btc_bitbsr* g)
@@ -988,6 +1041,27 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
     return BTC_OK;
 }
 
+// Whether the tile-wise kernel's tensor cores count a struct faster: dense 16x32 tiles, told
+// from a sample (a struct does not know its edges).  At 16x128 streaming wins at any density
+// (the complete graph on 4,096 vertices: 0.43 ms against 1.18).
+static bool struct_dense(const btc_bcsr_device* b, int tile_cols)
+{
+    if (tile_cols != 32) return false;
+    unsigned long long* h = host_slot_alloc();
+    void* d = nullptr;
+    bool dense = false;
+    if (h && cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess &&
+        launch_sample_bits(tile_cols, b->blocks, b->num_blocks, static_cast<unsigned long long*>(d), nullptr) == BTC_OK) {
+        if (cudaStreamSynchronize(nullptr) != cudaSuccess) return false;  // (the slot is given up)
+        dense = h[1] && dense_graph(tile_cols, (int64_t)((double)h[0] / (double)h[1] * (double)b->num_blocks), b->num_blocks,
+                                    b->n_row_blocks);
+    } else {
+        cudaGetLastError();
+    }
+    host_slot_free(h);
+    return dense;
+}
+
 static int count_struct(btc_bcsr_device* b, int tile_cols, float* kernel_ms,
                         unsigned long long* out)
 {
@@ -1015,9 +1089,8 @@ static int count_struct(btc_bcsr_device* b, int tile_cols, float* kernel_ms,
                      reinterpret_cast<unsigned long long*>(ss.done[dev].as<char>() + 8), b->result,
                      nullptr};
     int st = BTC_E_NOMEM;
-    // (tiles averaging more bits than default tau's half cannot be told from a struct: dense
-    // ones stream too)
-    if (b->n_row_blocks > 0 && (uint64_t)b->num_blocks >= 8ull * (uint64_t)b->n_row_blocks)
+    if (b->n_row_blocks > 0 && (uint64_t)b->num_blocks >= 8ull * (uint64_t)b->n_row_blocks &&
+        !struct_dense(b, tile_cols))
         st = count_struct_stream(b, tile_cols, scr);
     if (st == BTC_E_NOMEM)
         st = launch_count(tile_cols, b->indptr, b->indices, b->row_indices, b->blocks, b->num_blocks,

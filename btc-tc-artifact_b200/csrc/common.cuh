@@ -311,23 +311,24 @@ int launch_rowindex(const uint32_t* indptr, const uint32_t* indices, int32_t n_r
 // The grouped builder (group.cu).
 bool group_possible(int64_t n, uint64_t col_blocks);
 size_t group_scratch_words(uint32_t R);
-int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, int64_t rows,
-                const int32_t* rank, const GraphSeg* segs, const int64_t* e_off, uint32_t G,
-                const uint32_t* graph_rows, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
+int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
+                const int32_t* rank, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
                 uint64_t* grouped, uint32_t* edges, uint32_t* scratch, uint32_t* indptr, uint32_t* bsum,
                 unsigned long long* meta, cudaStream_t s);
-int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R, const uint32_t* graph_rows, uint32_t G,
+int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
                 const uint32_t* edges, const uint32_t* scratch, const uint32_t* indptr,
                 const unsigned long long* meta, uint32_t cap, uint32_t* indices, uint32_t* row_indices,
                 uint32_t* blocks, uint32_t* rowmask, uint32_t tiles_hint, cudaStream_t s);
 // indptr[R] = the tile count, the overflow flag and the host's status slots (bitmap.cu).
 int launch_finish_tiles(uint32_t* indptr, int32_t R, unsigned long long* meta, uint32_t cap,
                         unsigned long long* host_meta, cudaStream_t s);
+// Bits and number of up to 4,096 evenly spaced tiles (T > 0), to two words of mapped host memory.
+int launch_sample_bits(int tile_cols, const uint32_t* blocks, uint32_t T, unsigned long long* d_host, cudaStream_t s);
 // The (cell word, tile prefix) pairs of `words` words from the tiles, for a count that wants
 // them after a build that made none.
 int launch_cells(const uint32_t* indptr, const uint32_t* indices, const uint32_t* row_indices, uint32_t cap,
-                 const unsigned long long* d_tiles, uint64_t words, uint64_t wpr, const GraphSeg* segs,
-                 const uint32_t* graph_rows, uint32_t G, uint2* cellpp, cudaStream_t s);
+                 const unsigned long long* d_tiles, uint64_t words, uint64_t wpr, uint2* cellpp,
+                 cudaStream_t s);
 
 // Id locality of an edge list for the tile policy (policy.cu): sampled share of edges
 // with |u - v| < 128 over the share uniform ids would give.  e_off / nv (nullable): the

@@ -154,7 +154,17 @@ cudaError_t dev_alloc(void** ptr, size_t bytes)
 {
     cudaMemPool_t pool;
     cudaStream_t stream;
-    if (bytes >= kDirectBytes || !pool_for_current_device(&pool, &stream)) return cudaMalloc(ptr, bytes);
+    const bool pooled = pool_for_current_device(&pool, &stream);
+    if (bytes >= kDirectBytes || !pooled) {
+        cudaError_t e = cudaMalloc(ptr, bytes);
+        if (e == cudaErrorMemoryAllocation && pooled) {
+            // (the memory that the pool keeps may be what is missing)
+            cudaGetLastError();
+            cudaMemPoolTrimTo(pool, 0);
+            e = cudaMalloc(ptr, bytes);
+        }
+        return e;
+    }
     cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, pool, stream);
     if (e == cudaErrorMemoryAllocation) {
         // give the kept memory back and try once more

@@ -9,7 +9,7 @@
 //
 //   k_orient      edge -> (row, column) with row > column, range check, self-loops dropped;
 //                 counts the edges of each bucket of rows (up to kBuckets buckets).  With a
-//                 degree rank or a batch's vertex offsets the pair is stored, so that the
+//                 degree rank the pair is stored, so that the
 //                 random rank look-ups happen once.
 //   k_bucket_scan bucket starts
 //   k_scatter     tiles of 8192 edges sorted by bucket in shared memory, written in runs to
@@ -43,19 +43,7 @@ constexpr uint64_t kNone = ~0ull;
 // ---- orientation -----------------------------------------------------------------------
 constexpr int kOThreads = 512;
 
-// last g in [0, G) with off[g] <= x
-__device__ __forceinline__ uint32_t last_le(const int64_t* __restrict__ off, uint32_t G, int64_t x)
-{
-    uint32_t lo = 0, hi = G;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (off[mid] <= x) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
-__device__ __forceinline__ uint64_t pair_of(int32_t u, int32_t v, int32_t n, uint32_t vbase,
+__device__ __forceinline__ uint64_t pair_of(int32_t u, int32_t v, int32_t n,
                                             const int32_t* __restrict__ rank, bool& bad)
 {
     bad = (u < 0) | (v < 0) | (u >= n) | (v >= n);
@@ -65,15 +53,13 @@ __device__ __forceinline__ uint64_t pair_of(int32_t u, int32_t v, int32_t n, uin
         v = rank[v];
     }
     if (u == v) return kNone;
-    return ((uint64_t)(vbase + (uint32_t)max(u, v)) << 32) | (vbase + (uint32_t)min(u, v));
+    return ((uint64_t)(uint32_t)max(u, v) << 32) | (uint32_t)min(u, v);
 }
 
 // pairs (nullable): the oriented pairs, kNone for what is dropped.
-// segs (nullable): a batch, edge i of graph last_le(e_off, G, i).
 __global__ void __launch_bounds__(kOThreads)
 k_orient(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m, int32_t n,
-         const int32_t* __restrict__ rank, const GraphSeg* __restrict__ segs,
-         const int64_t* __restrict__ e_off, uint32_t G, int shift, uint64_t* __restrict__ pairs,
+         const int32_t* __restrict__ rank, int shift, uint64_t* __restrict__ pairs,
          uint32_t* __restrict__ hist, unsigned long long* __restrict__ bad_count)
 {
     __shared__ uint32_t s_hist[kBuckets];
@@ -81,11 +67,6 @@ k_orient(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64
     __syncthreads();
     constexpr int U = 8;
     uint32_t nbad = 0;
-    // a thread's edges are kOThreads apart within one run of U * kOThreads: neighbours in a
-    // batch mostly share a graph, so its search starts from the last one found
-    uint32_t g = 0;
-    int64_t g_lo = 0, g_hi = segs ? 0 : m;
-    GraphSeg sg{0u, n, 0u, 0u, 0u, 0u, 0ull};
     for (int64_t i0 = (int64_t)blockIdx.x * (U * kOThreads) + threadIdx.x; i0 < m + threadIdx.x;
          i0 += (int64_t)gridDim.x * (U * kOThreads)) {
         int32_t u[U], v[U];
@@ -99,14 +80,8 @@ k_orient(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64
 #pragma unroll
         for (int k = 0; k < U; ++k) {
             const int64_t i = i0 + k * kOThreads;
-            if (segs && i < m && (i < g_lo || i >= g_hi)) {
-                g = last_le(e_off, G, i);
-                g_lo = e_off[g];
-                g_hi = e_off[g + 1];
-                sg = segs[g];
-            }
             bool bad;
-            p[k] = pair_of(u[k], v[k], sg.n, sg.vbase, rank, bad);
+            p[k] = pair_of(u[k], v[k], n, rank, bad);
             if (i >= m) p[k] = kNone;
             else nbad += bad;
         }
@@ -172,7 +147,7 @@ k_scatter(const uint64_t* __restrict__ pairs, const int32_t* __restrict__ src, c
             const int64_t i = base + k * kSThreads;
             const int32_t u = i < m ? src[i] : 0, v = i < m ? dst[i] : 0;
             bool bad;
-            p[k] = pair_of(u, v, n, 0u, nullptr, bad);
+            p[k] = pair_of(u, v, n, nullptr, bad);
             if (i >= m) p[k] = kNone;
         }
     }
@@ -324,26 +299,10 @@ k_rb_scatter(const uint64_t* __restrict__ in, const uint32_t* __restrict__ d_m, 
 constexpr uint32_t kTileBytes = 32768;  // tile buffer, at most
 constexpr uint32_t kDirect = 1u << 18;  // looks at an edge from which a row block is written directly
 
-// First column block row block I can hold: its graph's first (0 for a single graph).
-template <int LOG2C>
-__device__ __forceinline__ uint32_t first_col_block(const uint32_t* __restrict__ graph_rows, uint32_t G,
-                                                    uint32_t I)
-{
-    if (!graph_rows) return 0u;
-    uint32_t lo = 0, hi = G;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (graph_rows[mid] <= I) lo = mid;
-        else hi = mid;
-    }
-    return (16u * graph_rows[lo]) >> LOG2C;
-}
-
 template <int LOG2C, int kTThreads>
 __global__ void __launch_bounds__(kTThreads)
 k_count_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ rb_end, uint32_t R,
-              uint32_t words, const uint32_t* __restrict__ graph_rows, uint32_t G,
-              uint32_t* __restrict__ indptr)
+              uint32_t words, uint32_t* __restrict__ indptr)
 {
     extern __shared__ uint32_t s_bm[];
     __shared__ uint32_t s_red[kTThreads / kWarp];
@@ -351,10 +310,9 @@ k_count_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
     __syncthreads();
     for (uint32_t I = blockIdx.x; I < R; I += gridDim.x) {
         const uint32_t e0 = I ? rb_end[I - 1] : 0u, e1 = rb_end[I];
-        const uint32_t cb0 = first_col_block<LOG2C>(graph_rows, G, I);
         uint32_t mine = 0;
         for (uint32_t e = e0 + threadIdx.x; e < e1; e += kTThreads) {
-            const uint32_t cb = ((edges[e] & 0x0fffffffu) >> LOG2C) - cb0;
+            const uint32_t cb = (edges[e] & 0x0fffffffu) >> LOG2C;
             const uint32_t bit = 1u << (cb & 31u);
             // read first: most edges of a dense row block find their bit set
             if (!(*(volatile uint32_t*)&s_bm[cb >> 5] & bit)) mine += !(atomicOr(&s_bm[cb >> 5], bit) & bit);
@@ -368,7 +326,7 @@ k_count_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
             indptr[I] = t;
         }
         for (uint32_t e = e0 + threadIdx.x; e < e1; e += kTThreads)
-            s_bm[(((edges[e] & 0x0fffffffu) >> LOG2C) - cb0) >> 5] = 0;
+            s_bm[((edges[e] & 0x0fffffffu) >> LOG2C) >> 5] = 0;
         __syncthreads();
     }
 }
@@ -376,8 +334,7 @@ k_count_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
 template <int LOG2C, int kTThreads>
 __global__ void __launch_bounds__(kTThreads)
 k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ rb_end, uint32_t R,
-              uint32_t words, const uint32_t* __restrict__ graph_rows, uint32_t G,
-              const uint32_t* __restrict__ indptr, const unsigned long long* __restrict__ d_tiles, uint32_t cap,
+              uint32_t words, const uint32_t* __restrict__ indptr, const unsigned long long* __restrict__ d_tiles, uint32_t cap,
               uint32_t* __restrict__ indices, uint32_t* __restrict__ row_indices, uint4* __restrict__ blocks,
               uint32_t* __restrict__ rowmask, uint32_t NT)
 {
@@ -430,7 +387,6 @@ k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
             hold(ne0, ne1);
             continue;
         }
-        const uint32_t cb0 = first_col_block<LOG2C>(graph_rows, G, I);
         auto each_edge = [&](auto f) {
 #pragma unroll
             for (int k = 0; k < kHeld; ++k)
@@ -438,7 +394,7 @@ k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
             for (uint32_t e = e0 + kHeld * kTThreads + threadIdx.x; e < e1; e += kTThreads) f(edges[e]);
         };
         each_edge([&](uint32_t x) {
-            const uint32_t cb = ((x & 0x0fffffffu) >> LOG2C) - cb0;
+            const uint32_t cb = (x & 0x0fffffffu) >> LOG2C;
             const uint32_t bit = 1u << (cb & 31u);
             if (!(*(volatile uint32_t*)&s_bm[cb >> 5] & bit)) atomicOr(&s_bm[cb >> 5], bit);
         });
@@ -447,7 +403,7 @@ k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
         __syncthreads();
         // tile numbers: a popcount prefix over the words that can hold a bit (columns stay
         // below the row block's last row), a run of words per thread
-        const uint32_t used = min(words, (((16u * I + 15u) >> LOG2C) - cb0) / 32u + 1u);
+        const uint32_t used = min(words, ((16u * I + 15u) >> LOG2C) / 32u + 1u);
         const uint32_t per = (used + 4 * kTThreads - 1) / (4 * kTThreads);  // in fours
         uint4* bm4 = reinterpret_cast<uint4*>(s_bm);
         uint4* pre4 = reinterpret_cast<uint4*>(s_pre);
@@ -472,7 +428,7 @@ k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
         // One edge: its tile's number, the tile's word (ORed where `tile` says) and mask.
         auto place = [&](uint32_t x, uint32_t tb, uint32_t nb, uint32_t* tile, uint32_t* mask) {
             const uint32_t c = x & 0x0fffffffu;
-            const uint32_t cb = (c >> LOG2C) - cb0;
+            const uint32_t cb = c >> LOG2C;
             const uint32_t t = s_pre[cb >> 5] + __popc(s_bm[cb >> 5] & ((1u << (cb & 31u)) - 1u)) - tb;
             if (t >= nb) return;
             const uint32_t cl = c & (C - 1), r = x >> 28;
@@ -480,7 +436,7 @@ k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
             // that finds the tile's mask empty names the tile
             if (atomicOr(&tile[(size_t)t * TW + r * WPR + (cl >> 5)], 1u << (cl & 31u)) == 0u &&
                 atomicOr(&mask[t], 1u << (r + (C == 128 ? (cl & 64u) / 4u : 0u))) == 0u) {
-                indices[t0 + tb + t] = cb0 + cb;
+                indices[t0 + tb + t] = cb;
                 row_indices[t0 + tb + t] = I;
             }
         };
@@ -558,8 +514,7 @@ static int bucket_shift(int64_t rows)
 // one, k_count_tiles 93 / 65), four above (R-MAT scale 22 in degree order averages 256).
 static int row_block_threads(int64_t m, uint32_t R) { return m <= 96ll * R ? 32 : 128; }
 
-// Whether the grouped builder takes a matrix of n columns (a batch: the union) whose row
-// blocks span at most col_blocks column blocks each.
+// Whether the grouped builder takes a matrix of n columns in col_blocks column blocks.
 bool group_possible(int64_t n, uint64_t col_blocks)
 {
     return n > 0 && n <= (1ll << 28) && (col_blocks + 31) / 32 <= gp::kMaxWords;
@@ -568,29 +523,28 @@ bool group_possible(int64_t n, uint64_t col_blocks)
 size_t group_scratch_words(uint32_t R) { return 3 * (size_t)gp::kBuckets + 1 + (size_t)R + 3; }
 
 // The edges grouped by row block and the row blocks' tile counts scanned into indptr.
-// pairs: m uint64 (only written with rank or segs); grouped: m uint64 of scratch whose
+// pairs: m uint64 (only written with rank); grouped: m uint64 of scratch whose
 // contents end up in `edges` (m words, may share memory with pairs); scratch:
 // group_scratch_words(R); bsum: scan scratch of R words.  Writes meta[kMetaBad] and
 // meta[kMetaTiles].
-int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, int64_t rows,
-                const int32_t* rank, const GraphSeg* segs, const int64_t* e_off, uint32_t G,
-                const uint32_t* graph_rows, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
+int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
+                const int32_t* rank, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
                 uint64_t* grouped, uint32_t* edges, uint32_t* scratch, uint32_t* indptr, uint32_t* bsum,
                 unsigned long long* meta, cudaStream_t s)
 {
-    const uint32_t R = (uint32_t)((rows + 15) / 16);
+    const uint32_t R = (uint32_t)(((int64_t)n + 15) / 16);
     uint32_t* hist = scratch;
     uint32_t* cursor = scratch + gp::kBuckets;
     uint32_t* base = cursor + gp::kBuckets;
     uint32_t* rb_end = base + gp::kBuckets + 1;  // offsets at first, then (moved on) ends
     unsigned long long* sum = reinterpret_cast<unsigned long long*>(scratch + (group_scratch_words(R) - 2) / 2 * 2);
-    const int shift = bucket_shift(rows);
+    const int shift = bucket_shift(n);
     if (cudaMemsetAsync(hist, 0, sizeof(uint32_t) * gp::kBuckets, s) != cudaSuccess) return BTC_E_CUDA;
-    const bool store = rank != nullptr || segs != nullptr;
+    const bool store = rank != nullptr;
     const int ogrid = (int)std::min<int64_t>((m + 8 * gp::kOThreads - 1) / (8 * gp::kOThreads),
                                              4 * (int64_t)device_sm_count());
     if (m > 0)
-        gp::k_orient<<<ogrid, gp::kOThreads, 0, s>>>(src, dst, m, n, rank, segs, e_off, G, shift,
+        gp::k_orient<<<ogrid, gp::kOThreads, 0, s>>>(src, dst, m, n, rank, shift,
                                                      store ? pairs : nullptr, hist, meta + kMetaBad);
     gp::k_bucket_scan<<<1, 1024, 0, s>>>(hist, base, cursor);
     static std::atomic<bool> scatter_ok[64];
@@ -608,7 +562,7 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, in
     const int threads = row_block_threads(m, R);
     const uint32_t grid = std::min<uint32_t>(R, 32u * device_sm_count() * (128 / threads));
     auto count = [&](auto kernel) {
-        kernel<<<grid, threads, 4 * words, s>>>(edges, rb_end, R, words, graph_rows, G, indptr);
+        kernel<<<grid, threads, 4 * words, s>>>(edges, rb_end, R, words, indptr);
     };
     if (tile_cols == 128)
         threads == 32 ? count(gp::k_count_tiles<7, 32>) : count(gp::k_count_tiles<7, 128>);
@@ -619,7 +573,7 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, in
 
 // Tiles, indices, row_indices and row masks from the grouped edges (indptr[R] set), against
 // `cap` tiles: nothing when meta[kMetaTiles] is above it.
-int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R, const uint32_t* graph_rows, uint32_t G,
+int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
                 const uint32_t* edges, const uint32_t* scratch, const uint32_t* indptr,
                 const unsigned long long* meta, uint32_t cap, uint32_t* indices, uint32_t* row_indices,
                 uint32_t* blocks, uint32_t* rowmask, uint32_t tiles_hint, cudaStream_t s)
@@ -640,7 +594,7 @@ int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R, const
     const uint32_t grid = std::min<uint32_t>(R, 32u * device_sm_count() * (128 / threads));
     auto write = [&](auto kernel, int which) {
         if (!gp::allow_smem(kernel, most, ok[which])) return BTC_E_CUDA;
-        kernel<<<grid, threads, smem, s>>>(edges, rb_end, R, words, graph_rows, G, indptr, meta + kMetaTiles, cap,
+        kernel<<<grid, threads, smem, s>>>(edges, rb_end, R, words, indptr, meta + kMetaTiles, cap,
                                            indices, row_indices, reinterpret_cast<uint4*>(blocks), rowmask, NT);
         return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
     };

@@ -34,8 +34,11 @@ struct btc_bitbsr {
     // build workspace
     btc200::DevBuf in_src, in_dst, keys0, keys1, sort_scratch, tile_base, meta, deg, rank, bitmap, prefix;
     bool cells = false;      // prefix holds the (cell word, tile prefix) pairs of the last build
-    bool row_store = false;  // the last build made the row store (its graph can be heavy)
-    bool row_index = false;  // the row index of the last build's graph has been enqueued
+    bool heavy = false;      // the last build's graph can average 8 tiles per row block: it has row masks
+    bool row_store = false;  // ... and the last build made the row store
+    bool row_index = false;  // the row index of the last build's graph has been made
+    bool cells_lazy = false; // ... and the pairs by a count, not by the build
+    bool captured = false;   // a caller's CUDA graph holds a rebuild, whose replays this handle does not see
     // count scratch
     btc200::DevBuf partials, done;
     btc200::PolicyWords policy;
@@ -119,15 +122,21 @@ btc200::RowStore row_store_of(const btc_bitbsr* g);
 // Reserves the row store of a graph with at most `entries` entries (BTC_E_NOMEM: the caller
 // goes on without one); no allocation when the buffers already hold it.
 int reserve_row_store(btc_bitbsr* g, uint64_t entries);
-// The row index of the row-wise count kernel, enqueued on s if this build's is not yet there.
-// Without the memory for it the kernel walks whole row blocks instead.
-// The cell pairs, enqueued on s if the last build made none (`words` of them; segs and
-// graph_rows for a batch).  Without the memory for them the count goes tile-wise.
-void ensure_cells(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, uint64_t words, uint64_t wpr,
-                  const btc200::GraphSeg* segs, const uint32_t* graph_rows, uint32_t G, cudaStream_t s);
-void ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s);
+// What the row-wise count kernel reads beside the tiles, enqueued on s where the last build
+// and the counts since have not made it: the cell pairs (`words` of them) and the row index.
+// True when this count may use them; without the memory for the pairs it goes tile-wise, and
+// without the index the kernel walks whole row blocks.  While s is capturing nothing is
+// allocated; and what a replay may find changed (a capturing s, a build still pending, a
+// captured rebuild) is made again by every count.
+bool ensure_cells(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, uint64_t words, uint64_t wpr,
+                  cudaStream_t s);
+bool ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s);
+bool stream_capturing(cudaStream_t s);
 
 int default_tau(int tile_cols);
+// Whether a graph of m edges in T tiles and R row blocks is dense enough for the row-wise
+// kernel's tensor cores to count it faster than the streaming count.
+bool dense_graph(int tile_cols, int64_t m, uint32_t T, int64_t R);
 int ensure_count_scratch(btc_bitbsr* g);
 // Counts tiles [tile_begin, tile_end) (clamped to the tile count) into g->result and,
 // when d_out2 is given, *d_out2.

@@ -96,3 +96,102 @@ def test_a_store_that_outgrows_its_first_build():
         g.rebuild(torch.from_numpy(s).cuda(), torch.from_numpy(d).cuda(), n, 32)
         assert g.count() == O.tc_merge(rp, col)
     g.free()
+
+
+def _captured(fn):
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        fn(s)
+    return graph
+
+
+@pytest.mark.parametrize("warm", [False, True])
+@pytest.mark.parametrize("deg", [False, True])
+def test_a_captured_lower_tau_count_makes_its_own_index(warm, deg):
+    """What a lower tau's kernels read beside the tiles is made by the first such count: not
+    allocated while capturing, and not taken for made by the handle when only a graph has it
+    (deg: grouped edges, no cell pairs from the build)."""
+    from btc_b200 import BitBSR
+    from oracle import oracle as O
+    n = 40000 if deg else 5000
+    s, d = _spread(n, (1 << 22) if deg else 150000, 40, 3)
+    rp, col, _ = O.lower_csr(s, d, n)
+    want = O.tc_merge(rp, col)
+    g = BitBSR(torch.from_numpy(s).cuda(), torch.from_numpy(d).cuda(), n, 32, orient_degree=deg)
+    if warm:
+        assert g.count(tau=4) == want
+    out = torch.zeros(1, dtype=torch.int64, device="cuda")
+    graph = _captured(lambda st: g.count_async(tau=4, stream=st, d_out=out.data_ptr()))
+    assert g.count(tau=4) == want  # before any replay
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        assert int(out.item()) == want
+    assert g.count(tau=4) == want
+    del graph
+    g.free()
+
+
+def test_a_replayed_batch_rebuild_leaves_no_stale_index():
+    """A captured rebuild is replayed on other edges of the same tiles (every id's last bit
+    flipped: the same triangles in other rows): a lower tau's count after it finds the index
+    of the new edges, whether a count before it made one or not."""
+    from btc_b200 import Batch
+    from oracle import oracle as O
+    gs, want = [], []
+    for k in range(3):
+        n = 2048 + 512 * k
+        s, d = _spread(n, 60000, 30, 20 + k)
+        rp, col, _ = O.lower_csr(s, d, n)
+        want.append(O.tc_merge(rp, col))
+        gs.append((s, d, n))
+    src, dst, off, nv = Batch.concat(gs)
+    d_src, d_dst = torch.from_numpy(src).cuda(), torch.from_numpy(dst).cuda()
+    args = dict(src=d_src, dst=d_dst, offsets=off, num_vertices=nv, tile_cols=32)
+    b = Batch(**args)
+    assert b.count(tau=4).tolist() == want
+    out = torch.zeros(len(gs), dtype=torch.int64, device="cuda")
+
+    def step(st):
+        b.rebuild(**args, stream=st, asynchronous=True)
+        b.count_async(out.data_ptr(), stream=st)
+
+    graph = _captured(step)
+    for _ in range(3):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert out.cpu().tolist() == want
+        assert b.count(tau=4).tolist() == want and b.count(tau=4).tolist() == want
+        d_src.bitwise_xor_(1)
+        d_dst.bitwise_xor_(1)
+    del graph
+    b.free()
+
+
+@pytest.mark.parametrize("tile_cols,n", [(32, 600), (32, 3000), (128, 2304)])
+def test_dense_graphs_take_the_tensor_cores_and_change_back(tile_cols, n):
+    """A dense graph makes no row store; rebuilds of the same geometry that turn sparse and
+    dense again are counted by whatever kernel the last tile count predicts."""
+    from btc_b200 import Batch, BitBSR, graphs as G
+    from oracle import oracle as O
+    ks, kd, _ = G.complete(n)
+    dense = torch.from_numpy(ks).cuda(), torch.from_numpy(kd).cuda()
+    want_d = n * (n - 1) * (n - 2) // 6
+    s, d = _spread(n, 40 * n, 20, 5)
+    rp, col, _ = O.lower_csr(s, d, n)
+    want_s = O.tc_merge(rp, col)
+    sparse = torch.from_numpy(s).cuda(), torch.from_numpy(d).cuda()
+    g = BitBSR(*dense, n, tile_cols)
+    assert g.count() == want_d and g.count(tau=0) == want_d
+    for asynchronous in (False, True):
+        for e, want in ((sparse, want_s), (sparse, want_s), (dense, want_d), (dense, want_d)):
+            g.rebuild(*e, n, tile_cols, asynchronous=asynchronous)
+            assert g.count() == want and g.count() == want
+            b = g.partition(3)
+            assert sum(int(g.count_tiles(x, y)) for x, y in zip(b[:-1], b[1:])) == want
+    g.free()
+    b = Batch([(ks, kd, n), (ks, kd, n)], tile_cols=tile_cols)
+    assert b.count().tolist() == [want_d, want_d]
+    b.free()
