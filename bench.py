@@ -182,24 +182,32 @@ class ClockSampler:
 
 
 def launches_per_step(n: int, tile_cols: int, orient_degree: bool, m: int, tiles: int) -> int:
-    """Kernels the engine launches per build + count (csrc/capi.cu build_into): the
-    bitmap builder (mark, chunk count, scan, emit, last indptr, fill) when the cell
-    bitmap is small enough, with the row index (five kernels) for graphs averaging 8 or
-    more tiles per row block, else the radix builder; plus the degree relabel and count."""
+    """Kernels the engine launches per enqueued build + count (csrc/capi.cu build_into): the
+    grouped builder for degree-ordered graphs of 2^22 edges or more, the bitmap builder for
+    other graphs with a small enough cell bitmap, and the row store of the streaming count
+    for graphs averaging 8 or more tiles per row block; plus the degree relabel and count."""
     R = (n + 15) // 16
     ncb = (n + tile_cols - 1) // tile_cols
     bm_bytes = 4 * R * ((ncb + 31) // 32)
-    if bm_bytes <= (4 << 30) and bm_bytes <= 32 * m + (64 << 20):
+    bitmap = bm_bytes <= (4 << 30) and bm_bytes <= 32 * m + (64 << 20)
+    group = n <= (1 << 28) and (ncb + 31) // 32 <= 4096 and (not bitmap or
+                                                             (orient_degree and m >= 1 << 22))
+    store = m >= 8 * R and tiles >= 8 * R
+    if group:
+        # orient, bucket scan, scatter, row-block count, scan (3), row-block scatter, tile
+        # count, scan (3), last indptr, tiles; the longest row block where no store finds it
+        k = 14 + (0 if store else 1)
+    elif bitmap:
         k = 4  # mark, chunk count + scan, emit (+ zero tiles, last indptr), fill
-        if m >= 8 * R and tiles >= 8 * R:
-            k += 5  # row index: totals, scan (reduce, scan, apply), fill
     else:
         t_bits = max(R - 1, 0).bit_length() + max(ncb - 1, 0).bit_length()
-        k = 1 + 3 * (-(-t_bits // 8)) + 2 + 1 + 1  # keys, sort, segment (2), fill, indptr
+        k = 1 + 3 * (-(-t_bits // 8)) + 2 + 1 + 1 + 1  # keys, sort, segment (2), fill, indptr, masks
+    if store:
+        k += 1 if orient_degree or R <= 32 * 148 else 2  # row store (long row blocks apart)
     if orient_degree:
         db = min(32, max(1, (2 * m).bit_length()))
         k += 1 + 1 + 1 + 3 * (-(-db // 8)) + 1  # degree, rank keys, set count, sort, scatter
-    return k + 1 + 1  # row-occupancy masks, count
+    return k + 1  # count
 
 
 def cpu_reference(rowptr, col, m_lower, budget_s=10.0):
@@ -955,7 +963,7 @@ def main():
     # capture of the same graph family when the full size is too large to capture).  Its
     # warp-instruction rate against the SMs' (4 schedulers per SM, one warp instruction
     # each per cycle, at the median SM clock sampled during the timed region) is the
-    # issue side of the bound; dependent-load latency is the other.
+    # issue side of the bound; the L1's shared-memory wavefronts are the other.
     prof = count_profile(args.workload, tile)
     traffic = int(prof["dram_bytes_per_launch"]) if prof else None
     warp_inst = float(prof["warp_instructions_per_launch"]) if prof else None

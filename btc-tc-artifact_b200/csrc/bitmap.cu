@@ -12,8 +12,8 @@
 //                chunk counts into chunk bases and the tile total
 //   k_bm_emit    per word: exclusive tile prefix (kept for k_fill_bm), indices /
 //                row_indices of each set cell, indptr at row-block starts; each CTA
-//                zeroes its chunk's tiles
-//   k_set_last   indptr[R], the overflow flag and the host's status words
+//                zeroes its chunk's tiles, the last one writes indptr[R] and the host's
+//                status words
 //   k_fill_bm    second pass over the edges: tile = prefix[word] + popc(lower bits of
 //                the word); OR the edge's bit into the tile; where the count wants row
 //                masks (8 or more tiles per row block), the edge whose OR finds its tile

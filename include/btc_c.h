@@ -201,7 +201,7 @@ BTC_API int btc_build_bitbsr(const int32_t* src, const int32_t* dst, int64_t m, 
  * when they are large enough (no allocation in steady state).
  *
  * BTC_BUILD_ASYNC (no counterpart in the reference): when the handle already holds tile
- * arrays from an earlier build and the cell-bitmap builder applies, the whole build is
+ * arrays from an earlier build and the radix builder does not apply, the whole build is
  * enqueued on `stream` against the arrays' capacity and the call returns without
  * waiting (otherwise the flag is ignored and the call waits as usual).  The inputs must
  * stay valid until `stream` has run the build.  A count enqueued after it reads the
@@ -214,7 +214,12 @@ BTC_API int btc_rebuild_bitbsr(btc_bitbsr* g, const int32_t* src, const int32_t*
                        int32_t n, int tile_cols, uint32_t flags, btc_stream_t stream);
 
 /* Counts the triangles of a handle: enqueues the count on `stream`, waits, and
- * writes *out_count.  tau: dense/sparse switch (BTC_TAU_DEFAULT for the engine's).
+ * writes *out_count.  tau: dense/sparse switch (BTC_TAU_DEFAULT for the engine's): a tile
+ * whose popcount exceeds it takes the tensor cores where a tile kernel counts.  At the
+ * default or above, graphs averaging 8 or more tiles per row block and not dense are counted
+ * from per-vertex rows instead; a lower tau keeps them on the tile kernels, whose index the
+ * first such count after a build makes (allocated then; never while `stream` is capturing,
+ * where the count goes without it).
  * kernel_ms (nullable): event time of the count kernel alone.  Replaces
  * count_triangles_16x{128,32}_adaptive (tc_16x128_adaptive.h:12, tc_16x32_adaptive.h:14). */
 BTC_API int btc_count(btc_bitbsr* g, int tau, btc_stream_t stream, unsigned long long* out_count,
@@ -236,8 +241,9 @@ BTC_API int btc_count(btc_bitbsr* g, int tau, btc_stream_t stream, unsigned long
  * context, and the next call repeats that lookup, so it too should come before any
  * capture.  All calls share the one array: calls whose kernels overlap on the GPU
  * (different streams, or several host threads) race and give wrong counts, so order
- * them.  It always runs the count's light variant (it has no per-tile row masks), so on
- * power-law graphs, where btc_count picks the heavy variant, it is exact but slower.
+ * them.  It always runs the tile-wise kernel's light variant (it has neither row masks nor
+ * per-vertex rows), so on power-law graphs, which btc_count counts from their rows, it is
+ * exact but slower.
  * Stream-ordered; does not wait for the result.  tau as in btc_count. */
 BTC_API int btc_count_bcsr_noalloc(const btc_bcsr_device* bcsr, int tile_cols, int tau,
                                    btc_stream_t stream, unsigned long long* d_out);
