@@ -485,6 +485,9 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     P.use_bitmap = !(flags & BTC_BUILD_RADIX) && bm_bytes <= (4ull << 30) &&
                    bm_bytes <= 32ull * (uint64_t)m + (64ull << 20);
     small = small && P.use_bitmap;
+    // An enqueued build is one that the bitmap takes, whichever builder then runs; on any other
+    // graph the call waits, and grows the arrays where they are too small.
+    const bool enqueued = (flags & BTC_BUILD_ASYNC) && P.use_bitmap;
     // Large edge lists are grouped by row block instead of marked and filled edge by edge
     // (see kGroupEdges), and so is what the bitmap does not take.
     P.col_blocks = (uint64_t)geom.n_col_blocks;
@@ -585,7 +588,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     uint64_t* sorted = nullptr;
     if (P.cap) {
         // repeated identical asynchronous rebuilds of device input replay a CUDA graph
-        const bool graphed = (flags & BTC_BUILD_ASYNC) && !(flags & BTC_INPUT_ON_HOST) &&
+        const bool graphed = enqueued && !(flags & BTC_INPUT_ON_HOST) &&
                              launch_build_graph(g, P, s);
         if (!graphed) BTC_TRY(enqueue_build(g, P, &sorted, s));
         // the build's status and tile count are in h_meta once the stream has run it
@@ -595,7 +598,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         BTC_CUDA_TRY(cudaEventRecord(g->meta_event, s));
         g->pending = true;
         g->pending_cap = P.cap;
-        if (flags & BTC_BUILD_ASYNC) return BTC_OK;  // resolved by the next wait
+        if (enqueued) return BTC_OK;  // resolved by the next wait
         const int st2 = resolve_build(g);
         if (small) {
             if (st2 == BTC_E_CUDA) return st2;

@@ -201,7 +201,8 @@ BTC_API int btc_build_bitbsr(const int32_t* src, const int32_t* dst, int64_t m, 
  * when they are large enough (no allocation in steady state).
  *
  * BTC_BUILD_ASYNC (no counterpart in the reference): when the handle already holds tile
- * arrays from an earlier build and the radix builder does not apply, the whole build is
+ * arrays from an earlier build and the graph is one the cell-bitmap builder takes (larger
+ * ones are grouped by row block instead, under the same rule), the whole build is
  * enqueued on `stream` against the arrays' capacity and the call returns without
  * waiting (otherwise the flag is ignored and the call waits as usual).  The inputs must
  * stay valid until `stream` has run the build.  A count enqueued after it reads the
