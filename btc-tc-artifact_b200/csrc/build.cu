@@ -14,6 +14,8 @@
 //   k_density        tile popcount histogram
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace btc200 {
 
 BuildGeom make_geom(int32_t n, int tile_cols)
@@ -54,13 +56,17 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v)
 // another counts in global memory as before.  4096 slots (32 KB of keys and counters):
 // at R-MAT s22 a CTA's table keeps ~17% of its increments (2048 slots: ~10%) and the
 // kernel takes 1.32 ms against 1.48.
-constexpr int kDegSlots = 4096;
+#ifndef DEG_SLOTS
+#define DEG_SLOTS 26624
+#define DEG_THREADS 1024
+#define DEG_U 4
+#endif
 constexpr uint32_t kDegFree = 0xffffffffu;
 
-__device__ __forceinline__ void degree_add(uint32_t v, uint32_t* __restrict__ keys,
-                                           uint32_t* __restrict__ cnt, uint32_t* __restrict__ deg)
+template <uint32_t kSlots>
+__device__ __forceinline__ void degree_add(uint32_t v, uint32_t* keys, uint32_t* cnt, uint32_t* __restrict__ deg)
 {
-    const uint32_t slot = (v * 0x9E3779B1u) >> (32 - 12);  // kDegSlots = 2^12
+    const uint32_t slot = __umulhi(v * 0x9E3779B1u, kSlots);
     uint32_t k = keys[slot];
     if (k == kDegFree) {
         const uint32_t prev = atomicCAS(&keys[slot], kDegFree, v);
@@ -70,26 +76,37 @@ __device__ __forceinline__ void degree_add(uint32_t v, uint32_t* __restrict__ ke
     else atomicAdd(&deg[v], 1u);
 }
 
-__global__ void __launch_bounds__(256)
+template <uint32_t kSlots, int kDThreads, int U>
+__global__ void __launch_bounds__(kDThreads)
 k_degree(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
          int64_t m, int32_t n, uint32_t* __restrict__ deg)
 {
-    static_assert(kDegSlots == 1 << 12, "degree_add hashes to 12 bits");
-    __shared__ uint32_t keys[kDegSlots], cnt[kDegSlots];
-    for (int i = threadIdx.x; i < kDegSlots; i += blockDim.x) {
+    extern __shared__ uint32_t s_deg[];
+    uint32_t* keys = s_deg;
+    uint32_t* cnt = s_deg + kSlots;
+    for (uint32_t i = threadIdx.x; i < kSlots; i += kDThreads) {
         keys[i] = kDegFree;
         cnt[i] = 0;
     }
     __syncthreads();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t u = src[i], v = dst[i];
-        if (u == v || u < 0 || v < 0 || u >= n || v >= n) continue;
-        degree_add((uint32_t)u, keys, cnt, deg);
-        degree_add((uint32_t)v, keys, cnt, deg);
+    const int64_t stride = (int64_t)gridDim.x * kDThreads;
+    for (int64_t i0 = (int64_t)blockIdx.x * kDThreads + threadIdx.x; i0 < m; i0 += U * stride) {
+        int32_t u[U], v[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int64_t i = i0 + k * stride;
+            u[k] = i < m ? src[i] : 0;  // (a pair of equal ids counts nothing)
+            v[k] = i < m ? dst[i] : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            if (u[k] == v[k] || u[k] < 0 || v[k] < 0 || u[k] >= n || v[k] >= n) continue;
+            degree_add<kSlots>((uint32_t)u[k], keys, cnt, deg);
+            degree_add<kSlots>((uint32_t)v[k], keys, cnt, deg);
+        }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kDegSlots; i += blockDim.x)
+    for (uint32_t i = threadIdx.x; i < kSlots; i += kDThreads)
         if (keys[i] != kDegFree && cnt[i]) atomicAdd(&deg[keys[i]], cnt[i]);
 }
 
@@ -365,7 +382,14 @@ int grid_for(int64_t work, int threads)
 int launch_degree(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, uint32_t* deg,
                   cudaStream_t s)
 {
-    if (m > 0) build_kernels::k_degree<<<grid_for(m, 256), 256, 0, s>>>(src, dst, m, n, deg);
+    if (m > 0) {
+        auto kernel = build_kernels::k_degree<DEG_SLOTS, DEG_THREADS, DEG_U>;
+        const int smem = 8 * DEG_SLOTS;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return BTC_E_CUDA;
+        const int64_t per = 232448 / (smem + 1024);
+        const int grid = (int)std::min<int64_t>((m + DEG_THREADS - 1) / DEG_THREADS, std::min<int64_t>(per, 2048 / DEG_THREADS) * device_sm_count());
+        kernel<<<grid, DEG_THREADS, smem, s>>>(src, dst, m, n, deg);
+    }
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 
