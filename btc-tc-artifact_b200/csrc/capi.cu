@@ -997,16 +997,19 @@ StructScratch& struct_scratch()
 // The streaming count of a struct whose row blocks average 8 or more tiles: the row masks
 // and the row store are made for this call, which costs a pass over the tiles (R-MAT scale
 // 18 in natural order, 16x128: 0.3 ms) and saves the tile-wise kernel's searches (22 ms).
-// BTC_E_NOMEM before anything is counted: the caller takes the tile-wise kernel.
+// BTC_E_NOMEM where there is no memory for them, or the tiles are not what they take
+// (launch_rowstore_check): the caller takes the tile-wise kernel.
 static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScratch scr)
 {
     struct Scratch {
         DevBuf rowmask, off, key, bits, first, meta;
+        unsigned long long* host = nullptr;
         bool idle = false;
         ~Scratch()
         {
             if (!idle && cudaDeviceSynchronize() != cudaSuccess) return;  // (given up: see DevBuf)
             for (DevBuf* d : {&rowmask, &off, &key, &bits, &first, &meta}) d->release_idle();
+            host_slot_free(host);
         }
     } w;
     const uint32_t T = b->num_blocks;
@@ -1015,6 +1018,13 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
     BTC_TRY(w.meta.reserve(sizeof(unsigned long long) * kMetaSlots));
     unsigned long long* meta = w.meta.as<unsigned long long>();
     BTC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(unsigned long long) * kMetaSlots, nullptr));
+    // a struct that the store is not made for is found out beside the counting: the count kernel
+    // then does nothing (as after a failed build), and the host learns it from the wait it has
+    if (!(w.host = host_slot_alloc())) return BTC_E_NOMEM;
+    void* d_host = nullptr;
+    BTC_CUDA_TRY(cudaHostGetDevicePointer(&d_host, w.host, 0));
+    BTC_TRY(launch_rowstore_check(tile_cols, b->indices, b->row_indices, T, b->n_row_blocks, meta + kMetaOverflow,
+                                  static_cast<unsigned long long*>(d_host), nullptr));
     BTC_TRY(launch_rowmask(tile_cols, b->blocks, T, nullptr, b->indptr, b->n_row_blocks,
                            w.rowmask.as<uint32_t>(), meta + kMetaRowMax, nullptr));
     // one entry per mask bit at most; counted (a wait) where 16 or 32 per tile is too much
@@ -1037,11 +1047,11 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
                             w.rowmask.as<uint32_t>(), nullptr, T, false, meta, rs, nullptr));
     BTC_TRY(launch_count_stream(rs, meta + kMetaRowChunks, tile_cols, b->n_row_blocks,
                                 ((uint32_t)b->n_row_blocks * 16u + 63) / 64, scr, nullptr, 0, nullptr,
-                                b->row_indices, b->indices, 0, T, true, false, nullptr,
+                                b->row_indices, b->indices, 0, T, true, false, meta,
                                 count_grid_size(tile_cols), nullptr));
     BTC_CUDA_TRY(cudaStreamSynchronize(nullptr));
     w.idle = true;
-    return BTC_OK;
+    return *static_cast<volatile unsigned long long*>(w.host) ? BTC_E_NOMEM : BTC_OK;
 }
 
 // Whether the tile-wise kernel's tensor cores count a struct faster: dense 16x32 tiles, told

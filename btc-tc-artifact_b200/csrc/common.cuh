@@ -274,13 +274,19 @@ inline uint64_t row_store_chunks(uint64_t entries, uint64_t R)
     return kRowRun + (entries + rows * (kRowChunk - 1)) / kRowChunk + blocks * (kRowRun - 1);
 }
 
-// Enqueues the row store of a Bit-BSR whose row masks exist (T = *d_tiles tiles, bounded by
-// cap, or cap when d_tiles is null; nothing when T > cap).  by_degree: the ids are in
-// descending-degree order.  meta:
-// the build's metadata slots (kMetaRowChunks zero: it counts the chunks handed out); also
-// raises meta[kMetaRowMax] to the most tiles in one row block.
+// Sets *bad and *d_host (a mapped host word) when a Bit-BSR that the engine did not build is not
+// one the row store and its count take: they are sized by 16 R columns (the count's table, the
+// 16-bit keys) and need ascending column blocks.  A tile whose first column is at or past 16 R
+// (a slab of rows of a wider matrix) is for the tile-wise kernel.
+int launch_rowstore_check(int tile_cols, const uint32_t* indices, const uint32_t* row_indices, uint32_t T,
+                          int32_t n_row_blocks, unsigned long long* bad, unsigned long long* d_host,
+                          cudaStream_t s);
 // *out += the set bits of mask[0, n).
 int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* out, cudaStream_t s);
+// Enqueues the row store of a Bit-BSR whose row masks exist (T = *d_tiles tiles, bounded by
+// cap, or cap when d_tiles is null; nothing when T > cap).  by_degree: the ids are in
+// descending-degree order.  meta: the build's metadata slots (kMetaRowChunks zero: it counts the
+// chunks handed out); also raises meta[kMetaRowMax] to the most tiles in one row block.
 int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indices, const uint32_t* blocks,
                     int32_t n_row_blocks, const uint32_t* rowmask, const unsigned long long* d_tiles,
                     uint32_t cap, bool by_degree, unsigned long long* meta, const RowStore& out,

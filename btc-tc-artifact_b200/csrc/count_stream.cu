@@ -40,7 +40,8 @@ constexpr int kPastWords = 64;
 static_assert(kPastWords == 2 * kWarp, "a lane ranks two words");
 static_assert(kGroup == 8 && kIdCap % (kGroups * kBatch) == 0, "a walk's rounds are whole");
 
-// Tables of fewer than 1,024 slots are for graphs whose rows they always hold.
+// Tables of fewer than 1,024 slots are for graphs whose rows they always hold (the engine's own
+// builds, and structs that launch_rowstore_check has passed).
 template <int W>
 constexpr bool kPastTable = W >= 1024;
 
@@ -238,10 +239,11 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
         uint32_t inside = 0;  // entries in the table
         auto put = [&](uint32_t slot, uint32_t x, uint32_t y) {
             if ((x | y) == 0u) return;
-            if (!kPastTable<W> || slot < (uint32_t)W) {
+            // (a small table's rows lie inside it: their store was checked or built so)
+            if (slot < (uint32_t)W) {
                 s.tab[slot] = make_uint2(x, y);
                 ++inside;
-            } else {
+            } else if (kPastTable<W>) {
                 const uint32_t pb = (slot - (uint32_t)W) % (32u * kPastWords);
                 atomicOr(&s.past[pb / 32], 1u << (pb & 31u));
             }

@@ -282,6 +282,25 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
     if (w == 0 && lane == 0 && longest) atomicMax(&meta[kMetaRowMax], (unsigned long long)longest);
 }
 
+// Raises *bad (and the host's word) where a caller's tiles are not what the store and its count
+// are sized by: column blocks ascending within a row block and below `limit`.
+__global__ void k_rs_check(const uint32_t* __restrict__ indices, const uint32_t* __restrict__ row_indices,
+                           uint32_t T, uint32_t limit, unsigned long long* __restrict__ bad,
+                           volatile unsigned long long* __restrict__ host_bad)
+{
+    bool ok = true;
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < T;
+         t += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t K = indices[t];
+        ok &= K < limit;
+        if (t > 0 && row_indices[t] == row_indices[t - 1]) ok &= indices[t - 1] < K;
+    }
+    if (!ok) {
+        *bad = 1ull;
+        *host_bad = 1ull;
+    }
+}
+
 __global__ void k_mask_popcount(const uint32_t* __restrict__ mask, uint32_t n,
                                 unsigned long long* __restrict__ out)
 {
@@ -294,6 +313,17 @@ __global__ void k_mask_popcount(const uint32_t* __restrict__ mask, uint32_t n,
 }
 
 }  // namespace rs
+
+int launch_rowstore_check(int tile_cols, const uint32_t* indices, const uint32_t* row_indices, uint32_t T,
+                          int32_t n_row_blocks, unsigned long long* bad, unsigned long long* d_host,
+                          cudaStream_t s)
+{
+    const uint64_t limit = (16ull * (uint64_t)n_row_blocks + tile_cols - 1) / tile_cols;
+    if (T)
+        rs::k_rs_check<<<std::min<uint32_t>((T + 255) / 256, 4u * device_sm_count()), 256, 0, s>>>(
+            indices, row_indices, T, (uint32_t)limit, bad, d_host);
+    return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+}
 
 int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* out, cudaStream_t s)
 {
