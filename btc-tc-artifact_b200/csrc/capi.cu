@@ -947,18 +947,8 @@ int btc_convert_coo_to_bcsr_16x32_gpu(btc_bcsr_device* b, const int32_t* d_rows,
 void btc_bcsr_free(btc_bcsr_device* b)
 {
     if (!b) return;
-    if (b->indptr || b->indices || b->blocks || b->row_indices || b->result) {
-        // (a failed wait gives the memory up: something may still use it)
-        if (cudaDeviceSynchronize() == cudaSuccess) {
-            dev_free(b->indptr);
-            dev_free(b->indices);
-            dev_free(b->blocks);
-            dev_free(b->row_indices);
-            dev_free(b->result);
-        } else {
-            cudaGetLastError();
-        }
-    }
+    void* const arrays[] = {b->indptr, b->indices, b->blocks, b->row_indices, b->result};
+    free_arrays(arrays, 5);
     b->indptr = b->indices = b->blocks = b->row_indices = nullptr;
     b->result = nullptr;
 }

@@ -65,6 +65,13 @@ __host__ __device__ __forceinline__ int log2_exact(int x)
 // call returns.  dev_free does not wait: nothing may be using the memory any more.
 cudaError_t dev_alloc(void** p, size_t bytes);
 void dev_free(void* p);
+// Waits for device `dev` (the current one when it is negative); the current device stays.  The
+// owner of memory on one device may be destroyed while another is current (a finaliser runs on
+// any thread), so a wait before a free names the memory's device.
+cudaError_t wait_device(int dev);
+// Waits for the device of the arrays (all on one, null ones among them) and frees them; a failed
+// wait gives the memory up: something may still use it.
+void free_arrays(void* const* arrays, int n);
 
 // A zeroed slot of kHostSlotWords uint64 in pinned, mapped, portable host memory (nullptr
 // without memory), and its return: nothing may be writing to it any more.
@@ -79,10 +86,12 @@ struct DevBuf {
     size_t bytes = 0;
     // Stream-ordered allocation, for an owner that uses the buffer on one stream only:
     // with `pool` and `stream` set, a growth frees and allocates in that stream's order
-    // (cudaFreeAsync / cudaMallocFromPoolAsync) instead of waiting for the whole device.  `pooled` records how the current allocation was made.
+    // (cudaFreeAsync / cudaMallocFromPoolAsync) instead of waiting for the whole device.
+    // `pooled` and `device` record how and where the current allocation was made.
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
     bool pooled = false;
+    int device = -1;
     int reserve(size_t need)
     {
         if (need <= bytes && ptr) return BTC_OK;
@@ -104,11 +113,12 @@ struct DevBuf {
     cudaError_t allocate(size_t b)
     {
         pooled = pool != nullptr && stream != nullptr;
+        if (cudaGetDevice(&device) != cudaSuccess) device = -1;
         return pooled ? cudaMallocFromPoolAsync(&ptr, b, pool, stream) : dev_alloc(&ptr, b);
     }
     void release()
     {
-        if (ptr && !pooled && cudaDeviceSynchronize() != cudaSuccess) {
+        if (ptr && !pooled && wait_device(device) != cudaSuccess) {
             cudaGetLastError();  // something may still use it: the memory is given up
             ptr = nullptr;
         }
@@ -390,7 +400,7 @@ struct PolicyWords {
     bool dirty = false;                  // a call did not come to its end
     void release()
     {
-        if (host && cudaDeviceSynchronize() != cudaSuccess) {
+        if (host && wait_device(dev.device) != cudaSuccess) {
             cudaGetLastError();
             host = nullptr;  // (something may still write to it)
             dev.release();

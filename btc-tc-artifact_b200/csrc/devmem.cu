@@ -175,10 +175,35 @@ cudaError_t dev_alloc(void** ptr, size_t bytes)
     return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
 }
 
+cudaError_t wait_device(int dev)
+{
+    int cur = 0;
+    if (dev < 0 || cudaGetDevice(&cur) != cudaSuccess || cur == dev) return cudaDeviceSynchronize();
+    cudaError_t e = cudaSetDevice(dev);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    const cudaError_t back = cudaSetDevice(cur);
+    return e != cudaSuccess ? e : back;
+}
+
 void dev_free(void* p)
 {
     // (cudaFree of pool memory returns it to its pool without a wait)
     if (p) cudaFree(p);
+}
+
+void free_arrays(void* const* arrays, int n)
+{
+    const void* any = nullptr;
+    for (int i = 0; i < n && !any; ++i) any = arrays[i];
+    if (!any) return;
+    cudaPointerAttributes a{};
+    const bool known = cudaPointerGetAttributes(&a, any) == cudaSuccess && a.type == cudaMemoryTypeDevice;
+    if (!known) cudaGetLastError();
+    if (wait_device(known ? a.device : -1) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    for (int i = 0; i < n; ++i) dev_free(arrays[i]);
 }
 
 }  // namespace btc200

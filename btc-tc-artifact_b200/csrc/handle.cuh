@@ -88,11 +88,23 @@ struct btc_bitbsr {
     }
     void release_all()
     {
-        // one wait for all the buffers that are not stream-ordered, and for the host slot
-        bool wait = h_meta != nullptr;
-        for_each_buf([&](btc200::DevBuf& b) { wait |= b.ptr && !b.pooled; });
-        if (wait && cudaDeviceSynchronize() != cudaSuccess) {
+        // one wait per device for all the buffers that are not stream-ordered, and for the host
+        // slot, which the kernels on the handle's device write
+        constexpr int kNone = -2;
+        int waited = kNone;
+        bool idle = true;
+        auto wait = [&](int dev) {
+            if (dev == waited) return;
+            waited = dev;
+            if (btc200::wait_device(dev) == cudaSuccess) return;
             cudaGetLastError();
+            idle = false;
+        };
+        if (h_meta) wait(device);
+        for_each_buf([&](btc200::DevBuf& b) {
+            if (b.ptr && !b.pooled) wait(b.device);
+        });
+        if (!idle) {
             for_each_buf([](btc200::DevBuf& b) { b.release(); });
             h_meta = nullptr;  // (given up: something may still write to it)
         }
