@@ -510,7 +510,7 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
     g->n_row_blocks = (int32_t)rows;
     g->input_edges = m;
     g->edges_known = false;
-    if (!g->h_meta && !(g->h_meta = host_slot_alloc())) return BTC_E_NOMEM;
+    if (!g->h_meta && !(g->h_meta = host_slot_alloc(&g->h_context))) return BTC_E_NOMEM;
     BTC_TRY(g->meta.reserve(sizeof(unsigned long long) * kMetaSlots));
     unsigned long long* meta = g->meta.as<unsigned long long>();
 

@@ -118,12 +118,12 @@ int ensure_count_scratch(btc_bitbsr* g)
 int ensure_host_meta(btc_bitbsr* g)
 {
     if (g->h_meta) return BTC_OK;
-    unsigned long long* p = host_slot_alloc();
+    unsigned long long* p = host_slot_alloc(&g->h_context);
     if (!p) return BTC_E_NOMEM;
     void* d = nullptr;
     if (cudaHostGetDevicePointer(&d, p, 0) != cudaSuccess) {
         cudaGetLastError();
-        host_slot_free(p);
+        host_slot_free(p, g->h_context);
         return BTC_E_CUDA;
     }
     g->h_meta = p;
@@ -994,12 +994,13 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
     struct Scratch {
         DevBuf rowmask, off, key, bits, first, meta;
         unsigned long long* host = nullptr;
+        unsigned long long context = 0;
         bool idle = false;
         ~Scratch()
         {
             if (!idle && cudaDeviceSynchronize() != cudaSuccess) return;  // (given up: see DevBuf)
             for (DevBuf* d : {&rowmask, &off, &key, &bits, &first, &meta}) d->release_idle();
-            host_slot_free(host);
+            host_slot_free(host, context);
         }
     } w;
     const uint32_t T = b->num_blocks;
@@ -1010,7 +1011,7 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
     BTC_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(unsigned long long) * kMetaSlots, nullptr));
     // a struct that the store is not made for is found out beside the counting: the count kernel
     // then does nothing (as after a failed build), and the host learns it from the wait it has
-    if (!(w.host = host_slot_alloc())) return BTC_E_NOMEM;
+    if (!(w.host = host_slot_alloc(&w.context))) return BTC_E_NOMEM;
     void* d_host = nullptr;
     BTC_CUDA_TRY(cudaHostGetDevicePointer(&d_host, w.host, 0));
     BTC_TRY(launch_rowstore_check(tile_cols, b->indices, b->row_indices, T, b->n_row_blocks, meta + kMetaOverflow,
@@ -1050,7 +1051,8 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
 static bool struct_dense(const btc_bcsr_device* b, int tile_cols)
 {
     if (tile_cols != 32) return false;
-    unsigned long long* h = host_slot_alloc();
+    unsigned long long context = 0;
+    unsigned long long* h = host_slot_alloc(&context);
     void* d = nullptr;
     bool dense = false;
     if (h && cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess &&
@@ -1061,7 +1063,7 @@ static bool struct_dense(const btc_bcsr_device* b, int tile_cols)
     } else {
         cudaGetLastError();
     }
-    host_slot_free(h);
+    host_slot_free(h, context);
     return dense;
 }
 

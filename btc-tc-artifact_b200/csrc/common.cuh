@@ -74,10 +74,11 @@ cudaError_t wait_device(int dev);
 void free_arrays(void* const* arrays, int n);
 
 // A zeroed slot of kHostSlotWords uint64 in pinned, mapped, portable host memory (nullptr
-// without memory), and its return: nothing may be writing to it any more.
+// without memory) of the current context, whose id is given with it, and its return: nothing may
+// be writing to it any more.
 constexpr size_t kHostSlotWords = 16;
-unsigned long long* host_slot_alloc();
-void host_slot_free(unsigned long long* s);
+unsigned long long* host_slot_alloc(unsigned long long* context);
+void host_slot_free(unsigned long long* s, unsigned long long context);
 
 // A grow-only device buffer.  reserve() keeps contents only when no reallocation
 // happens; callers treat it as scratch.
@@ -397,6 +398,7 @@ int launch_build_small(const SmallBuild& b, cudaStream_t s);
 struct PolicyWords {
     DevBuf dev;                          // two sums and a ticket
     unsigned long long* host = nullptr;  // a host slot
+    unsigned long long host_context = 0;
     bool dirty = false;                  // a call did not come to its end
     void release()
     {
@@ -406,7 +408,7 @@ struct PolicyWords {
             dev.release();
         }
         dev.release_idle();
-        host_slot_free(host);
+        host_slot_free(host, host_context);
         host = nullptr;
     }
 };

@@ -14,7 +14,9 @@
 #include <cuda.h>
 
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 namespace btc200 {
@@ -51,42 +53,54 @@ constexpr uint64_t kKeepBytes = 1ull << 30;
 constexpr size_t kDirectBytes = 256ull << 20;
 
 struct DevicePool {
-    cudaMemPool_t pool = nullptr;
+    cudaMemPool_t pool = nullptr;  // null: no pool support
     cudaStream_t stream = nullptr;
-    unsigned long long ctx_id = 0;  // the context it belongs to
-    bool tried = false;
 };
 
-// The current device's pool, made on first use in each context; false without pool support.
+// The id of the context the calling thread works in, made current if the thread had none yet (a
+// new thread's first call here comes before anything has bound it); 0 when it cannot be read.
+unsigned long long bound_context_id()
+{
+    unsigned long long id = current_context_id();
+    int dev = 0;
+    if (id == 0 && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess)
+        id = current_context_id();
+    return id;
+}
+
+// The current device's pool, made on first use in each context; false without pool support.  A
+// context's pool is kept for as long as the process runs: contexts come and go seldom, and one
+// that is met again (a second context on the device) finds its pool.
 bool pool_for_current_device(cudaMemPool_t* pool, cudaStream_t* stream)
 {
     static std::mutex mu;
-    static DevicePool pools[64];
+    static auto& pools = *new std::map<std::pair<int, unsigned long long>, DevicePool>;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    const unsigned long long id = current_context_id();
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const unsigned long long id = bound_context_id();
     std::lock_guard<std::mutex> lock(mu);
-    DevicePool& p = pools[dev];
-    if (!p.tried || (id != 0 && id != p.ctx_id)) {
-        p = DevicePool{};
-        p.tried = true;
-        int supported = 0;
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        uint64_t keep = kKeepBytes;
-        if (cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess ||
-            !supported || cudaMemPoolCreate(&p.pool, &props) != cudaSuccess) {
-            p.pool = nullptr;
-        } else if (cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
-                   cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) != cudaSuccess) {
-            cudaMemPoolDestroy(p.pool);
-            p.pool = nullptr;
-        }
-        if (!p.pool) cudaGetLastError();
-        p.ctx_id = id ? id : current_context_id();
+    const auto found = pools.find({dev, id});
+    if (found != pools.end()) {
+        *pool = found->second.pool;
+        *stream = found->second.stream;
+        return *pool != nullptr;
     }
+    DevicePool& p = pools[{dev, id}];
+    int supported = 0;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kKeepBytes;
+    if (cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, dev) != cudaSuccess ||
+        !supported || cudaMemPoolCreate(&p.pool, &props) != cudaSuccess) {
+        p.pool = nullptr;
+    } else if (cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+               cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaMemPoolDestroy(p.pool);
+        p.pool = nullptr;
+    }
+    if (!p.pool) cudaGetLastError();
     *pool = p.pool;
     *stream = p.stream;
     return p.pool != nullptr;
@@ -96,15 +110,15 @@ bool pool_for_current_device(cudaMemPool_t* pool, cudaStream_t* stream)
 
 // Pinned, mapped host slots of kHostSlotWords uint64, carved from blocks that stay until the
 // process ends (64 KB holds 512 handles; cudaHostAlloc and cudaFreeHost cost 0.01 to 5 ms a
-// handle).
+// handle).  A block belongs to the context that made it (a device reset takes its memory with
+// it), and its slots are handed out in that context only: whoever gives one back names it.
 namespace {
 
 constexpr size_t kSlotsPerBlock = 512;
 
 struct HostSlots {
     std::mutex mu;
-    std::vector<unsigned long long*> free_slots;
-    unsigned long long ctx_id = 0;  // a device reset takes the blocks with it
+    std::map<unsigned long long, std::vector<unsigned long long*>> free_slots;  // by context
 };
 HostSlots& host_slots()
 {
@@ -114,40 +128,34 @@ HostSlots& host_slots()
 
 }  // namespace
 
-unsigned long long* host_slot_alloc()
+unsigned long long* host_slot_alloc(unsigned long long* context)
 {
     HostSlots& h = host_slots();
-    const unsigned long long id = current_context_id();
+    *context = bound_context_id();
     std::lock_guard<std::mutex> lock(h.mu);
-    int devices = 0;
-    // (contexts of several devices share portable memory; one device's reset is told apart)
-    if (cudaGetDeviceCount(&devices) == cudaSuccess && devices == 1 && id != h.ctx_id) {
-        h.free_slots.clear();
-        h.ctx_id = id;
-    }
-    if (h.free_slots.empty()) {
+    std::vector<unsigned long long*>& free_slots = h.free_slots[*context];
+    if (free_slots.empty()) {
         void* p = nullptr;
         if (cudaHostAlloc(&p, sizeof(unsigned long long) * kHostSlotWords * kSlotsPerBlock,
                           cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
             cudaGetLastError();
             return nullptr;
         }
-        if (id == 0) h.ctx_id = current_context_id();  // (the allocation made the context)
         for (size_t i = kSlotsPerBlock; i-- > 0;)
-            h.free_slots.push_back(static_cast<unsigned long long*>(p) + i * kHostSlotWords);
+            free_slots.push_back(static_cast<unsigned long long*>(p) + i * kHostSlotWords);
     }
-    unsigned long long* s = h.free_slots.back();
-    h.free_slots.pop_back();
+    unsigned long long* s = free_slots.back();
+    free_slots.pop_back();
     std::memset(s, 0, sizeof(unsigned long long) * kHostSlotWords);
     return s;
 }
 
-void host_slot_free(unsigned long long* s)
+void host_slot_free(unsigned long long* s, unsigned long long context)
 {
     if (!s) return;
     HostSlots& h = host_slots();
     std::lock_guard<std::mutex> lock(h.mu);
-    h.free_slots.push_back(s);
+    h.free_slots[context].push_back(s);
 }
 
 cudaError_t dev_alloc(void** ptr, size_t bytes)

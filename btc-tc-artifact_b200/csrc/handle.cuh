@@ -44,7 +44,8 @@ struct btc_bitbsr {
     btc200::PolicyWords policy;
     btc200::DevBuf small;     // the one-launch builder's sums and barrier (small.cu), zero between launches
     bool small_dirty = false; // a launch may have left something in them
-    unsigned long long* h_meta = nullptr;  // pinned and mapped, 8 slots
+    unsigned long long* h_meta = nullptr;  // pinned and mapped, kHostSlotWords words
+    unsigned long long h_context = 0;      // ... of this context
     unsigned long long* d_hmeta = nullptr; // the device's address of h_meta
     bool edges_known = false;
     int64_t num_edges = 0;
@@ -110,7 +111,7 @@ struct btc_bitbsr {
         }
         policy.release();
         for_each_buf([](btc200::DevBuf& b) { b.release_idle(); });
-        btc200::host_slot_free(h_meta);
+        btc200::host_slot_free(h_meta, h_context);
         h_meta = nullptr;
         d_hmeta = nullptr;
         if (meta_event) cudaEventDestroy(meta_event);

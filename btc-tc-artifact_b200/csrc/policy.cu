@@ -122,7 +122,7 @@ int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n
         *L = pol::locality_host(src, dst, m, n, e_off, nv, G);
         return BTC_OK;
     }
-    if (!w.host && !(w.host = host_slot_alloc())) return BTC_E_NOMEM;
+    if (!w.host && !(w.host = host_slot_alloc(&w.host_context))) return BTC_E_NOMEM;
     void* d_host = nullptr;
     BTC_CUDA_TRY(cudaHostGetDevicePointer(&d_host, w.host, 0));
     const bool fresh = w.dev.ptr == nullptr;

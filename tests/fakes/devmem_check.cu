@@ -4,6 +4,8 @@
 
 #include "handle.cuh"
 
+#include <thread>
+
 namespace btc200 {
 void note_cuda_error(cudaError_t, const char*, const char*, int) {}
 }  // namespace btc200
@@ -39,10 +41,10 @@ static void handle_of_another_device()
     cudaSetDevice(1);
     btc_bitbsr g;
     g.device = 1;
-    g.h_meta = host_slot_alloc();
+    g.h_meta = host_slot_alloc(&g.h_context);
     EXPECT(g.indptr.reserve(100) == 0 && g.blocks.reserve(1000) == 0);
     EXPECT(g.policy.dev.reserve(24) == 0);
-    g.policy.host = host_slot_alloc();
+    g.policy.host = host_slot_alloc(&g.policy.host_context);
     cudaSetDevice(0);
     fake::log.clear();
     g.release_all();
@@ -84,12 +86,65 @@ static void arrays_of_another_device()
     free_arrays(p, 1);  // nothing held
 }
 
+// A program that builds from a new thread each time keeps one block of host slots.
+static void slots_of_many_threads()
+{
+    fake::devices = 1;
+    for (int i = 0; i < 20; ++i)
+        std::thread([] {
+            unsigned long long context = 0;
+            unsigned long long* s = host_slot_alloc(&context);
+            EXPECT(s && context == fake::context_id[0]);
+            host_slot_free(s, context);
+        }).join();
+    EXPECT(fake::pinned_made == 1);
+}
+
+// A slot freed after its context's end is not handed out again; the slots of the new context are.
+static void slots_across_a_reset()
+{
+    cudaSetDevice(0);
+    unsigned long long ca = 0, cb = 0, cc = 0;
+    unsigned long long* a = host_slot_alloc(&ca);
+    fake::reset(0);
+    unsigned long long* b = host_slot_alloc(&cb);
+    EXPECT(ca != cb && fake::pinned_made == 2);
+    host_slot_free(a, ca);
+    unsigned long long* c = host_slot_alloc(&cc);
+    EXPECT(cc == cb && c != a && c != b);
+    EXPECT(*reinterpret_cast<unsigned char*>(a) == 0xEE);  // nothing wrote to the dead memory
+    host_slot_free(b, cb);
+    EXPECT(host_slot_alloc(&cc) == b);
+}
+
+// Two contexts of one device in turn: one pool and one block each, and none more.
+static void contexts_in_turn()
+{
+    fake::devices = 1;
+    const unsigned long long first = fake::context_id[0];
+    for (int i = 0; i < 6; ++i) {
+        fake::context_id[0] = first + i % 2;
+        cudaSetDevice(0);
+        void* p = nullptr;
+        EXPECT(dev_alloc(&p, 64) == cudaSuccess);
+        dev_free(p);
+        unsigned long long context = 0;
+        unsigned long long* s = host_slot_alloc(&context);
+        EXPECT(context == first + i % 2);
+        host_slot_free(s, context);
+    }
+    EXPECT(fake::pools_made == 2 && fake::pinned_made == 2);
+}
+
 int main(int argc, char** argv)
 {
     const std::string name = argc > 1 ? argv[1] : "";
     if (name == "handle_of_another_device") handle_of_another_device();
     else if (name == "buffer_of_another_device") buffer_of_another_device();
     else if (name == "arrays_of_another_device") arrays_of_another_device();
+    else if (name == "slots_of_many_threads") slots_of_many_threads();
+    else if (name == "slots_across_a_reset") slots_across_a_reset();
+    else if (name == "contexts_in_turn") contexts_in_turn();
     else return 2;
     return failures ? 1 : 0;
 }
