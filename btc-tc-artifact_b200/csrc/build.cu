@@ -15,6 +15,7 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <atomic>
 
 namespace btc200 {
 
@@ -53,14 +54,17 @@ __device__ __forceinline__ uint32_t warp_sum(uint32_t v)
 // time the CTA sees it (compare-and-swap), later increments of it stay in shared memory,
 // and the table is added to the global counters once when the CTA ends.  Hubs appear
 // often and early, so they own slots in every CTA; a vertex whose slot is taken by
-// another counts in global memory as before.  4096 slots (32 KB of keys and counters):
-// at R-MAT s22 a CTA's table keeps ~17% of its increments (2048 slots: ~10%) and the
-// kernel takes 1.32 ms against 1.48.
-#ifndef DEG_SLOTS
-#define DEG_SLOTS 26624
-#define DEG_THREADS 1024
-#define DEG_U 4
-#endif
+// another counts in global memory as before.  The more slots, the more increments stay: 26,624
+// slots (208 KB, one CTA of 1,024 threads per SM) against 4,096 (six of 256) take a degree-
+// ordered R-MAT build, edge factor 16, from 268 to 228 us at scale 17, 1.26 to 1.12 ms at 20
+// and 5.65 to 5.21 at 22 (13,312 slots: 244 us, 1.16, 5.38), and change nothing on uniform ids
+// (n 10^6, 8M edges: 1.10 ms both).  Clearing and flushing a table that a short list does not
+// fill costs 2 us (8,192 edges: 71.2 us, 69.2 with 4,096 slots; 32,768 edges 98.4 / 98.0;
+// 131,072 130 / 135), so lists below kDegFewEdges take the small one.
+constexpr int64_t kDegFewEdges = 1 << 16;
+constexpr uint32_t kDegSlots = 26624, kDegFewSlots = 4096;
+constexpr int kDegThreads = 1024, kDegFewThreads = 256;
+constexpr int kDegEdges = 4;  // in flight per thread
 constexpr uint32_t kDegFree = 0xffffffffu;
 
 template <uint32_t kSlots>
@@ -76,11 +80,12 @@ __device__ __forceinline__ void degree_add(uint32_t v, uint32_t* keys, uint32_t*
     else atomicAdd(&deg[v], 1u);
 }
 
-template <uint32_t kSlots, int kDThreads, int U>
+template <uint32_t kSlots, int kDThreads>
 __global__ void __launch_bounds__(kDThreads)
 k_degree(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
          int64_t m, int32_t n, uint32_t* __restrict__ deg)
 {
+    constexpr int U = kDegEdges;
     extern __shared__ uint32_t s_deg[];
     uint32_t* keys = s_deg;
     uint32_t* cnt = s_deg + kSlots;
@@ -382,13 +387,19 @@ int grid_for(int64_t work, int threads)
 int launch_degree(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, uint32_t* deg,
                   cudaStream_t s)
 {
-    if (m > 0) {
-        auto kernel = build_kernels::k_degree<DEG_SLOTS, DEG_THREADS, DEG_U>;
-        const int smem = 8 * DEG_SLOTS;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return BTC_E_CUDA;
-        const int64_t per = 232448 / (smem + 1024);
-        const int grid = (int)std::min<int64_t>((m + DEG_THREADS - 1) / DEG_THREADS, std::min<int64_t>(per, 2048 / DEG_THREADS) * device_sm_count());
-        kernel<<<grid, DEG_THREADS, smem, s>>>(src, dst, m, n, deg);
+    if (m <= 0) return BTC_OK;
+    auto launch = [&](auto kernel, int threads, uint32_t slots, int per_sm) {
+        const int64_t ctas = std::min<int64_t>((m + threads - 1) / threads, (int64_t)per_sm * device_sm_count());
+        kernel<<<(unsigned)ctas, threads, 8 * slots, s>>>(src, dst, m, n, deg);
+    };
+    using namespace build_kernels;
+    if (m < kDegFewEdges) {
+        launch(k_degree<kDegFewSlots, kDegFewThreads>, kDegFewThreads, kDegFewSlots, 6);
+    } else {
+        auto kernel = k_degree<kDegSlots, kDegThreads>;
+        static std::atomic<unsigned long long> allowed[kMaxDevices];
+        if (!allow_dynamic_smem(reinterpret_cast<const void*>(kernel), 8 * kDegSlots, allowed)) return BTC_E_CUDA;
+        launch(kernel, kDegThreads, kDegSlots, 1);
     }
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }

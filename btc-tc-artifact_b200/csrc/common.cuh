@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 
@@ -441,6 +442,10 @@ static_assert(kMetaSlots <= kHostSlotWords, "a host slot holds the metadata");
 constexpr size_t kCountCtlBytes = 16;
 
 int device_sm_count();
+constexpr int kMaxDevices = 64;
+// Lets a kernel take `bytes` of dynamic shared memory on the current device: an opt-in that is
+// made once per device and context (done: the context it was made in, per device).
+bool allow_dynamic_smem(const void* kernel, size_t bytes, std::atomic<unsigned long long>* done);
 // Id of the calling thread's current context (0 when it cannot be read): a device reset
 // gives the device a new one.
 unsigned long long current_context_id();

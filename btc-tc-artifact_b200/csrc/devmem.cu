@@ -183,6 +183,20 @@ cudaError_t dev_alloc(void** ptr, size_t bytes)
     return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
 }
 
+bool allow_dynamic_smem(const void* kernel, size_t bytes, std::atomic<unsigned long long>* done)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+    const unsigned long long id = bound_context_id();
+    if (id != 0 && done[dev].load(std::memory_order_acquire) == id) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    done[dev].store(id, std::memory_order_release);
+    return true;
+}
+
 cudaError_t wait_device(int dev)
 {
     int cur = 0;

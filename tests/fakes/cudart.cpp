@@ -53,6 +53,11 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned)
     *s = reinterpret_cast<cudaStream_t>((uintptr_t)64);
     return cudaSuccess;
 }
+cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int value)
+{
+    fake::note("attribute" + std::to_string(value), fake::current);
+    return cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
