@@ -487,19 +487,26 @@ int rows_variant(int tile_cols, bool dense, bool seg)
     return (seg ? 3 : 0) + (tile_cols == 128 ? (dense ? 1 : 0) : 2);
 }
 
-// Resident CTAs per SM of a row-wise kernel variant (dynamic shared memory above 48 KB is
-// an opt-in per function, set here once per device); 0 on error.
+size_t rows_variant_smem(int v) { return v % 3 == 2 ? rows_smem_bytes<32>() : rows_smem_bytes<128>(); }
+
+// Dynamic shared memory above 48 KB is an opt-in per function.
+bool allow_rows_smem(int v)
+{
+    static std::atomic<unsigned long long> allowed[6][kMaxDevices];
+    return allow_dynamic_smem(reinterpret_cast<const void*>(rows_kernel(v)), rows_variant_smem(v), allowed[v]);
+}
+
+// Resident CTAs per SM of a row-wise kernel variant, cached per device; 0 on error.
 int rows_variant_blocks_per_sm(int v)
 {
-    static std::atomic<int> resident[64][6];
+    static std::atomic<int> resident[kMaxDevices][6];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
     int per_sm = resident[dev][v].load(std::memory_order_acquire);
     if (per_sm > 0) return per_sm;
-    const size_t smem = v % 3 == 2 ? rows_smem_bytes<32>() : rows_smem_bytes<128>();
-    const RowsKernel k = rows_kernel(v);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kRThreads, smem);
+    cudaError_t e = cudaErrorInvalidValue;
+    if (allow_rows_smem(v))
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rows_kernel(v), kRThreads, rows_variant_smem(v));
     if (e != cudaSuccess || per_sm < 1) {
         note_cuda_error(e, "k_count_rows launch set-up", __FILE__, __LINE__);
         return 0;
@@ -535,9 +542,9 @@ int launch_count_rows(int tile_cols, const uint32_t* indptr, const uint32_t* ind
     // the persistent grid is this kernel's resident CTAs, at most `grid` (the CTAs the
     // caller's scratch holds a partial sum for)
     const int v = rows_variant(tile_cols, dense, segs != nullptr);
-    const size_t smem = v % 3 == 2 ? rows_smem_bytes<32>() : rows_smem_bytes<128>();
+    const size_t smem = rows_variant_smem(v);
     const int per_sm = rows_variant_blocks_per_sm(v);
-    if (per_sm < 1) return BTC_E_CUDA;
+    if (per_sm < 1 || !allow_rows_smem(v)) return BTC_E_CUDA;
     if (per_sm * device_sm_count() < grid) grid = per_sm * device_sm_count();
     rows_kernel(v)<<<grid, kRThreads, smem, s>>>(indptr, indices, row_indices, blocks, num_tiles,
                                                  tile_begin, tile_end, n_row_blocks, tau, chunk, scr,

@@ -456,18 +456,24 @@ size_t stream_smem(int v)
     return v / 2 == 0 ? stream_smem_bytes<256>() : v / 2 == 1 ? stream_smem_bytes<512>() : stream_smem_bytes<1024>();
 }
 
-// Resident CTAs per SM of a variant (its dynamic shared memory is an opt-in, set here once
-// per device); 0 on error.
+// A variant's dynamic shared memory is an opt-in.
+bool allow_stream_smem(int v)
+{
+    static std::atomic<unsigned long long> allowed[kVariants][kMaxDevices];
+    return allow_dynamic_smem(reinterpret_cast<const void*>(stream_kernel(v)), stream_smem(v), allowed[v]);
+}
+
+// Resident CTAs per SM of a variant, cached per device; 0 on error.
 int stream_blocks_per_sm(int v)
 {
-    static std::atomic<int> resident[64][kVariants];
+    static std::atomic<int> resident[kMaxDevices][kVariants];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
     int per_sm = resident[dev][v].load(std::memory_order_acquire);
     if (per_sm > 0) return per_sm;
-    const StreamKernel k = stream_kernel(v);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stream_smem(v));
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kSThreads, stream_smem(v));
+    cudaError_t e = cudaErrorInvalidValue;
+    if (allow_stream_smem(v))
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stream_kernel(v), kSThreads, stream_smem(v));
     if (e != cudaSuccess || per_sm < 1) {
         note_cuda_error(e, "k_count_stream launch set-up", __FILE__, __LINE__);
         return 0;
@@ -499,7 +505,7 @@ int launch_count_stream(const RowStore& rs, const unsigned long long* rs_chunks,
     const int size = row_store_wide(n_row_blocks) ? 3 : max_col_blocks <= 256 ? 0 : max_col_blocks <= 512 ? 1 : 2;
     const int v = 2 * size + (graph_counts ? 1 : 0);
     const int per_sm = stream_blocks_per_sm(v);
-    if (per_sm < 1) return BTC_E_CUDA;
+    if (per_sm < 1 || !allow_stream_smem(v)) return BTC_E_CUDA;
     if (per_sm * device_sm_count() < grid) grid = per_sm * device_sm_count();
     stream_kernel(v)<<<grid, kSThreads, stream_smem(v), s>>>(
         rs.off, rs.key, rs.bits, rs.first_row, rs_chunks, (uint32_t)n_row_blocks, scr, graph_rows, num_graphs,

@@ -486,19 +486,6 @@ k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
     if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// Opt-in to a kernel's dynamic shared memory, once per device.
-template <class K>
-bool allow_smem(K kernel, size_t bytes, std::atomic<bool>* done)
-{
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    if (done[dev].load(std::memory_order_acquire)) return true;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-        return false;
-    done[dev].store(true, std::memory_order_release);
-    return true;
-}
-
 }  // namespace gp
 
 // Row bits below a bucket: at most kBuckets buckets of whole row blocks.
@@ -547,8 +534,9 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
         gp::k_orient<<<ogrid, gp::kOThreads, 0, s>>>(src, dst, m, n, rank, shift,
                                                      store ? pairs : nullptr, hist, meta + kMetaBad);
     gp::k_bucket_scan<<<1, 1024, 0, s>>>(hist, base, cursor);
-    static std::atomic<bool> scatter_ok[64];
-    if (!gp::allow_smem(gp::k_scatter, sizeof(gp::ScatterSmem), scatter_ok)) return BTC_E_CUDA;
+    static std::atomic<unsigned long long> scatter_ok[kMaxDevices];
+    if (!allow_dynamic_smem(reinterpret_cast<const void*>(&gp::k_scatter), sizeof(gp::ScatterSmem), scatter_ok))
+        return BTC_E_CUDA;
     if (m > 0)
         gp::k_scatter<<<(unsigned)((m + gp::kSTile - 1) / gp::kSTile), gp::kSThreads, sizeof(gp::ScatterSmem), s>>>(
             store ? pairs : nullptr, src, dst, m, n, shift, cursor, grouped);
@@ -589,11 +577,11 @@ int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
     const uint32_t NT = buf / tile_bytes;
     const size_t smem = buf + 4 * (size_t)NT + 8 * (size_t)words;
     const size_t most = gp::kTileBytes + 4 * (gp::kTileBytes / 64) + 8 * (size_t)gp::kMaxWords;
-    static std::atomic<bool> ok[4][64];
+    static std::atomic<unsigned long long> ok[4][kMaxDevices];
     const int threads = row_block_threads(m, R);
     const uint32_t grid = std::min<uint32_t>(R, 32u * device_sm_count() * (128 / threads));
     auto write = [&](auto kernel, int which) {
-        if (!gp::allow_smem(kernel, most, ok[which])) return BTC_E_CUDA;
+        if (!allow_dynamic_smem(reinterpret_cast<const void*>(kernel), most, ok[which])) return BTC_E_CUDA;
         kernel<<<grid, threads, smem, s>>>(edges, rb_end, R, words, indptr, meta + kMetaTiles, cap,
                                            indices, row_indices, reinterpret_cast<uint4*>(blocks), rowmask, NT);
         return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;

@@ -136,6 +136,25 @@ static void contexts_in_turn()
     EXPECT(fake::pools_made == 2 && fake::pinned_made == 2);
 }
 
+// A kernel's shared-memory opt-in is made once per context of each device.
+static void opt_ins()
+{
+    std::atomic<unsigned long long> done[kMaxDevices] = {};
+    int kernel = 0;
+    fake::log.clear();
+    for (int dev : {0, 0, 1, 0, 1}) {
+        cudaSetDevice(dev);
+        EXPECT(allow_dynamic_smem(&kernel, 100000, done));
+    }
+    EXPECT((fake::log == std::vector<std::string>{"attribute100000@0", "attribute100000@1"}));
+    fake::reset(0);
+    for (int dev : {0, 1, 0}) {
+        cudaSetDevice(dev);
+        EXPECT(allow_dynamic_smem(&kernel, 100000, done));
+    }
+    EXPECT(fake::log.size() == 3 && fake::log.back() == "attribute100000@0");
+}
+
 int main(int argc, char** argv)
 {
     const std::string name = argc > 1 ? argv[1] : "";
@@ -145,6 +164,7 @@ int main(int argc, char** argv)
     else if (name == "slots_of_many_threads") slots_of_many_threads();
     else if (name == "slots_across_a_reset") slots_across_a_reset();
     else if (name == "contexts_in_turn") contexts_in_turn();
+    else if (name == "opt_ins") opt_ins();
     else return 2;
     return failures ? 1 : 0;
 }
