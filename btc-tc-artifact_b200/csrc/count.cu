@@ -840,8 +840,11 @@ int launch_count(int tile_cols, const uint32_t* indptr, const uint32_t* indices,
     const int grid_tile = tile_blocks_per_sm(tile_cols) * device_sm_count();
     const int grid_most = grid_tile < grid_all ? grid_tile : grid_all;
     // no more warps than grabs of two tiles: the idle ones of a small graph still pass through
-    // the reduction at the end (Erdos-Renyi 256 / 24: 13.3 us with 592 CTAs, 11.8 without)
-    const int grid = (int)min((uint64_t)grid_most, max((uint64_t)span / (2 * kWarps) + 1, (uint64_t)1));
+    // the reduction at the end (Erdos-Renyi 256 / 24: 13.3 us with 592 CTAs, 11.8 without).  The
+    // bound is on the tiles that may be there, not on the hint: after an enqueued rebuild that
+    // is the previous graph's tile count, which says nothing of this one's work.
+    const uint64_t most_tiles = tile_end - tile_begin;
+    const int grid = (int)min((uint64_t)grid_most, most_tiles / (2 * kWarps) + 1);
     // Guided schedule: the first round of grabs is about half of an even share per warp
     // (2 to 64 tiles; later rounds halve it down to 2: a one-tile grab costs a contended
     // queue atomic per tile).  Fixed schedule: about an eighth of an even share (8 to 64 tiles);
