@@ -695,9 +695,11 @@ int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_o
     // tiles averaging more than half of tau's bits: the tensor-core path's graphs
     const bool dense = (uint64_t)g->input_edges * 2 > (uint64_t)tau * (uint64_t)g->num_tiles;
     const bool whole = tile_begin == 0 && tile_end == 0xffffffffu;
-    // A caller's lower tau asks for the tensor cores, which only the tile kernels use.
+    // A caller's lower tau asks for the tensor cores, which only the tile kernels use.  While an
+    // enqueued build is pending its tiles are not known (num_tiles is the graph's before it, of
+    // whatever size): the store it has made is used.
     if (g->row_store && tau >= default_tau(g->tile_cols) &&
-        !dense_graph(g->tile_cols, g->input_edges, g->num_tiles, g->n_row_blocks))
+        (g->pending || !dense_graph(g->tile_cols, g->input_edges, g->num_tiles, g->n_row_blocks)))
         return launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks, g->tile_cols, g->n_row_blocks,
                                    ((uint32_t)g->n + 63) / 64, scr, nullptr, 0, nullptr,
                                    g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), tile_begin,

@@ -56,3 +56,29 @@ def test_the_grid_does_not_shrink_on_the_last_graphs_tiles(tile_cols):
     assert int(out.item()) == want and g.count() == want
     assert changed < 4 * usual, (usual, changed)
     g.free()
+
+
+def test_a_pending_graph_is_counted_from_the_store_its_build_made():
+    """A large sparse graph enqueued after a small one looked dense (its edges over the small
+    one's tiles): the count went to the tile kernels and allocated their index."""
+    def uniform(n, m, seed):
+        e = np.random.default_rng(seed).integers(0, n, (2, m)).astype(np.int32)
+        return (*_cuda(e[0], e[1]), n)
+
+    large, small = uniform(40000, 600000, 1), uniform(300, 500, 2)
+    g = BitBSR(*large, 32)
+    want = g.count()
+
+    def cycle(asynchronous):
+        g.rebuild(*small, 32)
+        g.count()
+        g.rebuild(*large, 32, asynchronous=asynchronous)
+        got = torch.zeros(1, dtype=torch.int64, device="cuda")
+        g.count_async(d_out=got.data_ptr())
+        torch.cuda.synchronize()
+        assert int(got.item()) == want and g.count() == want
+        return g.info().device_bytes
+
+    held = cycle(False)
+    assert cycle(True) == held  # the tile kernels' index would have been allocated
+    g.free()
