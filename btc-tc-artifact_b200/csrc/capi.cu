@@ -986,12 +986,47 @@ StructScratch& struct_scratch()
 }
 }  // namespace
 
+// Device time of the kernels a struct count enqueues on the legacy stream, without the allocations
+// and waits between them: the sum over its spans.
+struct KernelTime {
+    static constexpr int kMost = 8;
+    cudaEvent_t at[kMost] = {};
+    int n = 0;
+    bool on;
+    explicit KernelTime(bool wanted) : on(wanted) {}
+    KernelTime(const KernelTime&) = delete;
+    KernelTime& operator=(const KernelTime&) = delete;
+    ~KernelTime()
+    {
+        for (int i = 0; i < n; ++i) cudaEventDestroy(at[i]);
+    }
+    // begins a span, or ends the one begun before
+    int mark()
+    {
+        if (!on || n == kMost) return BTC_OK;
+        BTC_CUDA_TRY(cudaEventCreate(&at[n]));
+        ++n;
+        BTC_CUDA_TRY(cudaEventRecord(at[n - 1], nullptr));
+        return BTC_OK;
+    }
+    // after the last span's work is done
+    float ms() const
+    {
+        float sum = 0.f;
+        for (int i = 0; i + 1 < n; i += 2) {
+            float t = 0.f;
+            if (cudaEventElapsedTime(&t, at[i], at[i + 1]) == cudaSuccess) sum += t;
+        }
+        return sum;
+    }
+};
+
 // The streaming count of a struct whose row blocks average 8 or more tiles: the row masks
 // and the row store are made for this call, which costs a pass over the tiles (R-MAT scale
 // 18 in natural order, 16x128: 0.3 ms) and saves the tile-wise kernel's searches (22 ms).
 // BTC_E_NOMEM where there is no memory for them, or the tiles are not what they take
 // (launch_rowstore_check): the caller takes the tile-wise kernel.
-static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScratch scr)
+static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScratch scr, KernelTime& kt)
 {
     struct Scratch {
         DevBuf rowmask, off, key, bits, first, meta;
@@ -1016,14 +1051,17 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
     if (!(w.host = host_slot_alloc(&w.context))) return BTC_E_NOMEM;
     void* d_host = nullptr;
     BTC_CUDA_TRY(cudaHostGetDevicePointer(&d_host, w.host, 0));
+    BTC_TRY(kt.mark());
     BTC_TRY(launch_rowstore_check(tile_cols, b->indices, b->row_indices, T, b->n_row_blocks, meta + kMetaOverflow,
                                   static_cast<unsigned long long*>(d_host), nullptr));
     BTC_TRY(launch_rowmask(tile_cols, b->blocks, T, nullptr, b->indptr, b->n_row_blocks,
                            w.rowmask.as<uint32_t>(), meta + kMetaRowMax, nullptr));
     // one entry per mask bit at most; counted (a wait) where 16 or 32 per tile is too much
     uint64_t entries = (uint64_t)T * (tile_cols == 128 ? 32 : 16);
-    if (entries > (16ull << 20)) {
-        BTC_TRY(launch_mask_popcount(w.rowmask.as<uint32_t>(), T, meta + kMetaUniq, nullptr));
+    const bool counted = entries > (16ull << 20);
+    if (counted) BTC_TRY(launch_mask_popcount(w.rowmask.as<uint32_t>(), T, meta + kMetaUniq, nullptr));
+    BTC_TRY(kt.mark());
+    if (counted) {
         unsigned long long bits = 0;
         BTC_CUDA_TRY(cudaMemcpy(&bits, meta + kMetaUniq, sizeof(bits), cudaMemcpyDeviceToHost));
         entries = bits;
@@ -1035,6 +1073,7 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
     BTC_TRY(w.key.reserve((wide ? sizeof(uint2) : sizeof(uint32_t)) * kRowLanes * chunks));
     BTC_TRY(w.bits.reserve(sizeof(uint4) * kRowLanes * chunks));
     BTC_TRY(w.first.reserve(sizeof(uint32_t) * (chunks / kRowRun + 1)));
+    BTC_TRY(kt.mark());
     const RowStore rs{w.off.as<uint32_t>(), w.key.ptr, w.bits.as<uint4>(), w.first.as<uint32_t>()};
     BTC_TRY(launch_rowstore(tile_cols, b->indptr, b->indices, b->blocks, b->n_row_blocks,
                             w.rowmask.as<uint32_t>(), nullptr, T, false, meta, rs, nullptr));
@@ -1042,6 +1081,7 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
                                 ((uint32_t)b->n_row_blocks * 16u + 63) / 64, scr, nullptr, 0, nullptr,
                                 b->row_indices, b->indices, 0, T, true, false, meta,
                                 count_grid_size(tile_cols), nullptr));
+    BTC_TRY(kt.mark());
     BTC_CUDA_TRY(cudaStreamSynchronize(nullptr));
     w.idle = true;
     return *static_cast<volatile unsigned long long*>(w.host) ? BTC_E_NOMEM : BTC_OK;
@@ -1050,15 +1090,21 @@ static int count_struct_stream(const btc_bcsr_device* b, int tile_cols, CountScr
 // Whether the tile-wise kernel's tensor cores count a struct faster: dense 16x32 tiles, told
 // from a sample (a struct does not know its edges).  At 16x128 streaming wins at any density
 // (the complete graph on 4,096 vertices: 0.43 ms against 1.18).
-static bool struct_dense(const btc_bcsr_device* b, int tile_cols)
+static bool struct_dense(const btc_bcsr_device* b, int tile_cols, KernelTime& kt)
 {
     if (tile_cols != 32) return false;
     unsigned long long context = 0;
     unsigned long long* h = host_slot_alloc(&context);
     void* d = nullptr;
     bool dense = false;
-    if (h && cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess &&
-        launch_sample_bits(tile_cols, b->blocks, b->num_blocks, static_cast<unsigned long long*>(d), nullptr) == BTC_OK) {
+    bool sampled = h && cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess;
+    if (sampled) {
+        kt.mark();
+        sampled = launch_sample_bits(tile_cols, b->blocks, b->num_blocks, static_cast<unsigned long long*>(d),
+                                     nullptr) == BTC_OK;
+        kt.mark();
+    }
+    if (sampled) {
         if (cudaStreamSynchronize(nullptr) != cudaSuccess) return false;  // (the slot is given up)
         dense = h[1] && dense_graph(tile_cols, (int64_t)((double)h[0] / (double)h[1] * (double)b->num_blocks), b->num_blocks,
                                     b->n_row_blocks);
@@ -1086,29 +1132,24 @@ static int count_struct(btc_bcsr_device* b, int tile_cols, float* kernel_ms,
         BTC_TRY(ss.done[dev].reserve(kCountCtlBytes));
         BTC_CUDA_TRY(cudaMemset(ss.done[dev].ptr, 0, kCountCtlBytes));
     }
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (kernel_ms) {
-        BTC_CUDA_TRY(cudaEventCreate(&e0));
-        BTC_CUDA_TRY(cudaEventCreate(&e1));
-        BTC_CUDA_TRY(cudaEventRecord(e0, nullptr));
-    }
+    KernelTime kt(kernel_ms != nullptr);
     CountScratch scr{ss.partials[dev].as<unsigned long long>(), ss.done[dev].as<unsigned int>(),
                      reinterpret_cast<unsigned long long*>(ss.done[dev].as<char>() + 8), b->result,
                      nullptr};
     int st = BTC_E_NOMEM;
     if (b->n_row_blocks > 0 && (uint64_t)b->num_blocks >= 8ull * (uint64_t)b->n_row_blocks &&
-        !struct_dense(b, tile_cols))
-        st = count_struct_stream(b, tile_cols, scr);
-    if (st == BTC_E_NOMEM)
+        !struct_dense(b, tile_cols, kt))
+        st = count_struct_stream(b, tile_cols, scr, kt);
+    if (st == BTC_E_NOMEM) {
+        BTC_TRY(kt.mark());
         st = launch_count(tile_cols, b->indptr, b->indices, b->row_indices, b->blocks, b->num_blocks,
                           b->n_row_blocks, default_tau(tile_cols), scr, nullptr);
-    if (st == BTC_OK && kernel_ms && cudaEventRecord(e1, nullptr) != cudaSuccess) st = BTC_E_CUDA;
+        if (st == BTC_OK) st = kt.mark();
+    }
     if (st == BTC_OK && cudaMemcpy(out, b->result, sizeof(unsigned long long),
                                    cudaMemcpyDeviceToHost) != cudaSuccess)
         st = BTC_E_CUDA;
-    if (st == BTC_OK && kernel_ms) cudaEventElapsedTime(kernel_ms, e0, e1);
-    if (e0) cudaEventDestroy(e0);
-    if (e1) cudaEventDestroy(e1);
+    if (st == BTC_OK && kernel_ms) *kernel_ms = kt.ms();
     return st;
 }
 

@@ -92,9 +92,10 @@ BTC_API int btc_convert_coo_to_bcsr_16x32_gpu(btc_bcsr_device* bcsr, const int32
 
 /* Replaces btc::count_triangles_16x128_adaptive (btc/operations/tc_16x128_adaptive.h:12-29)
  * and count_triangles_16x128_v5/_v4.  threshold_blocks selected the reference's v4/v5
- * variant; the engine has one kernel and accepts the argument for signature parity.
- * kernel_ms (nullable) receives the kernel-only event time.  The count is written to
- * *out_count and to bcsr->result.  Blocking. */
+ * variant; the engine picks its kernel itself and accepts the argument for signature parity.
+ * kernel_ms (nullable) receives the event time of the call's kernels (where the struct is
+ * counted from per-vertex rows, with those that make them), without its allocations, waits and
+ * copies.  The count is written to *out_count and to bcsr->result.  Blocking. */
 BTC_API int btc_count_triangles_16x128_adaptive(btc_bcsr_device* bcsr, int threshold_blocks,
                                         float* kernel_ms, unsigned long long* out_count);
 

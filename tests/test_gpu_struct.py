@@ -104,3 +104,25 @@ def test_struct_count_of_any_matrix(name, tile_cols):
     want = _want(a, runs)
     assert want > 0
     assert got == want and tile_wise == want
+
+
+def test_kernel_time_leaves_allocations_and_waits_out():
+    """A wide sparse struct: its per-vertex rows are half a gigabyte that every call allocates
+    and frees, over a quarter of the call.  A time that spans them is within 3% of the call's."""
+    import statistics
+    import time
+
+    import btc_b200
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    n = 3000000
+    e = torch.randint(0, n, (2, 2 * n), generator=gen, device="cuda", dtype=torch.int32)
+    b = btc_b200.BCSR_16x32_Device()
+    btc_b200.convert_coo_to_bcsr_16x32_gpu(b, btc_b200.CooMatrix(e[0].contiguous(), e[1].contiguous(), n))
+    kernel, wall = [], []
+    for _ in range(7):
+        t = time.perf_counter()
+        btc_b200.count_triangles_16x32_adaptive(b, kernel_ms=kernel)
+        wall.append((time.perf_counter() - t) * 1e3)
+    assert 0 < statistics.median(kernel) < 0.9 * statistics.median(wall), (kernel, wall)
+    b.free()
