@@ -590,7 +590,12 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         // repeated identical asynchronous rebuilds of device input replay a CUDA graph
         const bool graphed = enqueued && !(flags & BTC_INPUT_ON_HOST) &&
                              launch_build_graph(g, P, s);
-        if (!graphed) BTC_TRY(enqueue_build(g, P, &sorted, s));
+        if (!graphed) {
+            const int st = enqueue_build(g, P, &sorted, s);
+            if (st == kNotLaunched)
+                return build_into(g, src, dst, m, n, open_width ? 0 : tile_cols, flags, s, tiles_only, false);
+            BTC_TRY(st);
+        }
         // the build's status and tile count are in h_meta once the stream has run it
         // (k_set_last writes them through the mapping)
         if (!g->meta_event)
@@ -601,7 +606,10 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         if (enqueued) return BTC_OK;  // resolved by the next wait
         const int st2 = resolve_build(g);
         if (small) {
-            if (st2 == BTC_E_CUDA) return st2;
+            if (st2 == BTC_E_CUDA) {
+                if (g->h_meta[kMetaOverflow] != kGaveUp) return st2;
+                return build_into(g, src, dst, m, n, open_width ? 0 : tile_cols, flags, s, tiles_only, false);
+            }
             if (open_width) {
                 tile_cols = (int)g->h_meta[kHostTileCols];
                 if (tile_cols != 32 && tile_cols != 128) return BTC_E_CUDA;
@@ -731,8 +739,8 @@ int resolve_build(btc_bitbsr* g)
         return g->failed = BTC_E_CUDA;
     }
     const unsigned long long* h = g->h_meta;
-    g->small_dirty = g->small_dirty && h[kMetaOverflow] > 1;  // (2: a barrier of the small build gave up)
-    if (h[kMetaOverflow] > 1) {
+    g->small_dirty = g->small_dirty && h[kMetaOverflow] == kGaveUp;
+    if (h[kMetaOverflow] == kGaveUp) {
         g->failed = BTC_E_CUDA;
     } else if (h[kMetaBad] != 0) {
         g->failed = BTC_E_RANGE;

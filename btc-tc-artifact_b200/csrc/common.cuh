@@ -393,7 +393,12 @@ struct SmallBuild {
     unsigned int* bar;
     int64_t step;
     uint32_t samples;
+    uint32_t max_spins = 1u << 22;  // of a wait of one CTA for the others: seconds
 };
+// kNotLaunched: the device does not run that many CTAs together for this program (an SM limit, as
+// a multi-process service sets it); nothing was enqueued.
+constexpr int kNotLaunched = 1;
+constexpr unsigned long long kGaveUp = 2;  // meta[kMetaOverflow] of a build whose wait ran out
 int launch_build_small(const SmallBuild& b, cudaStream_t s);
 
 struct PolicyWords {

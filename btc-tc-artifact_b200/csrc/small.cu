@@ -14,8 +14,9 @@
 //   phase 3  tile prefix: pairs, indices, row_indices, indptr; tiles and row masks zeroed
 //   phase 4  tiles and row masks filled, the longest row-block list
 //
-// A barrier counts arrivals; its wait is bounded (a cooperative launch's CTAs are all
-// resident, so the bound is never met; past it the build reports failure).
+// A barrier counts arrivals; its wait is bounded (a cooperative launch's CTAs are all resident, so
+// the bound is not met unless they are kept from running; past it the build reports that it gave
+// up, and the caller builds otherwise).
 #include "common.cuh"
 
 #include <algorithm>
@@ -26,7 +27,6 @@ namespace sm {
 
 constexpr int kThreads = 256;
 constexpr int kEdges = 8;  // edges in flight per thread
-constexpr uint32_t kMaxSpins = 1u << 22;
 
 struct Args {
     const int32_t* src;
@@ -49,9 +49,10 @@ struct Args {
     unsigned int* bar;          // arrivals, CTAs done (zero at the start)
     int64_t step;               // the policy's sample
     uint32_t samples;
+    uint32_t max_spins;         // of a barrier's wait
 };
 
-__device__ __forceinline__ bool barrier(unsigned int* bar, unsigned target)
+__device__ __forceinline__ bool barrier(unsigned int* bar, unsigned target, uint32_t max_spins)
 {
     __shared__ int s_ok;
     __syncthreads();
@@ -59,9 +60,9 @@ __device__ __forceinline__ bool barrier(unsigned int* bar, unsigned target)
         __threadfence();
         atomicAdd(bar, 1u);
         uint32_t spins = 0;
-        while (*(volatile unsigned int*)bar < target && ++spins < kMaxSpins) {
+        while (*(volatile unsigned int*)bar < target && ++spins < max_spins) {
         }
-        s_ok = spins < kMaxSpins;
+        s_ok = spins < max_spins;
         __threadfence();
     }
     __syncthreads();
@@ -101,7 +102,7 @@ __device__ __forceinline__ bool build(const Args& a, uint32_t cap, uint32_t* s_s
     }
     nbad = __reduce_add_sync(kFull, nbad);
     if ((threadIdx.x & 31) == 0 && nbad) atomicAdd(&a.meta[kMetaBad], (unsigned long long)nbad);
-    if (!barrier(a.bar, 2 * G)) return false;
+    if (!barrier(a.bar, 2 * G, a.max_spins)) return false;
 
     // this CTA's words: whole runs of kThreads
     const uint32_t per = (W + G * kThreads - 1) / (G * kThreads) * kThreads;
@@ -111,7 +112,7 @@ __device__ __forceinline__ bool build(const Args& a, uint32_t cap, uint32_t* s_s
     uint32_t mine;
     cta_exclusive_scan<kThreads>(cnt, s_scan, mine);
     if (threadIdx.x == 0) a.counts[blockIdx.x] = mine;
-    if (!barrier(a.bar, 3 * G)) return false;
+    if (!barrier(a.bar, 3 * G, a.max_spins)) return false;
 
     uint32_t before = 0, all = 0;
     for (uint32_t b = threadIdx.x; b < G; b += kThreads) {
@@ -151,7 +152,7 @@ __device__ __forceinline__ bool build(const Args& a, uint32_t cap, uint32_t* s_s
             base += total;
         }
     }
-    if (!barrier(a.bar, 4 * G)) return false;
+    if (!barrier(a.bar, 4 * G, a.max_spins)) return false;
     if (!fits) return true;
 
     uint32_t longest = 0;
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(kThreads) k_build_small(Args a)
             if (expect) atomicAdd(&a.words3[1], expect);
         }
     }
-    bool ok = barrier(a.bar, gridDim.x);
+    bool ok = barrier(a.bar, gridDim.x, a.max_spins);
     int tile_cols = a.tile_cols;
     if (ok) {
         if (tile_cols == 0)
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(kThreads) k_build_small(Args a)
     // ---- the last CTA hands the status to the host and leaves the counters at zero --------
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (!ok) a.meta[kMetaOverflow] = 2ull;
+        if (!ok) a.meta[kMetaOverflow] = kGaveUp;
         __threadfence();
         if (atomicAdd(&a.bar[1], 1u) == gridDim.x - 1) {
             __threadfence();
@@ -254,21 +255,26 @@ static int small_grid(int64_t m)
 
 int launch_build_small(const SmallBuild& b, cudaStream_t s)
 {
-    static std::atomic<int> per_sm[64];
+    static std::atomic<int> per_sm[kMaxDevices];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BTC_E_CUDA;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return BTC_E_CUDA;
     int p = per_sm[dev].load(std::memory_order_relaxed);
     if (p == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, sm::k_build_small, sm::kThreads, 0) != cudaSuccess || p < 2)
-            return BTC_E_CUDA;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, sm::k_build_small, sm::kThreads, 0) != cudaSuccess || p < 2) {
+            cudaGetLastError();
+            return kNotLaunched;
+        }
         per_sm[dev].store(p, std::memory_order_relaxed);
     }
     sm::Args a{b.src, b.dst, b.m, b.n, b.tile_cols, b.words, b.counts, b.cellpp, b.indices, b.row_indices, b.indptr,
-               b.blocks, b.rowmask, b.cap128, b.cap32, b.meta, b.host, b.policy_sums, b.bar, b.step, b.samples};
+               b.blocks, b.rowmask, b.cap128, b.cap32, b.meta, b.host, b.policy_sums, b.bar, b.step, b.samples,
+               b.max_spins};
     void* args[] = {&a};
     const cudaError_t e = cudaLaunchCooperativeKernel(sm::k_build_small, dim3((unsigned)small_grid(b.m)),
                                                       dim3(sm::kThreads), args, 0, s);
-    return e == cudaSuccess ? BTC_OK : BTC_E_CUDA;
+    if (e == cudaSuccess) return BTC_OK;
+    cudaGetLastError();  // (refused: the next check of an error is not to find it)
+    return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported ? kNotLaunched : BTC_E_CUDA;
 }
 
 }  // namespace btc200

@@ -5,7 +5,27 @@ extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = fake::current; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { fake::current = d; fake::bound = true; return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int* n) { *n = fake::devices; return cudaSuccess; }
-cudaError_t cudaGetLastError(void) { return cudaSuccess; }
+cudaError_t cudaGetLastError(void)
+{
+    const cudaError_t e = fake::last_error;
+    fake::last_error = cudaSuccess;
+    return e;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void*, int, size_t, unsigned)
+{
+    *n = 4;
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t)
+{
+    *n = 4;
+    return cudaSuccess;
+}
+cudaError_t cudaLaunchCooperativeKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t)
+{
+    return fake::last_error = fake::cooperative;
+}
+cudaError_t cudaLaunchKernel(const void*, dim3, dim3, void**, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize(void)
 {
     fake::bound = true;
@@ -94,5 +114,9 @@ cudaError_t cudaGetDriverEntryPoint(const char* name, void** f, unsigned long lo
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*, dim3*, int*) {}
+unsigned __cudaPopCallConfiguration(dim3*, dim3*, size_t*, void*) { return 0; }
+cudaError_t __cudaGetKernel(cudaKernel_t*, const void*) { return cudaSuccess; }
+cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void**, size_t, cudaStream_t) { return cudaSuccess; }
 char __cudaInitModule(void**) { return 1; }
 }

@@ -21,6 +21,8 @@ inline std::map<void*, int> device_of;         // live device allocations
 inline std::map<void*, size_t> pinned;         // live pinned blocks
 inline std::map<CUcontext, unsigned long long> ids;
 inline int devices = 2;
+inline cudaError_t cooperative = cudaSuccess;  // what a cooperative launch answers
+inline cudaError_t last_error = cudaSuccess;
 inline int pools_made = 0, pinned_made = 0;
 inline unsigned long long context_id[2] = {101, 102};  // of each device's context
 inline thread_local int current = 0;

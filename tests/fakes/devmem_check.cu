@@ -1,5 +1,5 @@
-// Checks of csrc/devmem.cu and of the handle's release on a host-side CUDA runtime: one check
-// per name, exit code 0 when it holds.
+// Checks of csrc/devmem.cu, of the handle's release and of csrc/small.cu's launch on a host-side
+// CUDA runtime: one check per name, exit code 0 when it holds.
 #include "cudart.hpp"
 
 #include "handle.cuh"
@@ -8,6 +8,7 @@
 
 namespace btc200 {
 void note_cuda_error(cudaError_t, const char*, const char*, int) {}
+int device_sm_count() { return 148; }
 }  // namespace btc200
 
 using namespace btc200;
@@ -155,6 +156,21 @@ static void opt_ins()
     EXPECT(fake::log.size() == 3 && fake::log.back() == "attribute100000@0");
 }
 
+// A refused cooperative launch is told apart from an error, and leaves none behind.
+static void refused_launch()
+{
+    SmallBuild b{};
+    b.m = 100000;
+    b.n = 1000;
+    fake::cooperative = cudaErrorCooperativeLaunchTooLarge;
+    EXPECT(launch_build_small(b, nullptr) == kNotLaunched);
+    EXPECT(fake::last_error == cudaSuccess);
+    fake::cooperative = cudaErrorLaunchFailure;
+    EXPECT(launch_build_small(b, nullptr) == BTC_E_CUDA);
+    fake::cooperative = cudaSuccess;
+    EXPECT(launch_build_small(b, nullptr) == BTC_OK);
+}
+
 int main(int argc, char** argv)
 {
     const std::string name = argc > 1 ? argv[1] : "";
@@ -165,6 +181,7 @@ int main(int argc, char** argv)
     else if (name == "slots_across_a_reset") slots_across_a_reset();
     else if (name == "contexts_in_turn") contexts_in_turn();
     else if (name == "opt_ins") opt_ins();
+    else if (name == "refused_launch") refused_launch();
     else return 2;
     return failures ? 1 : 0;
 }

@@ -1,5 +1,6 @@
-"""CPU checks of the library's memory bookkeeping (csrc/devmem.cu, the handle's release) on a
-host-side CUDA runtime of two devices (tests/fakes): no GPU is touched."""
+"""CPU checks of the library's memory bookkeeping (csrc/devmem.cu, the handle's release) and of
+what it does with a refused launch, on a host-side CUDA runtime of two devices (tests/fakes): no
+GPU is touched."""
 from __future__ import annotations
 
 import os
@@ -10,7 +11,7 @@ import pytest
 from conftest import PKG, ROOT
 
 CHECKS = ["handle_of_another_device", "buffer_of_another_device", "arrays_of_another_device",
-          "slots_of_many_threads", "slots_across_a_reset", "contexts_in_turn", "opt_ins"]
+          "slots_of_many_threads", "slots_across_a_reset", "contexts_in_turn", "opt_ins", "refused_launch"]
 
 
 @pytest.fixture(scope="module")
@@ -20,6 +21,7 @@ def program(tmp_path_factory):
     subprocess.run(["nvcc", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "none",
                     "-I", os.path.join(PKG, "csrc"), "-I", os.path.join(ROOT, "include"), "-I", fakes,
                     os.path.join(fakes, "devmem_check.cu"), os.path.join(fakes, "cudart.cpp"), os.path.join(PKG, "csrc", "devmem.cu"),
+                    os.path.join(PKG, "csrc", "small.cu"),
                     "-o", str(exe)], check=True)
     return str(exe)
 
