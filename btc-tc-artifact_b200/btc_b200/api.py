@@ -302,6 +302,12 @@ def lite_select_tile_cols(nnz: int, num_rows: int, mode: int = 0) -> int:
     return int(lib().btc_lite_select_tile_cols(int(nnz), int(num_rows), int(mode)))
 
 
+def trim_memory(keep_bytes: int = 0) -> None:
+    """Gives the freed device memory the library keeps for its next handle back to the current
+    device, all but ``keep_bytes`` (btc_trim_memory)."""
+    check(lib().btc_trim_memory(int(keep_bytes)), "btc_trim_memory")
+
+
 def default_tau(tile_cols: int) -> int:
     return int(lib().btc_default_tau(int(tile_cols)))
 

@@ -769,7 +769,7 @@ btc_bitbsr* bitbsr_new_pooled(cudaMemPool_t pool, cudaStream_t s)
 
 extern "C" {
 
-int btc_abi_version(void) { return (1 << 16) | 0; }
+int btc_abi_version(void) { return (1 << 16) | 1; }
 
 int btc_default_tau(int tile_cols) { return default_tau(tile_cols); }
 

@@ -3,7 +3,7 @@
 // Handles that live for one graph allocate some 20 buffers; with cudaMalloc and cudaFree
 // each of them maps and unmaps memory and waits for the device.  The pool keeps up to
 // kKeepBytes of freed memory for the next handle; what is above that goes back to the
-// device at the next wait.  Allocations are made on a stream of the pool's own and are
+// device at the next wait, and all of it on btc_trim_memory.  Allocations are made on a stream of the pool's own and are
 // complete when dev_alloc returns, so a caller may use the memory on any stream; freed
 // memory is idle (dev_free's callers have waited), so it may be handed to any other.
 // Allocations of kDirectBytes and more come from cudaMalloc: the pool would not keep them
@@ -229,3 +229,13 @@ void free_arrays(void* const* arrays, int n)
 }
 
 }  // namespace btc200
+
+extern "C" int btc_trim_memory(uint64_t keep_bytes)
+{
+    using namespace btc200;
+    cudaMemPool_t pool;
+    cudaStream_t stream;
+    if (!pool_for_current_device(&pool, &stream)) return BTC_OK;  // (nothing is kept)
+    BTC_CUDA_TRY(cudaMemPoolTrimTo(pool, keep_bytes));
+    return BTC_OK;
+}

@@ -425,6 +425,12 @@ BTC_API int btc_server_stats_get(btc_server* s, btc_server_stats* st);
 /* Finishes every queued request, then stops the engine and frees the server. */
 BTC_API void btc_server_destroy(btc_server* s);
 
+/* Gives freed device memory that the library keeps for its next handle (up to 1 GiB on each
+ * device) back to the current device, all but keep_bytes of it, for the process's other
+ * allocators.  Memory in use stays; servers keep their own pools.  No counterpart in the
+ * reference, which frees through cudaFree. */
+BTC_API int btc_trim_memory(uint64_t keep_bytes);
+
 /* Default tau for a tile width (the value BTC_TAU_DEFAULT resolves to). */
 BTC_API int btc_default_tau(int tile_cols);
 

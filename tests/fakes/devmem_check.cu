@@ -156,6 +156,18 @@ static void opt_ins()
     EXPECT(fake::log.size() == 3 && fake::log.back() == "attribute100000@0");
 }
 
+// The kept memory is given back on the current device, down to what is asked for.
+static void trim()
+{
+    void* p = nullptr;
+    cudaSetDevice(1);
+    EXPECT(dev_alloc(&p, 64) == cudaSuccess);
+    dev_free(p);
+    fake::log.clear();
+    EXPECT(btc_trim_memory(4096) == BTC_OK && btc_trim_memory(0) == BTC_OK);
+    EXPECT((fake::log == std::vector<std::string>{"trim1to4096@1", "trim1to0@1"}));
+}
+
 // A refused cooperative launch is told apart from an error, and leaves none behind.
 static void refused_launch()
 {
@@ -182,6 +194,7 @@ int main(int argc, char** argv)
     else if (name == "contexts_in_turn") contexts_in_turn();
     else if (name == "opt_ins") opt_ins();
     else if (name == "refused_launch") refused_launch();
+    else if (name == "trim") trim();
     else return 2;
     return failures ? 1 : 0;
 }

@@ -11,7 +11,7 @@ import pytest
 from conftest import PKG, ROOT
 
 CHECKS = ["handle_of_another_device", "buffer_of_another_device", "arrays_of_another_device",
-          "slots_of_many_threads", "slots_across_a_reset", "contexts_in_turn", "opt_ins", "refused_launch"]
+          "slots_of_many_threads", "slots_across_a_reset", "contexts_in_turn", "opt_ins", "refused_launch", "trim"]
 
 
 @pytest.fixture(scope="module")
