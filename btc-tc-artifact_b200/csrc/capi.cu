@@ -83,17 +83,6 @@ bool dense_graph(int tile_cols, int64_t m, uint32_t T, int64_t R)
     return tile_cols == 128 ? per_tile > 896.0 : per_tile > 64.0 + (double)T / (double)R;
 }
 
-// Degree-ordered edge lists from this length on are grouped by row block (group.cu) instead
-// of marked and filled edge by edge: the tiles of a power-law graph this large do not stay
-// in L2 between zeroing and filling (R-MAT scale 18, 4.2M draws: 0.71 ms against 0.73 a
-// step; scale 19: 1.29 / 1.43; scale 22: build 9.3 -> 5.6 ms; scale 17: the same).  In
-// natural order the bitmap stays: meshes and communities have small tile arrays (27-point
-// mesh 100^3 0.61 ms against 0.69 grouped, 8 communities on 60,000 vertices 4.0 / 4.5) and a
-// power-law hub's row block is one CTA's work here (scale 18: 2.1 / 2.4); uniform graphs of
-// more than 3M edges would gain (800,000 vertices, 6.4M edges: 1.9 / 1.35 ms), but nothing
-// at hand tells them from a power-law graph.
-static constexpr int64_t kGroupEdges = 1 << 22;
-
 static constexpr uint64_t kMaxEdges = (1ull << 32) - (uint64_t)kSortTile;
 
 int ensure_count_scratch(btc_bitbsr* g)

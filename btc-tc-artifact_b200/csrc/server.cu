@@ -139,8 +139,6 @@ size_t slot_budget_in_use(btc_server* s, const Slot* except)
     return b;
 }
 
-// Device bytes a batch of m edges over `rows` row blocks may need (builder workspace,
-// bitmap, tiles at most one per edge), used to admit requests before building.
 // Cell-bitmap words of a request's part of a batch (row blocks x column-block words); a
 // batch holds at most kBatchWords of them, and a request of more than kSoloWords (a
 // large vertex range, however few its edges) runs alone through the single-graph builder,
@@ -159,11 +157,41 @@ bool runs_alone(const btc_server* s, const Request& q, int tile_cols)
     return q.m >= s->cfg.solo_edges || cell_words(q.n, tile_cols) > kSoloWords;
 }
 
-size_t batch_bytes_bound(int64_t m, int64_t rows, int tile_cols)
+// Device bytes a batch of `graphs` graphs, m edges, `rows` row blocks and `words` cell words may
+// need, used to admit requests before building: what batch_build_into and the count reserve, with
+// a tile per edge and the buffers' headroom.  A request that runs alone is built in degree order,
+// through a cell bitmap bounded by its edges or, a long list, grouped (16 bytes an edge).
+size_t batch_bytes_bound(int64_t m, int64_t rows, int64_t words, int64_t graphs, int tile_cols, bool alone)
 {
-    const size_t tw_bytes = (size_t)2 * tile_cols;  // 16 rows x tile_cols bits
-    const size_t m_ = (size_t)m;
-    return 8 * m_ + (m_ + 1) * (tw_bytes + 8) + (size_t)rows * 4 + (size_t)rows * 64 + (1 << 20);
+    const size_t m_ = (size_t)m, r = (size_t)rows;
+    size_t cells = 12 * ((size_t)words + r) + (size_t)words / 64;  // bitmap, pairs, chunk counts
+    if (alone) cells = std::min(cells, 3 * (32 * m_ + (64u << 20)));
+    if (alone && m >= btc200::kGroupEdges) cells = 16 * m_;
+    const size_t tiles = m_ * ((size_t)2 * tile_cols + 12);  // bits, column and row block, row mask
+    // per-vertex rows for the streaming count where the tiles can average 8 a row block; the other
+    // kernels' index is smaller
+    size_t store = 72 * r;
+    if (m_ >= 8 * r) {
+        const size_t chunk = btc200::kRowLanes * (sizeof(uint4) + (btc200::row_store_wide(rows) ? sizeof(uint2) : sizeof(uint32_t)));
+        store += (size_t)btc200::row_store_chunks(m_, r) * (chunk + 1);
+    }
+    const size_t sum = 8 * m_ + cells + tiles + 4 * r + store + 80 * (size_t)graphs;
+    return sum + sum / 8 + (1 << 20);
+}
+
+// Frees what the slots keep for their next batches, all but `except`'s; none of them is busy.
+void release_idle(btc_server* s, const Slot& except)
+{
+    for (Slot& o : s->slots) {
+        if (&o == &except) continue;
+        btc_batch_free(o.batch);
+        o.batch = nullptr;
+        o.d_src.release();
+        o.d_dst.release();
+        o.device_bytes = 0;
+    }
+    btc_free(s->solo);
+    s->solo = nullptr;
 }
 
 void publish(btc_server* s, Slot& sl, int status)
@@ -350,10 +378,12 @@ void engine_loop(btc_server* s)
                     s->cv.wait_for(lock, std::chrono::microseconds(any_busy ? 50 : 2000));
                     continue;
                 }
-                const size_t others = slot_budget_in_use(s, &sl);
-                const size_t budget = s->cfg.hbm_budget_bytes > others
-                                          ? (size_t)s->cfg.hbm_budget_bytes - others
-                                          : 0;
+                size_t others = 0, budget = 0;
+                auto look = [&] {
+                    others = slot_budget_in_use(s, &sl);
+                    budget = s->cfg.hbm_budget_bytes > others ? (size_t)s->cfg.hbm_budget_bytes - others : 0;
+                };
+                look();
                 sl.offsets.assign(1, 0);
                 sl.nv.clear();
                 int64_t m = 0, rows = 0, words = 0;
@@ -374,13 +404,12 @@ void engine_loop(btc_server* s)
                         continue;
                     }
                     const int64_t qr = ((int64_t)q.n + 15) / 16;
-                    const size_t need = batch_bytes_bound(m + qm, rows + qr, tile);
-                    const int64_t qw = cell_words(q.n, tile);
+                    const int64_t qw = cell_words(q.n, tile), graphs = (int64_t)sl.reqs.size() + 1;
+                    const size_t need = batch_bytes_bound(m + qm, rows + qr, words + qw, graphs, tile, alone);
                     if (!sl.reqs.empty() &&
                         (m + qm > s->cfg.max_batch_edges || need > budget || words + qw > kBatchWords))
                         break;
-                    if (sl.reqs.empty() && batch_bytes_bound(qm, qr, tile) > budget &&
-                        others == 0) {
+                    if (sl.reqs.empty() && need > budget && others == 0) {
                         btc_server_result r{};
                         r.id = q.id;
                         r.status = BTC_E_NOMEM;
@@ -392,7 +421,15 @@ void engine_loop(btc_server* s)
                         it = s->pending.erase(it);
                         continue;
                     }
-                    if (sl.reqs.empty() && batch_bytes_bound(qm, qr, tile) > budget) break;
+                    if (sl.reqs.empty() && need > budget) {
+                        bool any_busy = false;
+                        for (const Slot& o : s->slots) any_busy |= o.busy;
+                        if (any_busy) break;
+                        // nothing runs: what is missing is what the idle slots keep
+                        release_idle(s, sl);
+                        look();
+                        continue;
+                    }
                     m += qm;
                     rows += qr;
                     words += qw;
