@@ -298,7 +298,8 @@ int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* o
 // Enqueues the row store of a Bit-BSR whose row masks exist (T = *d_tiles tiles, bounded by
 // cap, or cap when d_tiles is null; nothing when T > cap).  by_degree: the ids are in
 // descending-degree order.  meta: the build's metadata slots (kMetaRowChunks zero: it counts the
-// chunks handed out); also raises meta[kMetaRowMax] to the most tiles in one row block.
+// chunks handed out); also raises meta[kMetaRowMax] to the most tiles and meta[kMetaRowLong] to the
+// most chunks in one row block.
 int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indices, const uint32_t* blocks,
                     int32_t n_row_blocks, const uint32_t* rowmask, const unsigned long long* d_tiles,
                     uint32_t cap, bool by_degree, unsigned long long* meta, const RowStore& out,
@@ -437,8 +438,8 @@ int policy_select(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, 
 
 // Device metadata slots of a build (uint64 each): valid keys, out-of-range flag, tile
 // count, unique edges, sort length, longest row-block list, tile-capacity overflow flag,
-// the chunk-scan ticket (CTAs of the chunk popcount that have finished), and the chunks of
-// the row store handed out.
+// the chunk-scan ticket (CTAs of the chunk popcount that have finished), and of the row store the
+// chunks handed out and the most that one row block has.
 enum {
     kMetaValid = 0,
     kMetaBad = 1,
@@ -449,7 +450,8 @@ enum {
     kMetaOverflow = 6,
     kMetaTicket = 7,
     kMetaRowChunks = 8,
-    kMetaSlots = 9
+    kMetaRowLong = 9,
+    kMetaSlots = 10
 };
 static_assert(kMetaSlots <= kHostSlotWords, "a host slot holds the metadata");
 

@@ -95,8 +95,8 @@ __device__ __forceinline__ uint32_t select_bit(uint32_t w, uint32_t r)
     return p;
 }
 
-// kGraphs: per-graph counts (graph_rows, graph_counts).
-template <int W, int kMinBlocks, bool kGraphs, bool kWide>
+// kGraphs: per-graph counts (graph_rows, graph_counts).  kRange: the tiles [tile_begin, tile_end).
+template <int W, int kMinBlocks, bool kGraphs, bool kWide, bool kRange>
 __global__ void __launch_bounds__(kSThreads, kMinBlocks)
 k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_words,
                const uint4* __restrict__ bits, const uint32_t* __restrict__ first_row,
@@ -104,7 +104,7 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
                CountScratch scr, const uint32_t* __restrict__ graph_rows, uint32_t num_graphs,
                unsigned long long* __restrict__ graph_counts, const uint32_t* __restrict__ row_indices,
                const uint32_t* __restrict__ indices, int log2c, uint32_t tile_begin, uint32_t tile_end,
-               bool whole, bool lower, const unsigned long long* __restrict__ build_meta)
+               bool lower, const unsigned long long* __restrict__ build_meta)
 {
     using Key = RowKey<kWide>;
     using KeyWord = typename Key::Word;
@@ -125,7 +125,7 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
     uint32_t cut_lo_u = 0, cut_lo_c = 0, cut_hi_u = 0xffffffffu, cut_hi_c = 0xffffffffu;
     if (build_meta) build_failed = (build_meta[kMetaBad] | build_meta[kMetaOverflow]) != 0ull;
     if (!build_failed) {
-        if (whole) {
+        if constexpr (!kRange) {
             e_hi = n_row_blocks ? kRowRun + (uint32_t)*rs_chunks : 0u;
         } else {
             if (build_meta) tile_end = (uint32_t)min((unsigned long long)tile_end, build_meta[kMetaTiles]);
@@ -285,7 +285,7 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
                 if (b.x) b.x &= b.x - 1;
                 else b.y &= b.y - 1;
             }
-            if (u < cut_lo_u || u >= cut_hi_u) {
+            if (kRange && (u < cut_lo_u || u >= cut_hi_u)) {
                 // a tile range's first or last row block: drop the columns outside it
                 uint32_t* w = reinterpret_cast<uint32_t*>(&b);
 #pragma unroll
@@ -375,33 +375,89 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
         __syncwarp();
     };
 
-    // Work queue: `per` chunks each, or one row block each.  A warp's first grab is its own
-    // index, later ones are numbered by an atomic.  A chunk of a hub row in natural order
-    // holds up to 1,024 neighbours with long rows, so grabs stay at one 32nd of an even
-    // share, one to eight chunks (R-MAT scale 18 in natural order: 2.83 ms with runs of
-    // four chunks and an eighth of a share, 2.05 with these).
+    // Work queue, `per` chunks each.  A warp's first grab is its own index, later ones are
+    // numbered by an atomic.  A chunk of a hub row in natural order holds up to 1,024 neighbours
+    // with long rows, so grabs stay at one 32nd of an even share, one to eight chunks (R-MAT scale
+    // 18 in natural order: 2.83 ms with runs of four chunks and an eighth of a share, 2.05 with
+    // these).
+    //
+    // The row blocks of a tile range lie anywhere in the store, so their chunks are numbered by
+    // pass: pass p has the chunks from p * per on of every row block, up to a little more than the
+    // average row block's; what longer ones have past that comes in slices, for which a grab looks
+    // at up to 32 row blocks, so that the slices that are not there (most of them where a hub has a
+    // hundred times the average) stay few beside the rest: a quarter of the first passes' grabs, and
+    // up to eight times that where the longest row block is 32 times the average.  (A row block per grab left
+    // a hub's to one warp: a quarter of R-MAT scale 20, edge factor 8, in natural order took 124
+    // ms; 6.6 like this.)
     __syncwarp();
     const uint64_t nwarps = (uint64_t)gridDim.x * kSWarps;
-    const uint32_t work = whole ? (e_hi > kRowRun ? e_hi - kRowRun : 0u) : I_hi - I_lo;
-    const uint64_t share = work / (nwarps * 32);
-    const uint32_t per = whole ? (uint32_t)(share < 1 ? 1 : (share > 8 ? 8 : share)) : 1u;
+    const uint32_t nb = I_hi - I_lo;
+    uint64_t work = e_hi > kRowRun ? e_hi - kRowRun : 0u;
+    uint32_t avg = 1, longest = 0;
+    if constexpr (kRange) {
+        avg = (uint32_t)max(rs_chunks[0] / max(n_row_blocks, 1u), 1ull);
+        longest = (uint32_t)rs_chunks[kMetaRowLong - kMetaRowChunks];
+        work = (uint64_t)avg * nb;
+    }
+    const uint64_t share = work / (nwarps * (kRange ? 8 : 32));
+    const uint32_t per = (uint32_t)(share < 1 ? 1 : (share > 8 ? 8 : share));
+    uint64_t grabs = (work + per - 1) / per, front = 0;
+    uint32_t groups = 1, width = 1, slice = 1, from = 0;
+    if constexpr (kRange) {
+        const uint32_t passes = (avg + avg / 4 + per - 1) / per;
+        from = passes * per;
+        front = (uint64_t)passes * nb;
+        grabs = front;
+        if (longest > from && nb) {
+            const uint64_t most = max(4 * nwarps, front / 4) * min(max(longest / (4 * avg), 1u), 8u);
+            const uint64_t slices = (longest - from + per - 1) / per;
+            width = (uint32_t)min((slices * nb + most - 1) / most, (uint64_t)kWarp);
+            groups = (nb + width - 1) / width;
+            slice = per * (uint32_t)((slices * groups + most - 1) / most);
+            grabs += (uint64_t)groups * ((longest - from + slice - 1) / slice);
+        }
+    }
     unsigned long long kq = (unsigned long long)blockIdx.x * kSWarps + warp;
-    while (kq * per < work) {
+    while (kq < grabs) {
         unsigned long long next = 0;
         if (lane == 0) next = nwarps + atomicAdd(scr.work, 1ull);
-        // chunks [e0, e1), row block by row block
-        uint32_t e0, e1, u;
-        if (whole) {
+        // chunks [e0, e1), row block by row block; of a range, lane l's chunks of its row block
+        uint32_t e0 = 0, e1 = 0, u = 0;
+        uint32_t lane_e0 = 0, lane_e1 = 0, lane_I = 0;
+        unsigned pieces = 0;
+        if constexpr (!kRange) {
             e0 = kRowRun + (uint32_t)(kq * per);
             e1 = min(e_hi, e0 + per);
             u = first_row[e0 / kRowRun];
         } else {
-            u = 16u * (I_lo + (uint32_t)kq);
-            e0 = off[u + (u >> 4)];
-            e1 = off[u + (u >> 4) + 16];
+            uint32_t a, b;
+            if (kq < front) {
+                lane_I = lane == 0 ? I_lo + (uint32_t)(kq % nb) : I_hi;
+                a = (uint32_t)(kq / nb) * per;
+                b = a + per;
+            } else {
+                const uint64_t x = kq - front;
+                lane_I = lane < width ? I_lo + (uint32_t)(x % groups) + lane * groups : I_hi;
+                a = from + (uint32_t)(x / groups) * slice;
+                b = a + slice;
+            }
+            if (lane_I < I_hi) {
+                const uint32_t first = off[17u * lane_I], end = off[17u * lane_I + 16];
+                lane_e0 = min(first + a, end);
+                lane_e1 = min(first + b, end);
+            }
+            pieces = __ballot_sync(kFull, lane_e0 < lane_e1);
         }
-        while (e0 < e1) {
-            const uint32_t I = u >> 4, l = min(lane, 16);
+        while (kRange ? pieces != 0u : e0 < e1) {
+            uint32_t I = u >> 4;
+            if constexpr (kRange) {
+                const int p = __ffs(pieces) - 1;
+                pieces &= pieces - 1;
+                I = __shfl_sync(kFull, lane_I, p);
+                e0 = __shfl_sync(kFull, lane_e0, p);
+                e1 = __shfl_sync(kFull, lane_e1, p);
+            }
+            const uint32_t l = min(lane, 16);
             const uint32_t o = off[17u * I + l];
             const uint32_t o1 = __shfl_down_sync(kFull, o, 1);
             const uint32_t fa = max(o, e0), fb = min(o1, e1);
@@ -420,10 +476,12 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
                 take_row(16u * I + r, __shfl_sync(kFull, o, r), __shfl_sync(kFull, o1, r),
                          __shfl_sync(kFull, fa, r), __shfl_sync(kFull, fb, r));
             }
-            // the next row block's first run
-            const uint32_t end = __shfl_sync(kFull, o, 16);
-            e0 = max(e0 + 1, (end + kRowRun - 1) / kRowRun * kRowRun);
-            if (e0 < e1) u = first_row[e0 / kRowRun];
+            if constexpr (!kRange) {
+                // the next row block's first run
+                const uint32_t end = __shfl_sync(kFull, o, 16);
+                e0 = max(e0 + 1, (end + kRowRun - 1) / kRowRun * kRowRun);
+                if (e0 < e1) u = first_row[e0 / kRowRun];
+            }
         }
         kq = __shfl_sync(kFull, next, 0);
     }
@@ -434,26 +492,29 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
     finish_count<kSThreads>(acc, scr, build_failed, s_red, &s_last);
 }
 
-using StreamKernel = decltype(&k_count_stream<1024, 3, false, false>);
+using StreamKernel = decltype(&k_count_stream<1024, 3, false, false, false>);
 
-// variant: 2 * (table size, then 32-bit keys) + (per-graph counts)
-constexpr int kVariants = 8;
+// variant: 3 * (table size, then 32-bit keys) + (per-graph counts, then tile ranges)
+constexpr int kVariants = 12;
+template <int W, int kMinBlocks, bool kWide>
+StreamKernel stream_kernel_of(int form)
+{
+    if (form == 0) return k_count_stream<W, kMinBlocks, false, kWide, false>;
+    if (form == 1) return k_count_stream<W, kMinBlocks, true, kWide, false>;
+    return k_count_stream<W, kMinBlocks, false, kWide, true>;
+}
 StreamKernel stream_kernel(int v)
 {
-    switch (v) {
-    case 0: return k_count_stream<256, 4, false, false>;
-    case 1: return k_count_stream<256, 4, true, false>;
-    case 2: return k_count_stream<512, 4, false, false>;
-    case 3: return k_count_stream<512, 4, true, false>;
-    case 4: return k_count_stream<1024, 3, false, false>;
-    case 5: return k_count_stream<1024, 3, true, false>;
-    case 6: return k_count_stream<1024, 3, false, true>;
-    default: return k_count_stream<1024, 3, true, true>;
+    switch (v / 3) {
+    case 0: return stream_kernel_of<256, 4, false>(v % 3);
+    case 1: return stream_kernel_of<512, 4, false>(v % 3);
+    case 2: return stream_kernel_of<1024, 3, false>(v % 3);
+    default: return stream_kernel_of<1024, 3, true>(v % 3);
     }
 }
 size_t stream_smem(int v)
 {
-    return v / 2 == 0 ? stream_smem_bytes<256>() : v / 2 == 1 ? stream_smem_bytes<512>() : stream_smem_bytes<1024>();
+    return v / 3 == 0 ? stream_smem_bytes<256>() : v / 3 == 1 ? stream_smem_bytes<512>() : stream_smem_bytes<1024>();
 }
 
 // A variant's dynamic shared memory is an opt-in.
@@ -503,14 +564,13 @@ int launch_count_stream(const RowStore& rs, const unsigned long long* rs_chunks,
                         bool lower, const unsigned long long* build_meta, int grid, cudaStream_t s)
 {
     const int size = row_store_wide(n_row_blocks) ? 3 : max_col_blocks <= 256 ? 0 : max_col_blocks <= 512 ? 1 : 2;
-    const int v = 2 * size + (graph_counts ? 1 : 0);
+    const int v = 3 * size + (!whole ? 2 : graph_counts ? 1 : 0);
     const int per_sm = stream_blocks_per_sm(v);
     if (per_sm < 1 || !allow_stream_smem(v)) return BTC_E_CUDA;
     if (per_sm * device_sm_count() < grid) grid = per_sm * device_sm_count();
     stream_kernel(v)<<<grid, kSThreads, stream_smem(v), s>>>(
         rs.off, rs.key, rs.bits, rs.first_row, rs_chunks, (uint32_t)n_row_blocks, scr, graph_rows, num_graphs,
-        graph_counts, row_indices, indices, tile_cols == 128 ? 7 : 5, tile_begin, tile_end, whole, lower,
-        build_meta);
+        graph_counts, row_indices, indices, tile_cols == 128 ? 7 : 5, tile_begin, tile_end, lower, build_meta);
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 

@@ -126,7 +126,7 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
         key[threadIdx.x] = 0;
         bits[threadIdx.x] = make_uint2(0u, 0u);
     }
-    uint32_t longest = 0;
+    uint32_t longest = 0, most_chunks = 0;
     auto row_block = [&](uint64_t I, uint32_t a, uint32_t b) {
         // ---- the rows' entries (lane r < 16: row r's) -----------------------------------
         uint32_t K = 0, m0 = 0, m1 = 0;
@@ -158,6 +158,7 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
             if (lane >= d) incl += y;
         }
         const uint32_t total = __shfl_sync(kFull, incl, 15);
+        most_chunks = max(most_chunks, total);
         if (w == 0 && lane == 0) {
             const uint32_t want = (total + kRowRun - 1) / kRowRun * kRowRun;
             tm.chunk = kRowRun + (want ? (uint32_t)atomicAdd(&meta[kMetaRowChunks], (unsigned long long)want) : 0u);
@@ -280,6 +281,7 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
         if (b - a <= len_hi && (len_lo == 0 || b - a > len_lo)) row_block(I, a, b);
     }
     if (w == 0 && lane == 0 && longest) atomicMax(&meta[kMetaRowMax], (unsigned long long)longest);
+    if (w == 0 && lane == 0 && most_chunks) atomicMax(&meta[kMetaRowLong], (unsigned long long)most_chunks);
 }
 
 // Raises *bad (and the host's word) where a caller's tiles are not what the store and its count
