@@ -195,8 +195,9 @@ def launches_per_step(n: int, tile_cols: int, orient_degree: bool, m: int, tiles
     store = m >= 8 * R and tiles >= 8 * R
     if group:
         # orient, bucket scan, scatter, row-block count, scan (3), row-block scatter, tile
-        # count, scan (3), last indptr, tiles; the longest row block where no store finds it
-        k = 14 + (0 if store else 1)
+        # count, scan (3), last indptr, tiles, and the heavy row blocks' mark, emit and fill; the
+        # longest row block where no store finds it
+        k = 17 + (0 if store else 1)
     elif bitmap:
         k = 4  # mark, chunk count + scan, emit (+ zero tiles, last indptr), fill
     else:

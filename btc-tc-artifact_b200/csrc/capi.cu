@@ -317,7 +317,7 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
         uint32_t* scratch = g->tile_base.as<uint32_t>();
         BTC_TRY(group_edges(P.d_src, P.d_dst, P.m, P.n, rank, geom.tile_cols, P.col_blocks,
                             k0, k1, g->keys0.as<uint32_t>(), scratch, g->indptr.as<uint32_t>(),
-                            scratch + group_scratch_words(R), meta, s));
+                            scratch + group_scratch_words(R, P.m, P.col_blocks), meta, s));
         if (P.cap) {
             BTC_TRY(launch_finish_tiles(g->indptr.as<uint32_t>(), geom.n_row_blocks, meta, P.cap, g->d_hmeta, s));
             BTC_TRY(enqueue_group_write(g, P, P.cap, s));
@@ -400,6 +400,14 @@ static bool launch_build_graph(btc_bitbsr* g, const BuildPlan& P, cudaStream_t s
     return cudaGraphLaunch(g->graph_exec, s) == cudaSuccess;
 }
 
+// The cell bitmap (one bit per (row block, column block)) replaces the sort when it is small next
+// to the edge list.
+static bool bitmap_takes(const BuildGeom& geom, int64_t m)
+{
+    const uint64_t bytes = 4 * bitmap_words_per_row(geom) * (uint64_t)geom.n_row_blocks;
+    return bytes <= (4ull << 30) && bytes <= 32ull * (uint64_t)m + (64ull << 20);
+}
+
 // tiles_only: the caller keeps the reference-shaped arrays alone, so no row store is made.
 static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
                       int tile_cols, uint32_t flags, cudaStream_t s, bool tiles_only = false,
@@ -415,6 +423,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     bool small = allow_small && !(flags & (BTC_ORIENT_DEGREE | BTC_BUILD_RADIX | BTC_BUILD_ASYNC)) &&
                  small_possible(m, n);
     const bool open_width = small && tile_cols == 0 && !(flags & BTC_INPUT_ON_HOST) && !policy_dense(m, n);
+    int skewed = -1;  // of the row blocks, where the policy's sample has told
     if (open_width) {
         tile_cols = 32;  // the larger cell grid, for the sizes below
     } else if (tile_cols == 0) {
@@ -426,7 +435,8 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         else if ((flags & BTC_BUILD_ASYNC) && (g->tile_cols == 32 || g->tile_cols == 128))
             tile_cols = g->tile_cols;
         else
-            BTC_TRY(policy_select(src, dst, m, n, flags & BTC_INPUT_ON_HOST, s, g->policy, &tile_cols, nullptr));
+            BTC_TRY(policy_select(src, dst, m, n, flags & BTC_INPUT_ON_HOST, s, g->policy, &tile_cols, nullptr,
+                                  bitmap_takes(make_geom(n, 32), m) ? nullptr : &skewed));
     }
     if (tile_cols != 32 && tile_cols != 128) return BTC_E_INVAL;
     BTC_CUDA_TRY(cudaGetDevice(&g->device));
@@ -466,13 +476,8 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         P.d_src = g->in_src.as<int32_t>();
         P.d_dst = g->in_dst.as<int32_t>();
     }
-    // The cell bitmap (one bit per (row block, column block)) replaces the sort when it
-    // is small next to the edge list; otherwise the radix path sorts tile keys.
-    const uint64_t wpr = bitmap_words_per_row(geom);
-    P.bm_words = wpr * (uint64_t)geom.n_row_blocks;
-    const uint64_t bm_bytes = 4 * P.bm_words;
-    P.use_bitmap = !(flags & BTC_BUILD_RADIX) && bm_bytes <= (4ull << 30) &&
-                   bm_bytes <= 32ull * (uint64_t)m + (64ull << 20);
+    P.bm_words = bitmap_words_per_row(geom) * (uint64_t)geom.n_row_blocks;
+    P.use_bitmap = !(flags & BTC_BUILD_RADIX) && bitmap_takes(geom, m);
     small = small && P.use_bitmap;
     // An enqueued build is one that the bitmap takes, whichever builder then runs; on any other
     // graph the call waits, and grows the arrays where they are too small.
@@ -481,13 +486,29 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     // (see kGroupEdges), and so is what the bitmap does not take.
     P.col_blocks = (uint64_t)geom.n_col_blocks;
     P.degree = (flags & BTC_ORIENT_DEGREE) && n > 0;
+    // (the first of the large buffers: the time of the degree count's atomics differs by up to a
+    // fifth with where its words lie, which is not to follow from the others' sizes)
+    if (P.degree) {
+        BTC_TRY(g->deg.reserve(sizeof(uint32_t) * (size_t)n));
+        BTC_TRY(g->rank.reserve(sizeof(int32_t) * (size_t)n));
+    }
     P.use_group = !(flags & BTC_BUILD_RADIX) && group_possible(n, P.col_blocks) &&
                   (!P.use_bitmap || (P.degree && m >= kGroupEdges));
+    // In natural order a hub's row block may have any share of the edges, and its row blocks' tiles
+    // are too much for a CTA each: such a list is sorted.
+    if (P.use_group && !P.degree) {
+        if (skewed < 0) {
+            bool is = false;
+            BTC_TRY(policy_skewed(src, dst, m, (flags & BTC_INPUT_ON_HOST) != 0, s, g->policy, &is));
+            skewed = is;
+        }
+        if (skewed) P.use_group = false;
+    }
     if (P.use_group) {
         const uint64_t R = (uint64_t)geom.n_row_blocks;
         if (g->keys0.reserve(sizeof(uint64_t) * (size_t)(m ? m : 1)) != BTC_OK ||
             g->keys1.reserve(sizeof(uint64_t) * (size_t)(m ? m : 1)) != BTC_OK ||
-            g->tile_base.reserve(sizeof(uint32_t) * (group_scratch_words((uint32_t)R) + ri_scan_blocks((uint32_t)R) + 1)) != BTC_OK) {
+            g->tile_base.reserve(sizeof(uint32_t) * (group_scratch_words((uint32_t)R, m, P.col_blocks) + ri_scan_blocks((uint32_t)R) + 1)) != BTC_OK) {
             if (!P.use_bitmap) return BTC_E_NOMEM;
             P.use_group = false;  // the bitmap may still fit
         }
@@ -506,10 +527,6 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     if (!P.use_group) {
         const size_t chunk_slots = P.use_bitmap ? bitmap_chunks(P.bm_words) : sort_tiles((size_t)m);
         BTC_TRY(g->tile_base.reserve(sizeof(uint32_t) * (chunk_slots + 1)));
-    }
-    if (P.degree) {
-        BTC_TRY(g->deg.reserve(sizeof(uint32_t) * (size_t)n));
-        BTC_TRY(g->rank.reserve(sizeof(int32_t) * (size_t)n));
     }
     if (P.use_bitmap) {
         BTC_TRY(g->bitmap.reserve(sizeof(uint32_t) * (P.bm_words ? P.bm_words : 1)));

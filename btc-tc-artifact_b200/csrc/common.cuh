@@ -339,13 +339,13 @@ int launch_rowindex(const uint32_t* indptr, const uint32_t* indices, int32_t n_r
 // at hand tells them from a power-law graph.
 constexpr int64_t kGroupEdges = 1 << 22;
 bool group_possible(int64_t n, uint64_t col_blocks);
-size_t group_scratch_words(uint32_t R);
+size_t group_scratch_words(uint32_t R, int64_t m, uint64_t col_blocks);
 int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
                 const int32_t* rank, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
                 uint64_t* grouped, uint32_t* edges, uint32_t* scratch, uint32_t* indptr, uint32_t* bsum,
                 unsigned long long* meta, cudaStream_t s);
 int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
-                const uint32_t* edges, const uint32_t* scratch, const uint32_t* indptr,
+                const uint32_t* edges, uint32_t* scratch, const uint32_t* indptr,
                 const unsigned long long* meta, uint32_t cap, uint32_t* indices, uint32_t* row_indices,
                 uint32_t* blocks, uint32_t* rowmask, uint32_t tiles_hint, cudaStream_t s);
 // indptr[R] = the tile count, the overflow flag and the host's status slots (bitmap.cu).
@@ -414,17 +414,20 @@ int launch_build_small(const SmallBuild& b, cudaStream_t s);
 
 struct PolicyWords {
     DevBuf dev;                          // two sums and a ticket
+    DevBuf skew;                         // counters of the skew sample, the most, a ticket
     unsigned long long* host = nullptr;  // a host slot
     unsigned long long host_context = 0;
     bool dirty = false;                  // a call did not come to its end
     void release()
     {
-        if (host && wait_device(dev.device) != cudaSuccess) {
+        if (host && wait_device(dev.ptr ? dev.device : skew.device) != cudaSuccess) {
             cudaGetLastError();
             host = nullptr;  // (something may still write to it)
             dev.release();
+            skew.release();
         }
         dev.release_idle();
+        skew.release_idle();
         host_slot_free(host, host_context);
         host = nullptr;
     }
@@ -433,8 +436,13 @@ int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n
                     const int64_t* e_off, const int32_t* nv, uint32_t G, cudaStream_t s, PolicyWords& w,
                     double* L);
 // btc_select_tile_policy with the caller's words.
+// skewed (nullable): also policy_skewed's answer, where a device sample is taken (else unchanged).
 int policy_select(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, uint32_t flags, cudaStream_t s,
-                  PolicyWords& w, int* tile_cols, int* tau);
+                  PolicyWords& w, int* tile_cols, int* tau, int* skewed = nullptr);
+// Whether one row block of 16 vertices has about a 1,024th of the oriented edges or more, by a sample
+// (a wait on device input).
+int policy_skewed(const int32_t* src, const int32_t* dst, int64_t m, bool on_host, cudaStream_t s, PolicyWords& w,
+                  bool* skewed);
 
 // Device metadata slots of a build (uint64 each): valid keys, out-of-range flag, tile
 // count, unique edges, sort length, longest row-block list, tile-capacity overflow flag,

@@ -16,11 +16,15 @@
 //                 space reserved per bucket (order inside a bucket is free)
 //   k_rb_count    edges per row block; scanned into the row blocks' offsets
 //   k_rb_scatter  every edge to its row block, as a 32-bit word (row in block << 28 | column)
-//   k_count_tiles one CTA per row block: distinct column blocks, by a shared bitmap
+//   k_count_tiles one CTA per row block: distinct column blocks, by a shared bitmap; a heavy row
+//                 block (heavy_edges) is only listed
+//   k_heavy_mark  the listed ones, a CTA per slice of their edges: bitmap in device memory, tiles
 //   (scan)        tile offsets
 //   k_write_tiles one CTA per row block: the bitmap again with a popcount prefix (tile order
 //                 is column order), indices, row_indices, tiles ORed in shared memory and
 //                 written once, row-occupancy masks
+//   k_heavy_emit  the listed ones: prefix, indices, row_indices, tiles and masks zeroed
+//   k_heavy_fill  ... and filled, a CTA per slice of their edges
 //
 // Needs columns below 2^28 and a row block's column bitmap in shared memory (kMaxWords
 // words).  Duplicate edges OR the same bit.
@@ -99,9 +103,11 @@ k_orient(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64
         if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
-// base[b] = edges of buckets below b (base[kBuckets] = all); cursor = the same.
+// base[b] = edges of buckets below b (base[kBuckets] = all); cursor = the same.  No row block is
+// listed as heavy yet.
 __global__ void __launch_bounds__(1024)
-k_bucket_scan(const uint32_t* __restrict__ hist, uint32_t* __restrict__ base, uint32_t* __restrict__ cursor)
+k_bucket_scan(const uint32_t* __restrict__ hist, uint32_t* __restrict__ base, uint32_t* __restrict__ cursor,
+              uint32_t* __restrict__ heavy_count)
 {
     __shared__ uint32_t s_warp[32];
     static_assert(kBuckets == 2048, "two buckets per thread");
@@ -111,6 +117,7 @@ k_bucket_scan(const uint32_t* __restrict__ hist, uint32_t* __restrict__ base, ui
     base[2 * threadIdx.x] = cursor[2 * threadIdx.x] = ex;
     base[2 * threadIdx.x + 1] = cursor[2 * threadIdx.x + 1] = ex + a;
     if (threadIdx.x == 1023) base[kBuckets] = total;
+    if (threadIdx.x == 0) *heavy_count = 0;
 }
 
 // ---- edges to buckets --------------------------------------------------------------------
@@ -219,10 +226,33 @@ __device__ __forceinline__ void tile_span(const uint64_t (&p)[kSItems], uint32_t
     span = s_mm[1] >= lo ? s_mm[1] - lo + 1 : 0u;
 }
 
-// cnt[I] += the edges of row block I.
+// Row blocks with so many edges that one CTA each would be the last to end (a clique's): above
+// 4,096 edges and a 512th of all, so there are fewer than 512 of them.  They are built by slices of
+// kSlice edges through bitmaps in device memory.  Cliques of 2,900 and 6,000 among sparse pairs on
+// 200,000 and 1M vertices, in degree order, 16x128: build 0.46 -> 0.36 and 1.45 -> 1.34 ms; where
+// there are none the three launches cost 8 us.
+constexpr uint32_t kMaxHeavy = 512;
+constexpr uint32_t kHeavyLeast = 4096;
+constexpr uint32_t kSlice = 2048;
+inline uint32_t heavy_edges(int64_t m) { return (uint32_t)std::max<int64_t>(kHeavyLeast, m / kMaxHeavy); }
+inline uint32_t heavy_most(int64_t m) { return (uint32_t)std::min<int64_t>(kMaxHeavy, m / kHeavyLeast); }
+struct Heavy {
+    uint32_t* count;
+    uint32_t* list;  // row blocks
+    uint32_t* done;  // slices marked
+    uint32_t* bm;    // a bitmap of `words` words each
+    uint32_t* pre;   // tiles of the row block before each word
+    uint32_t limit;  // edges of a row block that is not heavy, at most
+    uint32_t most;   // room in the arrays above
+};
+
+// cnt[I] += the edges of row block I.  Also zeroes the heavy row blocks' bitmaps.
 __global__ void __launch_bounds__(kSThreads)
-k_rb_count(const uint64_t* __restrict__ in, const uint32_t* __restrict__ d_m, uint32_t* __restrict__ cnt)
+k_rb_count(const uint64_t* __restrict__ in, const uint32_t* __restrict__ d_m, uint32_t* __restrict__ cnt,
+           uint32_t* __restrict__ bitmaps, uint32_t bitmap_words)
 {
+    for (uint32_t i = blockIdx.x * kSThreads + threadIdx.x; i < bitmap_words; i += gridDim.x * kSThreads)
+        bitmaps[i] = 0;
     __shared__ uint32_t s_cnt[kSpan];
     __shared__ uint32_t s_mm[2];
     const uint32_t m = *d_m;
@@ -302,14 +332,16 @@ constexpr uint32_t kDirect = 1u << 18;  // looks at an edge from which a row blo
 template <int LOG2C, int kTThreads>
 __global__ void __launch_bounds__(kTThreads)
 k_count_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ rb_end, uint32_t R,
-              uint32_t words, uint32_t* __restrict__ indptr)
+              uint32_t words, uint32_t* __restrict__ indptr, Heavy hv)
 {
     extern __shared__ uint32_t s_bm[];
     __shared__ uint32_t s_red[kTThreads / kWarp];
     for (uint32_t i = threadIdx.x; i < words; i += kTThreads) s_bm[i] = 0;
     __syncthreads();
     for (uint32_t I = blockIdx.x; I < R; I += gridDim.x) {
-        const uint32_t e0 = I ? rb_end[I - 1] : 0u, e1 = rb_end[I];
+        const uint32_t e0 = I ? rb_end[I - 1] : 0u, end = rb_end[I];
+        const bool heavy = end - e0 > hv.limit;
+        const uint32_t e1 = heavy ? e0 : end;
         uint32_t mine = 0;
         for (uint32_t e = e0 + threadIdx.x; e < e1; e += kTThreads) {
             const uint32_t cb = (edges[e] & 0x0fffffffu) >> LOG2C;
@@ -323,7 +355,15 @@ k_count_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
         if (threadIdx.x == 0) {
             uint32_t t = 0;
             for (int w = 0; w < kTThreads / kWarp; ++w) t += s_red[w];
-            indptr[I] = t;
+            if (!heavy) {
+                indptr[I] = t;
+            } else {
+                const uint32_t at = atomicAdd(hv.count, 1u);
+                if (at < hv.most) {
+                    hv.list[at] = I;
+                    hv.done[at] = 0;
+                }
+            }
         }
         for (uint32_t e = e0 + threadIdx.x; e < e1; e += kTThreads)
             s_bm[((edges[e] & 0x0fffffffu) >> LOG2C) >> 5] = 0;
@@ -336,7 +376,7 @@ __global__ void __launch_bounds__(kTThreads)
 k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ rb_end, uint32_t R,
               uint32_t words, const uint32_t* __restrict__ indptr, const unsigned long long* __restrict__ d_tiles, uint32_t cap,
               uint32_t* __restrict__ indices, uint32_t* __restrict__ row_indices, uint4* __restrict__ blocks,
-              uint32_t* __restrict__ rowmask, uint32_t NT)
+              uint32_t* __restrict__ rowmask, uint32_t NT, uint32_t heavy_limit)
 {
     if (*d_tiles > cap) return;  // more tiles than the arrays hold: the builder redoes this step
     constexpr int C = 1 << LOG2C;
@@ -383,7 +423,7 @@ k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
     for (; I < R; I += gridDim.x, e0 = ne0, e1 = ne1, t0 = nt0, t1 = nt1) {
         const uint32_t nt = t1 - t0;
         bounds(I + gridDim.x, ne0, ne1, nt0, nt1);
-        if (nt == 0) {  // uniform for the CTA
+        if (nt == 0 || e1 - e0 > heavy_limit) {  // uniform for the CTA
             hold(ne0, ne1);
             continue;
         }
@@ -486,6 +526,150 @@ k_write_tiles(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ r
     if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// ---- heavy row blocks ------------------------------------------------------------------------
+constexpr int kHThreads = 512;
+
+// The slices of the listed row blocks: f(h, I, first edge, end, slices of h) for this CTA's.
+template <class F>
+__device__ __forceinline__ void each_slice(const Heavy& hv, const uint32_t* __restrict__ rb_end, F f)
+{
+    static_assert(kMaxHeavy == kHThreads, "a row block per thread");
+    __shared__ uint32_t s_first[kMaxHeavy];  // slices of the row blocks before
+    __shared__ uint32_t s_scan[kHThreads / kWarp];
+    const uint32_t n = min(*hv.count, hv.most);
+    if (n == 0) return;
+    auto slices = [&](uint32_t h) -> uint32_t {
+        if (h >= n) return 0u;
+        const uint32_t I = hv.list[h];
+        return (rb_end[I] - (I ? rb_end[I - 1] : 0u) + kSlice - 1) / kSlice;
+    };
+    uint32_t total;
+    s_first[threadIdx.x] = cta_exclusive_scan<kHThreads>(slices(threadIdx.x), s_scan, total);
+    __syncthreads();
+    for (uint32_t s = blockIdx.x; s < total; s += gridDim.x) {
+        uint32_t h = 0, end = n;  // the last row block with s_first <= s
+        while (end - h > 1) {
+            const uint32_t mid = (h + end) >> 1;
+            if (s_first[mid] <= s) h = mid;
+            else end = mid;
+        }
+        const uint32_t I = hv.list[h];
+        const uint32_t e = (I ? rb_end[I - 1] : 0u) + (s - s_first[h]) * kSlice;
+        f(h, I, e, min(e + kSlice, rb_end[I]), (h + 1 < n ? s_first[h + 1] : total) - s_first[h]);
+    }
+}
+
+// The bitmaps of the row blocks' column blocks; a row block's last slice counts its tiles.
+template <int LOG2C>
+__global__ void __launch_bounds__(kHThreads)
+k_heavy_mark(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ rb_end, uint32_t words, Heavy hv,
+             uint32_t* __restrict__ indptr)
+{
+    extern __shared__ uint32_t s_bm[];
+    __shared__ uint32_t s_red[kHThreads / kWarp];
+    __shared__ int s_last;
+    each_slice(hv, rb_end, [&](uint32_t h, uint32_t I, uint32_t e0, uint32_t e1, uint32_t slices) {
+        uint32_t* bm = hv.bm + (size_t)h * words;
+        for (uint32_t w = threadIdx.x; w < words; w += kHThreads) s_bm[w] = 0;
+        __syncthreads();
+        for (uint32_t e = e0 + threadIdx.x; e < e1; e += kHThreads) {
+            const uint32_t cb = (edges[e] & 0x0fffffffu) >> LOG2C;
+            const uint32_t bit = 1u << (cb & 31u);
+            if (!(*(volatile uint32_t*)&s_bm[cb >> 5] & bit)) atomicOr(&s_bm[cb >> 5], bit);
+        }
+        __syncthreads();
+        for (uint32_t w = threadIdx.x; w < words; w += kHThreads)
+            if (s_bm[w]) atomicOr(&bm[w], s_bm[w]);
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(&hv.done[h], 1u) == slices - 1;
+        __syncthreads();
+        if (s_last) {
+            __threadfence();
+            uint32_t sum = 0;
+            for (uint32_t w = threadIdx.x; w < words; w += kHThreads) sum += __popc(__ldcg(&bm[w]));
+            uint32_t total;
+            cta_exclusive_scan<kHThreads>(sum, s_red, total);
+            if (threadIdx.x == 0) indptr[I] = total;
+        }
+        __syncthreads();
+    });
+}
+
+constexpr int kEThreads = 256;
+constexpr uint32_t kSegWords = 128;  // words a CTA of k_heavy_emit takes
+
+// Tile numbers before each word, indices and row_indices; tiles and masks zeroed.
+__global__ void __launch_bounds__(kEThreads)
+k_heavy_emit(uint32_t words, Heavy hv, const uint32_t* __restrict__ indptr,
+             const unsigned long long* __restrict__ d_tiles, uint32_t cap, uint32_t vec4,
+             uint32_t* __restrict__ indices, uint32_t* __restrict__ row_indices, uint4* __restrict__ blocks,
+             uint32_t* __restrict__ rowmask)
+{
+    if (*d_tiles > cap) return;
+    __shared__ uint32_t s_scan[kEThreads / kWarp];
+    const uint32_t segs = (words + kSegWords - 1) / kSegWords;
+    const uint32_t n = min(*hv.count, hv.most);
+    for (uint32_t u = blockIdx.x; u < n * segs; u += gridDim.x) {
+        const uint32_t h = u / segs, w0 = (u % segs) * kSegWords;
+        const uint32_t I = hv.list[h];
+        const uint32_t* bm = hv.bm + (size_t)h * words;
+        uint32_t sum = 0;
+        for (uint32_t w = threadIdx.x; w < w0; w += kEThreads) sum += __popc(bm[w]);
+        uint32_t base, total;
+        cta_exclusive_scan<kEThreads>(sum, s_scan, base);
+        const uint32_t w = w0 + threadIdx.x;
+        uint32_t x = threadIdx.x < kSegWords && w < words ? bm[w] : 0u;
+        uint32_t t = base + cta_exclusive_scan<kEThreads>(__popc(x), s_scan, total);
+        if (threadIdx.x < kSegWords && w < words) hv.pre[(size_t)h * words + w] = t;
+        const size_t t0 = indptr[I];
+        for (; x; x &= x - 1, ++t) {
+            indices[t0 + t] = w * 32 + (__ffs(x) - 1);
+            row_indices[t0 + t] = I;
+        }
+        for (uint32_t i = threadIdx.x; i < total; i += kEThreads) rowmask[t0 + base + i] = 0u;
+        for (size_t i = threadIdx.x; i < (size_t)total * vec4; i += kEThreads)
+            blocks[(t0 + base) * vec4 + i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+
+template <int LOG2C>
+__global__ void __launch_bounds__(kHThreads)
+k_heavy_fill(const uint32_t* __restrict__ edges, const uint32_t* __restrict__ rb_end, uint32_t words, Heavy hv,
+             const uint32_t* __restrict__ indptr, const unsigned long long* __restrict__ d_tiles, uint32_t cap,
+             uint32_t* __restrict__ blocks, uint32_t* __restrict__ rowmask)
+{
+    if (*d_tiles > cap) return;
+    constexpr int C = 1 << LOG2C, WPR = C / 32, TW = 16 * WPR, U = 4;
+    each_slice(hv, rb_end, [&](uint32_t h, uint32_t I, uint32_t e0, uint32_t e1, uint32_t) {
+        const uint32_t* bm = hv.bm + (size_t)h * words;
+        const uint32_t* pre = hv.pre + (size_t)h * words;
+        const size_t t0 = indptr[I];
+        for (uint32_t e = e0 + threadIdx.x; e < e1; e += U * kHThreads) {
+            uint32_t x[U], old[U];
+            size_t t[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) x[k] = e + k * kHThreads < e1 ? edges[e + k * kHThreads] : 0u;
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                const uint32_t cb = (x[k] & 0x0fffffffu) >> LOG2C;
+                t[k] = t0 + pre[cb >> 5] + __popc(bm[cb >> 5] & ((1u << (cb & 31u)) - 1u));
+            }
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                const uint32_t cl = x[k] & (C - 1), r = x[k] >> 28;
+                old[k] = 1u;
+                if (e + k * kHThreads < e1) old[k] = atomicOr(&blocks[t[k] * TW + r * WPR + (cl >> 5)], 1u << (cl & 31u));
+            }
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                const uint32_t cl = x[k] & (C - 1), r = x[k] >> 28;
+                if (old[k] == 0u) atomicOr(&rowmask[t[k]], 1u << (r + (C == 128 ? (cl & 64u) / 4u : 0u)));
+            }
+        }
+    });
+}
+
 }  // namespace gp
 
 // Row bits below a bucket: at most kBuckets buckets of whole row blocks.
@@ -507,12 +691,34 @@ bool group_possible(int64_t n, uint64_t col_blocks)
     return n > 0 && n <= (1ll << 28) && (col_blocks + 31) / 32 <= gp::kMaxWords;
 }
 
-size_t group_scratch_words(uint32_t R) { return 3 * (size_t)gp::kBuckets + 1 + (size_t)R + 3; }
+// Buckets, row-block ends, a sum; then the heavy row blocks' lists and bitmaps.
+static size_t group_front_words(uint32_t R) { return 3 * (size_t)gp::kBuckets + 1 + (size_t)R + 3; }
+static uint32_t bitmap_row_words(uint64_t col_blocks) { return (uint32_t)((col_blocks + 31) / 32); }
+
+size_t group_scratch_words(uint32_t R, int64_t m, uint64_t col_blocks)
+{
+    return group_front_words(R) + 1 + 2 * (size_t)gp::kMaxHeavy +
+           2 * (size_t)gp::heavy_most(m) * bitmap_row_words(col_blocks);
+}
+
+static gp::Heavy heavy_of(uint32_t* scratch, uint32_t R, int64_t m, uint64_t col_blocks)
+{
+    uint32_t* at = scratch + group_front_words(R);
+    gp::Heavy h{};
+    h.count = at;
+    h.list = at + 1;
+    h.done = h.list + gp::kMaxHeavy;
+    h.bm = h.done + gp::kMaxHeavy;
+    h.most = gp::heavy_most(m);
+    h.pre = h.bm + (size_t)h.most * bitmap_row_words(col_blocks);
+    h.limit = gp::heavy_edges(m);
+    return h;
+}
 
 // The edges grouped by row block and the row blocks' tile counts scanned into indptr.
 // pairs: m uint64 (only written with rank); grouped: m uint64 of scratch whose
 // contents end up in `edges` (m words, may share memory with pairs); scratch:
-// group_scratch_words(R); bsum: scan scratch of R words.  Writes meta[kMetaBad] and
+// group_scratch_words(R, m, col_blocks); bsum: scan scratch of R words.  Writes meta[kMetaBad] and
 // meta[kMetaTiles].
 int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
                 const int32_t* rank, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
@@ -524,7 +730,8 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
     uint32_t* cursor = scratch + gp::kBuckets;
     uint32_t* base = cursor + gp::kBuckets;
     uint32_t* rb_end = base + gp::kBuckets + 1;  // offsets at first, then (moved on) ends
-    unsigned long long* sum = reinterpret_cast<unsigned long long*>(scratch + (group_scratch_words(R) - 2) / 2 * 2);
+    unsigned long long* sum = reinterpret_cast<unsigned long long*>(scratch + (group_front_words(R) - 2) / 2 * 2);
+    const gp::Heavy hv = heavy_of(scratch, R, m, col_blocks);
     const int shift = bucket_shift(n);
     if (cudaMemsetAsync(hist, 0, sizeof(uint32_t) * gp::kBuckets, s) != cudaSuccess) return BTC_E_CUDA;
     const bool store = rank != nullptr;
@@ -533,7 +740,7 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
     if (m > 0)
         gp::k_orient<<<ogrid, gp::kOThreads, 0, s>>>(src, dst, m, n, rank, shift,
                                                      store ? pairs : nullptr, hist, meta + kMetaBad);
-    gp::k_bucket_scan<<<1, 1024, 0, s>>>(hist, base, cursor);
+    gp::k_bucket_scan<<<1, 1024, 0, s>>>(hist, base, cursor, hv.count);
     static std::atomic<unsigned long long> scatter_ok[kMaxDevices];
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(&gp::k_scatter), sizeof(gp::ScatterSmem), scatter_ok))
         return BTC_E_CUDA;
@@ -543,26 +750,30 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
     if (cudaMemsetAsync(rb_end, 0, sizeof(uint32_t) * (size_t)R, s) != cudaSuccess) return BTC_E_CUDA;
     const unsigned stiles = (unsigned)((m + gp::kSTile - 1) / gp::kSTile);
     const uint32_t* d_m = base + gp::kBuckets;
-    if (m > 0) gp::k_rb_count<<<stiles, gp::kSThreads, 0, s>>>(grouped, d_m, rb_end);
+    if (m > 0)
+        gp::k_rb_count<<<stiles, gp::kSThreads, 0, s>>>(grouped, d_m, rb_end, hv.bm,
+                                                        hv.most * bitmap_row_words(col_blocks));
     BTC_TRY(launch_scan_u32(rb_end, R, bsum, sum, s));
     if (m > 0) gp::k_rb_scatter<<<stiles, gp::kSThreads, 0, s>>>(grouped, d_m, rb_end, edges);
-    const uint32_t words = (uint32_t)((col_blocks + 31) / 32);
+    const uint32_t words = bitmap_row_words(col_blocks);
     const int threads = row_block_threads(m, R);
     const uint32_t grid = std::min<uint32_t>(R, 32u * device_sm_count() * (128 / threads));
-    auto count = [&](auto kernel) {
-        kernel<<<grid, threads, 4 * words, s>>>(edges, rb_end, R, words, indptr);
+    auto count = [&](auto kernel, auto mark) {
+        kernel<<<grid, threads, 4 * words, s>>>(edges, rb_end, R, words, indptr, hv);
+        if (hv.most)
+            mark<<<2 * device_sm_count(), gp::kHThreads, 4 * words, s>>>(edges, rb_end, words, hv, indptr);
     };
     if (tile_cols == 128)
-        threads == 32 ? count(gp::k_count_tiles<7, 32>) : count(gp::k_count_tiles<7, 128>);
+        count(threads == 32 ? gp::k_count_tiles<7, 32> : gp::k_count_tiles<7, 128>, gp::k_heavy_mark<7>);
     else
-        threads == 32 ? count(gp::k_count_tiles<5, 32>) : count(gp::k_count_tiles<5, 128>);
+        count(threads == 32 ? gp::k_count_tiles<5, 32> : gp::k_count_tiles<5, 128>, gp::k_heavy_mark<5>);
     return launch_scan_u32(indptr, R, bsum, meta + kMetaTiles, s);
 }
 
 // Tiles, indices, row_indices and row masks from the grouped edges (indptr[R] set), against
 // `cap` tiles: nothing when meta[kMetaTiles] is above it.
 int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
-                const uint32_t* edges, const uint32_t* scratch, const uint32_t* indptr,
+                const uint32_t* edges, uint32_t* scratch, const uint32_t* indptr,
                 const unsigned long long* meta, uint32_t cap, uint32_t* indices, uint32_t* row_indices,
                 uint32_t* blocks, uint32_t* rowmask, uint32_t tiles_hint, cudaStream_t s)
 {
@@ -580,15 +791,27 @@ int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
     static std::atomic<unsigned long long> ok[4][kMaxDevices];
     const int threads = row_block_threads(m, R);
     const uint32_t grid = std::min<uint32_t>(R, 32u * device_sm_count() * (128 / threads));
-    auto write = [&](auto kernel, int which) {
+    const gp::Heavy hv = heavy_of(scratch, R, m, col_blocks);
+    const uint32_t hwords = bitmap_row_words(col_blocks);
+    auto write = [&](auto kernel, int which, auto fill) {
         if (!allow_dynamic_smem(reinterpret_cast<const void*>(kernel), most, ok[which])) return BTC_E_CUDA;
         kernel<<<grid, threads, smem, s>>>(edges, rb_end, R, words, indptr, meta + kMetaTiles, cap,
-                                           indices, row_indices, reinterpret_cast<uint4*>(blocks), rowmask, NT);
+                                           indices, row_indices, reinterpret_cast<uint4*>(blocks), rowmask, NT,
+                                           hv.limit);
+        if (hv.most) {
+            gp::k_heavy_emit<<<4 * device_sm_count(), gp::kEThreads, 0, s>>>(
+                hwords, hv, indptr, meta + kMetaTiles, cap, tile_bytes / 16, indices, row_indices,
+                reinterpret_cast<uint4*>(blocks), rowmask);
+            fill<<<2 * device_sm_count(), gp::kHThreads, 0, s>>>(edges, rb_end, hwords, hv, indptr, meta + kMetaTiles,
+                                                                 cap, blocks, rowmask);
+        }
         return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
     };
     if (tile_cols == 128)
-        return threads == 32 ? write(gp::k_write_tiles<7, 32>, 0) : write(gp::k_write_tiles<7, 128>, 1);
-    return threads == 32 ? write(gp::k_write_tiles<5, 32>, 2) : write(gp::k_write_tiles<5, 128>, 3);
+        return threads == 32 ? write(gp::k_write_tiles<7, 32>, 0, gp::k_heavy_fill<7>)
+                             : write(gp::k_write_tiles<7, 128>, 1, gp::k_heavy_fill<7>);
+    return threads == 32 ? write(gp::k_write_tiles<5, 32>, 2, gp::k_heavy_fill<5>)
+                         : write(gp::k_write_tiles<5, 128>, 3, gp::k_heavy_fill<5>);
 }
 
 }  // namespace btc200

@@ -84,8 +84,10 @@ struct btc_bitbsr {
             b.pool = pool;
             b.stream = s;
         });
-        policy.dev.pool = pool;
-        policy.dev.stream = s;
+        for (btc200::DevBuf* b : {&policy.dev, &policy.skew}) {
+            b->pool = pool;
+            b->stream = s;
+        }
     }
     void release_all()
     {

@@ -19,7 +19,9 @@
 #include "common.cuh"
 #include "handle.cuh"
 
+#include <algorithm>
 #include <cstdlib>
+#include <vector>
 
 namespace btc200 {
 namespace pol {
@@ -28,6 +30,18 @@ constexpr int kThreads = 256;
 constexpr int kGrid = 64;
 constexpr uint32_t kSamples = kPolicySamples;
 constexpr int32_t kNear = kPolicyNear;
+// Skew of the row blocks (policy_skewed), for lists the grouped builder would take in natural order:
+// 65,536 samples over 16,384 counters leave at most some 20 in one where row blocks are alike; 64
+// in one are a row block of a 1,024th of the edges.  Above that the grouped builder's CTA for it
+// is the last to end (build, grouped / sorted: R-MAT scale 20, edge factor 2, 16x32 2.05 / 0.68 ms;
+// a vertex of 3.9M neighbours among 8M pairs 111 / 3.3 ms), below it the sort's passes cost more
+// (7-point grid 144^3: 0.54 / 0.95 ms).
+constexpr uint32_t kSkewSlots = 1u << 14;
+constexpr uint32_t kSkewed = 64;
+__host__ __device__ __forceinline__ uint32_t skew_slot(int32_t u, int32_t v)
+{
+    return ((uint32_t)(u > v ? u : v) >> 4) * 0x9E3779B1u >> (32 - 14);
+}
 
 // Sample i reads edge i * step.  Adds the number of local edges and their expectation
 // under uniform ids (per sampled edge: the chance that two uniform ids in [0, n) lie
@@ -76,6 +90,31 @@ __global__ void k_locality(const int32_t* __restrict__ src, const int32_t* __res
     }
 }
 
+// Sample i's row block, of the oriented edge, hashed to one of kSkewSlots counters: the most
+// samples that one counter got.
+__global__ void k_skew(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m, int64_t step,
+                       unsigned int* __restrict__ count, unsigned int* __restrict__ most_and_ticket,
+                       volatile unsigned long long* host)
+{
+    unsigned int most = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < kSamples;
+         i += (uint64_t)gridDim.x * kThreads) {
+        const int64_t e = (int64_t)i * step;
+        if (e >= m) break;
+        most = max(most, atomicAdd(&count[skew_slot(src[e], dst[e])], 1u) + 1u);
+    }
+    most = __reduce_max_sync(kFull, most);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&most_and_ticket[0], most);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&most_and_ticket[1], 1u) == gridDim.x - 1) {
+        *host = atomicMax(&most_and_ticket[0], 0u);
+        __threadfence_system();
+    }
+}
+
 double locality_host(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
                      const int64_t* e_off, const int32_t* nv, uint32_t G)
 {
@@ -96,6 +135,16 @@ double locality_host(const int32_t* src, const int32_t* dst, int64_t m, int32_t 
         expect += ng > 2 * kNear ? (2.0 * kNear - 1.0) / (double)ng : 1.0;
     }
     return expect > 0.0 ? local / expect : 0.0;
+}
+
+uint32_t skew_host(const int32_t* src, const int32_t* dst, int64_t m)
+{
+    const int64_t step = m > (int64_t)kSamples ? m / (int64_t)kSamples : 1;
+    std::vector<uint32_t> count(kSkewSlots, 0u);
+    uint32_t most = 0;
+    for (uint64_t i = 0; i < kSamples && (int64_t)i * step < m; ++i)
+        most = std::max(most, ++count[skew_slot(src[i * step], dst[i * step])]);
+    return most;
 }
 
 // Average degree 2m/n of at least 512.
@@ -144,14 +193,51 @@ int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n
     return BTC_OK;
 }
 
+// Enqueues the skew sample of a device edge list; its result is in w.host[2] after a wait.
+static int enqueue_skew(const int32_t* src, const int32_t* dst, int64_t m, cudaStream_t s, PolicyWords& w)
+{
+    if (!w.host && !(w.host = host_slot_alloc(&w.host_context))) return BTC_E_NOMEM;
+    void* d_host = nullptr;
+    BTC_CUDA_TRY(cudaHostGetDevicePointer(&d_host, w.host, 0));
+    const size_t bytes = sizeof(unsigned int) * (pol::kSkewSlots + 2);
+    BTC_TRY(w.skew.reserve(bytes));
+    BTC_CUDA_TRY(cudaMemsetAsync(w.skew.ptr, 0, bytes, s));
+    const int64_t step = m > (int64_t)pol::kSamples ? m / (int64_t)pol::kSamples : 1;
+    const int64_t samples = m < (int64_t)pol::kSamples ? m : (int64_t)pol::kSamples;
+    pol::k_skew<<<(unsigned)((samples + 4 * pol::kThreads - 1) / (4 * pol::kThreads)), pol::kThreads, 0, s>>>(
+        src, dst, m, step, w.skew.as<unsigned int>(), w.skew.as<unsigned int>() + pol::kSkewSlots,
+        static_cast<unsigned long long*>(d_host) + 2);
+    BTC_CUDA_TRY(cudaGetLastError());
+    return BTC_OK;
+}
+
+int policy_skewed(const int32_t* src, const int32_t* dst, int64_t m, bool on_host, cudaStream_t s, PolicyWords& w,
+                  bool* skewed)
+{
+    *skewed = false;
+    if (m <= 0) return BTC_OK;
+    if (on_host) {
+        *skewed = pol::skew_host(src, dst, m) >= pol::kSkewed;
+        return BTC_OK;
+    }
+    BTC_TRY(enqueue_skew(src, dst, m, s, w));
+    BTC_CUDA_TRY(cudaStreamSynchronize(s));
+    *skewed = *static_cast<volatile unsigned long long*>(w.host + 2) >= pol::kSkewed;
+    return BTC_OK;
+}
+
 int policy_select(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, uint32_t flags, cudaStream_t s,
-                  PolicyWords& w, int* tile_cols, int* tau)
+                  PolicyWords& w, int* tile_cols, int* tau, int* skewed)
 {
     if (n < 0 || m < 0 || !tile_cols || (m > 0 && (!src || !dst))) return BTC_E_INVAL;
     double L = 0.0;
     // (the locality decides only where neither the degree nor the ordering does)
-    if (!(flags & BTC_ORIENT_DEGREE) && !pol::dense(m, n))
+    if (!(flags & BTC_ORIENT_DEGREE) && !pol::dense(m, n)) {
+        const bool with_skew = skewed && m > 0 && !(flags & BTC_INPUT_ON_HOST);
+        if (with_skew) BTC_TRY(enqueue_skew(src, dst, m, s, w));  // (the wait below is for both)
         BTC_TRY(policy_locality(src, dst, m, n, (flags & BTC_INPUT_ON_HOST) != 0, nullptr, nullptr, 0, s, w, &L));
+        if (with_skew) *skewed = *static_cast<volatile unsigned long long*>(w.host + 2) >= pol::kSkewed;
+    }
     return btc_tile_policy_from_features(m, n, flags, L, tile_cols, tau);
 }
 

@@ -280,8 +280,17 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
         longest = max(longest, b - a);
         if (b - a <= len_hi && (len_lo == 0 || b - a > len_lo)) row_block(I, a, b);
     }
-    if (w == 0 && lane == 0 && longest) atomicMax(&meta[kMetaRowMax], (unsigned long long)longest);
-    if (w == 0 && lane == 0 && most_chunks) atomicMax(&meta[kMetaRowLong], (unsigned long long)most_chunks);
+    // the CTA's longest: one atomic each (a team's own were 12 us of R-MAT scale 22's rows)
+    __shared__ uint32_t s_long[2];
+    if (threadIdx.x < 2) s_long[threadIdx.x] = 0;
+    __syncthreads();
+    if (w == 0 && lane == 0) {
+        atomicMax(&s_long[0], longest);
+        atomicMax(&s_long[1], most_chunks);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_long[0]) atomicMax(&meta[kMetaRowMax], (unsigned long long)s_long[0]);
+    if (threadIdx.x == 0 && s_long[1]) atomicMax(&meta[kMetaRowLong], (unsigned long long)s_long[1]);
 }
 
 // Raises *bad (and the host's word) where a caller's tiles are not what the store and its count
