@@ -564,11 +564,13 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
     BTC_TRY(g->blocks.reserve(sizeof(uint32_t) * TW * (tiles ? tiles : 1)));
     BTC_TRY(g->rowmask.reserve(sizeof(uint32_t) * (tiles ? tiles : 1)));
     // the streaming count's row store, when the union averages 8 or more tiles per row block
-    // (then it has at least 8 edges per row block), is not dense, and there is the memory for it
+    // (then it has at least 8 edges per row block), the tile kernels do not win, and there is the
+    // memory for it
     b->heavy = rows > 0 && (uint64_t)tiles >= 8ull * rows && m < (int64_t)0xffffffffll;
-    b->row_store = b->heavy && !dense_graph(tile_cols, m, (uint32_t)tiles, rows) &&
+    b->row_store = b->heavy && !tiles_win(tile_cols, m, (uint32_t)tiles, (int64_t)rows, b->max_col_blocks, true) &&
                    // (an enqueued rebuild may fill the arrays to their capacity)
                    reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * batch_capacity(b))) == BTC_OK;
+    if (b->heavy && !b->row_store) reserve_row_index(g, batch_capacity(b));
     BTC_TRY(ensure_count_scratch(g));
     BTC_TRY(b->counts.reserve(sizeof(unsigned long long) * (size_t)G));
     BTC_TRY(batch_enqueue_tiles(b, d_src, d_dst, m, (uint32_t)tiles, s));

@@ -83,6 +83,35 @@ bool dense_graph(int tile_cols, int64_t m, uint32_t T, int64_t R)
     return tile_cols == 128 ? per_tile > 896.0 : per_tile > 64.0 + (double)T / (double)R;
 }
 
+// The streaming count takes a warp some 2 us a row however short it is (0.55 ns over the GPU); the
+// row-wise kernel takes the 16 rows of a tile together.  Where a row block's tiles are few and
+// shared, or its graph so small that no row block's list is long, the latter wins (count only,
+// streaming / row-wise, 400,000 vertices in all): 16x32, graphs
+// of 512 vertices and average degree 4 / 8 / 16 / 48 205 / 96, 253 / 115, 286 / 171, 371 / 336 us; of
+// 1,024 247 / 143 (8), 281 / 226 (16), communities 309 / 207, R-MAT 279 / 227; of 2,048 245 / 184
+// (8) but 281 / 308 (16) and R-MAT 288 / 354; 16x128, of 2,048 195 / 111 (4), 243 / 154 (8), 278 / 267
+// (16), 402 / 706 (48).  A 27-point mesh 51^3 in degree order, 16x32: 142 / 61 us, 102^3 896 / 282.
+// Nearly a tile an edge and at most five edges a vertex: uniform pairs, in whose lists nothing is
+// long (131,072 vertices, average degree 4 97 / 58, 8 119 / 95, 16 146 / 188; R-MAT scale 20, edge
+// factor 2, whose tiles hold 1.3 edges and up, 1.2 / 5.0 ms in natural order).
+// widest: 64-column blocks of the widest graph; cells: the build makes the cell pairs, without which
+// the tiles are searched for.  Below 1,024 row blocks both counts are launches.
+static bool short_rows(int tile_cols, int64_t m, uint64_t T, int64_t R, uint32_t widest, bool cells)
+{
+    if (R < 1024) return false;
+    const uint64_t r = (uint64_t)R, e = (uint64_t)m;
+    const bool few = T < 16 * r;
+    if (tile_cols == 32 && few && e >= 12 * T) return true;
+    if (cells && R >= 4096 && 10 * e <= 11 * T && e <= 80 * r) return true;
+    if (widest > 33) return false;  // 2,048 vertices
+    return tile_cols == 32 ? few || e <= 80 * r : few && e <= 128 * r;
+}
+
+bool tiles_win(int tile_cols, int64_t m, uint32_t T, int64_t R, uint32_t widest, bool cells)
+{
+    return dense_graph(tile_cols, m, T, R) || short_rows(tile_cols, m, T, R, widest, cells);
+}
+
 static constexpr uint64_t kMaxEdges = (1ull << 32) - (uint64_t)kSortTile;
 
 int ensure_count_scratch(btc_bitbsr* g)
@@ -220,20 +249,26 @@ bool ensure_cells(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap
     return made;
 }
 
+// The row index's buffers for up to `cap` tiles.
+static bool row_index_room(btc_bitbsr* g, uint32_t cap, bool capturing)
+{
+    const uint64_t R = (uint64_t)g->n_row_blocks;
+    const uint64_t ent = std::min<uint64_t>((uint64_t)g->input_edges, 16ull * cap);
+    return row_store_possible(g->input_edges, g->n_row_blocks) &&
+           room(g->row_off, sizeof(uint32_t) * (16 * R + 1), capturing) &&
+           room(g->row_ent, sizeof(uint2) * (size_t)ent, capturing) &&
+           room(g->row_tot, sizeof(uint32_t) * R, capturing) &&
+           room(g->row_bsum, sizeof(unsigned long long) + sizeof(uint32_t) * ((size_t)ri_scan_blocks((uint32_t)R) + 1),
+                capturing);
+}
+
+void reserve_row_index(btc_bitbsr* g, uint32_t cap) { (void)row_index_room(g, cap, false); }
+
 bool ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s)
 {
     const bool capturing = stream_capturing(s), keep = !capturing && !d_tiles && !g->captured;
     if (g->row_index && keep) return true;
-    const uint64_t R = (uint64_t)g->n_row_blocks;
-    const int64_t m = g->input_edges;
-    const uint64_t ent = std::min<uint64_t>((uint64_t)m, 16ull * cap);
-    if (!row_store_possible(m, g->n_row_blocks) ||
-        !room(g->row_off, sizeof(uint32_t) * (16 * R + 1), capturing) ||
-        !room(g->row_ent, sizeof(uint2) * (size_t)ent, capturing) ||
-        !room(g->row_tot, sizeof(uint32_t) * R, capturing) ||
-        !room(g->row_bsum, sizeof(unsigned long long) + sizeof(uint32_t) * ((size_t)ri_scan_blocks((uint32_t)R) + 1),
-              capturing))
-        return false;
+    if (!row_index_room(g, cap, capturing)) return false;
     unsigned long long* total = g->row_bsum.as<unsigned long long>();
     const bool made = launch_rowindex(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->n_row_blocks,
                                       g->rowmask.as<uint32_t>(), d_tiles, cap, g->row_tot.as<uint32_t>(),
@@ -449,9 +484,10 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     const bool prev_light = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks &&
                             g->num_tiles > 0 &&
                             (uint64_t)g->num_tiles < 8ull * (uint64_t)geom.n_row_blocks;
-    // ... and whether it is dense, which the row store does not help
-    const bool prev_dense = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks &&
-                            dense_graph(tile_cols, m, g->num_tiles, geom.n_row_blocks);
+    // ... and, with its tiles, whether the tile kernels count it faster than a row store does
+    const uint32_t widest = ((uint32_t)n + 63) / 64;
+    const bool prev_same = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks;
+    const uint32_t prev_tiles = g->num_tiles;
     g->tile_cols = tile_cols;
     g->n = n;
     g->n_row_blocks = geom.n_row_blocks;
@@ -585,7 +621,8 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         // tile-wise kernel, which needs no store.  So does a graph without the memory for it.
         // (A build by one launch decides when it knows the tiles.)
         P.heavy = !small && !tiles_only && P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light;
-        P.row_store = P.heavy && !prev_dense &&
+        P.row_store = P.heavy &&
+                      !(prev_same && tiles_win(tile_cols, m, prev_tiles, geom.n_row_blocks, widest, P.use_bitmap)) &&
                       reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * P.cap)) == BTC_OK;
         g->heavy = P.heavy;
         g->row_store = P.row_store;
@@ -626,9 +663,10 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
             if (st2 != BTC_OK) return st2;
             g->heavy = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
                        (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks;
-            g->row_store = g->heavy && !dense_graph(tile_cols, m, g->num_tiles, geom.n_row_blocks) &&
+            g->row_store = g->heavy && !tiles_win(tile_cols, m, g->num_tiles, geom.n_row_blocks, widest, P.use_bitmap) &&
                            reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * g->num_tiles)) == BTC_OK;
             if (g->row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, false, s));
+            else if (g->heavy) reserve_row_index(g, g->num_tiles);
             return BTC_OK;
         }
         if (st2 != BTC_E_CAPACITY) return st2;
@@ -654,7 +692,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     // per row block, the row store when it is not dense besides
     P.heavy = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
               (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks;
-    P.row_store = P.heavy && !dense_graph(tile_cols, m, g->num_tiles, geom.n_row_blocks) &&
+    P.row_store = P.heavy && !tiles_win(tile_cols, m, g->num_tiles, geom.n_row_blocks, widest, P.use_bitmap) &&
                   reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * tiles)) == BTC_OK;
     if (P.use_bitmap) {
         BTC_TRY(bitmap_emit_and_fill(geom, P.d_src, P.d_dst, m, P.degree ? g->rank.as<int32_t>() : nullptr,
@@ -682,6 +720,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
                                g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
                                meta + kMetaRowMax, s, !have_masks));
     if (P.row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, P.degree, s));
+    else if (P.heavy) reserve_row_index(g, g->num_tiles);  // (for a count that may be captured)
     g->heavy = P.heavy;
     g->row_store = P.row_store;
     return BTC_OK;

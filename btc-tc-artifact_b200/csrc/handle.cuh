@@ -152,6 +152,12 @@ int default_tau(int tile_cols);
 // Whether a graph of m edges in T tiles and R row blocks is dense enough for the row-wise
 // kernel's tensor cores to count it faster than the streaming count.
 bool dense_graph(int tile_cols, int64_t m, uint32_t T, int64_t R);
+// Whether the row-wise kernel counts it faster than the streaming one: dense, or of short rows
+// (widest: 64-column blocks of the widest graph; cells: the build makes the cell pairs).  Such a
+// graph gets no row store.
+bool tiles_win(int tile_cols, int64_t m, uint32_t T, int64_t R, uint32_t widest, bool cells);
+// Reserves the row-wise kernel's index for up to `cap` tiles, where there is the memory.
+void reserve_row_index(btc_bitbsr* g, uint32_t cap);
 int ensure_count_scratch(btc_bitbsr* g);
 // Counts tiles [tile_begin, tile_end) (clamped to the tile count) into g->result and,
 // when d_out2 is given, *d_out2.
