@@ -339,7 +339,7 @@ static uint32_t batch_capacity(const btc_batch* b)
 
 // The build after the tile count: emit (indices, row_indices, indptr, the (cell word, tile
 // prefix) pairs, the tiles zeroed), fill, row masks and, when reserved, the row store of
-// the streaming count -- all against `cap` tiles, the device tile count deciding (more than cap:
+// the streaming count or the row-wise kernel's index -- all against `cap` tiles, the device tile count deciding (more than cap:
 // nothing is built and the overflow flag is set).
 static int batch_enqueue_tiles(btc_batch* b, const int32_t* d_src, const int32_t* d_dst, int64_t m,
                                uint32_t cap, cudaStream_t s)
@@ -383,6 +383,7 @@ static int batch_enqueue_tiles(btc_batch* b, const int32_t* d_src, const int32_t
         BTC_TRY(launch_rowstore(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                                 g->blocks.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
                                 meta + kMetaTiles, cap, false, meta, row_store_of(g), s));
+    if (g->index_built) BTC_TRY(enqueue_row_index(g, meta + kMetaTiles, cap, s));
     return cudaGetLastError() == cudaSuccess ? BTC_OK : BTC_E_CUDA;
 }
 
@@ -570,7 +571,7 @@ static int batch_build_into(btc_batch* b, const int32_t* src, const int32_t* dst
     b->row_store = b->heavy && !tiles_win(tile_cols, m, (uint32_t)tiles, (int64_t)rows, b->max_col_blocks, true) &&
                    // (an enqueued rebuild may fill the arrays to their capacity)
                    reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * batch_capacity(b))) == BTC_OK;
-    if (b->heavy && !b->row_store) reserve_row_index(g, batch_capacity(b));
+    g->index_built = b->heavy && !b->row_store && reserve_row_index(g, batch_capacity(b));
     BTC_TRY(ensure_count_scratch(g));
     BTC_TRY(b->counts.reserve(sizeof(unsigned long long) * (size_t)G));
     BTC_TRY(batch_enqueue_tiles(b, d_src, d_dst, m, (uint32_t)tiles, s));

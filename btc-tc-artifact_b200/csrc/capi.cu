@@ -170,6 +170,7 @@ struct BuildPlan {
     uint32_t cap;  // > 0: the post-count steps run against this tile capacity
     bool heavy = false;      // the graph can average 8 tiles per row block: make its row masks
     bool row_store = false;  // ... and the streaming count's row store (rowstore.cu)
+    bool row_index = false;  // ... or the row-wise kernel's index
 };
 
 // Only a graph with at least 8 edges per row block can average 8 tiles per row block (every
@@ -262,20 +263,35 @@ static bool row_index_room(btc_bitbsr* g, uint32_t cap, bool capturing)
                 capturing);
 }
 
-void reserve_row_index(btc_bitbsr* g, uint32_t cap) { (void)row_index_room(g, cap, false); }
+bool reserve_row_index(btc_bitbsr* g, uint32_t cap) { return row_index_room(g, cap, false); }
+
+int enqueue_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s)
+{
+    unsigned long long* total = g->row_bsum.as<unsigned long long>();
+    return launch_rowindex(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->n_row_blocks,
+                           g->rowmask.as<uint32_t>(), d_tiles, cap, g->row_tot.as<uint32_t>(),
+                           reinterpret_cast<uint32_t*>(total + 1), total, g->row_off.as<uint32_t>(),
+                           g->row_ent.as<uint2>(), g->row_ent.bytes / sizeof(uint2), s);
+}
 
 bool ensure_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s)
 {
+    if (g->index_built) return true;
     const bool capturing = stream_capturing(s), keep = !capturing && !d_tiles && !g->captured;
     if (g->row_index && keep) return true;
     if (!row_index_room(g, cap, capturing)) return false;
-    unsigned long long* total = g->row_bsum.as<unsigned long long>();
-    const bool made = launch_rowindex(g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(), g->n_row_blocks,
-                                      g->rowmask.as<uint32_t>(), d_tiles, cap, g->row_tot.as<uint32_t>(),
-                                      reinterpret_cast<uint32_t*>(total + 1), total, g->row_off.as<uint32_t>(),
-                                      g->row_ent.as<uint2>(), g->row_ent.bytes / sizeof(uint2), s) == BTC_OK;
+    const bool made = enqueue_row_index(g, d_tiles, cap, s) == BTC_OK;
     if (keep) g->row_index = made;
     return made;
+}
+
+// Tiles the handle's arrays hold room for at its width.  What a build reserves beside them follows
+// this, not its own tiles: the next rebuild is enqueued against it, and is not to allocate then.
+static uint32_t tile_capacity(const btc_bitbsr* g)
+{
+    const uint64_t c = std::min<uint64_t>(std::min<uint64_t>(g->indices.bytes, g->row_indices.bytes),
+                                          g->rowmask.bytes) / 4;
+    return (uint32_t)std::min<uint64_t>(std::min<uint64_t>(c, g->blocks.bytes / (2 * (size_t)g->tile_cols)), 0xffffffffull);
 }
 
 static int enqueue_group_write(btc_bitbsr* g, const BuildPlan& P, uint32_t cap, cudaStream_t s)
@@ -346,6 +362,7 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
                                          g->rowmask.as<uint32_t>(), P.heavy, P.row_store));
             // (the fill pass set the row masks, or found the longest row-block list)
             if (P.row_store) BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s));
+            if (P.row_index) BTC_TRY(enqueue_row_index(g, meta + kMetaTiles, P.cap, s));
         }
     } else if (P.use_group) {
         const uint32_t R = (uint32_t)geom.n_row_blocks;
@@ -386,13 +403,15 @@ static void build_key(const btc_bitbsr* g, const BuildPlan& P, BuildGraphKey* k)
                        g->keys1.ptr, g->sort_scratch.ptr, g->deg.ptr, g->rank.ptr, g->bitmap.ptr,
                        g->prefix.ptr, g->tile_base.ptr, g->indices.ptr, g->row_indices.ptr,
                        g->indptr.ptr, g->blocks.ptr, g->rowmask.ptr, g->d_hmeta, g->rs_off.ptr,
-                       g->rs_key.ptr, g->rs_bits.ptr, g->rs_first.ptr};
+                       g->rs_key.ptr, g->rs_bits.ptr, g->rs_first.ptr, g->row_off.ptr, g->row_ent.ptr,
+                       g->row_tot.ptr, g->row_bsum.ptr};
     static_assert(sizeof(w) / sizeof(w[0]) == kBuildKeyPtrs, "key layout");
     for (int i = 0; i < kBuildKeyPtrs; ++i) k->ptr[i] = w[i];
     k->m = P.m;
     k->n = P.n;
     k->tile_cols = P.geom.tile_cols;
-    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.heavy ? 0x20000000u : 0u) | (P.use_group ? 0x40000000u : 0u);
+    k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.use_group ? 0x40000000u : 0u) |
+               (P.heavy ? 0x20000000u : 0u) | (P.row_index ? 0x10000000u : 0u);
     k->cap = P.cap;
 }
 
@@ -551,7 +570,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         if (P.use_group) P.use_bitmap = false;
     }
     g->cells = P.use_bitmap;
-    g->heavy = g->row_store = g->row_index = g->cells_lazy = false;
+    g->heavy = g->row_store = g->row_index = g->cells_lazy = g->index_built = false;
     if ((flags & BTC_BUILD_ASYNC) && stream_capturing(s)) g->captured = true;
     size_t key_cap = P.use_bitmap || P.use_group ? 0 : (size_t)m;
     if (P.degree && (size_t)n > key_cap) key_cap = (size_t)n;
@@ -606,11 +625,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     // a count above the capacity is redone below at the right size.  A first build
     // waits for the count in between.
     if ((P.use_bitmap || P.use_group) && g->indices.ptr && g->row_indices.ptr && g->blocks.ptr && g->rowmask.ptr) {
-        uint64_t c = g->indices.bytes / 4;
-        c = std::min<uint64_t>(c, g->row_indices.bytes / 4);
-        c = std::min<uint64_t>(c, g->blocks.bytes / (4 * TW));
-        c = std::min<uint64_t>(c, g->rowmask.bytes / 4);
-        P.cap = (uint32_t)std::min<uint64_t>(c, 0xffffffffull);
+        P.cap = tile_capacity(g);
         const uint64_t rows = std::min<uint64_t>(g->indices.bytes / 4,
                                                  std::min<uint64_t>(g->row_indices.bytes / 4, g->rowmask.bytes / 4));
         P.cap32 = (uint32_t)std::min<uint64_t>(rows, g->blocks.bytes / 64);
@@ -624,8 +639,11 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         P.row_store = P.heavy &&
                       !(prev_same && tiles_win(tile_cols, m, prev_tiles, geom.n_row_blocks, widest, P.use_bitmap)) &&
                       reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * P.cap)) == BTC_OK;
+        // (the index needs the cell pairs beside it, which the bitmap builder makes)
+        P.row_index = P.heavy && !P.row_store && P.use_bitmap && reserve_row_index(g, P.cap);
         g->heavy = P.heavy;
         g->row_store = P.row_store;
+        g->index_built = P.row_index;
     }
 
     uint64_t* sorted = nullptr;
@@ -664,9 +682,10 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
             g->heavy = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
                        (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks;
             g->row_store = g->heavy && !tiles_win(tile_cols, m, g->num_tiles, geom.n_row_blocks, widest, P.use_bitmap) &&
-                           reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * g->num_tiles)) == BTC_OK;
+                           reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * tile_capacity(g))) == BTC_OK;
             if (g->row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, false, s));
-            else if (g->heavy) reserve_row_index(g, g->num_tiles);
+            g->index_built = g->heavy && !g->row_store && reserve_row_index(g, tile_capacity(g));
+            if (g->index_built) BTC_TRY(enqueue_row_index(g, nullptr, g->num_tiles, s));
             return BTC_OK;
         }
         if (st2 != BTC_E_CAPACITY) return st2;
@@ -693,7 +712,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     P.heavy = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
               (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks;
     P.row_store = P.heavy && !tiles_win(tile_cols, m, g->num_tiles, geom.n_row_blocks, widest, P.use_bitmap) &&
-                  reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * tiles)) == BTC_OK;
+                  reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * tile_capacity(g))) == BTC_OK;
     if (P.use_bitmap) {
         BTC_TRY(bitmap_emit_and_fill(geom, P.d_src, P.d_dst, m, P.degree ? g->rank.as<int32_t>() : nullptr,
                                      g->bitmap.as<uint32_t>(), g->tile_base.as<uint32_t>(),
@@ -720,9 +739,11 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
                                g->indptr.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(),
                                meta + kMetaRowMax, s, !have_masks));
     if (P.row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, P.degree, s));
-    else if (P.heavy) reserve_row_index(g, g->num_tiles);  // (for a count that may be captured)
+    P.row_index = P.heavy && !P.row_store && reserve_row_index(g, tile_capacity(g)) && P.use_bitmap;
+    if (P.row_index) BTC_TRY(enqueue_row_index(g, nullptr, g->num_tiles, s));
     g->heavy = P.heavy;
     g->row_store = P.row_store;
+    g->index_built = P.row_index;
     return BTC_OK;
 }
 

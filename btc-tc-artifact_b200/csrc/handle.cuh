@@ -5,7 +5,7 @@
 
 // Arguments and buffers of an enqueued build (a cached build graph replays only when
 // they are unchanged).
-constexpr int kBuildKeyPtrs = 23;
+constexpr int kBuildKeyPtrs = 27;
 struct BuildGraphKey {
     const void* ptr[kBuildKeyPtrs];
     int64_t m;
@@ -27,9 +27,9 @@ struct btc_bitbsr {
     // row store of the streaming count (rowstore.cu): row starts, column blocks, bits and
     // the row of every run of chunks
     btc200::DevBuf rs_off, rs_key, rs_bits, rs_first;
-    // row index of the row-wise count kernel (rowindex.cu), made by the first count that
-    // takes it: per-vertex list offsets and (column block, tile) entries, plus the scan's
-    // scratch
+    // row index of the row-wise count kernel (rowindex.cu), made by the build of a graph that takes
+    // it, else by the first count that does: per-vertex list offsets and (column block, tile)
+    // entries, plus the scan's scratch
     btc200::DevBuf row_off, row_ent, row_tot, row_bsum;
     // build workspace
     btc200::DevBuf in_src, in_dst, keys0, keys1, sort_scratch, tile_base, meta, deg, rank, bitmap, prefix;
@@ -37,6 +37,7 @@ struct btc_bitbsr {
     bool heavy = false;      // the last build's graph can average 8 tiles per row block: it has row masks
     bool row_store = false;  // ... and the last build made the row store
     bool row_index = false;  // the row index of the last build's graph has been made
+    bool index_built = false; // ... by the build itself, and so by each of its replays
     bool cells_lazy = false; // ... and the pairs by a count, not by the build
     bool captured = false;   // a caller's CUDA graph holds a rebuild, whose replays this handle does not see
     // count scratch
@@ -156,8 +157,10 @@ bool dense_graph(int tile_cols, int64_t m, uint32_t T, int64_t R);
 // (widest: 64-column blocks of the widest graph; cells: the build makes the cell pairs).  Such a
 // graph gets no row store.
 bool tiles_win(int tile_cols, int64_t m, uint32_t T, int64_t R, uint32_t widest, bool cells);
-// Reserves the row-wise kernel's index for up to `cap` tiles, where there is the memory.
-void reserve_row_index(btc_bitbsr* g, uint32_t cap);
+// Reserves the row-wise kernel's index for up to `cap` tiles (false without the memory), and
+// enqueues it after the tiles and row masks.
+bool reserve_row_index(btc_bitbsr* g, uint32_t cap);
+int enqueue_row_index(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap, cudaStream_t s);
 int ensure_count_scratch(btc_bitbsr* g);
 // Counts tiles [tile_begin, tile_end) (clamped to the tile count) into g->result and,
 // when d_out2 is given, *d_out2.

@@ -122,3 +122,28 @@ def test_batches(name, tile_cols):
     del graph
     fresh.free()
     b.free()
+
+
+@pytest.mark.parametrize("deg", [False, True])
+def test_the_build_makes_the_row_wise_index(deg):
+    """A count behind an enqueued rebuild is one kernel: what it reads beside the tiles is made by
+    the build (it had been made again by every such count)."""
+    from torch.profiler import ProfilerActivity, profile
+    n = 600
+    s, d, _ = G.complete(n)
+    ts, td = torch.from_numpy(s).cuda(), torch.from_numpy(d).cuda()
+    g = BitBSR(ts, td, n, 32, orient_degree=deg)
+    assert g.count() == n * (n - 1) * (n - 2) // 6
+    out = torch.zeros(1, dtype=torch.int64, device="cuda")
+    for _ in range(3):
+        g.rebuild(td, ts, n, 32, orient_degree=deg, asynchronous=True)
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            g.count_async(d_out=out.data_ptr())
+            torch.cuda.synchronize()
+        assert int(out.item()) == n * (n - 1) * (n - 2) // 6
+        names = [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+        if not names:
+            pytest.skip("no kernel records on this machine")
+        assert len(names) == 1 and "k_count_rows" in names[0], names
+    g.free()
