@@ -653,22 +653,21 @@ int btc_batch_count(btc_batch* b, int tau, btc_stream_t stream, unsigned long lo
     const unsigned long long* build_meta = b->pending ? g->meta.as<unsigned long long>() : nullptr;
     const uint32_t cap = b->pending ? b->pending_cap : g->num_tiles;
     if (b->row_store && tau >= default_tau(g->tile_cols)) {
-        BTC_TRY(launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks, g->tile_cols, g->n_row_blocks, b->max_col_blocks, scr,
+        BTC_TRY(launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks,
+                                    g->tile_cols, g->n_row_blocks, b->max_col_blocks, scr,
                                     b->row_off.as<uint32_t>(), (uint32_t)b->num_graphs, counts,
                                     g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), 0, cap, true, true,
                                     build_meta, count_grid_size(g->tile_cols), stream));
     } else {
-    const bool index = b->heavy && ensure_row_index(g, build_meta ? build_meta + kMetaTiles : nullptr, cap, stream);
-    BTC_TRY(launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
-                         g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(),
-                         cap, g->n_row_blocks, tau, scr,
-                         stream, b->row_off.as<uint32_t>(), (uint32_t)b->num_graphs, counts,
-                         g->rowmask.as<uint32_t>(), g->prefix.as<uint2>(), 0,
-                         g->meta.as<unsigned long long>() + kMetaRowMax, 0, 0xffffffffu, build_meta,
-                         g->num_tiles,
-                         index ? g->row_off.as<uint32_t>() : nullptr,
-                         index ? g->row_ent.as<uint2>() : nullptr, false,
-                         b->segs.as<GraphSeg>()));
+        const bool index =
+            b->heavy && ensure_row_index(g, build_meta ? build_meta + kMetaTiles : nullptr, cap, stream);
+        BTC_TRY(launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
+                             g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(), cap, g->n_row_blocks, tau,
+                             scr, stream, b->row_off.as<uint32_t>(), (uint32_t)b->num_graphs, counts,
+                             g->rowmask.as<uint32_t>(), g->prefix.as<uint2>(), 0,
+                             g->meta.as<unsigned long long>() + kMetaRowMax, 0, 0xffffffffu, build_meta,
+                             g->num_tiles, index ? g->row_off.as<uint32_t>() : nullptr,
+                             index ? g->row_ent.as<uint2>() : nullptr, false, b->segs.as<GraphSeg>()));
     }
     if (h_counts) {
         BTC_CUDA_TRY(cudaMemcpyAsync(h_counts, counts, bytes, cudaMemcpyDeviceToHost, stream));

@@ -1,6 +1,7 @@
 // capi.cu -- the C ABI (include/btc_c.h): handles, build pipeline, count calls and
-// the reference-shaped struct surface.  Host code only; kernels live in radix.cu,
-// build.cu and count.cu.
+// the reference-shaped struct surface.  Host code only; the builders' kernels live in bitmap.cu,
+// group.cu, small.cu, build.cu and radix.cu, the counts' in count.cu, count_rows.cu and
+// count_stream.cu.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -173,8 +174,6 @@ struct BuildPlan {
     bool row_index = false;  // ... or the row-wise kernel's index
 };
 
-// Only a graph with at least 8 edges per row block can average 8 tiles per row block (every
-// tile holds an edge).
 // Graphs the one-launch builder takes, when the call waits: it saves about 17 us of launches
 // and waits whatever the size (Erdos-Renyi, a step: 1,000 vertices 83 -> 66 us, 16,384 / 16
 // 112 -> 91, 40,000 / 26, 520,000 draws 184 -> 168), which from 2^19 edges on is a few percent
@@ -189,6 +188,8 @@ static bool small_possible(int64_t m, int32_t n)
     return bitmap_words_per_row(g) * (uint64_t)g.n_row_blocks <= (1ull << 20);
 }
 
+// Only a graph with at least 8 edges per row block can average 8 tiles per row block (every
+// tile holds an edge).
 static bool row_store_possible(int64_t m, int32_t n_row_blocks)
 {
     return n_row_blocks > 0 && m >= 8 * (int64_t)n_row_blocks && m < (int64_t)0xffffffffll;
@@ -296,7 +297,7 @@ static uint32_t tile_capacity(const btc_bitbsr* g)
 
 static int enqueue_group_write(btc_bitbsr* g, const BuildPlan& P, uint32_t cap, cudaStream_t s)
 {
-    return group_write(P.geom.tile_cols, P.col_blocks, P.m, (uint32_t)P.geom.n_row_blocks,
+    return group_write(P.geom.tile_cols, P.col_blocks, P.m, (uint32_t)P.geom.n_row_blocks, !P.degree,
                        g->keys0.as<uint32_t>(), g->tile_base.as<uint32_t>(), g->indptr.as<uint32_t>(),
                        g->meta.as<unsigned long long>(), cap, g->indices.as<uint32_t>(),
                        g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(), g->rowmask.as<uint32_t>(),
@@ -367,7 +368,7 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
     } else if (P.use_group) {
         const uint32_t R = (uint32_t)geom.n_row_blocks;
         uint32_t* scratch = g->tile_base.as<uint32_t>();
-        BTC_TRY(group_edges(P.d_src, P.d_dst, P.m, P.n, rank, geom.tile_cols, P.col_blocks,
+        BTC_TRY(group_edges(P.d_src, P.d_dst, P.m, P.n, rank, !P.degree, geom.tile_cols, P.col_blocks,
                             k0, k1, g->keys0.as<uint32_t>(), scratch, g->indptr.as<uint32_t>(),
                             scratch + group_scratch_words(R, P.m, P.col_blocks), meta, s));
         if (P.cap) {
@@ -549,12 +550,14 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     }
     P.use_group = !(flags & BTC_BUILD_RADIX) && group_possible(n, P.col_blocks) &&
                   (!P.use_bitmap || (P.degree && m >= kGroupEdges));
-    // In natural order a hub's row block may have any share of the edges, and its row blocks' tiles
-    // are too much for a CTA each: such a list is sorted.
+    // In natural order a hub's row block may have any share of the edges, and its tiles are too much
+    // for a CTA: such a list is sorted.
     if (P.use_group && !P.degree) {
         if (skewed < 0) {
             bool is = false;
-            BTC_TRY(policy_skewed(src, dst, m, (flags & BTC_INPUT_ON_HOST) != 0, s, g->policy, &is));
+            double unused = 0.0;
+            BTC_TRY(policy_locality(src, dst, m, n, (flags & BTC_INPUT_ON_HOST) != 0, nullptr, nullptr, 0, s,
+                                    g->policy, &unused, &is));
             skewed = is;
         }
         if (skewed) P.use_group = false;
@@ -563,7 +566,8 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         const uint64_t R = (uint64_t)geom.n_row_blocks;
         if (g->keys0.reserve(sizeof(uint64_t) * (size_t)(m ? m : 1)) != BTC_OK ||
             g->keys1.reserve(sizeof(uint64_t) * (size_t)(m ? m : 1)) != BTC_OK ||
-            g->tile_base.reserve(sizeof(uint32_t) * (group_scratch_words((uint32_t)R, m, P.col_blocks) + ri_scan_blocks((uint32_t)R) + 1)) != BTC_OK) {
+            g->tile_base.reserve(sizeof(uint32_t) * (group_scratch_words((uint32_t)R, m, P.col_blocks) +
+                                                     ri_scan_blocks((uint32_t)R) + 1)) != BTC_OK) {
             if (!P.use_bitmap) return BTC_E_NOMEM;
             P.use_group = false;  // the bitmap may still fit
         }
@@ -774,10 +778,11 @@ int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_o
     // whatever size): the store it has made is used.
     if (g->row_store && tau >= default_tau(g->tile_cols) &&
         (g->pending || !dense_graph(g->tile_cols, g->input_edges, g->num_tiles, g->n_row_blocks)))
-        return launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks, g->tile_cols, g->n_row_blocks,
-                                   ((uint32_t)g->n + 63) / 64, scr, nullptr, 0, nullptr,
-                                   g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), tile_begin,
-                                   std::min(tile_end, cap), whole, true, build_meta, count_grid_size(g->tile_cols), s);
+        return launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks,
+                                   g->tile_cols, g->n_row_blocks, ((uint32_t)g->n + 63) / 64, scr, nullptr, 0,
+                                   nullptr, g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), tile_begin,
+                                   std::min(tile_end, cap), whole, true, build_meta,
+                                   count_grid_size(g->tile_cols), s);
     const uint64_t wpr = bitmap_words_per_row(make_geom(g->n, g->tile_cols));
     bool cells = g->cells && !g->cells_lazy, index = false;
     if (g->heavy) {

@@ -306,14 +306,15 @@ int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indic
                     cudaStream_t s);
 
 // The streaming count (count_stream.cu) of the sample tiles [tile_begin, tile_end), or of
-// all of them with `whole`.  rs_chunks: the store's meta[kMetaRowChunks].  max_col_blocks: the most 64-column blocks a row's columns can
-// span.  lower: the matrix is a lower triangle (every handle's is; a caller's
-// Bit-BSR need not be).  grid: the CTAs scr.partials has room for.
+// all of them with `whole`.  rs_chunks: the store's meta[kMetaRowChunks], with meta[kMetaRowLong]
+// behind it.  max_col_blocks: the most 64-column blocks a row's columns can span.  lower: the
+// matrix is a lower triangle (every handle's is; a caller's Bit-BSR need not be).  grid: the CTAs
+// scr.partials has room for.
 int stream_blocks_per_sm_max();
 int launch_count_stream(const RowStore& rs, const unsigned long long* rs_chunks, int tile_cols,
-                        int32_t n_row_blocks, uint32_t max_col_blocks, CountScratch scr, const uint32_t* graph_rows, uint32_t num_graphs,
-                        unsigned long long* graph_counts, const uint32_t* row_indices,
-                        const uint32_t* indices, uint32_t tile_begin, uint32_t tile_end, bool whole,
+                        int32_t n_row_blocks, uint32_t max_col_blocks, CountScratch scr,
+                        const uint32_t* graph_rows, uint32_t num_graphs, unsigned long long* graph_counts,
+                        const uint32_t* row_indices, const uint32_t* indices, uint32_t tile_begin, uint32_t tile_end, bool whole,
                         bool lower, const unsigned long long* build_meta, int grid, cudaStream_t s);
 
 // Row index of the row-wise count kernel (rowindex.cu): for vertex u, ent[off[u],
@@ -327,24 +328,23 @@ int launch_rowindex(const uint32_t* indptr, const uint32_t* indices, int32_t n_r
                     uint32_t* tot, uint32_t* bsum, unsigned long long* total, uint32_t* off,
                     uint2* ent, uint64_t ent_cap, cudaStream_t s);
 
-// The grouped builder (group.cu).
-// Degree-ordered edge lists from this length on are grouped by row block (group.cu) instead
-// of marked and filled edge by edge: the tiles of a power-law graph this large do not stay
-// in L2 between zeroing and filling (R-MAT scale 18, 4.2M draws: 0.71 ms against 0.73 a
-// step; scale 19: 1.29 / 1.43; scale 22: build 9.3 -> 5.6 ms; scale 17: the same).  In
+// The grouped builder (group.cu).  Degree-ordered edge lists from this length on are grouped by row
+// block instead of marked and filled edge by edge: the tiles of a power-law graph this large do not
+// stay in L2 between zeroing and filling (R-MAT scale 18, 4.2M draws: 0.71 ms against 0.73 a
+// step; scale 19: 1.29 / 1.43; scale 22: build 8.7 -> 5.2 ms; scale 17: the same).  In
 // natural order the bitmap stays: meshes and communities have small tile arrays (27-point
-// mesh 100^3 0.61 ms against 0.69 grouped, 8 communities on 60,000 vertices 4.0 / 4.5) and a
-// power-law hub's row block is one CTA's work here (scale 18: 2.1 / 2.4); uniform graphs of
+// mesh 100^3 0.61 ms against 0.69 grouped, 8 communities on 60,000 vertices 4.0 / 4.5) and hubs
+// unbalance the row blocks (scale 18: 2.1 / 2.4); uniform graphs of
 // more than 3M edges would gain (800,000 vertices, 6.4M edges: 1.9 / 1.35 ms), but nothing
 // at hand tells them from a power-law graph.
 constexpr int64_t kGroupEdges = 1 << 22;
 bool group_possible(int64_t n, uint64_t col_blocks);
 size_t group_scratch_words(uint32_t R, int64_t m, uint64_t col_blocks);
 int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
-                const int32_t* rank, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
+                const int32_t* rank, bool balanced, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
                 uint64_t* grouped, uint32_t* edges, uint32_t* scratch, uint32_t* indptr, uint32_t* bsum,
                 unsigned long long* meta, cudaStream_t s);
-int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
+int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R, bool balanced,
                 const uint32_t* edges, uint32_t* scratch, const uint32_t* indptr,
                 const unsigned long long* meta, uint32_t cap, uint32_t* indices, uint32_t* row_indices,
                 uint32_t* blocks, uint32_t* rowmask, uint32_t tiles_hint, cudaStream_t s);
@@ -361,7 +361,8 @@ int launch_cells(const uint32_t* indptr, const uint32_t* indices, const uint32_t
 
 // Id locality of an edge list for the tile policy (policy.cu): sampled share of edges
 // with |u - v| < 128 over the share uniform ids would give.  e_off / nv (nullable): the
-// batch layout, each edge measured against its own graph's vertex count.
+// batch layout, each edge measured against its own graph's vertex count.  skewed (nullable): whether
+// one row block of 16 vertices has about a 1,024th of the oriented edges or more, by the same sample.
 constexpr uint32_t kPolicySamples = 1u << 16;
 constexpr int32_t kPolicyNear = 128;  // |u - v| below this counts as local
 // One sampled edge: is it local, and the chance that two uniform ids are (2^20 = 1).
@@ -414,7 +415,7 @@ int launch_build_small(const SmallBuild& b, cudaStream_t s);
 
 struct PolicyWords {
     DevBuf dev;                          // two sums and a ticket
-    DevBuf skew;                         // counters of the skew sample, the most, a ticket
+    DevBuf skew;                         // counters of the samples' row blocks, and the most
     unsigned long long* host = nullptr;  // a host slot
     unsigned long long host_context = 0;
     bool dirty = false;                  // a call did not come to its end
@@ -434,15 +435,11 @@ struct PolicyWords {
 };
 int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, bool on_host,
                     const int64_t* e_off, const int32_t* nv, uint32_t G, cudaStream_t s, PolicyWords& w,
-                    double* L);
+                    double* L, bool* skewed = nullptr);
 // btc_select_tile_policy with the caller's words.
-// skewed (nullable): also policy_skewed's answer, where a device sample is taken (else unchanged).
+// skewed (nullable): set where the sample is taken, else unchanged.
 int policy_select(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, uint32_t flags, cudaStream_t s,
                   PolicyWords& w, int* tile_cols, int* tau, int* skewed = nullptr);
-// Whether one row block of 16 vertices has about a 1,024th of the oriented edges or more, by a sample
-// (a wait on device input).
-int policy_skewed(const int32_t* src, const int32_t* dst, int64_t m, bool on_host, cudaStream_t s, PolicyWords& w,
-                  bool* skewed);
 
 // Device metadata slots of a build (uint64 each): valid keys, out-of-range flag, tile
 // count, unique edges, sort length, longest row-block list, tile-capacity overflow flag,

@@ -43,6 +43,7 @@
 #include <cstddef>
 #include <cstdlib>
 
+#include <algorithm>
 #include <atomic>
 
 namespace btc200 {
@@ -815,10 +816,20 @@ static int tile_blocks_per_sm(int tile_cols)
 // launch runs at most its own kernel's resident CTAs).
 int count_grid_size(int tile_cols)
 {
-    const int rows = rows_blocks_per_sm(tile_cols);
-    const int tile = tile_blocks_per_sm(tile_cols);
-    const int most = rows > tile ? rows : tile, stream = stream_blocks_per_sm_max();
-    return (most > stream ? most : stream) * device_sm_count();
+    // (asked several times a step: the variants' own caches cost a device query each)
+    static std::atomic<int> cache[kMaxDevices][2];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = -1;
+    const int w = tile_cols == 128 ? 0 : 1;
+    if (dev >= 0) {
+        const int v = cache[dev][w].load(std::memory_order_relaxed);
+        if (v > 0) return v;
+    }
+    const int rows = rows_blocks_per_sm(tile_cols), tile = tile_blocks_per_sm(tile_cols);
+    const int stream = stream_blocks_per_sm_max();
+    const int grid = std::max(rows, std::max(tile, stream)) * device_sm_count();
+    if (dev >= 0 && rows > 0 && stream > 0) cache[dev][w].store(grid, std::memory_order_relaxed);
+    return grid;
 }
 
 int launch_count(int tile_cols, const uint32_t* indptr, const uint32_t* indices,

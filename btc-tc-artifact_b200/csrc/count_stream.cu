@@ -8,8 +8,8 @@
 //  * u's row (its entries: 64-column block K and 64 bits) is scattered into a warp's table
 //    of W slots, slot K - K0 with K0 the row's first column block; slots without an entry
 //    hold zeros.  Entries past the table (K - K0 >= W) stay in the store and are found by a
-//    bitmap of their column blocks with ranks; on degree-ordered power-law graphs W = 1024 covers 99.9% of the look-ups
-//    (R-MAT scale 20).
+//    bitmap of their column blocks with ranks; on degree-ordered power-law graphs W = 1024
+//    covers 99.9% of the look-ups (R-MAT scale 20).
 //  * u's neighbours v are picked out of its entries' bits one per lane, and the 16-entry
 //    chunks of their rows are listed in shared memory.  Four groups of eight lanes take
 //    four chunks each per round: a chunk is one 32-byte (64 with 32-bit keys) and one
@@ -558,9 +558,9 @@ int stream_blocks_per_sm_max()
 }
 
 int launch_count_stream(const RowStore& rs, const unsigned long long* rs_chunks, int tile_cols,
-                        int32_t n_row_blocks, uint32_t max_col_blocks, CountScratch scr, const uint32_t* graph_rows, uint32_t num_graphs,
-                        unsigned long long* graph_counts, const uint32_t* row_indices,
-                        const uint32_t* indices, uint32_t tile_begin, uint32_t tile_end, bool whole,
+                        int32_t n_row_blocks, uint32_t max_col_blocks, CountScratch scr,
+                        const uint32_t* graph_rows, uint32_t num_graphs, unsigned long long* graph_counts,
+                        const uint32_t* row_indices, const uint32_t* indices, uint32_t tile_begin, uint32_t tile_end, bool whole,
                         bool lower, const unsigned long long* build_meta, int grid, cudaStream_t s)
 {
     const int size = row_store_wide(n_row_blocks) ? 3 : max_col_blocks <= 256 ? 0 : max_col_blocks <= 512 ? 1 : 2;

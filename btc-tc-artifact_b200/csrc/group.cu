@@ -701,7 +701,8 @@ size_t group_scratch_words(uint32_t R, int64_t m, uint64_t col_blocks)
            2 * (size_t)gp::heavy_most(m) * bitmap_row_words(col_blocks);
 }
 
-static gp::Heavy heavy_of(uint32_t* scratch, uint32_t R, int64_t m, uint64_t col_blocks)
+// balanced: no row block has a share of the edges that is worth slices; none is heavy.
+static gp::Heavy heavy_of(uint32_t* scratch, uint32_t R, int64_t m, uint64_t col_blocks, bool balanced)
 {
     uint32_t* at = scratch + group_front_words(R);
     gp::Heavy h{};
@@ -709,19 +710,19 @@ static gp::Heavy heavy_of(uint32_t* scratch, uint32_t R, int64_t m, uint64_t col
     h.list = at + 1;
     h.done = h.list + gp::kMaxHeavy;
     h.bm = h.done + gp::kMaxHeavy;
-    h.most = gp::heavy_most(m);
+    h.most = balanced ? 0u : gp::heavy_most(m);
     h.pre = h.bm + (size_t)h.most * bitmap_row_words(col_blocks);
-    h.limit = gp::heavy_edges(m);
+    h.limit = balanced ? 0xffffffffu : gp::heavy_edges(m);
     return h;
 }
 
 // The edges grouped by row block and the row blocks' tile counts scanned into indptr.
 // pairs: m uint64 (only written with rank); grouped: m uint64 of scratch whose
-// contents end up in `edges` (m words, may share memory with pairs); scratch:
+// contents end up in `edges` (m words, may share memory with pairs); balanced: see heavy_of; scratch:
 // group_scratch_words(R, m, col_blocks); bsum: scan scratch of R words.  Writes meta[kMetaBad] and
 // meta[kMetaTiles].
 int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
-                const int32_t* rank, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
+                const int32_t* rank, bool balanced, int tile_cols, uint64_t col_blocks, uint64_t* pairs,
                 uint64_t* grouped, uint32_t* edges, uint32_t* scratch, uint32_t* indptr, uint32_t* bsum,
                 unsigned long long* meta, cudaStream_t s)
 {
@@ -731,7 +732,7 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
     uint32_t* base = cursor + gp::kBuckets;
     uint32_t* rb_end = base + gp::kBuckets + 1;  // offsets at first, then (moved on) ends
     unsigned long long* sum = reinterpret_cast<unsigned long long*>(scratch + (group_front_words(R) - 2) / 2 * 2);
-    const gp::Heavy hv = heavy_of(scratch, R, m, col_blocks);
+    const gp::Heavy hv = heavy_of(scratch, R, m, col_blocks, balanced);
     const int shift = bucket_shift(n);
     if (cudaMemsetAsync(hist, 0, sizeof(uint32_t) * gp::kBuckets, s) != cudaSuccess) return BTC_E_CUDA;
     const bool store = rank != nullptr;
@@ -772,7 +773,7 @@ int group_edges(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
 
 // Tiles, indices, row_indices and row masks from the grouped edges (indptr[R] set), against
 // `cap` tiles: nothing when meta[kMetaTiles] is above it.
-int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
+int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R, bool balanced,
                 const uint32_t* edges, uint32_t* scratch, const uint32_t* indptr,
                 const unsigned long long* meta, uint32_t cap, uint32_t* indices, uint32_t* row_indices,
                 uint32_t* blocks, uint32_t* rowmask, uint32_t tiles_hint, cudaStream_t s)
@@ -784,14 +785,15 @@ int group_write(int tile_cols, uint64_t col_blocks, int64_t m, uint32_t R,
     // 15%, 32 KB 20%
     const uint32_t tile_bytes = 2u * (uint32_t)tile_cols;
     uint32_t buf = 4096;
-    while (buf < (tile_cols == 128 ? gp::kTileBytes / 2 : gp::kTileBytes) && (uint64_t)buf * R * 2 < 3ull * tiles_hint * tile_bytes) buf *= 2;
+    const uint32_t buf_most = tile_cols == 128 ? gp::kTileBytes / 2 : gp::kTileBytes;
+    while (buf < buf_most && (uint64_t)buf * R * 2 < 3ull * tiles_hint * tile_bytes) buf *= 2;
     const uint32_t NT = buf / tile_bytes;
     const size_t smem = buf + 4 * (size_t)NT + 8 * (size_t)words;
     const size_t most = gp::kTileBytes + 4 * (gp::kTileBytes / 64) + 8 * (size_t)gp::kMaxWords;
     static std::atomic<unsigned long long> ok[4][kMaxDevices];
     const int threads = row_block_threads(m, R);
     const uint32_t grid = std::min<uint32_t>(R, 32u * device_sm_count() * (128 / threads));
-    const gp::Heavy hv = heavy_of(scratch, R, m, col_blocks);
+    const gp::Heavy hv = heavy_of(scratch, R, m, col_blocks, balanced);
     const uint32_t hwords = bitmap_row_words(col_blocks);
     auto write = [&](auto kernel, int which, auto fill) {
         if (!allow_dynamic_smem(reinterpret_cast<const void*>(kernel), most, ok[which])) return BTC_E_CUDA;

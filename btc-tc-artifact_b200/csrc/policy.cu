@@ -30,7 +30,7 @@ constexpr int kThreads = 256;
 constexpr int kGrid = 64;
 constexpr uint32_t kSamples = kPolicySamples;
 constexpr int32_t kNear = kPolicyNear;
-// Skew of the row blocks (policy_skewed), for lists the grouped builder would take in natural order:
+// Skew of the row blocks, for lists the grouped builder would take in natural order:
 // 65,536 samples over 16,384 counters leave at most some 20 in one where row blocks are alike; 64
 // in one are a row block of a 1,024th of the edges.  Above that the grouped builder's CTA for it
 // is the last to end (build, grouped / sorted: R-MAT scale 20, edge factor 2, 16x32 2.05 / 0.68 ms;
@@ -46,73 +46,77 @@ __host__ __device__ __forceinline__ uint32_t skew_slot(int32_t u, int32_t v)
 // Sample i reads edge i * step.  Adds the number of local edges and their expectation
 // under uniform ids (per sampled edge: the chance that two uniform ids in [0, n) lie
 // closer than kNear, about (2 kNear - 1) / n), scaled by 2^20 to stay integer.  With
-// e_off / nv (a batch), an edge's n is its own graph's.  out: two sums and a ticket, zero at
-// the start; the last CTA hands the sums to the host (mapped memory) and zeroes them.
+// e_off / nv (a batch), an edge's n is its own graph's.  skew (nullable): kSkewSlots counters of the
+// samples' row blocks (of the oriented edge, hashed) and the most that one got.  out: two sums and a
+// ticket.  All are zero at the start; the last CTA hands the sums and the most to the host (mapped
+// memory) and zeroes them.
 __global__ void k_locality(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m,
                            int32_t n, const int64_t* __restrict__ e_off, const int32_t* __restrict__ nv,
-                           uint32_t G, int64_t step, unsigned long long* __restrict__ out,
-                           volatile unsigned long long* host)
+                           uint32_t G, int64_t step, unsigned int* __restrict__ skew,
+                           unsigned long long* __restrict__ out, volatile unsigned long long* host)
 {
+    constexpr int U = 4;  // samples in flight per thread
     unsigned long long local = 0, expect = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < kSamples;
-         i += (uint64_t)gridDim.x * kThreads) {
-        const int64_t e = (int64_t)i * step;
-        if (e >= m) break;
-        int32_t ng = n;
-        if (e_off) {
-            uint32_t lo = 0, hi = G;  // last g with e_off[g] <= e
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (e_off[mid] <= e) lo = mid;
-                else hi = mid;
-            }
-            ng = nv[lo];
+    unsigned int most = 0;
+    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i0 < kSamples; i0 += U * stride) {
+        int32_t u[U], v[U];
+        int64_t e[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const uint64_t i = i0 + k * stride;
+            e[k] = i < kSamples && (int64_t)i * step < m ? (int64_t)i * step : -1;
+            u[k] = e[k] >= 0 ? src[e[k]] : 0;
+            v[k] = e[k] >= 0 ? dst[e[k]] : 0;
         }
-        const int32_t u = src[e], v = dst[e];
-        policy_sample(u, v, ng, local, expect);
+        if (skew) {
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+                if (e[k] >= 0) most = max(most, atomicAdd(&skew[skew_slot(u[k], v[k])], 1u) + 1u);
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            if (e[k] < 0) continue;
+            int32_t ng = n;
+            if (e_off) {
+                uint32_t lo = 0, hi = G;  // last g with e_off[g] <= e
+                while (hi - lo > 1) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (e_off[mid] <= e[k]) lo = mid;
+                    else hi = mid;
+                }
+                ng = nv[lo];
+            }
+            policy_sample(u[k], v[k], ng, local, expect);
+        }
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
         local += __shfl_xor_sync(kFull, local, d);
         expect += __shfl_xor_sync(kFull, expect, d);
     }
+    most = __reduce_max_sync(kFull, most);
     if ((threadIdx.x & 31) == 0) {
         atomicAdd(&out[0], local);
         atomicAdd(&out[1], expect);
+        if (skew) atomicMax(&skew[kSkewSlots], most);
         __threadfence();
     }
+    __shared__ bool s_last;
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&out[2], 1ull) == gridDim.x - 1) {
-        host[0] = atomicExch(&out[0], 0ull);
-        host[1] = atomicExch(&out[1], 0ull);
-        out[2] = 0ull;
-        __threadfence_system();
-    }
-}
-
-// Sample i's row block, of the oriented edge, hashed to one of kSkewSlots counters: the most
-// samples that one counter got.
-__global__ void k_skew(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m, int64_t step,
-                       unsigned int* __restrict__ count, unsigned int* __restrict__ most_and_ticket,
-                       volatile unsigned long long* host)
-{
-    unsigned int most = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < kSamples;
-         i += (uint64_t)gridDim.x * kThreads) {
-        const int64_t e = (int64_t)i * step;
-        if (e >= m) break;
-        most = max(most, atomicAdd(&count[skew_slot(src[e], dst[e])], 1u) + 1u);
-    }
-    most = __reduce_max_sync(kFull, most);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(&most_and_ticket[0], most);
-        __threadfence();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(&out[2], 1ull) == gridDim.x - 1;
+        if (s_last) {
+            host[0] = atomicExch(&out[0], 0ull);
+            host[1] = atomicExch(&out[1], 0ull);
+            if (skew) host[2] = atomicMax(&skew[kSkewSlots], 0u);
+            out[2] = 0ull;
+            __threadfence_system();
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&most_and_ticket[1], 1u) == gridDim.x - 1) {
-        *host = atomicMax(&most_and_ticket[0], 0u);
-        __threadfence_system();
-    }
+    if (s_last && skew)
+        for (uint32_t i = threadIdx.x; i <= kSkewSlots; i += kThreads) skew[i] = 0u;
 }
 
 double locality_host(const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
@@ -163,26 +167,32 @@ bool policy_dense(int64_t m, int32_t n) { return pol::dense(m, n); }
 // handle keeps them: an allocation, a memset and a copy back cost a small graph's step 15 us).
 int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, bool on_host,
                     const int64_t* e_off, const int32_t* nv, uint32_t G, cudaStream_t s, PolicyWords& w,
-                    double* L)
+                    double* L, bool* skewed)
 {
     *L = 0.0;
+    if (skewed) *skewed = false;
     if (m <= 0) return BTC_OK;
     if (on_host) {
         *L = pol::locality_host(src, dst, m, n, e_off, nv, G);
+        if (skewed) *skewed = pol::skew_host(src, dst, m) >= pol::kSkewed;
         return BTC_OK;
     }
     if (!w.host && !(w.host = host_slot_alloc(&w.host_context))) return BTC_E_NOMEM;
     void* d_host = nullptr;
     BTC_CUDA_TRY(cudaHostGetDevicePointer(&d_host, w.host, 0));
-    const bool fresh = w.dev.ptr == nullptr;
+    const bool fresh = w.dev.ptr == nullptr, fresh_skew = w.skew.ptr == nullptr;
     BTC_TRY(w.dev.reserve(3 * sizeof(unsigned long long)));
     // (a call that failed on its way may have left something in them)
     if (fresh || w.dirty) BTC_CUDA_TRY(cudaMemsetAsync(w.dev.ptr, 0, 3 * sizeof(unsigned long long), s));
+    constexpr size_t skew_bytes = sizeof(unsigned int) * (pol::kSkewSlots + 1);
+    if (skewed) BTC_TRY(w.skew.reserve(skew_bytes));
+    if (w.skew.ptr && (fresh_skew || w.dirty)) BTC_CUDA_TRY(cudaMemsetAsync(w.skew.ptr, 0, skew_bytes, s));
+    unsigned int* skew = skewed ? w.skew.as<unsigned int>() : nullptr;
     w.dirty = true;
     const int64_t step = m > (int64_t)pol::kSamples ? m / (int64_t)pol::kSamples : 1;
     const int64_t samples = m < (int64_t)pol::kSamples ? m : (int64_t)pol::kSamples;
     const int grid = (int)((samples + 4 * pol::kThreads - 1) / (4 * pol::kThreads));
-    pol::k_locality<<<grid, pol::kThreads, 0, s>>>(src, dst, m, n, e_off, nv, G, step,
+    pol::k_locality<<<grid, pol::kThreads, 0, s>>>(src, dst, m, n, e_off, nv, G, step, skew,
                                                    w.dev.as<unsigned long long>(),
                                                    static_cast<unsigned long long*>(d_host));
     BTC_CUDA_TRY(cudaGetLastError());
@@ -190,39 +200,7 @@ int policy_locality(const int32_t* src, const int32_t* dst, int64_t m, int32_t n
     w.dirty = false;
     const volatile unsigned long long* h = w.host;
     *L = h[1] ? (double)h[0] / (double)h[1] : 0.0;
-    return BTC_OK;
-}
-
-// Enqueues the skew sample of a device edge list; its result is in w.host[2] after a wait.
-static int enqueue_skew(const int32_t* src, const int32_t* dst, int64_t m, cudaStream_t s, PolicyWords& w)
-{
-    if (!w.host && !(w.host = host_slot_alloc(&w.host_context))) return BTC_E_NOMEM;
-    void* d_host = nullptr;
-    BTC_CUDA_TRY(cudaHostGetDevicePointer(&d_host, w.host, 0));
-    const size_t bytes = sizeof(unsigned int) * (pol::kSkewSlots + 2);
-    BTC_TRY(w.skew.reserve(bytes));
-    BTC_CUDA_TRY(cudaMemsetAsync(w.skew.ptr, 0, bytes, s));
-    const int64_t step = m > (int64_t)pol::kSamples ? m / (int64_t)pol::kSamples : 1;
-    const int64_t samples = m < (int64_t)pol::kSamples ? m : (int64_t)pol::kSamples;
-    pol::k_skew<<<(unsigned)((samples + 4 * pol::kThreads - 1) / (4 * pol::kThreads)), pol::kThreads, 0, s>>>(
-        src, dst, m, step, w.skew.as<unsigned int>(), w.skew.as<unsigned int>() + pol::kSkewSlots,
-        static_cast<unsigned long long*>(d_host) + 2);
-    BTC_CUDA_TRY(cudaGetLastError());
-    return BTC_OK;
-}
-
-int policy_skewed(const int32_t* src, const int32_t* dst, int64_t m, bool on_host, cudaStream_t s, PolicyWords& w,
-                  bool* skewed)
-{
-    *skewed = false;
-    if (m <= 0) return BTC_OK;
-    if (on_host) {
-        *skewed = pol::skew_host(src, dst, m) >= pol::kSkewed;
-        return BTC_OK;
-    }
-    BTC_TRY(enqueue_skew(src, dst, m, s, w));
-    BTC_CUDA_TRY(cudaStreamSynchronize(s));
-    *skewed = *static_cast<volatile unsigned long long*>(w.host + 2) >= pol::kSkewed;
+    if (skewed) *skewed = h[2] >= pol::kSkewed;
     return BTC_OK;
 }
 
@@ -233,10 +211,10 @@ int policy_select(const int32_t* src, const int32_t* dst, int64_t m, int32_t n, 
     double L = 0.0;
     // (the locality decides only where neither the degree nor the ordering does)
     if (!(flags & BTC_ORIENT_DEGREE) && !pol::dense(m, n)) {
-        const bool with_skew = skewed && m > 0 && !(flags & BTC_INPUT_ON_HOST);
-        if (with_skew) BTC_TRY(enqueue_skew(src, dst, m, s, w));  // (the wait below is for both)
-        BTC_TRY(policy_locality(src, dst, m, n, (flags & BTC_INPUT_ON_HOST) != 0, nullptr, nullptr, 0, s, w, &L));
-        if (with_skew) *skewed = *static_cast<volatile unsigned long long*>(w.host + 2) >= pol::kSkewed;
+        bool is = false;
+        BTC_TRY(policy_locality(src, dst, m, n, (flags & BTC_INPUT_ON_HOST) != 0, nullptr, nullptr, 0, s, w, &L,
+                                skewed ? &is : nullptr));
+        if (skewed) *skewed = is;
     }
     return btc_tile_policy_from_features(m, n, flags, L, tile_cols, tau);
 }

@@ -6,8 +6,8 @@
 // has a bit: the column blocks u has lower neighbours in.  All lists sit in one array in
 // vertex order; vertex u's list is ent[off[u], off[u+1]).  Entries number at most the
 // unique edges (every listed tile row holds at least one edge), so the caller sizes ent
-// by the input edge count.  Built by the first count that takes the row-wise kernel, from the
-// per-tile row-occupancy masks (row blocks averaging 8 or more tiles), in three steps:
+// by the input edge count.  Built by the build of a graph that the row-wise kernel counts, else by
+// the first count that takes it, from the per-tile row-occupancy masks (row blocks averaging 8 or more tiles), in three steps:
 //   k_ri_totals   one warp per row block: popcount of its tiles' masks
 //   scan          exclusive prefix of the totals (per-CTA reduce, one-CTA scan of the
 //                 CTA sums, per-CTA down-sweep)

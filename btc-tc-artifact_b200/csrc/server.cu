@@ -172,7 +172,8 @@ size_t batch_bytes_bound(int64_t m, int64_t rows, int64_t words, int64_t graphs,
     // kernels' index is smaller
     size_t store = 72 * r;
     if (m_ >= 8 * r) {
-        const size_t chunk = btc200::kRowLanes * (sizeof(uint4) + (btc200::row_store_wide(rows) ? sizeof(uint2) : sizeof(uint32_t)));
+        const size_t keys = btc200::row_store_wide(rows) ? sizeof(uint2) : sizeof(uint32_t);
+        const size_t chunk = btc200::kRowLanes * (sizeof(uint4) + keys);
         store += (size_t)btc200::row_store_chunks(m_, r) * (chunk + 1);
     }
     const size_t sum = 8 * m_ + cells + tiles + 4 * r + store + 80 * (size_t)graphs;
