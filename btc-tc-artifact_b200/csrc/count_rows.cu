@@ -1,6 +1,6 @@
-// count_rows.cu -- the count kernel for graphs whose row blocks hold many dense tiles, and for
-// any graph of many tiles under a tau below the default (its sparse path; otherwise such
-// graphs stream, count_stream.cu): row-wise matching with flattened work units.
+// count_rows.cu -- the count kernel for graphs whose row blocks hold many tiles and that are dense
+// or of short rows, and for any graph of many tiles under a tau below the default (its sparse
+// path; otherwise such graphs stream, count_stream.cu): row-wise matching with flattened work units.
 //
 // Computes what btc/operations/tc_16x128_mma_v5.h:9-211 and tc_16x32_mma_v6.h:9-238
 // compute -- for every set bit (r, c) of every sample tile S = (I, J_L) of L, with c in

@@ -22,7 +22,7 @@
 // wavefronts.  One full ncu capture each: R-MAT scale 20 in degree order L1 73%, issue 56%, DRAM
 // 4%, L2 hits 92%, 876M warp instructions in 1.38 ms (2.85 ms by the row-wise kernel over the
 // tiles); 8 communities on 32,768 vertices L1 95%, issue 53%, 0.65 ms (3.18).  R-MAT scale 22:
-// 21.9 GB of DRAM traffic at 2.0 TB/s, issue 46%, 10.9 ms (77.8 GB, 20.8 ms).
+// 21.6 GB of DRAM traffic at 2.0 TB/s, issue 47%, 10.8 ms (77.8 GB, 20.8 ms).
 #include "count_common.cuh"
 
 #include <atomic>

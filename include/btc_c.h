@@ -218,10 +218,10 @@ BTC_API int btc_rebuild_bitbsr(btc_bitbsr* g, const int32_t* src, const int32_t*
 /* Counts the triangles of a handle: enqueues the count on `stream`, waits, and
  * writes *out_count.  tau: dense/sparse switch (BTC_TAU_DEFAULT for the engine's): a tile
  * whose popcount exceeds it takes the tensor cores where a tile kernel counts.  At the
- * default or above, graphs averaging 8 or more tiles per row block and not dense are counted
- * from per-vertex rows instead; a lower tau keeps them on the tile kernels, whose index the
- * first such count after a build makes (allocated then; never while `stream` is capturing,
- * where the count goes without it).
+ * default or above, graphs averaging 8 or more tiles per row block that are neither dense nor of
+ * short rows are counted from per-vertex rows instead; a lower tau keeps them on the tile
+ * kernels, whose index the first such count after a build makes (allocated then; never while
+ * `stream` is capturing, where the count goes without it).
  * kernel_ms (nullable): event time of the count kernel alone.  Replaces
  * count_triangles_16x{128,32}_adaptive (tc_16x128_adaptive.h:12, tc_16x32_adaptive.h:14). */
 BTC_API int btc_count(btc_bitbsr* g, int tau, btc_stream_t stream, unsigned long long* out_count,
