@@ -463,6 +463,39 @@ static bool bitmap_takes(const BuildGeom& geom, int64_t m)
     return bytes <= (4ull << 30) && bytes <= 32ull * (uint64_t)m + (64ull << 20);
 }
 
+static int mark_tail(btc_bitbsr* g, cudaStream_t s)
+{
+    if (!g->meta_event)
+        BTC_CUDA_TRY(cudaEventCreateWithFlags(&g->meta_event, cudaEventDisableTiming));
+    BTC_CUDA_TRY(cudaEventRecord(g->meta_event, s));
+    g->tail = true;
+    return BTC_OK;
+}
+
+// (inside a capture the event is one from outside it)
+static int wait_tail(btc_bitbsr* g, cudaStream_t s)
+{
+    if (g->tail)
+        BTC_CUDA_TRY(cudaStreamWaitEvent(s, g->meta_event,
+                                         stream_capturing(s) ? cudaEventWaitExternal : cudaEventWaitDefault));
+    return BTC_OK;
+}
+
+// After a build whose tiles the host knows (row masks made where they average 8 per row block): the
+// row store, or the row-wise kernel's index, or neither.
+static int finish_known(btc_bitbsr* g, const BuildPlan& P, uint32_t widest, bool tiles_only, cudaStream_t s)
+{
+    const int64_t R = P.geom.n_row_blocks;
+    const uint32_t T = g->num_tiles;
+    g->heavy = !tiles_only && row_store_possible(P.m, P.geom.n_row_blocks) && (uint64_t)T >= 8ull * (uint64_t)R;
+    g->row_store = g->heavy && !tiles_win(g->tile_cols, P.m, T, R, widest, P.use_bitmap) &&
+                   reserve_row_store(g, std::min<uint64_t>((uint64_t)P.m, 32ull * tile_capacity(g))) == BTC_OK;
+    if (g->row_store) BTC_TRY(enqueue_row_store(g, nullptr, T, P.degree, s));
+    g->index_built = g->heavy && !g->row_store && P.use_bitmap && reserve_row_index(g, tile_capacity(g));
+    if (g->index_built) BTC_TRY(enqueue_row_index(g, nullptr, T, s));
+    return g->row_store || g->index_built ? mark_tail(g, s) : BTC_OK;
+}
+
 // tiles_only: the caller keeps the reference-shaped arrays alone, so no row store is made.
 static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int64_t m, int32_t n,
                       int tile_cols, uint32_t flags, cudaStream_t s, bool tiles_only = false,
@@ -473,6 +506,8 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     if (flags & ~(BTC_INPUT_ON_HOST | BTC_ORIENT_DEGREE | BTC_BUILD_RADIX | BTC_BUILD_ASYNC))
         return BTC_E_INVAL;
     if (g->pending) resolve_build(g);  // an enqueued build still owns the buffers
+    BTC_TRY(wait_tail(g, s));
+    g->tail = false;
     // A small graph in natural order is built by one launch (small.cu), which also picks the
     // tile width where it is open: device input, and not the degree's to decide.
     bool small = allow_small && !(flags & (BTC_ORIENT_DEGREE | BTC_BUILD_RADIX | BTC_BUILD_ASYNC)) &&
@@ -499,12 +534,12 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     BuildPlan P{};
     P.geom = make_geom(n, tile_cols);
     const BuildGeom& geom = P.geom;
-    // the previous build of this handle, when it had the same geometry, predicts whether
-    // the graph averages 8 or more tiles per row block (the row store's condition)
-    const bool prev_light = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks &&
-                            g->num_tiles > 0 &&
-                            (uint64_t)g->num_tiles < 8ull * (uint64_t)geom.n_row_blocks;
-    // ... and, with its tiles, whether the tile kernels count it faster than a row store does
+    // What an enqueued build cannot know: the previous graph of this handle, at the same width,
+    // predicts whether this one averages 8 or more tiles per row block (the row store's condition)
+    const bool prev_light = g->tile_cols == tile_cols && g->num_tiles > 0 &&
+                            (uint64_t)g->num_tiles < 8ull * (uint64_t)g->n_row_blocks;
+    // ... and, when it had the same geometry, whether the tile kernels count it faster than a row
+    // store does
     const uint32_t widest = ((uint32_t)n + 63) / 64;
     const bool prev_same = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks;
     const uint32_t prev_tiles = g->num_tiles;
@@ -634,12 +669,13 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
                                                  std::min<uint64_t>(g->row_indices.bytes / 4, g->rowmask.bytes / 4));
         P.cap32 = (uint32_t)std::min<uint64_t>(rows, g->blocks.bytes / 64);
         P.cap128 = (uint32_t)std::min<uint64_t>(rows, g->blocks.bytes / 256);
-        // The row store of the streaming count.  A rebuild whose previous graph of the same
-        // geometry averaged fewer than 8 tiles per row block skips it (a mesh counts faster
-        // tile-wise); should this graph average more after all, the count takes the
-        // tile-wise kernel, which needs no store.  So does a graph without the memory for it.
-        // (A build by one launch decides when it knows the tiles.)
-        P.heavy = !small && !tiles_only && P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light;
+        // The row store of the streaming count.  A build that waits decides when it knows the tiles
+        // (the store is then enqueued after the wait, where the count would have been).  An enqueued
+        // one goes by the previous graph: where that averaged fewer than 8 tiles per row block it
+        // makes none (a mesh counts faster tile-wise); should this graph average more after all,
+        // the count takes the tile-wise kernel, which needs no store.  So does a graph without
+        // the memory for it.
+        P.heavy = enqueued && !tiles_only && P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light;
         P.row_store = P.heavy &&
                       !(prev_same && tiles_win(tile_cols, m, prev_tiles, geom.n_row_blocks, widest, P.use_bitmap)) &&
                       reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * P.cap)) == BTC_OK;
@@ -682,16 +718,8 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
             }
             if (st2 == BTC_E_CAPACITY)
                 return build_into(g, src, dst, m, n, tile_cols, flags, s, tiles_only, false);
-            if (st2 != BTC_OK) return st2;
-            g->heavy = !tiles_only && row_store_possible(m, geom.n_row_blocks) &&
-                       (uint64_t)g->num_tiles >= 8ull * (uint64_t)geom.n_row_blocks;
-            g->row_store = g->heavy && !tiles_win(tile_cols, m, g->num_tiles, geom.n_row_blocks, widest, P.use_bitmap) &&
-                           reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * tile_capacity(g))) == BTC_OK;
-            if (g->row_store) BTC_TRY(enqueue_row_store(g, nullptr, g->num_tiles, false, s));
-            g->index_built = g->heavy && !g->row_store && reserve_row_index(g, tile_capacity(g));
-            if (g->index_built) BTC_TRY(enqueue_row_index(g, nullptr, g->num_tiles, s));
-            return BTC_OK;
         }
+        if (st2 == BTC_OK) return finish_known(g, P, widest, tiles_only, s);
         if (st2 != BTC_E_CAPACITY) return st2;
         // more tiles than the arrays hold: redo the post-count steps at the right size
         BTC_CUDA_TRY(cudaMemsetAsync(meta + kMetaOverflow, 0, sizeof(unsigned long long), s));
@@ -748,7 +776,7 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     g->heavy = P.heavy;
     g->row_store = P.row_store;
     g->index_built = P.row_index;
-    return BTC_OK;
+    return mark_tail(g, s);
 }
 
 int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_out2,
@@ -759,6 +787,7 @@ int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_o
     if (tau < 0) return BTC_E_INVAL;
     if (!g->pending && g->failed != BTC_OK) return g->failed;
     BTC_TRY(ensure_count_scratch(g));
+    BTC_TRY(wait_tail(g, s));
     CountScratch scr{g->partials.as<unsigned long long>(), g->done.as<unsigned int>(),
                      reinterpret_cast<unsigned long long*>(g->done.as<char>() + 8),
                      g->result.as<unsigned long long>(), d_out2};
@@ -776,8 +805,10 @@ int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_o
     // A caller's lower tau asks for the tensor cores, which only the tile kernels use.  While an
     // enqueued build is pending its tiles are not known (num_tiles is the graph's before it, of
     // whatever size): the store it has made is used.
-    if (g->row_store && tau >= default_tau(g->tile_cols) &&
-        (g->pending || !dense_graph(g->tile_cols, g->input_edges, g->num_tiles, g->n_row_blocks)))
+    // Once they are known, a mesh and a dense graph take the tile kernels all the same.
+    const bool streams = g->pending || ((uint64_t)g->num_tiles >= 8ull * (uint64_t)g->n_row_blocks &&
+                                        !dense_graph(g->tile_cols, g->input_edges, g->num_tiles, g->n_row_blocks));
+    if (g->row_store && tau >= default_tau(g->tile_cols) && streams)
         return launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks,
                                    g->tile_cols, g->n_row_blocks, ((uint32_t)g->n + 63) / 64, scr, nullptr, 0,
                                    nullptr, g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), tile_begin,

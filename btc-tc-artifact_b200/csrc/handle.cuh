@@ -56,6 +56,10 @@ struct btc_bitbsr {
     uint32_t pending_cap = 0;  // tile capacity the enqueued build ran against
     int failed = 0;  // status of the last build (BTC_OK once resolved without error)
     cudaEvent_t meta_event = nullptr;
+    // A build that has waited may enqueue more after its wait (the row store, its index, the
+    // tiles themselves where the arrays grew); meta_event then marks the end, which a count or
+    // a rebuild on any stream waits for.
+    bool tail = false;
     // CUDA graph of a repeated asynchronous rebuild (captured on the second identical call)
     cudaGraphExec_t graph_exec = nullptr;
     BuildGraphKey graph_key{};

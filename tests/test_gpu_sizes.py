@@ -1,0 +1,128 @@
+"""One handle rebuilt with graphs of changing sizes and kinds: each is counted by the kernel its
+own tiles ask for, waiting and enqueued, on the build's stream and on another."""
+from __future__ import annotations
+
+import statistics
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from btc_b200 import BitBSR, graphs as G  # noqa: E402
+from oracle import oracle as O  # noqa: E402
+
+
+def _cuda(g):
+    return torch.from_numpy(g[0]).cuda(), torch.from_numpy(g[1]).cuda(), g[2]
+
+
+def _uniform(n, m, seed):
+    e = np.random.default_rng(seed).integers(0, n, (2, m)).astype(np.int32)
+    return e[0], e[1], n
+
+
+def _want(g):
+    rp, col, _ = O.lower_csr(*g)
+    return O.tc_merge(rp, col)
+
+
+def _us(f):
+    for _ in range(3):
+        f()
+    t = []
+    for _ in range(7):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        f()
+        torch.cuda.synchronize()
+        t.append((time.perf_counter() - t0) * 1e6)
+    return statistics.median(t)
+
+
+@pytest.mark.parametrize("asynchronous", [False, True])
+@pytest.mark.parametrize("make,k", [(G.stencil27, 50), (G.stencil7, 70)])
+def test_meshes_of_changing_size_stay_with_the_tile_kernel(make, k, asynchronous):
+    """Two mesh sizes in turn on one handle, against a handle each: the work is the same (two to
+    three and a half times when a changed size made a row store and streamed)."""
+    graphs = [_cuda(make(k)), _cuda(make(k + 1))]
+    one = [BitBSR(*g) for g in graphs]
+    both = BitBSR(*graphs[0])
+    out = torch.zeros(1, dtype=torch.int64, device="cuda")
+
+    def step(h, g):
+        h.rebuild(*g, asynchronous=asynchronous)
+        if asynchronous:
+            h.count_async(d_out=out.data_ptr())
+        else:
+            h.count()
+
+    for g, h in zip(graphs, one):
+        both.rebuild(*g)
+        assert both.count() == h.count()
+    apart = sum(_us(lambda h=h, g=g: step(h, g)) for h, g in zip(one, graphs))
+    in_turn = _us(lambda: [step(both, g) for g in graphs])
+    assert in_turn < 1.6 * apart, (in_turn, apart)
+    for h in one + [both]:
+        h.free()
+
+
+@pytest.mark.parametrize("deg", [False, True])
+@pytest.mark.parametrize("tile_cols", [32, 128])
+def test_kinds_in_turn(tile_cols, deg):
+    """Meshes, uniform, power-law and dense graphs of several sizes through one handle."""
+    graphs = [G.stencil27(18), _uniform(9000, 150000, 1), G.rmat_raw_np(13, 16, 2), G.complete(300), G.stencil7(40),
+              _uniform(70000, 140000, 3), _uniform(9000, 600000, 4)]
+    want = [_want(g) for g in graphs]
+    cuda = [_cuda(g) for g in graphs]
+    h = BitBSR(*cuda[0], tile_cols, orient_degree=deg)
+    for g in cuda:  # room for each
+        h.rebuild(*g, tile_cols, orient_degree=deg)
+    other = torch.cuda.Stream()
+    out = torch.zeros(1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    rng = np.random.default_rng(6)
+    for i in rng.integers(0, len(graphs), 40):
+        mode = int(rng.integers(3))
+        h.rebuild(*cuda[i], tile_cols, orient_degree=deg, asynchronous=mode == 1)
+        if mode == 2:  # a build that has waited, counted on another stream
+            h.count_async(stream=other, d_out=out.data_ptr())
+            other.synchronize()
+            assert int(out.item()) == want[i], i
+        else:
+            assert h.count() == want[i], i
+        b = h.partition(3)
+        assert sum(int(h.count_tiles(x, y).item()) for x, y in zip(b[:-1], b[1:])) == want[i], i
+    h.free()
+
+
+@pytest.mark.parametrize("make", [lambda: G.rmat_raw_np(15, 16, 7), lambda: _uniform(9000, 150000, 8)])
+def test_count_captured_right_after_a_waiting_build(make):
+    """What a waiting build enqueues after its wait is waited for by a count captured on another
+    stream, and by a rebuild on another stream."""
+    host = make()
+    g, want = _cuda(host), _want(host)
+    h = BitBSR(*g)
+    assert h.count() == want
+    side, out = torch.cuda.Stream(), torch.zeros(1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    h.rebuild(*g)
+    with torch.cuda.graph(graph, stream=side):
+        h.count_async(stream=side, d_out=out.data_ptr())
+    for _ in range(5):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert int(out.item()) == want
+    for _ in range(5):
+        h.rebuild(*g)
+        h.rebuild(*g, stream=side)
+        h.count_async(d_out=out.data_ptr())
+        torch.cuda.synchronize()
+        assert int(out.item()) == want
+    graph.reset()
+    h.free()
