@@ -171,6 +171,7 @@ struct BuildPlan {
     uint32_t cap;  // > 0: the post-count steps run against this tile capacity
     bool heavy = false;      // the graph can average 8 tiles per row block: make its row masks
     bool row_store = false;  // ... and the streaming count's row store (rowstore.cu)
+    bool open = false;       // ... both only if it does (by the device's tile count)
     bool row_index = false;  // ... or the row-wise kernel's index
 };
 
@@ -214,11 +215,12 @@ int reserve_row_store(btc_bitbsr* g, uint64_t entries)
 
 // The row store after the tiles and row masks (T = *d_tiles bounded by cap, or cap itself).
 static int enqueue_row_store(btc_bitbsr* g, const unsigned long long* d_tiles, uint32_t cap,
-                             bool by_degree, cudaStream_t s)
+                             bool by_degree, cudaStream_t s, bool open = false)
 {
     return launch_rowstore(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
                            g->blocks.as<uint32_t>(), g->n_row_blocks, g->rowmask.as<uint32_t>(), d_tiles,
-                           cap, by_degree, g->meta.as<unsigned long long>(), row_store_of(g), s);
+                           cap, by_degree, g->meta.as<unsigned long long>(), row_store_of(g), s,
+                           open ? 8ull * (uint64_t)g->n_row_blocks : 0ull);
 }
 
 bool stream_capturing(cudaStream_t s)
@@ -360,9 +362,10 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
                                          g->prefix.as<uint2>(), g->indices.as<uint32_t>(),
                                          g->row_indices.as<uint32_t>(), g->indptr.as<uint32_t>(),
                                          g->blocks.as<uint32_t>(), meta, P.cap, g->d_hmeta, s,
-                                         g->rowmask.as<uint32_t>(), P.heavy, P.row_store));
+                                         g->rowmask.as<uint32_t>(), P.heavy && !P.open,
+                                         P.row_store && !P.open));
             // (the fill pass set the row masks, or found the longest row-block list)
-            if (P.row_store) BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s));
+            if (P.row_store) BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s, P.open));
             if (P.row_index) BTC_TRY(enqueue_row_index(g, meta + kMetaTiles, P.cap, s));
         }
     } else if (P.use_group) {
@@ -374,9 +377,8 @@ static int enqueue_build(btc_bitbsr* g, const BuildPlan& P, uint64_t** sorted_ou
         if (P.cap) {
             BTC_TRY(launch_finish_tiles(g->indptr.as<uint32_t>(), geom.n_row_blocks, meta, P.cap, g->d_hmeta, s));
             BTC_TRY(enqueue_group_write(g, P, P.cap, s));
-            if (P.row_store)
-                BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s));
-            else
+            if (P.row_store) BTC_TRY(enqueue_row_store(g, meta + kMetaTiles, P.cap, P.degree, s, P.open));
+            if (!P.row_store || P.open)
                 BTC_TRY(launch_rowmask(geom.tile_cols, g->blocks.as<uint32_t>(), P.cap,
                                        meta + kMetaTiles, g->indptr.as<uint32_t>(), geom.n_row_blocks,
                                        g->rowmask.as<uint32_t>(), meta + kMetaRowMax, s, false));
@@ -412,7 +414,7 @@ static void build_key(const btc_bitbsr* g, const BuildPlan& P, BuildGraphKey* k)
     k->n = P.n;
     k->tile_cols = P.geom.tile_cols;
     k->flags = P.flags | (P.row_store ? 0x80000000u : 0u) | (P.use_group ? 0x40000000u : 0u) |
-               (P.heavy ? 0x20000000u : 0u) | (P.row_index ? 0x10000000u : 0u);
+               (P.heavy ? 0x20000000u : 0u) | (P.row_index ? 0x10000000u : 0u) | (P.open ? 0x08000000u : 0u);
     k->cap = P.cap;
 }
 
@@ -534,14 +536,12 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
     BuildPlan P{};
     P.geom = make_geom(n, tile_cols);
     const BuildGeom& geom = P.geom;
-    // What an enqueued build cannot know: the previous graph of this handle, at the same width,
-    // predicts whether this one averages 8 or more tiles per row block (the row store's condition)
-    const bool prev_light = g->tile_cols == tile_cols && g->num_tiles > 0 &&
-                            (uint64_t)g->num_tiles < 8ull * (uint64_t)g->n_row_blocks;
-    // ... and, when it had the same geometry, whether the tile kernels count it faster than a row
-    // store does
+    // What an enqueued build cannot know: the previous graph of this handle, when it had the same
+    // geometry, predicts whether this one averages 8 or more tiles per row block (the row store's
+    // condition) and, with its tiles, whether the tile kernels count it faster than a row store does
     const uint32_t widest = ((uint32_t)n + 63) / 64;
     const bool prev_same = g->tile_cols == tile_cols && g->n_row_blocks == geom.n_row_blocks;
+    const bool prev_light = g->num_tiles > 0 && (uint64_t)g->num_tiles < 8ull * (uint64_t)g->n_row_blocks;
     const uint32_t prev_tiles = g->num_tiles;
     g->tile_cols = tile_cols;
     g->n = n;
@@ -671,19 +671,23 @@ static int build_into(btc_bitbsr* g, const int32_t* src, const int32_t* dst, int
         P.cap128 = (uint32_t)std::min<uint64_t>(rows, g->blocks.bytes / 256);
         // The row store of the streaming count.  A build that waits decides when it knows the tiles
         // (the store is then enqueued after the wait, where the count would have been).  An enqueued
-        // one goes by the previous graph: where that averaged fewer than 8 tiles per row block it
+        // one whose previous graph of the same geometry averaged fewer than 8 tiles per row block
         // makes none (a mesh counts faster tile-wise); should this graph average more after all,
         // the count takes the tile-wise kernel, which needs no store.  So does a graph without
-        // the memory for it.
-        P.heavy = enqueued && !tiles_only && P.cap && row_store_possible(m, geom.n_row_blocks) && !prev_light;
+        // the memory for it.  After such a graph of another geometry, of whose size nothing follows
+        // for this one, the device decides: two launches that may find nothing to do.
+        P.heavy = enqueued && !tiles_only && P.cap && row_store_possible(m, geom.n_row_blocks) &&
+                  !(prev_same && prev_light);
         P.row_store = P.heavy &&
                       !(prev_same && tiles_win(tile_cols, m, prev_tiles, geom.n_row_blocks, widest, P.use_bitmap)) &&
                       reserve_row_store(g, std::min<uint64_t>((uint64_t)m, 32ull * P.cap)) == BTC_OK;
+        P.open = P.row_store && prev_light;
         // (the index needs the cell pairs beside it, which the bitmap builder makes)
         P.row_index = P.heavy && !P.row_store && P.use_bitmap && reserve_row_index(g, P.cap);
         g->heavy = P.heavy;
         g->row_store = P.row_store;
         g->index_built = P.row_index;
+        g->open = P.open;
     }
 
     uint64_t* sorted = nullptr;
@@ -806,30 +810,39 @@ int count_handle(btc_bitbsr* g, int tau, cudaStream_t s, unsigned long long* d_o
     // enqueued build is pending its tiles are not known (num_tiles is the graph's before it, of
     // whatever size): the store it has made is used.
     // Once they are known, a mesh and a dense graph take the tile kernels all the same.
-    const bool streams = g->pending || ((uint64_t)g->num_tiles >= 8ull * (uint64_t)g->n_row_blocks &&
+    const bool open = g->pending && g->open;
+    const uint64_t many = 8ull * (uint64_t)g->n_row_blocks;
+    const bool streams = g->pending || ((uint64_t)g->num_tiles >= many &&
                                         !dense_graph(g->tile_cols, g->input_edges, g->num_tiles, g->n_row_blocks));
+    const uint64_t wpr = bitmap_words_per_row(make_geom(g->n, g->tile_cols));
+    auto tiles_count = [&](const uint32_t* rowmask, const uint2* cellpp, bool index, uint32_t hint) {
+        return launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
+                            g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(),
+                            cap, g->n_row_blocks, tau, scr, s, nullptr, 0, nullptr, rowmask, cellpp, wpr,
+                            g->meta.as<unsigned long long>() + kMetaRowMax, tile_begin, tile_end,
+                            build_meta, hint, index ? g->row_off.as<uint32_t>() : nullptr,
+                            index ? g->row_ent.as<uint2>() : nullptr, dense);
+    };
+    if (open) {
+        scr.tiles_below = many;
+        BTC_TRY(tiles_count(nullptr, nullptr, false, g->num_tiles));
+        scr.tiles_below = ~0ull;
+        scr.tiles_from = many;
+    }
     if (g->row_store && tau >= default_tau(g->tile_cols) && streams)
         return launch_count_stream(row_store_of(g), g->meta.as<unsigned long long>() + kMetaRowChunks,
                                    g->tile_cols, g->n_row_blocks, ((uint32_t)g->n + 63) / 64, scr, nullptr, 0,
                                    nullptr, g->row_indices.as<uint32_t>(), g->indices.as<uint32_t>(), tile_begin,
                                    std::min(tile_end, cap), whole, true, build_meta,
                                    count_grid_size(g->tile_cols), s);
-    const uint64_t wpr = bitmap_words_per_row(make_geom(g->n, g->tile_cols));
     bool cells = g->cells && !g->cells_lazy, index = false;
-    if (g->heavy) {
+    if (g->heavy && (g->pending || g->num_tiles >= many)) {
         const unsigned long long* d_tiles = build_meta ? build_meta + kMetaTiles : nullptr;
         cells = ensure_cells(g, d_tiles, cap, wpr * (uint64_t)g->n_row_blocks, wpr, s);
         index = cells && ensure_row_index(g, d_tiles, cap, s);
     }
-    return launch_count(g->tile_cols, g->indptr.as<uint32_t>(), g->indices.as<uint32_t>(),
-                        g->row_indices.as<uint32_t>(), g->blocks.as<uint32_t>(),
-                        cap, g->n_row_blocks, tau, scr, s,
-                        nullptr, 0, nullptr, g->rowmask.as<uint32_t>(),
-                        cells ? g->prefix.as<uint2>() : nullptr, wpr,
-                        g->meta.as<unsigned long long>() + kMetaRowMax, tile_begin, tile_end,
-                        build_meta, g->num_tiles,
-                        index ? g->row_off.as<uint32_t>() : nullptr,
-                        index ? g->row_ent.as<uint2>() : nullptr, dense);
+    return tiles_count(g->rowmask.as<uint32_t>(), cells ? g->prefix.as<uint2>() : nullptr, index,
+                       open ? (uint32_t)std::max<uint64_t>(g->num_tiles, many) : g->num_tiles);
 }
 
 int resolve_build(btc_bitbsr* g)

@@ -232,6 +232,9 @@ struct CountScratch {
     // optional device alias of mapped pinned host memory that also receives the count
     // (written by the last CTA, no copy-engine hop)
     unsigned long long* result_host = nullptr;
+    // A count behind an enqueued build (build_meta) whose tiles the host cannot guess is launched for
+    // few and for many: the launch whose bounds the tiles are outside of leaves everything as it is.
+    unsigned long long tiles_from = 0, tiles_below = ~0ull;
 };
 
 int count_grid_size(int tile_cols);
@@ -303,7 +306,7 @@ int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* o
 int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indices, const uint32_t* blocks,
                     int32_t n_row_blocks, const uint32_t* rowmask, const unsigned long long* d_tiles,
                     uint32_t cap, bool by_degree, unsigned long long* meta, const RowStore& out,
-                    cudaStream_t s);
+                    cudaStream_t s, unsigned long long least = 0);
 
 // The streaming count (count_stream.cu) of the sample tiles [tile_begin, tile_end), or of
 // all of them with `whole`.  rs_chunks: the store's meta[kMetaRowChunks], with meta[kMetaRowLong]
@@ -459,6 +462,11 @@ enum {
     kMetaSlots = 10
 };
 static_assert(kMetaSlots <= kHostSlotWords, "a host slot holds the metadata");
+
+__device__ __forceinline__ bool count_is_another(const CountScratch& scr, const unsigned long long* build_meta)
+{
+    return build_meta && (build_meta[kMetaTiles] < scr.tiles_from || build_meta[kMetaTiles] >= scr.tiles_below);
+}
 
 // Queue/completion words of the count kernel: done (u32) at byte 0, work (u64) at 8.
 constexpr size_t kCountCtlBytes = 16;

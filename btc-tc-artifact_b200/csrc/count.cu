@@ -313,6 +313,7 @@ k_count(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indice
     __shared__ unsigned long long s_red[kWarps];
     __shared__ int s_last;
 
+    if (count_is_another(scr, build_meta)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     WarpSmem<C>& s = smem_all[warp];
     const unsigned lt = lanemask_lt();

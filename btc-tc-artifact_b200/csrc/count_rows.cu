@@ -90,6 +90,7 @@ k_count_rows(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ i
     __shared__ unsigned long long s_red[kRWarps];
     __shared__ int s_last;
 
+    if (count_is_another(scr, build_meta)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     RowSmem<C>& s = reinterpret_cast<RowSmem<C>*>(rows_smem_raw)[warp];
     const unsigned lt = lanemask_lt();

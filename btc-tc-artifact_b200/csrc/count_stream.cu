@@ -112,6 +112,7 @@ k_count_stream(const uint32_t* __restrict__ off, const void* __restrict__ key_wo
     extern __shared__ __align__(16) unsigned char stream_smem_raw[];
     __shared__ unsigned long long s_red[kSWarps];
     __shared__ int s_last;
+    if (count_is_another(scr, build_meta)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int grp = lane / kGroup, sub = lane % kGroup;
     StreamSmem<W>& s = reinterpret_cast<StreamSmem<W>*>(stream_smem_raw)[warp];

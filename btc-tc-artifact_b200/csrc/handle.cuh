@@ -60,6 +60,9 @@ struct btc_bitbsr {
     // tiles themselves where the arrays grew); meta_event then marks the end, which a count or
     // a rebuild on any stream waits for.
     bool tail = false;
+    // An enqueued build whose row store is made only if the graph averages 8 tiles per row block:
+    // the count behind it is launched for either case.
+    bool open = false;
     // CUDA graph of a repeated asynchronous rebuild (captured on the second identical call)
     cudaGraphExec_t graph_exec = nullptr;
     BuildGraphKey graph_key{};

@@ -91,7 +91,8 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
           const uint32_t* __restrict__ blocks, uint32_t R, const uint32_t* __restrict__ rowmask,
           const unsigned long long* __restrict__ d_tiles, uint32_t cap,
           unsigned long long* __restrict__ meta, uint32_t* __restrict__ off, void* __restrict__ key_words,
-          uint4* __restrict__ bit_words, uint32_t* __restrict__ first_row, uint32_t len_lo, uint32_t len_hi)
+          uint4* __restrict__ bit_words, uint32_t* __restrict__ first_row, uint32_t len_lo, uint32_t len_hi,
+          unsigned long long least)
 {
     constexpr int TW = 16 * (C / 32);
     constexpr int kPerTile = C == 128 ? 32 : 16;
@@ -117,7 +118,8 @@ k_rs_fill(const uint32_t* __restrict__ indptr, const uint32_t* __restrict__ indi
     };
     __shared__ Warp s_all[kWarps];
     __shared__ Team s_team[kTeams];
-    if (d_tiles && *d_tiles > cap) return;  // overflowed tile arrays: nothing was built
+    // overflowed tile arrays: nothing was built; fewer tiles than asked for: no store is wanted
+    if (d_tiles && (*d_tiles > cap || *d_tiles < least)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int team = warp / kTeam, w = warp % kTeam;
     Warp& s = s_all[warp];
@@ -345,7 +347,7 @@ int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* o
 int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indices, const uint32_t* blocks,
                     int32_t n_row_blocks, const uint32_t* rowmask, const unsigned long long* d_tiles,
                     uint32_t cap, bool by_degree, unsigned long long* meta, const RowStore& out,
-                    cudaStream_t s)
+                    cudaStream_t s, unsigned long long least)
 {
     const uint32_t R = n_row_blocks > 0 ? (uint32_t)n_row_blocks : 0u;
     if (R == 0) return BTC_OK;
@@ -364,7 +366,7 @@ int launch_rowstore(int tile_cols, const uint32_t* indptr, const uint32_t* indic
     auto launch = [&](auto kernel, uint32_t per_cta, uint32_t len_lo, uint32_t len_hi) {
         const uint32_t grid = std::min((R + per_cta - 1) / per_cta, sms * 16);
         kernel<<<grid, rs::kThreads, 0, s>>>(indptr, indices, blocks, R, rowmask, d_tiles, cap, meta, out.off,
-                                             out.key, out.bits, out.first_row, len_lo, len_hi);
+                                             out.key, out.bits, out.first_row, len_lo, len_hi, least);
     };
     auto fill = [&](auto one, auto team) {
         if (!few) launch(one, rs::kWarps, 0, by_degree ? kAny : kLong);
