@@ -299,7 +299,7 @@ int launch_rowstore_check(int tile_cols, const uint32_t* indices, const uint32_t
 // *out += the set bits of mask[0, n).
 int launch_mask_popcount(const uint32_t* mask, uint32_t n, unsigned long long* out, cudaStream_t s);
 // Enqueues the row store of a Bit-BSR whose row masks exist (T = *d_tiles tiles, bounded by
-// cap, or cap when d_tiles is null; nothing when T > cap).  by_degree: the ids are in
+// cap, or cap when d_tiles is null; nothing when T > cap or *d_tiles < least).  by_degree: the ids are in
 // descending-degree order.  meta: the build's metadata slots (kMetaRowChunks zero: it counts the
 // chunks handed out); also raises meta[kMetaRowMax] to the most tiles and meta[kMetaRowLong] to the
 // most chunks in one row block.
